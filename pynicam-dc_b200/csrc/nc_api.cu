@@ -337,6 +337,7 @@ struct nc_handle {
   cudaGraphExec_t gexec = nullptr;
   bool use_graph = true;
   bool have_state = false;
+  int sms = 148;        // multiprocessors of the device
   int sstep[4] = {0, 0, 0, 0};
   int nstage = 0;
   double dtl = 0, dts = 0;
@@ -819,6 +820,22 @@ static int trc_rhog(nc_handle* h) {
   return 0;
 }
 
+// Levels per chunk of a kernel whose blocks march over the levels of a tile:
+// all of them where the tiles fill the SMs (4 blocks each; a chunk repeats its
+// first half level and re-reads the tile's coefficients), else enough chunks
+// for that, of at least 4 levels.
+static int tile_chunks(const nc_handle* h, int blocks, int levels) {
+  const int want = 4 * h->sms;
+  const int n = std::max(1, std::min((want + blocks - 1) / blocks, levels / 4));
+  return (levels + n - 1) / n;
+}
+// Levels per thread of a column kernel split along the levels
+static int column_chunks(const nc_handle* h, int levels) {
+  const long long want = 4LL * 1024 * h->sms;
+  const long long n = std::max(1LL, std::min((want + h->D.npt2 - 1) / h->D.npt2, (long long)levels / 4));
+  return (int)((levels + n - 1) / n);
+}
+
 template <class R>
 static int run_step(nc_handle* h) {
   cudaStream_t s = h->stream;
@@ -826,12 +843,18 @@ static int run_step(nc_handle* h) {
   h->phase = 0;
   const Dims& D = h->D;
   const unsigned gkl = grid_cols_kl(h);
-  // pole kernels: one thread per pole column (6 * LP) or per pole level (kall * LP);
-  // LP = 2 per ensemble member
-  const unsigned pcb = (unsigned)((6 * D.LP + 31) / 32);
-  const unsigned pkb = (unsigned)((D.KA * D.LP + 127) / 128);
+  // pole kernels: one thread per pole point (6 * LP * kall) or per pole level
+  // (kall * LP), in blocks of a warp to spread the few threads over SMs; LP = 2
+  // per ensemble member.  They stay launches of their own on the pole stream:
+  // folded into the tiled kernels they raised those kernels' register use into
+  // spills (path 1 at gl08 mixed 1.12 -> 1.68 ms)
+  const unsigned ppb = (unsigned)((D.npl + 31) / 32);
+  const unsigned pkb = (unsigned)((D.KA * D.LP + 31) / 32);
   const unsigned npt_blocks = (unsigned)((D.npt + kBlock - 1) / kBlock);
   const unsigned npl_blocks = (unsigned)((D.npl + kBlock - 1) / kBlock);
+  // blocks of the point kernels (a thread per pole point, per regional point)
+  auto pblk = [&](int tb) { return (int)((D.npl + h->blk[tb] - 1) / h->blk[tb]); };
+  auto rblk = [&](int tb) { return (int)((D.npt + h->blk[tb] - 1) / h->blk[tb]); };
   // per-level tiled kernels: (levels kmin..kmax, tiles, regions)
   const dim3 vagrid((unsigned)((D.kmax - D.kmin + VA_NK) / VA_NK),
                     (unsigned)(((D.G - 2 + DD_DX - 1) / DD_DX) * ((D.G - 2 + DD_DY - 1) / DD_DY)), (unsigned)D.L);
@@ -860,28 +883,30 @@ static int run_step(nc_handle* h) {
       a.vvx = F(h->vv[0]); a.vvy = F(h->vv[1]); a.vvz = F(h->vv[2]);
       return a;
     };
-    // regional and pole columns: same kernel, launched with the matching pointers
-    k_diag<<<(unsigned)((D.npt2 + h->blk[TB_DIAG] - 1) / h->blk[TB_DIAG]), h->blk[TB_DIAG], 0, s>>>(diag_args(false), 0);
+    // regional and pole points in one launch
+    k_diag<<<pblk(TB_DIAG) + rblk(TB_DIAG), h->blk[TB_DIAG], 0, s>>>(diag_args(false), diag_args(true), pblk(TB_DIAG));
     TRY(check_launch(h, "diag"));
-    k_diag<<<pcb, 32, 0, ps>>>(diag_args(true), 1);
-    TRY(check_launch(h, "diag_pl"));
+    TRY(fork_pl(h));
     PHASE();
     // ---- momentum advection
-    AdvMomArgs<R> am;
-    am.rg = RG<R>(h->P[0]); am.rvx = RG<R>(h->P[1]); am.rvy = RG<R>(h->P[2]); am.rvz = RG<R>(h->P[3]); am.rw = RG<R>(h->P[4]);
-    am.vvx = RG<R>(h->vv[0]); am.vvy = RG<R>(h->vv[1]); am.vvz = RG<R>(h->vv[2]);
-    am.gvx = RG<R>(h->gadv[0]); am.gvy = RG<R>(h->gadv[1]); am.gvz = RG<R>(h->gadv[2]); am.gw = RG<R>(h->gadv[3]);
+    AdvMomArgs<R> am, amp;
+    for (int pole = 0; pole < 2; ++pole) {
+      AdvMomArgs<R>& x = pole ? amp : am;
+      auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
+      x.rg = F(h->P[0]); x.rvx = F(h->P[1]); x.rvy = F(h->P[2]); x.rvz = F(h->P[3]); x.rw = F(h->P[4]);
+      x.vvx = F(h->vv[0]); x.vvy = F(h->vv[1]); x.vvz = F(h->vv[2]);
+      x.gvx = F(h->gadv[0]); x.gvy = F(h->gadv[1]); x.gvz = F(h->gadv[2]); x.gw = F(h->gadv[3]);
+    }
     {
       // interior cells, levels kmin..kmax (see k_advmom_t)
-      const dim3 gt((unsigned)(((D.G - 2 + 31) / 32) * ((D.G - 2 + 7) / 8)), 1, (unsigned)D.L);
-      k_advmom_t<<<gt, 256, 0, s>>>(am);
+      const int tiles = ((D.G - 2 + 31) / 32) * ((D.G - 2 + 7) / 8);
+      const int nk = tile_chunks(h, tiles * D.L, D.kmax - D.kmin + 1);
+      const dim3 gt((unsigned)tiles, (unsigned)((D.kmax - D.kmin + nk) / nk), (unsigned)D.L);
+      if (gt.y > 1) k_advmom_t<R, true><<<gt, 256, 0, s>>>(am, nk);
+      else k_advmom_t<R, false><<<gt, 256, 0, s>>>(am, nk);
     }
     TRY(check_launch(h, "advmom"));
-    AdvMomArgs<R> amp;
-    amp.rg = PL<R>(h->P[0]); amp.rvx = PL<R>(h->P[1]); amp.rvy = PL<R>(h->P[2]); amp.rvz = PL<R>(h->P[3]); amp.rw = PL<R>(h->P[4]);
-    amp.vvx = PL<R>(h->vv[0]); amp.vvy = PL<R>(h->vv[1]); amp.vvz = PL<R>(h->vv[2]);
-    amp.gvx = PL<R>(h->gadv[0]); amp.gvy = PL<R>(h->gadv[1]); amp.gvz = PL<R>(h->gadv[2]); amp.gw = PL<R>(h->gadv[3]);
-    k_advmom_pl<<<pcb, 32, 0, ps>>>(amp);
+    k_advmom_pl<<<ppb, 32, 0, ps>>>(amp);
     TRY(check_launch(h, "advmom_pl"));
     PHASE();
     // ---- hyperdiffusion
@@ -892,9 +917,9 @@ static int run_step(nc_handle* h) {
       src.f[n] = RG<R>(*sf[n]); srcp.f[n] = PL<R>(*sf[n]);
       o1.f[n] = RG<R>(h->vt[n]); o1p.f[n] = PL<R>(h->vt[n]);
     }
-    k_hdiff1<<<(unsigned)((D.npt2 + h->blk[TB_HDIFF1] - 1) / h->blk[TB_HDIFF1]), h->blk[TB_HDIFF1], 0, s>>>(src, o1);
+    k_hdiff1<<<rblk(TB_HDIFF1), h->blk[TB_HDIFF1], 0, s>>>(src, o1);
     TRY(check_launch(h, "hdiff1"));
-    k_hdiff1_pl<<<pkb, 128, 0, ps>>>(srcp, o1p);
+    k_hdiff1_pl<<<pkb, 32, 0, ps>>>(srcp, o1p);
     TRY(check_launch(h, "hdiff1_pl"));
     TRY(comm<R>(h, {h->vt[0], h->vt[1], h->vt[2], h->vt[3], h->vt[4], h->vt[5]}));
     PHASE();
@@ -906,41 +931,43 @@ static int run_step(nc_handle* h) {
     }
     {
       // interior cells; the exchange below fills the halo rows
-      const dim3 gt((unsigned)((D.G - 2 + HD_DX - 1) / HD_DX), (unsigned)((D.G - 2 + HD_DY - 1) / HD_DY),
-                    (unsigned)D.L);
-      const dim3 gl2((unsigned)((D.KA + HD_NK - 1) / HD_NK), gt.x * gt.y, gt.z);
+      const int tiles = ((D.G - 2 + HD_DX - 1) / HD_DX) * ((D.G - 2 + HD_DY - 1) / HD_DY);
+      const dim3 gl2((unsigned)((D.KA + HD_NK - 1) / HD_NK), (unsigned)tiles, (unsigned)D.L);
       k_hdiff2_m<<<gl2, HD_DX * HD_DY, hdiff2_m_smem<R>(), s>>>(vin, RG<R>(h->P[0]), o2);
       TRY(check_launch(h, "hdiff2"));
     }
-    k_hdiff2_pl<<<pkb, 128, 0, ps>>>(vinp, PL<R>(h->P[0]), o2p);
+    k_hdiff2_pl<<<pkb, 32, 0, ps>>>(vinp, PL<R>(h->P[0]), o2p);
     TRY(check_launch(h, "hdiff2_pl"));
     TRY(comm<R>(h, {h->vt2[0], h->vt2[1], h->vt2[2], h->vt2[3], h->vt2[4], h->vt2[5]}));
     PHASE();
     // ---- large-step tendency
-    for (int pole = 0; pole < 2; ++pole) {
-      GtendArgs<R> ga;
-      auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
-      for (int n = 0; n < 6; ++n) { ga.vt2.f[n] = F(h->vt2[n]); ga.gT0[n] = F(h->gT0[n]); }
-      ga.lapT = F(h->vt[4]);
-      ga.vx = F(h->vx); ga.vy = F(h->vy); ga.vz = F(h->vz); ga.w = F(h->w);
-      ga.rhog = F(h->P[0]); ga.gvx = F(h->gadv[0]); ga.gvy = F(h->gadv[1]); ga.gvz = F(h->gadv[2]);
-      ga.gw = F(h->gadv[3]); ga.frhog = F(h->frhog);
-      if (!pole) k_gtend<<<(unsigned)((D.npt2 + h->blk[TB_GTEND] - 1) / h->blk[TB_GTEND]), h->blk[TB_GTEND], 0, s>>>(ga, 0);
-      else k_gtend<<<pcb, 32, 0, ps>>>(ga, 1);
-      TRY(check_launch(h, pole ? "gtend_pl" : "gtend"));
+    {
+      GtendArgs<R> gt[2];
+      for (int pole = 0; pole < 2; ++pole) {
+        GtendArgs<R>& ga = gt[pole];
+        auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
+        for (int n = 0; n < 6; ++n) { ga.vt2.f[n] = F(h->vt2[n]); ga.gT0[n] = F(h->gT0[n]); }
+        ga.lapT = F(h->vt[4]);
+        ga.vx = F(h->vx); ga.vy = F(h->vy); ga.vz = F(h->vz); ga.w = F(h->w);
+        ga.rhog = F(h->P[0]); ga.gvx = F(h->gadv[0]); ga.gvy = F(h->gadv[1]); ga.gvz = F(h->gadv[2]);
+        ga.gw = F(h->gadv[3]); ga.frhog = F(h->frhog);
+      }
+      k_gtend<<<pblk(TB_GTEND) + rblk(TB_GTEND), h->blk[TB_GTEND], 0, s>>>(gt[0], gt[1], pblk(TB_GTEND));
+      TRY(check_launch(h, "gtend"));
     }
     PHASE();
     // ---- vi_small_step (mod_vi.py:104-1590)
-    k_split_init<<<(unsigned)((D.npt + h->blk[TB_SPLIT] - 1) / h->blk[TB_SPLIT]), h->blk[TB_SPLIT], 0, s>>>(RG<R>(h->P0[0]), RG<R>(h->P0[1]), RG<R>(h->P0[2]), RG<R>(h->P0[3]), RG<R>(h->P0[4]),
-                                                RG<R>(h->P0[5]), prog_reg<R>(h), RG<R>(h->PSa[0]), RG<R>(h->PSa[1]), RG<R>(h->PSa[2]),
-                                                RG<R>(h->PSa[3]), RG<R>(h->PSa[4]), RG<R>(h->PSa[5]), RG<R>(h->PM[0]), RG<R>(h->PM[1]),
-                                                RG<R>(h->PM[2]), RG<R>(h->PM[3]), RG<R>(h->PM[4]), D.npt, nl == 0);
-    TRY(check_launch(h, "split_init"));
-    k_split_init<<<npl_blocks, kBlock, 0, ps>>>(PL<R>(h->P0[0]), PL<R>(h->P0[1]), PL<R>(h->P0[2]), PL<R>(h->P0[3]), PL<R>(h->P0[4]),
-                                                PL<R>(h->P0[5]), prog_pl<R>(h), PL<R>(h->PSa[0]), PL<R>(h->PSa[1]), PL<R>(h->PSa[2]),
-                                                PL<R>(h->PSa[3]), PL<R>(h->PSa[4]), PL<R>(h->PSa[5]), PL<R>(h->PM[0]), PL<R>(h->PM[1]),
-                                                PL<R>(h->PM[2]), PL<R>(h->PM[3]), PL<R>(h->PM[4]), D.npl, nl == 0);
-    TRY(check_launch(h, "split_init_pl"));
+    {
+      SplitArgs<R> sp[2];
+      for (int pole = 0; pole < 2; ++pole) {
+        auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
+        for (int n = 0; n < 6; ++n) { sp[pole].P0[n] = F(h->P0[n]); sp[pole].P[n] = F(h->P[n]); sp[pole].PS[n] = F(h->PSa[n]); }
+        for (int n = 0; n < 5; ++n) sp[pole].PM[n] = F(h->PM[n]);
+      }
+      k_split_init<<<pblk(TB_SPLIT) + rblk(TB_SPLIT), h->blk[TB_SPLIT], 0, s>>>(sp[0], (int)D.npt, sp[1], D.npl,
+                                                                               pblk(TB_SPLIT), nl == 0);
+      TRY(check_launch(h, "split_init"));
+    }
     auto dd3d = [&](FieldPair* v4) -> int {
       Four<R> v, vp;
       Three<R> o, op;
@@ -948,10 +975,12 @@ static int run_step(nc_handle* h) {
       for (int d = 0; d < 3; ++d) { o.f[d] = RG<R>(h->vtmp2[d]); op.f[d] = PL<R>(h->vtmp2[d]); }
       // interior cells only: halo rows are filled by the exchange below and the
       // boundary levels of vtmp2 stay zero from allocation
-      const dim3 gt((unsigned)((D.G - 2 + DD_DX - 1) / DD_DX), (unsigned)((D.G - 2 + DD_DY - 1) / DD_DY), (unsigned)D.L);
-      k_dd3d_m<R, true><<<gt, DD_DX * DD_DY, dd3d_m_smem<R>(), s>>>(v, o);
+      const unsigned tx = (unsigned)((D.G - 2 + DD_DX - 1) / DD_DX), ty = (unsigned)((D.G - 2 + DD_DY - 1) / DD_DY);
+      const int nk = tile_chunks(h, (int)(tx * ty) * D.L, D.kmax - D.kmin + 1);
+      const dim3 gt(tx, ty, (unsigned)(D.L * ((D.kmax - D.kmin + nk) / nk)));
+      k_dd3d_m<R, true><<<gt, DD_DX * DD_DY, dd3d_m_smem<R>(), s>>>(v, o, nk);
       TRY(check_launch(h, "dd3d"));
-      k_dd3d_pl<<<pkb, 128, 0, ps>>>(vp, op);
+      k_dd3d_pl<<<pkb, 32, 0, ps>>>(vp, op);
       TRY(check_launch(h, "dd3d_pl"));
       return comm<R>(h, {h->vtmp2[0], h->vtmp2[1], h->vtmp2[2]});
     };
@@ -960,28 +989,30 @@ static int run_step(nc_handle* h) {
       TRY(dd3d(v4));
     }
     PHASE();
-    for (int pole = 0; pole < 2; ++pole) {
-      Vp0Args<R> va;
-      auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
-      auto F64 = [&](FieldPair& f) { return pole ? f.p : f.r; };
-      va.P = pole ? prog_pl<R>(h) : prog_reg<R>(h);
-      va.vx = F(h->vx); va.vy = F(h->vy); va.vz = F(h->vz); va.eth = F(h->eth); va.pregd = F64(h->pregd);
-      va.rhogd = F64(h->rhogd);
-      for (int d = 0; d < 3; ++d) va.vt.f[d] = F(h->vtmp2[d]);
-      for (int n = 0; n < 6; ++n) { va.gT0[n] = F(h->gT0[n]); va.gT[n] = F(h->gT[n]); }
-      va.Mc = F64(h->Mc); va.Mu = F64(h->Mu); va.Ml = F64(h->Ml); va.ethtot0 = F(h->ethtot0);
-      va.dt = h->dts;
-      if (!pole) {
-        Vp0H<R> vh;
-        for (int n = 0; n < 8; ++n) vh.out[n] = RG<R>(h->vph[n]);
-        k_vp0_hl<<<lvgrid_vp, VP_DX * VP_DY, 0, s>>>(va, vh);
-        TRY(check_launch(h, "vp0_h"));
-        k_vp0_cr<<<(unsigned)((D.npt2 + h->blk[TB_VP0C] - 1) / h->blk[TB_VP0C]), h->blk[TB_VP0C], 0, s>>>(va, vh);
-        TRY(check_launch(h, "vp0_c"));
-      } else {
-        k_vp0<<<pcb, 32, 0, ps>>>(va, 1);
-        TRY(check_launch(h, "vp0_pl"));
+    {
+      Vp0Args<R> v0[2];
+      for (int pole = 0; pole < 2; ++pole) {
+        Vp0Args<R>& va = v0[pole];
+        auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
+        auto F64 = [&](FieldPair& f) { return pole ? f.p : f.r; };
+        va.P = pole ? prog_pl<R>(h) : prog_reg<R>(h);
+        va.vx = F(h->vx); va.vy = F(h->vy); va.vz = F(h->vz); va.eth = F(h->eth); va.pregd = F64(h->pregd);
+        va.rhogd = F64(h->rhogd);
+        for (int d = 0; d < 3; ++d) va.vt.f[d] = F(h->vtmp2[d]);
+        for (int n = 0; n < 6; ++n) { va.gT0[n] = F(h->gT0[n]); va.gT[n] = F(h->gT[n]); }
+        va.Mc = F64(h->Mc); va.Mu = F64(h->Mu); va.Ml = F64(h->Ml); va.ethtot0 = F(h->ethtot0);
+        va.dt = h->dts;
       }
+      Vp0H<R> vh;
+      for (int n = 0; n < 8; ++n) vh.out[n] = RG<R>(h->vph[n]);
+      k_vp0_hl<<<lvgrid_vp, VP_DX * VP_DY, 0, s>>>(v0[0], vh);
+      TRY(check_launch(h, "vp0_h"));
+      const int tb = h->blk[TB_VP0C];
+      const int nk = column_chunks(h, D.KA);
+      k_vp0_cr<<<dim3((unsigned)((D.npt2 + tb - 1) / tb), (unsigned)((D.KA + nk - 1) / nk)), tb, 0, s>>>(v0[0], vh, nk);
+      TRY(check_launch(h, "vp0_c"));
+      k_vp0_pl<<<ppb, 32, 0, ps>>>(v0[1]);
+      TRY(check_launch(h, "vp0_pl"));
     }
     PHASE();
     const int nitr = h->sstep[nl];
@@ -995,28 +1026,29 @@ static int run_step(nc_handle* h) {
         TRY(dd3d(v4));
       }
       PHASE();
-      for (int pole = 0; pole < 2; ++pole) {
-        Path1Args<R> pa;
-        auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
-        for (int n = 0; n < 6; ++n) { pa.PS[n] = F(PS[n]); pa.gT[n] = F(h->gT[n]); }
-        pa.rhog = F(h->P[0]);
-        for (int d = 0; d < 3; ++d) { pa.vt.f[d] = F(h->vtmp2[d]); pa.dvh[d] = F(PN[1 + d]); }
-        for (int n = 0; n < 5; ++n) pa.PM[n] = F(h->PM[n]);
-        pa.dt = h->dts; pa.rweight = rweight; pa.RovCV = RovCV;
-        if (!pole) {
-          k_path1_l<<<lvgrid, DD_DX * DD_DY, 0, s>>>(pa);
-          TRY(check_launch(h, "path1"));
-        } else {
-          k_path1<<<pcb, 32, 0, ps>>>(pa, 1);
-          TRY(check_launch(h, "path1_pl"));
+      {
+        Path1Args<R> p1[2];
+        for (int pole = 0; pole < 2; ++pole) {
+          Path1Args<R>& pa = p1[pole];
+          auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
+          for (int n = 0; n < 6; ++n) { pa.PS[n] = F(PS[n]); pa.gT[n] = F(h->gT[n]); }
+          pa.rhog = F(h->P[0]);
+          for (int d = 0; d < 3; ++d) { pa.vt.f[d] = F(h->vtmp2[d]); pa.dvh[d] = F(PN[1 + d]); }
+          for (int n = 0; n < 5; ++n) pa.PM[n] = F(h->PM[n]);
+          pa.dt = h->dts; pa.rweight = rweight; pa.RovCV = RovCV;
         }
+        k_path1_l<<<lvgrid, DD_DX * DD_DY, 0, s>>>(p1[0]);
+        TRY(check_launch(h, "path1"));
+        k_path1_pl<<<ppb, 32, 0, ps>>>(p1[1]);
+        TRY(check_launch(h, "path1_pl"));
       }
       TRY(comm<R>(h, {PN[1], PN[2], PN[3]}));
       PHASE();
+      VimainArgs<R> vi[2];
       for (int pole = 0; pole < 2; ++pole) {
-        VimainArgs<R> va;
+        VimainArgs<R>& va = vi[pole];
         auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
-      auto F64 = [&](FieldPair& f) { return pole ? f.p : f.r; };
+        auto F64 = [&](FieldPair& f) { return pole ? f.p : f.r; };
         for (int n = 0; n < 6; ++n) { va.PS[n] = F(PS[n]); va.P[n] = F(h->P[n]); va.gT[n] = F(h->gT[n]); }
         va.eth = F(h->eth); va.ethtot0 = F(h->ethtot0); va.gT0e = F(h->gT0[5]);
         va.Mc = F64(h->Mc); va.Mu = F64(h->Mu); va.Ml = F64(h->Ml);
@@ -1024,30 +1056,46 @@ static int run_step(nc_handle* h) {
         va.dwe[0] = F(PN[0]); va.dwe[1] = F(PN[4]); va.dwe[2] = F(PN[5]);
         va.PM0 = F(h->PM[0]); va.PM4 = F(h->PM[4]);
         va.dt = h->dts; va.rweight = rweight; va.RovCV = RovCV;
-        if (!pole) {
-          if constexpr (std::is_same<R, float>::value) k_vimain_a_m<<<vagrid, DD_DX * DD_DY, 0, s>>>(va);
-          else k_vimain_a_l<<<lvgrid, DD_DX * DD_DY, 0, s>>>(va);
-          TRY(check_launch(h, "vimain_a"));
-          if (h->C.gam_unit) k_vi_solve<R, true><<<(unsigned)((D.npt2 + h->blk[TB_VISOLVE] - 1) / h->blk[TB_VISOLVE]), h->blk[TB_VISOLVE], 0, s>>>(va);
-          else k_vi_solve<R, false><<<(unsigned)((D.npt2 + h->blk[TB_VISOLVE] - 1) / h->blk[TB_VISOLVE]), h->blk[TB_VISOLVE], 0, s>>>(va);
+      }
+      if constexpr (std::is_same<R, float>::value) k_vimain_a_m<<<vagrid, DD_DX * DD_DY, 0, s>>>(vi[0]);
+      else k_vimain_a_l<<<lvgrid, DD_DX * DD_DY, 0, s>>>(vi[0]);
+      TRY(check_launch(h, "vimain_a"));
+      {
+        const int ncol = D.L * (D.G - 2) * (D.G - 2);
+        const size_t sm = vi_col_smem(D.KA);
+        if (ncol <= h->sms * 9 * 128) {   // one wave of the column kernel's nine 128-thread blocks per SM
+          const unsigned nb = (unsigned)((ncol + VC_COLS - 1) / VC_COLS);
+          if (h->C.gam_unit) k_vi_col<R, true, false><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
+          else k_vi_col<R, false, false><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
           TRY(check_launch(h, "vi_solve"));
-          k_vi_energy_p<<<(unsigned)((D.npt + h->blk[TB_VIENERGY] - 1) / h->blk[TB_VIENERGY]), h->blk[TB_VIENERGY], 0, s>>>(va);
-          TRY(check_launch(h, "vi_energy"));
         } else {
-          k_vimain_a<<<pkb, 128, 0, ps>>>(va, 1);
-          TRY(check_launch(h, "vimain_a_pl"));
-          k_vimain_b<<<pcb, 32, 0, ps>>>(va, 1);
-          TRY(check_launch(h, "vimain_b_pl"));
+          const int tb = h->blk[TB_VISOLVE];
+          const unsigned nb = (unsigned)((D.npt2 + tb - 1) / tb);
+          if (h->C.gam_unit) k_vi_solve<R, true><<<nb, tb, 0, s>>>(vi[0]);
+          else k_vi_solve<R, false><<<nb, tb, 0, s>>>(vi[0]);
+          TRY(check_launch(h, "vi_solve"));
+          k_vi_energy_p<<<(unsigned)((D.npt + h->blk[TB_VIENERGY] - 1) / h->blk[TB_VIENERGY]), h->blk[TB_VIENERGY], 0, s>>>(vi[0]);
+          TRY(check_launch(h, "vi_energy"));
         }
+        k_vimain_a_pl<<<pkb, 32, 0, ps>>>(vi[1]);
+        TRY(check_launch(h, "vimain_a_pl"));
+        k_vi_col<R, false, true><<<(6 * D.LP + VC_COLS - 1) / VC_COLS, 32 * VC_MAXW, sm, ps>>>(vi[1]);
+        TRY(check_launch(h, "vi_solve_pl"));
       }
       TRY(comm<R>(h, {PN[0], PN[4], PN[5]}));
       PHASE();
     }
     FieldPair* PSf = (nitr % 2 == 0) ? h->PSa : h->PSb;
-    k_post<<<(unsigned)((D.npt2 + h->blk[TB_POST] - 1) / h->blk[TB_POST]), h->blk[TB_POST], 0, s>>>(prog_reg<R>(h), RG<R>(PSf[0]), RG<R>(PSf[1]), RG<R>(PSf[2]), RG<R>(PSf[3]), RG<R>(PSf[4]), RG<R>(PSf[5]), 0);
-    TRY(check_launch(h, "post"));
-    k_post<<<pcb, 32, 0, ps>>>(prog_pl<R>(h), PL<R>(PSf[0]), PL<R>(PSf[1]), PL<R>(PSf[2]), PL<R>(PSf[3]), PL<R>(PSf[4]), PL<R>(PSf[5]), 1);
-    TRY(check_launch(h, "post_pl"));
+    {
+      PostArgs<R> po[2];
+      for (int pole = 0; pole < 2; ++pole)
+        for (int n = 0; n < 6; ++n) {
+          po[pole].P[n] = pole ? PL<R>(h->P[n]) : RG<R>(h->P[n]);
+          po[pole].PS[n] = pole ? PL<R>(PSf[n]) : RG<R>(PSf[n]);
+        }
+      k_post<<<pblk(TB_POST) + rblk(TB_POST), h->blk[TB_POST], 0, s>>>(po[0], po[1], pblk(TB_POST));
+      TRY(check_launch(h, "post"));
+    }
     TRY(comm<R>(h, {h->PM[0], h->PM[1], h->PM[2], h->PM[3], h->PM[4]}));
     PHASE();
     if (!last) {
@@ -1600,12 +1648,22 @@ static int make_f32_geometry(nc_handle* h) {
 }
 
 static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
+  {
+    int dev = 0;
+    CU(cudaGetDevice(&dev));
+    CU(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, dev));
+  }
   // the multi-level hyperdiffusion kernel takes more than the default 48 KB of
   // dynamic shared memory in its float64 instance
   CU(cudaFuncSetAttribute(k_hdiff2_m<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<double>()));
   CU(cudaFuncSetAttribute(k_hdiff2_m<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<float>()));
   CU(cudaFuncSetAttribute(k_dd3d_m<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double>()));
   CU(cudaFuncSetAttribute(k_dd3d_m<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float>()));
+  // the column kernel of vi_main: five doubles per level of 32 columns (164 KB at NC_MAXK levels)
+  for (const void* f : {(const void*)k_vi_col<double, true, false>, (const void*)k_vi_col<double, false, false>,
+                        (const void*)k_vi_col<double, false, true>, (const void*)k_vi_col<float, true, false>,
+                        (const void*)k_vi_col<float, false, false>, (const void*)k_vi_col<float, false, true>})
+    CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vi_col_smem(NC_MAXK)));
   ArrTab T;
   for (int n = 0; n < narrays; ++n) {
     if (!arrays[n].name || !arrays[n].data) return fail(NC_ERR_ARG, "null array entry");

@@ -160,7 +160,7 @@ template <> __device__ __forceinline__ const GeomT<float>& geom<float>() { retur
 #define NC_F32_VP0H 5
 #endif
 #ifndef NC_F32_VP0C
-#define NC_F32_VP0C 4
+#define NC_F32_VP0C 3
 #endif
 #ifndef NC_F32_PATH1
 #define NC_F32_PATH1 6

@@ -13,8 +13,8 @@ struct Prog { R* v[6]; };   // RHOG, RHOGVX, RHOGVY, RHOGVZ, RHOGW, RHOGE
 // Pre_Post: diagnostics (kernels/diag.py:53-143), BNDCND_all
 // (share/mod_bndcnd.py:182-264 with kernels/bndcnd.py), th/eth and the
 // deviations (mod_dynamics.py:1043-1057), then the merged velocity of the
-// momentum advection (kernels/advconvmom.py:54-78).  One thread per column,
-// regional and pole columns alike.
+// momentum advection (kernels/advconvmom.py:54-78), regional and pole points
+// alike.
 // ---------------------------------------------------------------------------
 template <class R>
 struct DiagArgs {
@@ -26,208 +26,133 @@ struct DiagArgs {
 };
 
 template <class R>
-__device__ void diag_column(const Col c, const MetT<R> m, const DiagArgs<R>& a, double gx, double gy, double gz) {
-  const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
-  R** P = const_cast<R**>(a.P.v);
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    double RHOG = P[0][p];
-    double rho = RHOG / m.GSGAM2[p];
-    a.vx[p] = P[1][p] / RHOG;
-    a.vy[p] = P[2][p] / RHOG;
-    a.vz[p] = P[3][p] / RHOG;
-    double ein = P[5][p] / RHOG;
-    double q0 = a.Pqw[0][p] / RHOG;
-    double qd, cv;
-    moist_qd_cv([&](int n) { return (double)a.Pqw[n][p] / RHOG; }, q0, qd, cv);
-    double tem = ein / cv;
-    a.tem[p] = tem;
-    a.pre[p] = rho * tem * (qd * cC.Rdry + q0 * cC.Rvap);
-    a.rho[p] = rho;
-    a.ein[p] = ein;
-    if (k >= kmin + 1 && k <= kmax) {
-      int pm = c.at(k - 1);
-      a.w[p] = P[4][p] / (mc(m.C2W, c, 0, 2, k) * RHOG + mc(m.C2W, c, 1, 2, k) * P[0][pm]);
-    }
-  }
-  // ---- boundary conditions: TEM top/bottom, FREE top, RIGID bottom
-  const int pT = c.at(kmax + 1), pK = c.at(kmax), pKm = c.at(kmax - 1);
-  const int pB = c.at(kmin - 1), pN = c.at(kmin), pNp = c.at(kmin + 1);
-  double tem_top = a.tem[pK];
-  double tem_btm = a.tem[pN];
-  double pre_top = a.pre[pKm] - a.rho[pK] * (m.PHI[pT] - m.PHI[pKm]);
-  double pre_btm = a.pre[pNp] - a.rho[pN] * (m.PHI[pB] - m.PHI[pNp]);
-  double rho_top = pre_top / (cC.Rdry * tem_top);
-  double rho_btm = pre_btm / (cC.Rdry * tem_btm);
-  a.tem[pT] = tem_top; a.tem[pB] = tem_btm;
-  a.pre[pT] = pre_top; a.pre[pB] = pre_btm;
-  a.rho[pT] = rho_top; a.rho[pB] = rho_btm;
-  double rgT = rho_top * m.GSGAM2[pT];
-  double rgB = rho_btm * m.GSGAM2[pB];
-  P[0][pT] = rgT; P[0][pB] = rgB;
-  double einT = cC.CVdry * tem_top, einB = cC.CVdry * tem_btm;
-  a.ein[pT] = einT; a.ein[pB] = einB;
-  P[5][pT] = rgT * einT; P[5][pB] = rgB * einB;
-  double rgK = P[0][pK], rgN = P[0][pN];
-  double vT[3], vB[3];
-  for (int d = 0; d < 3; ++d) {
-    vT[d] = 1.0 * (P[1 + d][pK] / rgK) * rgT;
-    vB[d] = -1.0 * (P[1 + d][pN] / rgN) * rgB;
-    P[1 + d][pT] = vT[d];
-    P[1 + d][pB] = vB[d];
-  }
-  R* dv[3] = {a.vx, a.vy, a.vz};
-  for (int d = 0; d < 3; ++d) {
-    dv[d][pT] = P[1 + d][pT] / P[0][pT];
-    dv[d][pB] = P[1 + d][pB] / P[0][pB];
-  }
-  const int kT = kmax + 1;
-  double rwT = -(mc(m.C2WGz, c, 0, 6, kT) * vT[0] + mc(m.C2WGz, c, 1, 6, kT) * P[1][pK] +
-                 mc(m.C2WGz, c, 2, 6, kT) * vT[1] + mc(m.C2WGz, c, 3, 6, kT) * P[2][pK] +
-                 mc(m.C2WGz, c, 4, 6, kT) * vT[2] + mc(m.C2WGz, c, 5, 6, kT) * P[3][pK]);
-  P[4][pT] = rwT;
-  P[4][pN] = 0.0;
-  P[4][pB] = 0.0;
-  a.w[pT] = rwT / (mc(m.C2W, c, 0, 2, kT) * rgT + mc(m.C2W, c, 1, 2, kT) * rgK);
-  a.w[pN] = P[4][pN] / (mc(m.C2W, c, 0, 2, kmin) * rgN + mc(m.C2W, c, 1, 2, kmin) * rgB);
-  a.w[pB] = 0.0;
-  // ---- eth, deviations, merged velocity
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    double pre = a.pre[p], rho = a.rho[p];
-    a.eth[p] = a.ein[p] + pre / rho;
-    a.pregd[p] = (pre - m.pre_bs[p]) * m.GSGAM2[p];
-    a.rhogd[p] = (rho - m.rho_bs[p]) * m.GSGAM2[p];
-    if (k >= kmin && k <= kmax) {
-      double wc = cC.cfact[k] * a.w[c.at(k + 1)] + cC.dfact[k] * a.w[p];
-      a.vvx[p] = a.vx[p] + div_r(wc * gx);
-      a.vvy[p] = a.vy[p] + div_r(wc * gy);
-      a.vvz[p] = a.vz[p] + div_r(wc * gz);
-    } else {
-      a.vvx[p] = 0.0; a.vvy[p] = 0.0; a.vvz[p] = 0.0;
-    }
-  }
-}
-
-// diag_column with the second pass (eth, deviations, merged velocity) fused
-// into the first for the levels kmin+1..kmax-1, whose inputs do not depend on
-// the boundary rows: level k-1 is finished while level k is diagnosed, from
-// values carried in registers.  The four levels next to and on the boundary
-// rows are finished after the boundary conditions, as in diag_column.  Same
-// expressions, same results.
-template <class R>
-__device__ void diag_column_fused(const Col c, const MetT<R> m, const DiagArgs<R>& a, double gx, double gy, double gz) {
-  const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
-  R** P = const_cast<R**>(a.P.v);
-  auto finish = [&](int k, int p, double pre, double rho, double ein, double vxk, double vyk, double vzk,
-                    double wk, double wk1) {
-    a.eth[p] = ein + pre / rho;
-    a.pregd[p] = (pre - m.pre_bs[p]) * m.GSGAM2[p];
-    a.rhogd[p] = (rho - m.rho_bs[p]) * m.GSGAM2[p];
-    if (k >= kmin && k <= kmax) {
-      double wc = cC.cfact[k] * wk1 + cC.dfact[k] * wk;
-      a.vvx[p] = vxk + div_r(wc * gx);
-      a.vvy[p] = vyk + div_r(wc * gy);
-      a.vvz[p] = vzk + div_r(wc * gz);
-    } else {
-      a.vvx[p] = 0.0; a.vvy[p] = 0.0; a.vvz[p] = 0.0;
-    }
+__device__ void diag_point(const Col c, const MetT<R> m, const DiagArgs<R>& a, int k, double gx, double gy, double gz) {
+  const int kmin = cD.kmin, kmax = cD.kmax;
+  if (k == kmin - 1 || k == kmax + 1) return;   // written with the row next to them
+  R* const* P = a.P.v;
+  struct D {
+    double rhog, rho, vx, vy, vz, ein, tem, pre;
   };
-  double pp = 0.0, pr = 0.0, pe = 0.0, px = 0.0, py = 0.0, pz = 0.0, pw = 0.0;   // level k-1
-  double rg_prev = 0.0;
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    double RHOG = P[0][p];
-    double rho = RHOG / m.GSGAM2[p];
-    const auto rr = recip_of(RHOG);   // five quotients by RHOG
-    const double vx = div_by(P[1][p], rr), vy = div_by(P[2][p], rr), vz = div_by(P[3][p], rr);
-    a.vx[p] = vx;
-    a.vy[p] = vy;
-    a.vz[p] = vz;
-    double ein = div_by(P[5][p], rr);
-    double q0 = div_by(a.Pqw[0][p], rr);
+  auto diag = [&](int kk) -> D {
+    const int p = c.at(kk);
+    D d;
+    d.rhog = P[0][p];
+    d.rho = d.rhog / m.GSGAM2[p];
+    const auto rr = recip_of(d.rhog);   // the quotients by RHOG
+    d.vx = div_by(P[1][p], rr);
+    d.vy = div_by(P[2][p], rr);
+    d.vz = div_by(P[3][p], rr);
+    d.ein = div_by(P[5][p], rr);
+    const double q0 = div_by(a.Pqw[0][p], rr);
     double qd, cv;
     moist_qd_cv([&](int n) { return div_by(a.Pqw[n][p], rr); }, q0, qd, cv);
-    double tem = ein / cv;
-    const double pre = rho * tem * (qd * cC.Rdry + q0 * cC.Rvap);
+    d.tem = d.ein / cv;
+    d.pre = d.rho * d.tem * (qd * cC.Rdry + q0 * cC.Rvap);
+    return d;
+  };
+  auto put = [&](int p, double tem, double pre, double rho, double ein) {
     a.tem[p] = tem;
     a.pre[p] = pre;
     a.rho[p] = rho;
     a.ein[p] = ein;
-    double w = 0.0;
-    if (k >= kmin + 1 && k <= kmax) {
-      w = P[4][p] / (mc(m.C2W, c, 0, 2, k) * RHOG + mc(m.C2W, c, 1, 2, k) * rg_prev);
-      a.w[p] = w;
+  };
+  auto w_at = [&](int kk) -> double {   // kmin+1..kmax
+    const int p = c.at(kk);
+    return P[4][p] / (mc(m.C2W, c, 0, 2, kk) * (double)P[0][p] + mc(m.C2W, c, 1, 2, kk) * (double)P[0][c.at(kk - 1)]);
+  };
+  auto finish = [&](int kk, int p, double pre, double rho, double ein, double vx, double vy, double vz, double wk,
+                    double wk1) {
+    a.eth[p] = ein + pre / rho;
+    a.pregd[p] = (pre - m.pre_bs[p]) * m.GSGAM2[p];
+    a.rhogd[p] = (rho - m.rho_bs[p]) * m.GSGAM2[p];
+    if (kk >= kmin && kk <= kmax) {
+      const double wc = cC.cfact[kk] * wk1 + cC.dfact[kk] * wk;
+      a.vvx[p] = vx + div_r(wc * gx);
+      a.vvy[p] = vy + div_r(wc * gy);
+      a.vvz[p] = vz + div_r(wc * gz);
+    } else {
+      a.vvx[p] = 0.0; a.vvy[p] = 0.0; a.vvz[p] = 0.0;
     }
-    if (k - 1 >= kmin + 1 && k - 1 <= kmax - 1) finish(k - 1, c.at(k - 1), pp, pr, pe, px, py, pz, pw, w);
-    pp = pre; pr = rho; pe = ein; px = vx; py = vy; pz = vz; pw = w;
-    rg_prev = RHOG;
+  };
+  const int p = c.at(k);
+  const D d = diag(k);
+  if (k < kmin || k > kmax) {   // beyond the boundary rows
+    a.vx[p] = d.vx; a.vy[p] = d.vy; a.vz[p] = d.vz;
+    put(p, d.tem, d.pre, d.rho, d.ein);
+    return;
   }
-  // ---- boundary conditions: TEM top/bottom, FREE top, RIGID bottom
-  const int pT = c.at(kmax + 1), pK = c.at(kmax), pKm = c.at(kmax - 1);
-  const int pB = c.at(kmin - 1), pN = c.at(kmin), pNp = c.at(kmin + 1);
-  double tem_top = a.tem[pK];
-  double tem_btm = a.tem[pN];
-  double pre_top = a.pre[pKm] - a.rho[pK] * (m.PHI[pT] - m.PHI[pKm]);
-  double pre_btm = a.pre[pNp] - a.rho[pN] * (m.PHI[pB] - m.PHI[pNp]);
-  double rho_top = pre_top / (cC.Rdry * tem_top);
-  double rho_btm = pre_btm / (cC.Rdry * tem_btm);
-  a.tem[pT] = tem_top; a.tem[pB] = tem_btm;
-  a.pre[pT] = pre_top; a.pre[pB] = pre_btm;
-  a.rho[pT] = rho_top; a.rho[pB] = rho_btm;
-  double rgT = rho_top * m.GSGAM2[pT];
-  double rgB = rho_btm * m.GSGAM2[pB];
-  P[0][pT] = rgT; P[0][pB] = rgB;
-  double einT = cC.CVdry * tem_top, einB = cC.CVdry * tem_btm;
-  a.ein[pT] = einT; a.ein[pB] = einB;
-  P[5][pT] = rgT * einT; P[5][pB] = rgB * einB;
-  double rgK = P[0][pK], rgN = P[0][pN];
-  double vT[3], vB[3];
-  for (int d = 0; d < 3; ++d) {
-    vT[d] = 1.0 * (P[1 + d][pK] / rgK) * rgT;
-    vB[d] = -1.0 * (P[1 + d][pN] / rgN) * rgB;
-    P[1 + d][pT] = vT[d];
-    P[1 + d][pB] = vB[d];
+  if (k > kmin && k < kmax) {
+    const double wk = w_at(k), wk1 = w_at(k + 1);
+    finish(k, p, d.pre, d.rho, d.ein, d.vx, d.vy, d.vz, wk, wk1);
+    a.vx[p] = d.vx; a.vy[p] = d.vy; a.vz[p] = d.vz;
+    put(p, d.tem, d.pre, d.rho, d.ein);
+    a.w[p] = wk;
+    return;
   }
+  // ---- the rows at a boundary, from the stored (rounded) values: TEM top and
+  // bottom, FREE top, RIGID bottom
+  const bool top = k == kmax;
+  const int kb = top ? kmax + 1 : kmin - 1, ki = top ? kmax - 1 : kmin + 1;
+  const int pb = c.at(kb), pi = c.at(ki);
+  const R tem = d.tem, rho = d.rho, pre = d.pre, ein = d.ein, vx = d.vx, vy = d.vy, vz = d.vz;
+  const R pre_i = diag(ki).pre;
+  const double tem_b = tem;
+  const double pre_b = pre_i - rho * (m.PHI[pb] - m.PHI[pi]);
+  const double rho_b = pre_b / (cC.Rdry * tem_b);
+  const double rg = P[0][p], rgb = rho_b * m.GSGAM2[pb], ein_b = cC.CVdry * tem_b;
+  const R Pp[3] = {P[1][p], P[2][p], P[3][p]};
+  double vb[3];
+#pragma unroll
+  for (int n = 0; n < 3; ++n) vb[n] = (top ? 1.0 : -1.0) * (Pp[n] / rg) * rgb;
+  const R rgbR = rgb;
+  R wR, wbR;      // w at the half levels k and k+1 of the row inside (top), at kmin and kmin+1 (bottom)
+  if (top) {
+    const double rwT = -(mc(m.C2WGz, c, 0, 6, kb) * vb[0] + mc(m.C2WGz, c, 1, 6, kb) * Pp[0] +
+                         mc(m.C2WGz, c, 2, 6, kb) * vb[1] + mc(m.C2WGz, c, 3, 6, kb) * Pp[1] +
+                         mc(m.C2WGz, c, 4, 6, kb) * vb[2] + mc(m.C2WGz, c, 5, 6, kb) * Pp[2]);
+    wR = w_at(k);
+    wbR = rwT / (mc(m.C2W, c, 0, 2, kb) * rgb + mc(m.C2W, c, 1, 2, kb) * rg);
+    a.w[p] = wR;
+    a.w[pb] = wbR;
+    P[4][pb] = rwT;
+  } else {
+    wbR = w_at(kmin + 1);
+    wR = R(0.0) / (mc(m.C2W, c, 0, 2, kmin) * rg + mc(m.C2W, c, 1, 2, kmin) * rgb);
+    a.w[p] = wR;
+    a.w[pb] = 0.0;
+    P[4][p] = 0.0;
+    P[4][pb] = 0.0;
+  }
+  finish(k, p, pre, rho, ein, vx, vy, vz, wR, wbR);
+  a.vx[p] = vx; a.vy[p] = vy; a.vz[p] = vz;
+  put(p, tem, pre, rho, ein);
+  // the boundary row
+  finish(kb, pb, R(pre_b), R(rho_b), R(ein_b), 0.0, 0.0, 0.0, 0.0, 0.0);
+  put(pb, tem_b, pre_b, rho_b, ein_b);
+  P[0][pb] = rgb;
+  P[5][pb] = rgb * ein_b;
   R* dv[3] = {a.vx, a.vy, a.vz};
-  for (int d = 0; d < 3; ++d) {
-    dv[d][pT] = P[1 + d][pT] / P[0][pT];
-    dv[d][pB] = P[1 + d][pB] / P[0][pB];
-  }
-  const int kT = kmax + 1;
-  double rwT = -(mc(m.C2WGz, c, 0, 6, kT) * vT[0] + mc(m.C2WGz, c, 1, 6, kT) * P[1][pK] +
-                 mc(m.C2WGz, c, 2, 6, kT) * vT[1] + mc(m.C2WGz, c, 3, 6, kT) * P[2][pK] +
-                 mc(m.C2WGz, c, 4, 6, kT) * vT[2] + mc(m.C2WGz, c, 5, 6, kT) * P[3][pK]);
-  P[4][pT] = rwT;
-  P[4][pN] = 0.0;
-  P[4][pB] = 0.0;
-  a.w[pT] = rwT / (mc(m.C2W, c, 0, 2, kT) * rgT + mc(m.C2W, c, 1, 2, kT) * rgK);
-  a.w[pN] = P[4][pN] / (mc(m.C2W, c, 0, 2, kmin) * rgN + mc(m.C2W, c, 1, 2, kmin) * rgB);
-  a.w[pB] = 0.0;
-  // ---- the levels next to the boundary rows
-  const int rest[4] = {kmin - 1, kmin, kmax, kmax + 1};
-  for (int r = 0; r < 4; ++r) {
-    const int k = rest[r];
-    const int p = c.at(k);
-    const double wk1 = (k >= kmin && k <= kmax) ? a.w[c.at(k + 1)] : 0.0;
-    finish(k, p, a.pre[p], a.rho[p], a.ein[p], a.vx[p], a.vy[p], a.vz[p], a.w[p], wk1);
+#pragma unroll
+  for (int n = 0; n < 3; ++n) {
+    P[1 + n][pb] = vb[n];
+    dv[n][pb] = R(vb[n]) / rgbR;
   }
 }
 
-// eight 128-thread blocks per SM (64 registers): measured faster than the
-// uncapped 84 registers
+// A thread per point (a column per thread was bound by the chain of a level's
+// loads, stores and divisions: 4 us a level at any grid level); w at the
+// half levels k and k+1 is formed by both neighbours.
 template <class R>
-__global__ void __launch_bounds__(128, NC_MINB(R, 8, NC_F32_DIAG)) k_diag(DiagArgs<R> a, int pole) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  if (!pole) {
-    diag_column_fused(col_reg(i, j, l), met_of<R>(false), a, (double)P2(CG.GRD_x, 0, i, j, l),
-                      (double)P2(CG.GRD_x, 1, i, j, l), (double)P2(CG.GRD_x, 2, i, j, l));
+__global__ void __launch_bounds__(128, NC_MINB(R, 8, NC_F32_DIAG)) k_diag(const __grid_constant__ DiagArgs<R> a, const __grid_constant__ DiagArgs<R> ap, int npb) {
+  Pt q;
+  if ((int)blockIdx.x < npb) {
+    if (!pole_point((int)(blockIdx.x * blockDim.x + threadIdx.x), q)) return;
+    const R* X = CG.GRD_x_pl + (q.g * cD.LP + q.lp) * 3;
+    diag_point(col_pl(q.g, q.lp), met_of<R>(true), ap, q.k, (double)X[0], (double)X[1], (double)X[2]);
   } else {
-    const R* X = CG.GRD_x_pl;
-    diag_column(col_pl(g, lp), met_of<R>(true), a, (double)X[(g * cD.LP + lp) * 3 + 0],
-                (double)X[(g * cD.LP + lp) * 3 + 1], (double)X[(g * cD.LP + lp) * 3 + 2]);
+    if (!reg_point((int)((blockIdx.x - npb) * blockDim.x + threadIdx.x), q)) return;
+    diag_point(col_reg(q.i, q.j, q.l), met_of<R>(false), a, q.k, (double)P2(CG.GRD_x, 0, q.i, q.j, q.l),
+               (double)P2(CG.GRD_x, 1, q.i, q.j, q.l), (double)P2(CG.GRD_x, 2, q.i, q.j, q.l));
   }
 }
 
@@ -252,8 +177,12 @@ struct AdvMomArgs {
 // the large-step tendencies derived from them are replaced by the exchanges).
 // Arithmetic and association order are those of the reference's expressions
 // (kernels/advconv.py, kernels/advconvmom.py), as in the pole kernel.
-template <class R>
-__global__ void __launch_bounds__(256, NC_MINB(R, 2, NC_F32_ADVMOM)) k_advmom_t(AdvMomArgs<R> a) {
+// The levels are split into gridDim.y chunks of nk where the tiles alone leave
+// SMs idle (see tile_chunks); a chunk walks two levels below its first
+// without storing them, for the projection and the flux that its first needs.
+// (SPLIT; the unsplit instance keeps the registers of the chunk's bounds)
+template <class R, bool SPLIT>
+__global__ void __launch_bounds__(256, NC_MINB(R, 2, NC_F32_ADVMOM)) k_advmom_t(AdvMomArgs<R> a, int nk) {
   constexpr int TXD = 32, TYD = 8;
   constexpr int PX = TXD + 2, PY = TYD + 2;
   __shared__ R s_rv[3][PY * PX], s_vv[3][PY * PX], s_rg[PY * PX];
@@ -278,7 +207,8 @@ __global__ void __launch_bounds__(256, NC_MINB(R, 2, NC_F32_ADVMOM)) k_advmom_t(
   }
   R vmh_lo[3] = {R(0.0), R(0.0), R(0.0)};
   R gwc_prev = R(0.0);
-  for (int k = kmin; k <= kmax; ++k) {
+  const int ka = SPLIT ? kmin + (int)blockIdx.y * nk : kmin, kb = SPLIT ? min(ka + nk - 1, kmax) : kmax;
+  for (int k = SPLIT ? max(ka - 2, kmin) : kmin; k <= kb; ++k) {
     for (int p = tid; p < PX * PY; p += blockDim.x) {
       const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
       const bool ok = ii < G && jj < G;
@@ -331,11 +261,13 @@ __global__ void __launch_bounds__(256, NC_MINB(R, 2, NC_F32_ADVMOM)) k_advmom_t(
       const R dvy = dv[1] - (R(2.0) * rh * (CC.OHM * s_vv[0][c0]));
       const R dvz = dv[2];
       const R prd = dvx * gx + dvy * gy + dvz * gz;
-      a.gvx[p] = dvx - prd * gx;
-      a.gvy[p] = dvy - prd * gy;
-      a.gvz[p] = dvz - prd * gz;
       const R gwc = prd * CC.alpha;
-      a.gw[p] = (k >= kmin + 1) ? (CG.C2W[p] * gwc + CG.C2W[n + p] * gwc_prev) : R(0.0);
+      if (!SPLIT || k >= ka) {
+        a.gvx[p] = dvx - prd * gx;
+        a.gvy[p] = dvy - prd * gy;
+        a.gvz[p] = dvz - prd * gz;
+        a.gw[p] = (k >= kmin + 1) ? (CG.C2W[p] * gwc + CG.C2W[n + p] * gwc_prev) : R(0.0);
+      }
       gwc_prev = gwc;
     }
     __syncthreads();
@@ -376,37 +308,37 @@ __device__ R advconv_pl_at(int g, int lp, int k, const Col& c, const MetT<R>& m,
 }
 
 template <class R>
-__global__ void k_advmom_pl(AdvMomArgs<R> a) {
-  int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= 6 * cD.LP) return;
-  int g = t / cD.LP, lp = t % cD.LP;
+__global__ void k_advmom_pl(const __grid_constant__ AdvMomArgs<R> a) {
+  Pt q_;
+  if (!pole_point((int)(blockIdx.x * blockDim.x + threadIdx.x), q_)) return;
+  const int g = q_.g, lp = q_.lp, k = q_.k;
   const Col c = col_pl(g, lp);
-  const MetT<R> m = met_of<R>(true);
-  const R* X = CG.GRD_x_pl;
-  const R gx = div_r(X[(g * cD.LP + lp) * 3 + 0]), gy = div_r(X[(g * cD.LP + lp) * 3 + 1]),
-               gz = div_r(X[(g * cD.LP + lp) * 3 + 2]);
-  R gwc_prev = R(0.0);
-  for (int k = 0; k < cD.KA; ++k) {
-    int p = c.at(k);
-    if (k < cD.kmin || k > cD.kmax) {
-      a.gvx[p] = R(0.0); a.gvy[p] = R(0.0); a.gvz[p] = R(0.0); a.gw[p] = R(0.0);
-      continue;
-    }
-    R dv[3];
-    const R* vv[3] = {a.vvx, a.vvy, a.vvz};
-    for (int s = 0; s < 3; ++s) dv[s] = advconv_pl_at(g, lp, k, c, m, a.rvx, a.rvy, a.rvz, a.rw, vv[s]);
-    R rh = a.rg[p];
-    R dvx = dv[0] - (-R(2.0) * rh * (CC.OHM * a.vvy[p]));
-    R dvy = dv[1] - (R(2.0) * rh * (CC.OHM * a.vvx[p]));
-    R dvz = dv[2];
-    R prd = dvx * gx + dvy * gy + dvz * gz;
-    a.gvx[p] = dvx - prd * gx;
-    a.gvy[p] = dvy - prd * gy;
-    a.gvz[p] = dvz - prd * gz;
-    R gwc = prd * CC.alpha;
-    a.gw[p] = (k >= cD.kmin + 1) ? (mc(m.C2W, c, 0, 2, k) * gwc + mc(m.C2W, c, 1, 2, k) * gwc_prev) : R(0.0);
-    gwc_prev = gwc;
+  const int p = c.at(k);
+  if (k < cD.kmin || k > cD.kmax) {
+    a.gvx[p] = R(0.0); a.gvy[p] = R(0.0); a.gvz[p] = R(0.0); a.gw[p] = R(0.0);
+    return;
   }
+  const MetT<R> m = met_of<R>(true);
+  const R* X = CG.GRD_x_pl + (g * cD.LP + lp) * 3;
+  const R gx = div_r(X[0]), gy = div_r(X[1]), gz = div_r(X[2]);
+  auto conv = [&](int kk, R dv[3]) -> R {   // the tendency at kk and its vertical component
+    const int q = c.at(kk);
+    dv[0] = advconv_pl_at(g, lp, kk, c, m, a.rvx, a.rvy, a.rvz, a.rw, a.vvx);
+    dv[1] = advconv_pl_at(g, lp, kk, c, m, a.rvx, a.rvy, a.rvz, a.rw, a.vvy);
+    dv[2] = advconv_pl_at(g, lp, kk, c, m, a.rvx, a.rvy, a.rvz, a.rw, a.vvz);
+    const R rh = a.rg[q];
+    dv[0] = dv[0] - (-R(2.0) * rh * (CC.OHM * a.vvy[q]));
+    dv[1] = dv[1] - (R(2.0) * rh * (CC.OHM * a.vvx[q]));
+    return dv[0] * gx + dv[1] * gy + dv[2] * gz;
+  };
+  R dv[3], below[3];
+  const R prd = conv(k, dv);
+  a.gvx[p] = dv[0] - prd * gx;
+  a.gvy[p] = dv[1] - prd * gy;
+  a.gvz[p] = dv[2] - prd * gz;
+  a.gw[p] = (k >= cD.kmin + 1) ? (mc(m.C2W, c, 0, 2, k) * (prd * CC.alpha) +
+                                  mc(m.C2W, c, 1, 2, k) * (conv(k - 1, below) * CC.alpha))
+                               : R(0.0);
 }
 
 // ---------------------------------------------------------------------------
@@ -420,41 +352,8 @@ template <class R>
 struct SixOut { R* f[6]; };
 
 template <class R>
-__global__ void k_hdiff1(Six<R> src, SixOut<R> out) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l;
-  if (!col_of(t, i, j, l)) return;
-  const bool in = interior(i, j);
-  // the column's seven laplacian coefficients, loaded once for all levels
-  R cl[7];
-#pragma unroll
-  for (int m = 0; m < 7; ++m) cl[m] = in ? P2(CG.coef_lap, m, i, j, l) : R(0.0);
-  for (int k = 0; k < cD.KA; ++k) {
-    int p = ix(i, j, k, l);
-#pragma unroll
-    for (int n = 0; n < 6; ++n) {
-      R v = R(0.0);
-      if (in) {
-        const R* s = src.f[n];
-        const R* bs = (n == 4) ? CG.tem_bs : CG.rho_bs;
-        // lap7 (kernels/oprtlaplacian.py:41-55) with the reference-state
-        // deviation for TEM and RHO
-        auto scl = [&](int m) {
-          const int q = ix(i + kNbI[m], j + kNbJ[m], k, l);
-          return (n >= 4) ? s[q] - bs[q] : s[q];
-        };
-        v = cl[0] * scl(0);
-#pragma unroll
-        for (int m = 1; m < 7; ++m) v = v + cl[m] * scl(m);
-      }
-      out.f[n][p] = -v;
-    }
-  }
-}
-
-template <class R>
-__global__ void k_hdiff1_pl(Six<R> src, SixOut<R> out) {
-  int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void k_hdiff1_pl(const __grid_constant__ Six<R> src, const __grid_constant__ SixOut<R> out) {
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= cD.KA * cD.LP) return;
   int k = t / cD.LP, lp = t % cD.LP;
   for (int n = 0; n < 6; ++n) {
@@ -470,6 +369,38 @@ __global__ void k_hdiff1_pl(Six<R> src, SixOut<R> out) {
     out.f[n][ipl(0, k, lp)] = -row;
     for (int g = 1; g < 6; ++g) out.f[n][ipl(g, k, lp)] = -R(0.0);
   }
+}
+
+// A thread per point: with a column per thread the stores of one field held
+// back the loads of the next (5.4 us a level at every grid level).
+template <class R>
+__global__ void k_hdiff1(Six<R> src, SixOut<R> out) {
+  Pt c;
+  const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (!reg_point(p, c)) return;
+  if (!interior(c.i, c.j)) {
+#pragma unroll
+    for (int n = 0; n < 6; ++n) out.f[n][p] = -R(0.0);
+    return;
+  }
+  const int G = cD.G;
+  const int nb[7] = {p, p + 1, p + 1 + G, p + G, p - 1, p - 1 - G, p - G};
+  R cl[7], v[6];
+#pragma unroll
+  for (int m = 0; m < 7; ++m) cl[m] = P2c(CG.coef_lap, m, c.i, c.j, c.l);
+#pragma unroll
+  for (int n = 0; n < 6; ++n) {
+    const R* s = src.f[n];
+    const R* bs = (n == 4) ? CG.tem_bs : CG.rho_bs;
+    // lap7 (kernels/oprtlaplacian.py:41-55) with the reference-state
+    // deviation for TEM and RHO
+    auto scl = [&](int m) { return (n >= 4) ? __ldg(s + nb[m]) - __ldg(bs + nb[m]) : __ldg(s + nb[m]); };
+    v[n] = cl[0] * scl(0);
+#pragma unroll
+    for (int m = 1; m < 7; ++m) v[n] = v[n] + cl[m] * scl(m);
+  }
+#pragma unroll
+  for (int n = 0; n < 6; ++n) out.f[n][p] = -v[n];
 }
 
 // The three vertex weights of each triangle of the Kh-weighted diffusion,
@@ -524,6 +455,53 @@ template <class R>
 constexpr int hdiff2_m_smem() {
   return ((18 + 12) * (HD_DX + 1) * (HD_DY + 1) + 7 * (HD_DX + 2) * (HD_DY + 2)) * (int)sizeof(R);
 }
+template <class R>
+__global__ void k_hdiff2_pl(const __grid_constant__ Six<R> vt, const R* rhog, const __grid_constant__ SixOut<R> out) {
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= cD.KA * cD.LP) return;
+  int k = t / cD.LP, lp = t % cD.LP;
+  for (int n = 0; n < 6; ++n) {
+    const R* s = vt.f[n];
+    R row = R(0.0);
+    if (n < 4) {
+      for (int v = 0; v < 6; ++v) {
+        R tv = CG.coef_lap_pl[v * cD.LP + lp] * s[ipl(v, k, lp)];
+        row = (v == 0) ? tv : row + tv;
+      }
+    } else {
+      // kernels/oprtdiffusion.py:137-177
+      const R fac = (n == 4) ? CC.CVdry : CC.hdiff_fact_rho;
+      R sn = s[ipl(0, k, lp)];
+      R vt_[5][3];
+      for (int v = 1; v <= 5; ++v) {
+        int vp1 = (v == 5) ? 1 : v + 1;
+        R sij = s[ipl(v, k, lp)], sp1 = s[ipl(vp1, k, lp)];
+        for (int d = 0; d < 3; ++d) {
+          const R* cI = CG.coef_intp_pl + ((v * cD.LP + lp) * 3 + d) * 3;
+          R c0 = cI[0], c1 = cI[1], c2 = cI[2];
+          vt_[v - 1][d] = div3((R(2.0) * c0 - c1 - c2) * sn + (-c0 + R(2.0) * c1 - c2) * sij + (-c0 - c1 + R(2.0) * c2) * sp1);
+        }
+      }
+      R khn = rhog[ipl(0, k, lp)] * fac * hdiff_kh<R>(vt.f[4][ipl(0, k, lp)], k);
+      for (int v = 1; v <= 5; ++v) {
+        int vm1 = (v == 1) ? 5 : v - 1;
+        R khv = rhog[ipl(v, k, lp)] * fac * hdiff_kh<R>(vt.f[4][ipl(v, k, lp)], k);
+        R kavg = R(0.5) * (khn + khv);
+        R sd = R(0.0);
+        for (int d = 0; d < 3; ++d) {
+          R cdv = CG.coef_diff_pl[(v * cD.LP + lp) * 3 + d];
+          R tv = cdv * (vt_[vm1 - 1][d] + vt_[v - 1][d]);
+          sd = (d == 0) ? tv : sd + tv;
+        }
+        R contrib = kavg * sd;
+        row = (v == 1) ? contrib : row + contrib;
+      }
+    }
+    out.f[n][ipl(0, k, lp)] = -row;
+    for (int g = 1; g < 6; ++g) out.f[n][ipl(g, k, lp)] = -R(0.0);
+  }
+}
+
 template <class R>
 __global__ void __launch_bounds__(HD_DX * HD_DY, NC_MINB(R, 2, 4)) k_hdiff2_m(Six<R> vt, const R* rhog,
                                                                             SixOut<R> out) {
@@ -635,53 +613,6 @@ __global__ void __launch_bounds__(HD_DX * HD_DY, NC_MINB(R, 2, 4)) k_hdiff2_m(Si
   }
 }
 
-template <class R>
-__global__ void k_hdiff2_pl(Six<R> vt, const R* rhog, SixOut<R> out) {
-  int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  int k = t / cD.LP, lp = t % cD.LP;
-  for (int n = 0; n < 6; ++n) {
-    const R* s = vt.f[n];
-    R row = R(0.0);
-    if (n < 4) {
-      for (int v = 0; v < 6; ++v) {
-        R tv = CG.coef_lap_pl[v * cD.LP + lp] * s[ipl(v, k, lp)];
-        row = (v == 0) ? tv : row + tv;
-      }
-    } else {
-      // kernels/oprtdiffusion.py:137-177
-      const R fac = (n == 4) ? CC.CVdry : CC.hdiff_fact_rho;
-      R sn = s[ipl(0, k, lp)];
-      R vt_[5][3];
-      for (int v = 1; v <= 5; ++v) {
-        int vp1 = (v == 5) ? 1 : v + 1;
-        R sij = s[ipl(v, k, lp)], sp1 = s[ipl(vp1, k, lp)];
-        for (int d = 0; d < 3; ++d) {
-          const R* cI = CG.coef_intp_pl + ((v * cD.LP + lp) * 3 + d) * 3;
-          R c0 = cI[0], c1 = cI[1], c2 = cI[2];
-          vt_[v - 1][d] = div3((R(2.0) * c0 - c1 - c2) * sn + (-c0 + R(2.0) * c1 - c2) * sij + (-c0 - c1 + R(2.0) * c2) * sp1);
-        }
-      }
-      R khn = rhog[ipl(0, k, lp)] * fac * hdiff_kh<R>(vt.f[4][ipl(0, k, lp)], k);
-      for (int v = 1; v <= 5; ++v) {
-        int vm1 = (v == 1) ? 5 : v - 1;
-        R khv = rhog[ipl(v, k, lp)] * fac * hdiff_kh<R>(vt.f[4][ipl(v, k, lp)], k);
-        R kavg = R(0.5) * (khn + khv);
-        R sd = R(0.0);
-        for (int d = 0; d < 3; ++d) {
-          R cdv = CG.coef_diff_pl[(v * cD.LP + lp) * 3 + d];
-          R tv = cdv * (vt_[vm1 - 1][d] + vt_[v - 1][d]);
-          sd = (d == 0) ? tv : sd + tv;
-        }
-        R contrib = kavg * sd;
-        row = (v == 1) ? contrib : row + contrib;
-      }
-    }
-    out.f[n][ipl(0, k, lp)] = -row;
-    for (int g = 1; g < 6; ++g) out.f[n][ipl(g, k, lp)] = -R(0.0);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Large-step tendency: hyperdiffusion tendency (mod_numfilter.py:1519-1578)
 // + horizontalize (mod_numfilter.py:1364-1369) + g_TEND = adv + f
@@ -698,9 +629,10 @@ struct GtendArgs {
 };
 
 template <class R>
-__device__ void gtend_column(const Col c, const MetT<R> m, const GtendArgs<R>& a, int i, int j, int l, int g, int lp) {
-  for (int k = 0; k < cD.KA; ++k) {
-    int p = c.at(k);
+__device__ void gtend_point(const Col c, const MetT<R> m, const GtendArgs<R>& a, int i, int j, int k, int l, int g,
+                            int lp) {
+  {
+    const int p = c.at(k);
     R rg = a.rhog[p];
     R rgh = R(0.0);
     if (k >= cD.kmin) rgh = mc(m.C2W, c, 0, 2, k) * rg + mc(m.C2W, c, 1, 2, k) * a.rhog[c.at(k - 1)];
@@ -742,12 +674,14 @@ __device__ void gtend_column(const Col c, const MetT<R> m, const GtendArgs<R>& a
 }
 
 template <class R>
-__global__ void k_gtend(GtendArgs<R> a, int pole) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  if (!pole) gtend_column(col_reg(i, j, l), met_of<R>(false), a, i, j, l, 0, 0);
-  else gtend_column(col_pl(g, lp), met_of<R>(true), a, 0, 0, 0, g, lp);
+__global__ void k_gtend(const __grid_constant__ GtendArgs<R> a, const __grid_constant__ GtendArgs<R> ap, int npb) {
+  Pt q;
+  if ((int)blockIdx.x < npb) {
+    if (pole_point((int)(blockIdx.x * blockDim.x + threadIdx.x), q))
+      gtend_point(col_pl(q.g, q.lp), met_of<R>(true), ap, 0, 0, q.k, 0, q.g, q.lp);
+  } else if (reg_point((int)((blockIdx.x - npb) * blockDim.x + threadIdx.x), q)) {
+    gtend_point(col_reg(q.i, q.j, q.l), met_of<R>(false), a, q.i, q.j, q.k, q.l, 0, 0);
+  }
 }
 
 }  // namespace nc

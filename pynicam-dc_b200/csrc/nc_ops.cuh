@@ -52,6 +52,34 @@ __device__ __forceinline__ bool map_col(int pole, int t, int& i, int& j, int& l,
   return true;
 }
 
+// Thread -> grid point of a launch whose first npb blocks (along x) take the
+// pole points and the others the regional points, halo ring included.  A
+// thread per point: where a level needs its neighbours' half-level values it
+// forms them again, so no thread walks a column.
+struct Pt {
+  int i, j, k, l, g, lp;
+};
+__device__ __forceinline__ bool pole_point(int t, Pt& q) {
+  if (t >= 6 * cD.KA * cD.LP) return false;
+  q.lp = t % cD.LP;
+  q.k = (t / cD.LP) % cD.KA;
+  q.g = t / (cD.LP * cD.KA);
+  q.i = q.j = q.l = 0;
+  return true;
+}
+__device__ __forceinline__ bool reg_point(int t, Pt& q) {
+  if (t >= cD.npti) return false;
+  const int G = cD.G;
+  q.i = t % G;
+  int r = t / G;
+  q.j = r % G;
+  r /= G;
+  q.k = r % cD.KA;
+  q.l = r / cD.KA;
+  q.g = q.lp = 0;
+  return true;
+}
+
 // Metric selection by column kind
 template <class R>
 struct MetT {

@@ -63,8 +63,53 @@ constexpr int dd3d_m_smem() {
 // barrier is needed at the end of a level, and the corner tile alone waits
 // for its singular-point fix.
 
+// pole 3-D divergence damping (kernels/oprt3ddivdamp.py:176-237)
+template <class R>
+__global__ void k_dd3d_pl(const __grid_constant__ Four<R> v, const __grid_constant__ Three<R> out) {
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= cD.KA * cD.LP) return;
+  int k = t / cD.LP, lp = t % cD.LP;
+  for (int g = 0; g < 6; ++g)
+    for (int d = 0; d < 3; ++d) out.f[d][ipl(g, k, lp)] = R(0.0);
+  if (k < cD.kmin || k > cD.kmax) return;
+  auto rw = [&](int g, int kk) -> R {
+    if (kk <= cD.kmin || kk > cD.kmax) return R(0.0);
+    int q = ipl(g, kk, lp), qm = ipl(g, kk - 1, lp);
+    const R* cz = CG.C2WGz_pl;
+    R h = cz[q * 6 + 0] * v.f[0][q] + cz[q * 6 + 1] * v.f[0][qm] + cz[q * 6 + 2] * v.f[1][q] +
+               cz[q * 6 + 3] * v.f[1][qm] + cz[q * 6 + 4] * v.f[2][q] + cz[q * 6 + 5] * v.f[2][qm];
+    return h * gam_at(CG.RGAMH_pl, q) + v.f[3][q] * CG.RGSQRTH_pl[q];
+  };
+  R vm[6][3];
+  for (int g = 0; g < 6; ++g) {
+    int q = ipl(g, k, lp);
+    for (int d = 0; d < 3; ++d) vm[g][d] = v.f[d][q] * gam_at(CG.RGAM_pl, q);
+  }
+  R sclt[5];
+  for (int v_ = 1; v_ <= 5; ++v_) {
+    int vp1 = (v_ == 5) ? 1 : v_ + 1;
+    R sw = div3((rw(0, k + 1) + rw(v_, k + 1) + rw(vp1, k + 1)) - (rw(0, k) + rw(v_, k) + rw(vp1, k))) * CC.rdgz[k];
+    const R* cI = CG.coef_intp_pl + (v_ * cD.LP + lp) * 9;
+    sclt[v_ - 1] = cI[0] * vm[0][0] + cI[1] * vm[v_][0] + cI[2] * vm[vp1][0] + cI[3] * vm[0][1] + cI[4] * vm[v_][1] +
+                   cI[5] * vm[vp1][1] + cI[6] * vm[0][2] + cI[7] * vm[v_][2] + cI[8] * vm[vp1][2] + sw;
+  }
+  for (int d = 0; d < 3; ++d) {
+    R row = R(0.0);
+    for (int v_ = 1; v_ <= 5; ++v_) {
+      int vm1 = (v_ == 1) ? 5 : v_ - 1;
+      R pair = sclt[vm1 - 1] + sclt[v_ - 1];
+      R tv = CG.coef_diff_pl[(v_ * cD.LP + lp) * 3 + d] * pair;
+      row = (v_ == 1) ? tv : row + tv;
+    }
+    out.f[d][ipl(0, k, lp)] = row;
+  }
+}
+
+// The levels are split into chunks of nk where the tiles alone leave SMs idle
+// (see tile_chunks); blockIdx.z counts (region, chunk).
 template <class R, bool CDR>
-__global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4))) k_dd3d_m(Four<R> v, Three<R> out) {
+__global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4))) k_dd3d_m(Four<R> v, Three<R> out,
+                                                                                           int nk) {
   constexpr int PX = DD_DX + 2, PY = DD_DY + 2, NP = PX * PY;
   constexpr int TX = DD_DX + 1, TY = DD_DY + 1, NT = TX * TY;
   extern __shared__ __align__(16) unsigned char dd_smem[];
@@ -73,7 +118,8 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4
   R* s_rw = s_vm + 3 * NP;                     // [2][NP]
   R* s_ti = s_rw + 2 * NP;                     // [NT]
   R* s_tj = s_ti + NT;                         // [NT]
-  const int l = blockIdx.z;
+  const int l = (int)blockIdx.z % cD.L;
+  const int ka = cD.kmin + (int)blockIdx.z / cD.L * nk, kb = min(ka + nk - 1, cD.kmax);
   const int i0 = 1 + blockIdx.x * DD_DX, j0 = 1 + blockIdx.y * DD_DY;
   const int G = cD.G, gmax = cD.G - 2;
   const int tid = threadIdx.x, tx = tid % DD_DX, ty = tid / DD_DX;
@@ -92,9 +138,19 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4
 #pragma unroll
     for (int m = 0; m < (CDR ? 18 : 1); ++m) cd[m] = P2c(CG.coef_diff, m, i, j, l);
   }
-  for (int p = tid; p < NP; p += blockDim.x) s_rw[p] = R(0.0);   // rwv(kmin) = 0
+  // vertical mass flux at half level k (q: the point at k)
+  auto rwv = [&](int q) -> R {
+    const int qm = q - cD.planei;
+    const R h = cz[q] * v.f[0][q] + cz[n + q] * v.f[0][qm] + cz[2 * n + q] * v.f[1][q] + cz[3 * n + q] * v.f[1][qm] +
+                cz[4 * n + q] * v.f[2][q] + cz[5 * n + q] * v.f[2][qm];
+    return h * gam_at(CG.RGAMH, q) + v.f[3][q] * CG.RGSQRTH[q];
+  };
+  for (int p = tid; p < NP; p += blockDim.x) {   // at the chunk's first level (zero at kmin)
+    const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
+    s_rw[p] = (ka > cD.kmin && ii < G && jj < G) ? rwv(ix(ii, jj, ka, l)) : R(0.0);
+  }
   int cur = 0;
-  for (int k = cD.kmin; k <= cD.kmax; ++k) {
+  for (int k = ka; k <= kb; ++k) {
     const bool up = (k + 1 <= cD.kmax);   // rwv(k+1) = 0 above kmax
     for (int p = tid; p < NP; p += blockDim.x) {
       const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
@@ -181,80 +237,10 @@ __device__ __forceinline__ TileLv tile_level(int kbase) {
   return t;
 }
 
-// pole 3-D divergence damping (kernels/oprt3ddivdamp.py:176-237)
-template <class R>
-__global__ void k_dd3d_pl(Four<R> v, Three<R> out) {
-  int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  int k = t / cD.LP, lp = t % cD.LP;
-  for (int g = 0; g < 6; ++g)
-    for (int d = 0; d < 3; ++d) out.f[d][ipl(g, k, lp)] = R(0.0);
-  if (k < cD.kmin || k > cD.kmax) return;
-  auto rw = [&](int g, int kk) -> R {
-    if (kk <= cD.kmin || kk > cD.kmax) return R(0.0);
-    int q = ipl(g, kk, lp), qm = ipl(g, kk - 1, lp);
-    const R* cz = CG.C2WGz_pl;
-    R h = cz[q * 6 + 0] * v.f[0][q] + cz[q * 6 + 1] * v.f[0][qm] + cz[q * 6 + 2] * v.f[1][q] +
-               cz[q * 6 + 3] * v.f[1][qm] + cz[q * 6 + 4] * v.f[2][q] + cz[q * 6 + 5] * v.f[2][qm];
-    return h * gam_at(CG.RGAMH_pl, q) + v.f[3][q] * CG.RGSQRTH_pl[q];
-  };
-  R vm[6][3];
-  for (int g = 0; g < 6; ++g) {
-    int q = ipl(g, k, lp);
-    for (int d = 0; d < 3; ++d) vm[g][d] = v.f[d][q] * gam_at(CG.RGAM_pl, q);
-  }
-  R sclt[5];
-  for (int v_ = 1; v_ <= 5; ++v_) {
-    int vp1 = (v_ == 5) ? 1 : v_ + 1;
-    R sw = div3((rw(0, k + 1) + rw(v_, k + 1) + rw(vp1, k + 1)) - (rw(0, k) + rw(v_, k) + rw(vp1, k))) * CC.rdgz[k];
-    const R* cI = CG.coef_intp_pl + (v_ * cD.LP + lp) * 9;
-    sclt[v_ - 1] = cI[0] * vm[0][0] + cI[1] * vm[v_][0] + cI[2] * vm[vp1][0] + cI[3] * vm[0][1] + cI[4] * vm[v_][1] +
-                   cI[5] * vm[vp1][1] + cI[6] * vm[0][2] + cI[7] * vm[v_][2] + cI[8] * vm[vp1][2] + sw;
-  }
-  for (int d = 0; d < 3; ++d) {
-    R row = R(0.0);
-    for (int v_ = 1; v_ <= 5; ++v_) {
-      int vm1 = (v_ == 1) ? 5 : v_ - 1;
-      R pair = sclt[vm1 - 1] + sclt[v_ - 1];
-      R tv = CG.coef_diff_pl[(v_ * cD.LP + lp) * 3 + d] * pair;
-      row = (v_ == 1) ? tv : row + tv;
-    }
-    out.f[d][ipl(0, k, lp)] = row;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // post-COMM 2-D divergence damping (kernels/divdamppostcomm.py:29-81):
-// gd = coef * OPRT_divdamp(-vtmp2), then horizontalize (interior).
+// gd = coef * OPRT_divdamp(-vtmp2), then horizontalize.
 // ---------------------------------------------------------------------------
-template <class R>
-__device__ void divdamp2d_at(const CThree<R>& vt, int i, int j, int k, int l, R gd[3]) {
-  if (!interior(i, j)) {
-    for (int d = 0; d < 3; ++d) gd[d] = CC.divdamp_coef * R(0.0);
-    return;
-  }
-  auto sc = [&](int ii, int jj, R& sTI, R& sTJ) {
-    int a = ix(ii, jj, k, l), b = ix(ii + 1, jj, k, l), c = ix(ii + 1, jj + 1, k, l), d = ix(ii, jj + 1, k, l);
-    auto C = [&](int dir, int p, int t) { return P2(CG.coef_intp, (dir * 3 + p) * 2 + t, ii, jj, l); };
-    R x0 = -vt.f[0][a], x1 = -vt.f[0][b], x2 = -vt.f[0][c], x3 = -vt.f[0][d];
-    R y0 = -vt.f[1][a], y1 = -vt.f[1][b], y2 = -vt.f[1][c], y3 = -vt.f[1][d];
-    R z0 = -vt.f[2][a], z1 = -vt.f[2][b], z2 = -vt.f[2][c], z3 = -vt.f[2][d];
-    sTI = C(0, 0, 0) * x0 + C(0, 1, 0) * x1 + C(0, 2, 0) * x2 + C(1, 0, 0) * y0 + C(1, 1, 0) * y1 + C(1, 2, 0) * y2 +
-          C(2, 0, 0) * z0 + C(2, 1, 0) * z1 + C(2, 2, 0) * z2;
-    sTJ = C(0, 0, 1) * x0 + C(0, 1, 1) * x2 + C(0, 2, 1) * x3 + C(1, 0, 1) * y0 + C(1, 1, 1) * y2 + C(1, 2, 1) * y3 +
-          C(2, 0, 1) * z0 + C(2, 1, 1) * z2 + C(2, 2, 1) * z3;
-  };
-  R aTI, aTJ, bTI, bTJ, cTI, cTJ, dTI, dTJ;
-  sc(i, j, aTI, aTJ);
-  sc(i - 1, j, bTI, bTJ);
-  sc(i - 1, j - 1, cTI, cTJ);
-  sc(i, j - 1, dTI, dTJ);
-  R o[3];
-  for (int d = 0; d < 3; ++d) o[d] = CC.divdamp_coef * ddivd(i, j, l, d, aTI, aTJ, bTI, cTJ, cTI, dTJ);
-  horiz_reg(i, j, l, o[0], o[1], o[2]);
-  gd[0] = o[0]; gd[1] = o[1]; gd[2] = o[2];
-}
-
 // pole 2-D divergence damping of -vtmp2 at (g,k,lp) (kernels/oprtdivdamp.py:125-173
 // then horizontalize over all g)
 template <class R>
@@ -292,23 +278,6 @@ __device__ void divdamp2d_pl_at(const CThree<R>& vt, int g, int k, int lp, R gd[
 // k with the first-layer remedy and the tangent-plane projection.
 // P(ii,jj,kk) gives the pressure; returns Pgrad (3 comps).
 // ---------------------------------------------------------------------------
-template <class R, class PF>
-__device__ void presgrad_reg(int i, int j, int k, int l, const Col& c, const MetT<R>& m, PF P, R out[3]) {
-  const int kmin = cD.kmin, kmax = cD.kmax;
-  out[0] = out[1] = out[2] = R(0.0);
-  if (k >= kmin && k <= kmax) {
-    const int kk = (k == kmin) ? kmin + 1 : k;
-    R gh[3] = {R(0.0), R(0.0), R(0.0)};
-    if (interior(i, j)) grad7(i, j, kk, l, [&](int ii, int jj, int k2) { return P(ii, jj, k2) * gam_at(CG.RGAM, ix(ii, jj, k2, l)); }, gh);
-    auto pvmh = [&](int k2, int d) {
-      return (mc(m.C2WGz, c, 2 * d, 6, k2) * P(i, j, k2) + mc(m.C2WGz, c, 2 * d + 1, 6, k2) * P(i, j, k2 - 1)) *
-             gam_at(m.RGAMH, c.at(k2));
-    };
-    for (int d = 0; d < 3; ++d) out[d] = gh[d] + (pvmh(kk + 1, d) - pvmh(kk, d)) * CC.rdgz[kk];
-  }
-  if (interior(i, j)) horiz_reg(i, j, l, out[0], out[1], out[2]);
-}
-
 template <class R, class PF>
 __device__ void presgrad_pl(int g, int k, int lp, const Col& c, const MetT<R>& m, PF P, R out[3]) {
   const int kmin = cD.kmin, kmax = cD.kmax;
@@ -392,15 +361,18 @@ struct Vp0Args {
   double dt;                    // small-step dt
 };
 
-// One pole column of vp0.  In the mixed form the horizontal operators run in
+// One pole point of vp0.  In the mixed form the horizontal operators run in
 // float32 (R) and the vertical part -- buoyancy and vertical pressure gradient
 // of the float64 deviations, gz, the implicit matrix and the vertical-momentum
 // tendency -- in float64, as in the regional column kernel k_vp0_cr.
-template <class R, bool POLE>
-__device__ void vp0_column(const Vp0Args<R>& a, int i, int j, int l, int g, int lp) {
-  const Col c = POLE ? col_pl(g, lp) : col_reg(i, j, l);
-  const MetT<R> m = met_of<R>(POLE);
-  const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
+template <class R>
+__global__ void k_vp0_pl(const __grid_constant__ Vp0Args<R> a) {
+  Pt q_;
+  if (!pole_point((int)(blockIdx.x * blockDim.x + threadIdx.x), q_)) return;
+  const int g = q_.g, lp = q_.lp, k = q_.k;
+  const Col c = col_pl(g, lp);
+  const MetT<R> m = met_of<R>(true);
+  const int kmin = cD.kmin, kmax = cD.kmax;
   const R* const* P = a.P.v;
   const double dt = a.dt;
   // column-local half-level values (float64)
@@ -428,22 +400,11 @@ __device__ void vp0_column(const Vp0Args<R>& a, int i, int j, int l, int g, int 
   auto pwh = [&](int k) -> R { return R(-gz(k) * (double)P[4][c.at(k)]); };
   auto PF = [&](int k, int d) -> R { return P[1 + d][c.at(k)]; };
   auto PEF = [&](int k, int d) -> R { return P[1 + d][c.at(k)] * a.eth[c.at(k)]; };
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
+  {
+    const int p = c.at(k);
     // horizontal divergences
     R div1 = R(0.0), div2 = R(0.0);
-    if (!POLE) {
-      if (interior(i, j)) {
-        div1 = div7<R>(i, j, k, l, [&](int ii, int jj, int kk, int d) {
-          int q = ix(ii, jj, kk, l);
-          return P[1 + d][q] * gam_at(CG.RGAM, q);
-        });
-        div2 = div7<R>(i, j, k, l, [&](int ii, int jj, int kk, int d) {
-          int q = ix(ii, jj, kk, l);
-          return (P[1 + d][q] * a.eth[q]) * gam_at(CG.RGAM, q);
-        });
-      }
-    } else if (g == 0) {
+    if (g == 0) {
       div1 = div_pl<R>(lp, k, [&](int q, int d) { return P[1 + d][q]; });
       div2 = div_pl<R>(lp, k, [&](int q, int d) { return P[1 + d][q] * a.eth[q]; });
     }
@@ -453,13 +414,8 @@ __device__ void vp0_column(const Vp0Args<R>& a, int i, int j, int l, int g, int 
       return P[4][q] * (CC.afact[kk] * a.eth[q] + CC.bfact[kk] * a.eth[c.at(kk - 1)]);
     });
     R dd[3], dpg[3];
-    if (!POLE) {
-      divdamp2d_at(a.vt, i, j, k, l, dd);
-      presgrad_reg(i, j, k, l, c, m, [&](int ii, int jj, int kk) { return R(a.pregd[ix(ii, jj, kk, l)]); }, dpg);
-    } else {
-      divdamp2d_pl_at(a.vt, g, k, lp, dd);
-      presgrad_pl(g, k, lp, c, m, [&](int gg, int kk) { return R(a.pregd[ipl(gg, kk, lp)]); }, dpg);
-    }
+    divdamp2d_pl_at(a.vt, g, k, lp, dd);
+    presgrad_pl(g, k, lp, c, m, [&](int gg, int kk) { return R(a.pregd[ipl(gg, kk, lp)]); }, dpg);
     R pw = R(0.0);
     if (k >= kmin && k <= kmax)
       pw = a.vx[p] * dpg[0] + a.vy[p] * dpg[1] + a.vz[p] * dpg[2] + mc(m.W2C, c, 0, 2, k) * pwh(k + 1) +
@@ -660,15 +616,19 @@ __global__ void __launch_bounds__(VP_DX * VP_DY, NC_MINB(R, 4, NC_F32_VP0H)) k_v
 // k and k-1 are carried in registers.  Each value is the expression of
 // vp0_column (the pole form), so regional and pole columns round alike.
 // 256-thread blocks capped at 64 registers (four per SM; measured faster
-// than three at 74 registers)
+// than three at 74 registers).  blockIdx.y takes a chunk of nk levels: a whole
+// column per thread walked 42 levels at 9 us each, however few the columns;
+// a chunk forms the half-level values of its first two levels again.
 #define NC_VP0C_BLOCK 256
 template <class R>
-__global__ void __launch_bounds__(NC_VP0C_BLOCK, NC_MINB(R, 4, NC_F32_VP0C)) k_vp0_cr(Vp0Args<R> a, Vp0H<R> h) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(NC_VP0C_BLOCK, NC_MINB(R, 3, NC_F32_VP0C)) k_vp0_cr(Vp0Args<R> a, Vp0H<R> h,
+                                                                                   int nk) {
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   int i, j, l;
   if (!col_of(t, i, j, l)) return;
   const Col c = col_reg(i, j, l);
   const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
+  const int ka = (int)blockIdx.y * nk, kb = min(ka + nk, KA);
   const int n = cD.npti;
   const bool in = interior(i, j);
   const R* const* P = a.P.v;
@@ -679,101 +639,100 @@ __global__ void __launch_bounds__(NC_VP0C_BLOCK, NC_MINB(R, 4, NC_F32_VP0C)) k_v
   const R* w2c = CG.W2C;
   const double GCVovR = cC.GRAV * cC.CVdry / cC.Rdry;
   const double ACVovRt2 = cC.alpha * cC.CVdry / cC.Rdry / (dt * dt);
-  // values at level k (index 0) and k-1 (index m), carried upward
-  double vA0 = 0.0, vE0 = 0.0;            // vertical fluxes of rhog / rhoge at half level k
-  double gz0 = 0.0, gzm = 0.0;            // gz at k and k-1
-  double eh0 = 0.0, ehm = 0.0;            // half-level eth at k and k-1
-  double pwh0 = 0.0, dpgw0 = 0.0, dbuo0 = 0.0, vint0 = 0.0;
-  for (int k = 0; k < KA; ++k) {
-    const int p = c.at(k);
-    const int kn = k + 1;
-    // ---- half-level values at kn = k+1
-    double vA1 = 0.0, vE1 = 0.0, gz1 = 0.0, eh1 = 0.0, pwh1 = 0.0, dpgw1 = 0.0, dbuo1 = 0.0, vint1 = 0.0;
-    if (kn < KA) {
-      const int q = c.at(kn), qm = c.at(kn - 1);
-      if (kn > kmin && kn <= kmax) {
-        const double rgh = gam_at(CG.RGAMH, q), rsq = CG.RGSQRTH[q];
-        const double z0 = cz[q], z1 = cz[n + q], z2 = cz[2 * n + q], z3 = cz[3 * n + q], z4 = cz[4 * n + q],
-                     z5 = cz[5 * n + q];
-        const double px = P[1][q], pxm = P[1][qm], py = P[2][q], pym = P[2][qm], pz = P[3][q], pzm = P[3][qm];
-        const double e = a.eth[q], em = a.eth[qm], w = P[4][q];
-        const double hA = z0 * px + z1 * pxm + z2 * py + z3 * pym + z4 * pz + z5 * pzm;
-        vA1 = hA * rgh + 1.0 * w * rsq;
-        const double hE = z0 * (px * e) + z1 * (pxm * em) + z2 * (py * e) + z3 * (pym * em) + z4 * (pz * e) +
-                          z5 * (pzm * em);
-        vE1 = hE * rgh + 1.0 * (w * (cC.afact[kn] * e + cC.bfact[kn] * em)) * rsq;
-        // vertical kinetic-energy term of rhogkin
-        const double den = c2w[q] * P[0][q] + c2w[n + q] * P[0][qm];
-        vint1 = 0.5 * (w * w) / den;
-        // buoyancy and vertical pressure gradient
-        dbuo1 = -GRAV * (c2w[q] * a.rhogd[q] + c2w[n + q] * a.rhogd[qm]);
-        dpgw1 = gam_at(CG.GAM2H, q) * (a.pregd[q] * CG.RGSGAM2[q] - a.pregd[qm] * CG.RGSGAM2[qm]) * cC.rdgzh[kn];
-      }
-      if (kn >= kmin && kn <= kmax + 1) {
-        const int kk = kn;   // kn >= kmin here, so the clamp of rhog_h / eth_h is inactive
-        const double rh = c2w[q] * P[0][q] + c2w[n + q] * P[0][c.at(kk - 1)];
-        gz1 = GRAV - (dpgw1 - dbuo1) / rh;
-        pwh1 = -gz1 * P[4][q];
-        eh1 = cC.afact[kk] * a.eth[q] + cC.bfact[kk] * a.eth[c.at(kk - 1)];
-      }
+  // half-level values; those at level k (h0) and k-1 (hm) are carried upward
+  struct Half {
+    double vA, vE, gz, eh, pwh, dpgw, dbuo, vint;   // vertical fluxes of rhog / rhoge, gz, eth, ...
+  };
+  auto half = [&](int kn) -> Half {
+    Half r{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (kn < kmin || kn > kmax + 1) return r;
+    const int q = c.at(kn), qm = c.at(kn - 1);
+    const double e = __ldg(a.eth + q), em = __ldg(a.eth + qm), w = __ldg(P[4] + q);
+    const double c0 = __ldg(c2w + q), c1 = __ldg(c2w + n + q);
+    const double r0 = __ldg(P[0] + q), r1 = __ldg(P[0] + qm);
+    const double rh = c0 * r0 + c1 * r1;
+    if (kn > kmin && kn <= kmax) {
+      const double rgh = gam_at(CG.RGAMH, q), rsq = __ldg(CG.RGSQRTH + q);
+      const double z0 = __ldg(cz + q), z1 = __ldg(cz + n + q), z2 = __ldg(cz + 2 * n + q), z3 = __ldg(cz + 3 * n + q),
+                   z4 = __ldg(cz + 4 * n + q), z5 = __ldg(cz + 5 * n + q);
+      const double px = __ldg(P[1] + q), pxm = __ldg(P[1] + qm), py = __ldg(P[2] + q), pym = __ldg(P[2] + qm),
+                   pz = __ldg(P[3] + q), pzm = __ldg(P[3] + qm);
+      const double hA = z0 * px + z1 * pxm + z2 * py + z3 * pym + z4 * pz + z5 * pzm;
+      r.vA = hA * rgh + 1.0 * w * rsq;
+      const double hE = z0 * (px * e) + z1 * (pxm * em) + z2 * (py * e) + z3 * (pym * em) + z4 * (pz * e) +
+                        z5 * (pzm * em);
+      r.vE = hE * rgh + 1.0 * (w * (cC.afact[kn] * e + cC.bfact[kn] * em)) * rsq;
+      // vertical kinetic-energy term of rhogkin
+      r.vint = 0.5 * (w * w) / rh;
+      // buoyancy and vertical pressure gradient
+      r.dbuo = -GRAV * (c0 * __ldg(a.rhogd + q) + c1 * __ldg(a.rhogd + qm));
+      r.dpgw = gam_at(CG.GAM2H, q) * (__ldg(a.pregd + q) * __ldg(CG.RGSGAM2 + q) - __ldg(a.pregd + qm) * __ldg(CG.RGSGAM2 + qm)) *
+               cC.rdgzh[kn];
     }
+    r.gz = GRAV - (r.dpgw - r.dbuo) / rh;
+    r.pwh = -r.gz * w;
+    r.eh = cC.afact[kn] * e + cC.bfact[kn] * em;
+    return r;
+  };
+  double gzm = 0.0, ehm = 0.0;
+  if (ka > 0) {
+    const Half x = half(ka - 1);
+    gzm = x.gz;
+    ehm = x.eh;
+  }
+  Half h0 = half(ka);
+  for (int k = ka; k < kb; ++k) {
+    const int p = c.at(k);
+    const Half h1 = half(k + 1);   // zero at KA
     // ---- level k
     const bool hk = in && k >= kmin && k <= kmax;
     const bool kin = k >= kmin && k <= kmax;
-    const double div1 = hk ? h.out[0][p] : 0.0, div2 = hk ? h.out[1][p] : 0.0;
-    const double drhog = kin ? -div1 - (vA1 - vA0) * cC.rdgz[k] : 0.0;
-    const double drhoge = kin ? -div2 - (vE1 - vE0) * cC.rdgz[k] : 0.0;
-    double dd[3], dpg[3];
+    // every load of the level before its stores
+    double hv[8], g[6];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      dd[d] = hk ? h.out[2 + d][p] : 0.0;
-      dpg[d] = hk ? h.out[5 + d][p] : 0.0;
+    for (int d = 0; d < 8; ++d) hv[d] = hk ? __ldg(h.out[d] + p) : R(0.0);
+#pragma unroll
+    for (int d = 0; d < 6; ++d) g[d] = __ldg(a.gT0[d] + p);
+    const double rg0 = __ldg(P[0] + p), eth = __ldg(a.eth + p), phi = __ldg(CG.PHI + p);
+    const double* dd = hv + 2;
+    const double* dpg = hv + 5;
+    double pw = 0.0, drhog = 0.0, drhoge = 0.0, kin0 = 0.0;
+    if (kin) {
+      drhog = -hv[0] - (h1.vA - h0.vA) * cC.rdgz[k];
+      drhoge = -hv[1] - (h1.vE - h0.vE) * cC.rdgz[k];
+      const double w0 = __ldg(w2c + p), w1 = __ldg(w2c + n + p);
+      pw = __ldg(a.vx + p) * dpg[0] + __ldg(a.vy + p) * dpg[1] + __ldg(a.vz + p) * dpg[2] + w0 * h1.pwh + w1 * h0.pwh;
+      const double vx = __ldg(P[1] + p), vy = __ldg(P[2] + p), vz = __ldg(P[3] + p);
+      const double kh = 0.5 * (vx * vx + vy * vy + vz * vz) / rg0;
+      kin0 = kh + w0 * h1.vint + w1 * h0.vint;
     }
-    double pw = 0.0;
-    if (kin)
-      pw = a.vx[p] * dpg[0] + a.vy[p] * dpg[1] + a.vz[p] * dpg[2] + w2c[p] * pwh1 + w2c[n + p] * pwh0;
-    a.gT[0][p] = a.gT0[0][p] + drhog;
-    a.gT[1][p] = a.gT0[1][p] - dpg[0] + dd[0] + 0.0;
-    a.gT[2][p] = a.gT0[2][p] - dpg[1] + dd[1] + 0.0;
-    a.gT[3][p] = a.gT0[3][p] - dpg[2] + dd[2] + 0.0;
-    a.gT[4][p] = a.gT0[4][p] + 0.0 * cC.alpha - dpgw0 + dbuo0;
-    a.gT[5][p] = a.gT0[5][p] + drhoge + pw;
     if (k >= kmin + 1 && k <= kmax) {
       const int pm = c.at(k - 1), pp = c.at(k + 1);
       const double rg = cC.rdgz[k], rgm = cC.rdgz[k - 1];
-      const double Ca = (CG.RGSGAM2[p] * rg + CG.RGSGAM2[pm] * rgm) * gam_at(CG.GAM2H, p);
+      const double rs = __ldg(CG.RGSGAM2 + p);
+      const double Ca = (rs * rg + __ldg(CG.RGSGAM2 + pm) * rgm) * gam_at(CG.GAM2H, p);
       const double Cb = cC.dfact[k] - cC.cfact[k - 1];
-      const double Cu1 = CG.RGSGAM2[p] * rg * gam_at(CG.GAM2H, pp);
+      const double Cu1 = rs * rg * gam_at(CG.GAM2H, pp);
       const double rgh2 = gam_at(CG.RGAMH, p) * gam_at(CG.RGAMH, p);
       const double Cu2 = gam_at(CG.GAM2H, pp) * rgh2 * GCVovR;
-      const double Cl1 = CG.RGSGAM2[p] * rg * gam_at(CG.GAM2H, pm);
+      const double Cl1 = rs * rg * gam_at(CG.GAM2H, pm);
       const double Cl2 = gam_at(CG.GAM2H, pm) * rgh2 * GCVovR;
       const double rgh = cC.rdgzh[k];
-      a.Mc[p] = ACVovRt2 / CG.RGSQRTH[p] + rgh * (Ca * eh0 - Cb * (gz0 + GCVovR));
-      a.Mu[p] = -rgh * (Cu1 * eh1 + cC.cfact[k] * (gz1 + Cu2));
+      a.Mc[p] = ACVovRt2 / __ldg(CG.RGSQRTH + p) + rgh * (Ca * h0.eh - Cb * (h0.gz + GCVovR));
+      a.Mu[p] = -rgh * (Cu1 * h1.eh + cC.cfact[k] * (h1.gz + Cu2));
       a.Ml[p] = -rgh * (Cl1 * ehm - cC.dfact[k - 1] * (gzm + Cl2));
     }
-    double kin0 = 0.0;
-    if (kin) {
-      const double rg = P[0][p], vx = P[1][p], vy = P[2][p], vz = P[3][p];
-      const double kh = 0.5 * (vx * vx + vy * vy + vz * vz) / rg;
-      kin0 = kh + w2c[p] * vint1 + w2c[n + p] * vint0;
-    }
-    a.ethtot0[p] = a.eth[p] + kin0 / P[0][p] + CG.PHI[p];
-    vA0 = vA1; vE0 = vE1;
-    gzm = gz0; gz0 = gz1;
-    ehm = eh0; eh0 = eh1;
-    pwh0 = pwh1; dpgw0 = dpgw1; dbuo0 = dbuo1; vint0 = vint1;
+    a.gT[0][p] = g[0] + drhog;
+    a.gT[1][p] = g[1] - dpg[0] + dd[0] + 0.0;
+    a.gT[2][p] = g[2] - dpg[1] + dd[1] + 0.0;
+    a.gT[3][p] = g[3] - dpg[2] + dd[2] + 0.0;
+    a.gT[4][p] = g[4] + 0.0 * cC.alpha - h0.dpgw + h0.dbuo;
+    a.gT[5][p] = g[5] + drhoge + pw;
+    a.ethtot0[p] = eth + kin0 / rg0 + phi;
+    gzm = h0.gz;
+    ehm = h0.eh;
+    h0 = h1;
   }
-}
-
-template <class R>
-__global__ void k_vp0(Vp0Args<R> a, int pole) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  if (!pole) vp0_column<R, false>(a, i, j, l, 0, 0);
-  else vp0_column<R, true>(a, 0, 0, 0, g, lp);
 }
 
 // ---------------------------------------------------------------------------
@@ -791,49 +750,48 @@ struct Path1Args {
   R dt, rweight, RovCV;
 };
 
-template <class R, bool POLE>
-__device__ void path1_column(const Path1Args<R>& a, int i, int j, int l, int g, int lp) {
-  const Col c = POLE ? col_pl(g, lp) : col_reg(i, j, l);
-  const MetT<R> m = met_of<R>(POLE);
-  const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
-  const R dt = a.dt;
-  auto pregs = [&](int base_q, int kk) -> R {  // preg_prim_split with clamped boundary rows
-    int k2 = kk < kmin ? kmin : (kk > kmax ? kmax : kk);
-    return a.PS[5][base_q + (int)k2 * c.ks] * a.RovCV;
+// One pole point; the points at kmin and kmax also write the boundary rows
+// kmin-1 and kmax+1 from their values.
+template <class R>
+__global__ void k_path1_pl(const __grid_constant__ Path1Args<R> a) {
+  Pt q_;
+  if (!pole_point((int)(blockIdx.x * blockDim.x + threadIdx.x), q_)) return;
+  const int g = q_.g, lp = q_.lp, k = q_.k;
+  const Col c = col_pl(g, lp);
+  const MetT<R> m = met_of<R>(true);
+  const int kmin = cD.kmin, kmax = cD.kmax;
+  if (k == kmin - 1 || k == kmax + 1) return;
+  auto pregs = [&](int gg, int kk) -> R {  // preg_prim_split with clamped boundary rows
+    const int k2 = kk < kmin ? kmin : (kk > kmax ? kmax : kk);
+    return a.PS[5][ipl(gg, k2, lp)] * a.RovCV;
   };
-  R vals[3][2];  // values at kmin and kmax for the boundary rows
-  R* const* out = a.dvh;
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    R dd[3], pg[3];
-    if (!POLE) {
-      divdamp2d_at(a.vt, i, j, k, l, dd);
-      presgrad_reg(i, j, k, l, c, m, [&](int ii, int jj, int kk) { return pregs(ix(ii, jj, 0, l), kk); }, pg);
-    } else {
-      divdamp2d_pl_at(a.vt, g, k, lp, dd);
-      presgrad_pl(g, k, lp, c, m, [&](int gg, int kk) { return pregs((int)gg * cD.KA * cD.LP + lp, kk); }, pg);
-    }
-    for (int d = 0; d < 3; ++d) {
-      R drv = a.gT[1 + d][p] - pg[d] + dd[d] + R(0.0);
-      R v = a.PS[1 + d][p] + drv * dt;
-      out[d][p] = v;
-      if (k == kmin) vals[d][0] = v;
-      if (k == kmax) vals[d][1] = v;
-    }
-  }
-  const int pT = c.at(kmax + 1), pK = c.at(kmax), pB = c.at(kmin - 1), pN = c.at(kmin);
+  const int p = c.at(k);
+  R dd[3], pg[3];
+  divdamp2d_pl_at(a.vt, g, k, lp, dd);
+  presgrad_pl(g, k, lp, c, m, pregs, pg);
+#pragma unroll
   for (int d = 0; d < 3; ++d) {
-    out[d][pT] = R(1.0) * (vals[d][1] / a.rhog[pK]) * a.rhog[pT];
-    out[d][pB] = -R(1.0) * (vals[d][0] / a.rhog[pN]) * a.rhog[pB];
-  }
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    for (int d = 0; d < 3; ++d) a.PM[1 + d][p] = a.PM[1 + d][p] + out[d][p] * a.rweight;
+    const R drv = a.gT[1 + d][p] - pg[d] + dd[d] + R(0.0);
+    const R v = a.PS[1 + d][p] + drv * a.dt;
+    a.dvh[d][p] = v;
+    a.PM[1 + d][p] = a.PM[1 + d][p] + v * a.rweight;
+    if (k == kmin) {
+      const int pB = c.at(kmin - 1);
+      const R vB = -R(1.0) * (v / a.rhog[p]) * a.rhog[pB];
+      a.dvh[d][pB] = vB;
+      a.PM[1 + d][pB] = a.PM[1 + d][pB] + vB * a.rweight;
+    }
+    if (k == kmax) {
+      const int pT = c.at(kmax + 1);
+      const R vT = R(1.0) * (v / a.rhog[p]) * a.rhog[pT];
+      a.dvh[d][pT] = vT;
+      a.PM[1 + d][pT] = a.PM[1 + d][pT] + vT * a.rweight;
+    }
   }
 }
 
 // Regional path 1, one block per (level, tile): same stencils and
-// arithmetic as path1_column.  The blocks at kmin and kmax also write the
+// arithmetic as k_path1_pl.  The blocks at kmin and kmax also write the
 // boundary rows kmin-1 and kmax+1 from the values they computed.
 template <class R>
 __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, 6, NC_F32_PATH1))) k_path1_l(Path1Args<R> a) {
@@ -958,15 +916,6 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, 6, NC_F32_PA
   }
 }
 
-template <class R>
-__global__ void k_path1(Path1Args<R> a, int pole) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  if (!pole) path1_column<R, false>(a, i, j, l, 0, 0);
-  else path1_column<R, true>(a, 0, 0, 0, g, lp);
-}
-
 // ---------------------------------------------------------------------------
 // vi_main (kernels/vimain.py:127-262): horizontal divergences (kernel A),
 // then per column the flux convergences, the tridiagonal Thomas solve
@@ -989,45 +938,19 @@ struct VimainArgs {
 };
 
 template <class R>
-__global__ void k_vimain_a(VimainArgs<R> a, int pole) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l;
-  if (!pole) {
-    if (!col_of(t, i, j, l)) return;
-    const bool in = interior(i, j);
-    for (int k = 0; k < cD.KA; ++k) {
-      int p = ix(i, j, k, l);
+__global__ void k_vimain_a_pl(const __grid_constant__ VimainArgs<R> a) {
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t < cD.KA * cD.LP) {
+    const int k = t / cD.LP, lp = t % cD.LP;
+    for (int g = 0; g < 6; ++g) {
+      const int p = ipl(g, k, lp);
       R h1 = R(0.0), h2 = R(0.0), h3 = R(0.0);
-      if (in && k >= cD.kmin && k <= cD.kmax) {
-        h1 = div7<R>(i, j, k, l, [&](int ii, int jj, int kk, int d) {
-          int q = ix(ii, jj, kk, l);
-          return a.dvh.f[d][q] * gam_at(CG.RGAM, q);
-        });
-        h2 = div7<R>(i, j, k, l, [&](int ii, int jj, int kk, int d) {
-          int q = ix(ii, jj, kk, l);
-          return (a.dvh.f[d][q] * a.eth[q]) * gam_at(CG.RGAM, q);
-        });
-        h3 = div7<R>(i, j, k, l, [&](int ii, int jj, int kk, int d) {
-          int q = ix(ii, jj, kk, l);
-          return ((a.P[1 + d][q] + a.dvh.f[d][q]) * a.ethtot0[q]) * gam_at(CG.RGAM, q);
-        });
+      if (g == 0 && k >= cD.kmin && k <= cD.kmax) {
+        h1 = div_pl<R>(lp, k, [&](int q, int d) { return a.dvh.f[d][q]; });
+        h2 = div_pl<R>(lp, k, [&](int q, int d) { return a.dvh.f[d][q] * a.eth[q]; });
+        h3 = div_pl<R>(lp, k, [&](int q, int d) { return (a.P[1 + d][q] + a.dvh.f[d][q]) * a.ethtot0[q]; });
       }
       a.hdiv[0][p] = h1; a.hdiv[1][p] = h2; a.hdiv[2][p] = h3;
-    }
-  } else {
-    int tp = t;
-    if (tp < cD.KA * cD.LP) {
-      int k = (int)(tp / cD.LP), lp = (int)(tp % cD.LP);
-      for (int g = 0; g < 6; ++g) {
-        int p = ipl(g, k, lp);
-        R h1 = R(0.0), h2 = R(0.0), h3 = R(0.0);
-        if (g == 0 && k >= cD.kmin && k <= cD.kmax) {
-          h1 = div_pl<R>(lp, k, [&](int q, int d) { return a.dvh.f[d][q]; });
-          h2 = div_pl<R>(lp, k, [&](int q, int d) { return a.dvh.f[d][q] * a.eth[q]; });
-          h3 = div_pl<R>(lp, k, [&](int q, int d) { return (a.P[1 + d][q] + a.dvh.f[d][q]) * a.ethtot0[q]; });
-        }
-        a.hdiv[0][p] = h1; a.hdiv[1][p] = h2; a.hdiv[2][p] = h3;
-      }
     }
   }
 }
@@ -1166,125 +1089,255 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, 4, 5))) k_vi
   }
 }
 
-// One pole column of vi_main.  In the mixed form the flux convergences and
-// the energy update run in float32 (R) and the tridiagonal solve in float64,
-// as in the regional kernels k_vi_solve / k_vi_energy_p.
-template <class R, bool POLE>
-__device__ void vimain_column(const VimainArgs<R>& a, const Col c) {
+// vi_main, column part: flux convergences of diff_vh, the Thomas solve
+// (kernels/virhowsolver.py:42-120), rhog_split1, the kinetic energies and the
+// energy update, for the interior regional columns (the halo columns of the
+// outputs are replaced by the exchange that follows) and the pole columns.
+//
+// One block takes VC_COLS columns (a lane each) and splits the levels over its
+// warps: each warp assembles the right-hand side of its levels marching upward,
+// warp 0 walks the two sweeps of the elimination on operands in shared memory
+// (five doubles per level and column: 54 KB at 42 levels), then each warp
+// finishes its levels, again marching upward; a part of the column repeats one
+// level (assembly) or two (finish) of its neighbour instead of exchanging them.
+// A column per thread was bound by its chain of loads and divisions (gl05 z40
+// float64: 6 us a level, whatever the number of columns) and kept the sweep's
+// factors in local memory; the finish in the same launch finds the fields that
+// both parts read in L2.
+// Slots, by level (kmin..kmax+1) and lane:
+//   0 horizontal part of the half-level mass flux
+//   1 the right-hand side, then the solution
+//   2 Mu, then the sweep's gamma      3 Ml      4 Mc
+#define VC_COLS 32
+#define VC_MAXW 8
+static inline size_t vi_col_smem(int KA) { return (size_t)5 * KA * VC_COLS * sizeof(double); }
+
+// the contiguous part [lo, hi) of the levels first..last that a warp takes
+__device__ __forceinline__ void warp_levels(int first, int last, int& lo, int& hi) {
+  const int nw = (int)(blockDim.x / 32), w = (int)(threadIdx.x / 32);
+  const int per = (last - first + nw) / nw;
+  lo = first + w * per;
+  hi = min(lo + per, last + 1);
+}
+
+template <class R, bool GU, bool POLE>
+__device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* sm) {
+  const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax, kT = kmax + 1;
+  const int lane = (int)(threadIdx.x % 32);
+  const int ni = cD.G - 2;
+  const int ncol = POLE ? 6 * cD.LP : cD.L * ni * ni;
+  const int t0 = blk * VC_COLS + lane;
+  const bool act = t0 < ncol;              // surplus lanes repeat the last column and store nothing
+  const int t = act ? t0 : ncol - 1;
+  const Col c = POLE ? col_pl(t / cD.LP, t % cD.LP) : col_reg(1 + t % ni, 1 + (t / ni) % ni, t / (ni * ni));
   const MetT<R> m = met_of<R>(POLE);
-  const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
-  const double dt = a.dt;
-  const R dtR = R(a.dt);
-  const double Rdry = cC.Rdry, CVdry = cC.CVdry;
-  auto PSk = [&](int comp, int k) -> R {  // PROG_split with clamped RHOGE boundary rows
-    if (comp == 5) k = k < kmin ? kmin : (k > kmax ? kmax : k);
-    return a.PS[comp][c.at(k)];
+  const double dt = a.dt, Rdry = cC.Rdry, CVdry = cC.CVdry, RovCV = a.RovCV;
+  const R* const* DV = a.dvh.f;
+  double* s0 = sm + lane;
+  double* s1 = s0 + KA * VC_COLS;
+  double* s2 = s1 + KA * VC_COLS;
+  double* s3 = s2 + KA * VC_COLS;
+  double* s4 = s3 + KA * VC_COLS;
+  auto S = [](double* s, int k) -> double& { return s[k * VC_COLS]; };
+  auto cz = [&](int comp, int q) -> R { return __ldg(POLE ? m.C2WGz + q * 6 + comp : m.C2WGz + comp * cD.npti + q); };
+  auto two = [&](const R* w, int comp, int q) -> R { return __ldg(POLE ? w + q * 2 + comp : w + comp * cD.npti + q); };
+  int lo, hi;
+  // ---- right-hand side on kmin+1..kmax
+  warp_levels(kmin + 1, kmax, lo, hi);
+  if (lo < hi) {
+    const double CVovRt2 = CVdry / Rdry / (dt * dt);
+    double f0m, f1m, f2m, em;             // diff_vh and eth one level below
+    auto flux = [&](int k, double& hd, double& he) {   // half-level fluxes at k; level k becomes the one below
+      const int p = c.at(k);
+      const double f0 = __ldg(DV[0] + p), f1 = __ldg(DV[1] + p), f2 = __ldg(DV[2] + p), e = __ldg(a.eth + p);
+      const double z0 = cz(0, p), z1 = cz(1, p), z2 = cz(2, p), z3 = cz(3, p), z4 = cz(4, p), z5 = cz(5, p);
+      const double g = GU ? 1.0 : (double)__ldg(m.RGAMH + p);
+      hd = (z0 * f0 + z1 * f0m + z2 * f1 + z3 * f1m + z4 * f2 + z5 * f2m) * g;
+      he = (z0 * (f0 * e) + z1 * (f0m * em) + z2 * (f1 * e) + z3 * (f1m * em) + z4 * (f2 * e) + z5 * (f2m * em)) * g;
+      f0m = f0; f1m = f1; f2m = f2; em = e;
+    };
+    double hD = 0.0, hE = 0.0;            // zero at kmin (and at kmax+1)
+    {
+      const int k = (lo - 1 > kmin) ? lo - 2 : lo - 1;
+      const int q = c.at(k);
+      f0m = __ldg(DV[0] + q); f1m = __ldg(DV[1] + q); f2m = __ldg(DV[2] + q); em = __ldg(a.eth + q);
+      if (lo - 1 > kmin) flux(lo - 1, hD, hE);
+    }
+    double T1m = 0.0, T2m = 0.0;
+    for (int k = lo - 1; k < hi; ++k) {
+      const int p = c.at(k);
+      double hDn = 0.0, hEn = 0.0;
+      if (k < kmax) flux(k + 1, hDn, hEn);
+      const double drhog = -__ldg(a.hdiv[0] + p) - (hDn - hD) * cC.rdgz[k];
+      const double drhoge = -__ldg(a.hdiv[1] + p) - (hEn - hE) * cC.rdgz[k];
+      const double g1 = __ldg(a.gT[0] + p) + drhog;
+      const double gp = (__ldg(a.gT[5] + p) + drhoge) * Rdry / CVdry;
+      const double rgm = GU ? 1.0 : (double)__ldg(m.RGAM + p);
+      const double T1 = (__ldg(a.PS[5] + p) * RovCV + dt * gp) * __ldg(m.RGSGAM2 + p);
+      const double T2 = (__ldg(a.PS[0] + p) + dt * g1) * (rgm * rgm);
+      if (k >= lo) {
+        const double rgh = GU ? 1.0 : (double)__ldg(m.RGAMH + p);
+        const double Sw = __ldg(a.gT[4] + p) + 0.0 * cC.alpha;
+        const double mu = __ldg(a.Mu + p), ml = __ldg(a.Ml + p);
+        double b = ((__ldg(a.PS[4] + p) * cC.alpha + dt * Sw) * (rgh * rgh) - (T1 - T1m) * dt * cC.rdgzh[k] -
+                    (T2 * cC.afact[k] + T2m * cC.bfact[k]) * dt * cC.GRAV) *
+                   CVovRt2;
+        if (k == kmin + 1) {
+          const double rw_kmin = 0.0 * __ldg(m.RGSGAM2H + c.at(kmin));
+          b = b - ml * rw_kmin;
+          S(s1, kmin) = rw_kmin;
+        }
+        if (k == kmax) {
+          const int pT = c.at(kT);
+          const double top = -(cz(0, pT) * __ldg(DV[0] + pT) + cz(1, pT) * __ldg(DV[0] + p) + cz(2, pT) * __ldg(DV[1] + pT) +
+                               cz(3, pT) * __ldg(DV[1] + p) + cz(4, pT) * __ldg(DV[2] + pT) + cz(5, pT) * __ldg(DV[2] + p));
+          const double rw_top = top * __ldg(m.RGSGAM2H + pT);
+          b = b - mu * rw_top;
+          S(s1, kT) = rw_top;
+        }
+        S(s0, k) = hD;
+        S(s1, k) = b;
+        S(s2, k) = mu;
+        S(s3, k) = ml;
+        S(s4, k) = __ldg(a.Mc + p);
+      }
+      T1m = T1; T2m = T2; hD = hDn; hE = hEn;
+    }
+  }
+  __syncthreads();
+  // ---- Thomas sweeps, one lane per column; the operands of the next level are
+  // read before this level's are overwritten
+  if (threadIdx.x < 32) {
+    const int k0 = kmin + 1;
+    double beta = S(s4, k0), u = S(s1, k0) / beta;
+    double mu = S(s2, k0);
+    double mc_ = S(s4, k0 + 1), ml = S(s3, k0 + 1), b = S(s1, k0 + 1), mu1 = S(s2, k0 + 1);   // k0+1 <= kT < KA
+    S(s1, k0) = u;
+    for (int k = k0 + 1; k <= kmax; ++k) {
+      const int kn = min(k + 1, kmax);
+      const double mcn = S(s4, kn), mln = S(s3, kn), bn = S(s1, kn), mun = S(s2, kn);
+      const double gg = mu / beta;
+      beta = mc_ - ml * gg;
+      u = (b - ml * u) / beta;
+      S(s2, k - 1) = gg;      // gamma of level k beside the level below, whose Mu is spent
+      S(s1, k) = u;
+      mu = mu1;
+      mu1 = mun; mc_ = mcn; ml = mln; b = bn;
+    }
+    double x = u, un = S(s1, kmax - 1), gn = S(s2, kmax - 1);
+    for (int k = kmax - 1; k >= k0; --k) {
+      const int kn = max(k - 1, k0);
+      const double un1 = S(s1, kn), gn1 = S(s2, kn);
+      x = un - gn * x;
+      S(s1, k) = x;
+      un = un1; gn = gn1;
+    }
+  }
+  __syncthreads();
+  // ---- rhogw_split1, rhog_split1, the kinetic energies before and after, the
+  // total-energy advection and rhoge_split1 on every level
+  warp_levels(0, KA - 1, lo, hi);
+  if (lo >= hi) return;
+  const R dtR = R(dt);
+  struct W { double rws, v2; };          // rhogw_split1 and its mass flux at half level k
+  auto wat = [&](int k) -> W {
+    W w{0.0, 0.0};
+    if (k < kmin || k > kT) return w;
+    const int p = c.at(k);
+    w.rws = S(s1, k) * __ldg(m.GSGAM2H + p);
+    if (k > kmin && k <= kmax) w.v2 = S(s0, k) + 1.0 * w.rws * __ldg(m.RGSQRTH + p);
+    return w;
   };
-  auto preg0 = [&](int k) -> double { return (double)PSk(5, k) * a.RovCV; };
-  auto DV = [&](int k, int d) -> R { return a.dvh.f[d][c.at(k)]; };
-  auto DVE = [&](int k, int d) -> R { return a.dvh.f[d][c.at(k)] * a.eth[c.at(k)]; };
-  // grhog1 and gpre on every level
-  double grhog1[NC_MAXK], gpre[NC_MAXK];
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    R drhog = fluxconv_col(c, m, k, a.hdiv[0][p], R(0.0), DV, [&](int kk) { return PSk(4, kk); });
-    R drhoge = fluxconv_col(c, m, k, a.hdiv[1][p], R(0.0), DVE, [&](int kk) { return R(0.0); });
-    grhog1[k] = (double)a.gT[0][p] + (double)drhog;
-    double grhoge1 = (double)a.gT[5][p] + (double)drhoge;
-    gpre[k] = grhoge1 * Rdry / CVdry;
+  auto rsat = [&](int k, double v2, double v2n) -> double {   // rhog_split1 at level k
+    const int p = c.at(k);
+    double drhog2 = 0.0;
+    if (k >= kmin && k <= kmax) drhog2 = -__ldg(a.hdiv[0] + p) - (v2n - v2) * cC.rdgz[k];
+    return __ldg(a.PS[0] + p) + (__ldg(a.gT[0] + p) + drhog2) * dt;
+  };
+  struct L { R rg, r0, r1, vx, vy, vz, x1, y1, z1, et; };   // the values of one level
+  auto lat = [&](int k, double rs) -> L {
+    const int p = c.at(k);
+    L q;
+    q.rg = __ldg(a.P[0] + p);
+    q.r0 = __ldg(a.PS[0] + p);
+    q.r1 = R(rs);
+    q.vx = __ldg(a.P[1] + p); q.vy = __ldg(a.P[2] + p); q.vz = __ldg(a.P[3] + p);
+    q.x1 = q.vx + __ldg(DV[0] + p); q.y1 = q.vy + __ldg(DV[1] + p); q.z1 = q.vz + __ldg(DV[2] + p);
+    q.et = __ldg(a.ethtot0 + p);
+    return q;
+  };
+  struct H { R k10, k11, fl; };          // half-level kinetic energies and total-energy flux
+  auto half = [&](int k, const L& u, const L& d, double rws) -> H {   // between the levels k (u) and k-1 (d)
+    const int p = c.at(k);
+    H h;
+    const R c0 = two(m.C2W, 0, p), c1 = two(m.C2W, 1, p), w = __ldg(a.P[4] + p);
+    const R w0 = w + __ldg(a.PS[4] + p), w1 = w + R(rws);
+    h.k10 = R(0.5) * (w0 * w0) / (c0 * (u.rg + u.r0) + c1 * (d.rg + d.r0));
+    h.k11 = R(0.5) * (w1 * w1) / (c0 * (u.rg + u.r1) + c1 * (d.rg + d.r1));
+    const R f = cz(0, p) * (u.x1 * u.et) + cz(1, p) * (d.x1 * d.et) + cz(2, p) * (u.y1 * u.et) +
+                cz(3, p) * (d.y1 * d.et) + cz(4, p) * (u.z1 * u.et) + cz(5, p) * (d.z1 * d.et);
+    h.fl = f * (GU && !POLE ? R(1.0) : gam_at(m.RGAMH, p)) +
+           R(1.0) * (w1 * (CC.afact[k] * u.et + CC.bfact[k] * d.et)) * __ldg(m.RGSQRTH + p);
+    return h;
+  };
+  W wc = wat(lo), wn = wat(lo + 1);
+  double rs = rsat(lo, wc.v2, wn.v2);
+  L cur = lat(lo, rs);
+  H hc{R(0.0), R(0.0), R(0.0)};
+  if (lo > kmin && lo <= kmax) {
+    const L below = lat(lo - 1, rsat(lo - 1, wat(lo - 1).v2, wc.v2));
+    hc = half(lo, cur, below, wc.rws);
   }
-  // Thomas solve (kernels/virhowsolver.py:67-120), float64
-  const int kT = kmax + 1;
-  double rw_top = -((double)mc(m.C2WGz, c, 0, 6, kT) * DV(kT, 0) + (double)mc(m.C2WGz, c, 1, 6, kT) * DV(kmax, 0) +
-                    (double)mc(m.C2WGz, c, 2, 6, kT) * DV(kT, 1) + (double)mc(m.C2WGz, c, 3, 6, kT) * DV(kmax, 1) +
-                    (double)mc(m.C2WGz, c, 4, 6, kT) * DV(kT, 2) + (double)mc(m.C2WGz, c, 5, 6, kT) * DV(kmax, 2));
-  const double CVovRt2 = CVdry / Rdry / (dt * dt);
-  const double rw_kmin = 0.0 * (double)m.RGSGAM2H[c.at(kmin)];
-  const double rw_kmaxp1 = rw_top * (double)m.RGSGAM2H[c.at(kT)];
-  const int N = kmax - kmin;
-  double u[NC_MAXK], gam[NC_MAXK];
-  double beta = 0.0;
-  for (int n = 0; n < N; ++n) {
-    int k = kmin + 1 + n;
-    int p = c.at(k), pm = c.at(k - 1);
-    double rg2 = (double)gam_at(m.RGAMH, p) * (double)gam_at(m.RGAMH, p);
-    double rgam2 = (double)gam_at(m.RGAM, p) * (double)gam_at(m.RGAM, p);
-    double rgam2m = (double)gam_at(m.RGAM, pm) * (double)gam_at(m.RGAM, pm);
-    double Sw = (double)a.gT[4][p] + 0.0 * cC.alpha;
-    double S = (((double)PSk(4, k) * cC.alpha + dt * Sw) * rg2 -
-                ((preg0(k) + dt * gpre[k]) * (double)m.RGSGAM2[p] - (preg0(k - 1) + dt * gpre[k - 1]) * (double)m.RGSGAM2[pm]) *
-                    dt * cC.rdgzh[k] -
-                (((double)PSk(0, k) + dt * grhog1[k]) * rgam2 * cC.afact[k] +
-                 ((double)PSk(0, k - 1) + dt * grhog1[k - 1]) * rgam2m * cC.bfact[k]) *
-                    dt * cC.GRAV) *
-               CVovRt2;
-    if (n == 0) S = S - a.Ml[c.at(kmin + 1)] * rw_kmin;
-    if (n == N - 1) S = S - a.Mu[c.at(kmax)] * rw_kmaxp1;
-    double Mc = a.Mc[p], Ml = a.Ml[p];
-    if (n == 0) {
-      beta = Mc;
-      u[0] = S / beta;
-    } else {
-      double gg = a.Mu[pm] / beta;
-      beta = Mc - Ml * gg;
-      u[n] = (S - Ml * u[n - 1]) / beta;
-      gam[n] = gg;
+  for (int k = lo; k < hi; ++k) {
+    const int p = c.at(k);
+    const W wnn = wat(k + 2);
+    double rsn = 0.0;
+    L up = cur;
+    H hn{R(0.0), R(0.0), R(0.0)};
+    if (k + 1 < KA) {
+      rsn = rsat(k + 1, wn.v2, wnn.v2);
+      up = lat(k + 1, rsn);
+      if (k + 1 > kmin && k < kmax) hn = half(k + 1, up, cur, wn.rws);
     }
-  }
-  R rws1[NC_MAXK];
-  for (int k = 0; k < KA; ++k) rws1[k] = R(0.0);
-  {
-    double x = u[N - 1];
-    rws1[kmin + N] = R(x * (double)m.GSGAM2H[c.at(kmin + N)]);
-    for (int n = N - 2; n >= 0; --n) {
-      x = u[n] - gam[n + 1] * x;
-      rws1[kmin + 1 + n] = R(x * (double)m.GSGAM2H[c.at(kmin + 1 + n)]);
+    R kin10 = R(0.0), kin11 = R(0.0), adv = R(0.0);
+    if (k >= kmin && k <= kmax) {
+      const R x0 = cur.vx + __ldg(a.PS[1] + p), y0 = cur.vy + __ldg(a.PS[2] + p), z0 = cur.vz + __ldg(a.PS[3] + p);
+      const R w0 = two(m.W2C, 0, p), w1 = two(m.W2C, 1, p);
+      kin10 = R(0.5) * (x0 * x0 + y0 * y0 + z0 * z0) / (cur.rg + cur.r0) + w0 * hn.k10 + w1 * hc.k10;
+      kin11 = R(0.5) * (cur.x1 * cur.x1 + cur.y1 * cur.y1 + cur.z1 * cur.z1) / (cur.rg + cur.r1) + w0 * hn.k11 +
+              w1 * hc.k11;
+      adv = -__ldg(a.hdiv[2] + p) - (hn.fl - hc.fl) * CC.rdgz[k];
     }
-    rws1[kmin] = R(rw_kmin * (double)m.GSGAM2H[c.at(kmin)]);
-    rws1[kT] = R(rw_kmaxp1 * (double)m.GSGAM2H[c.at(kT)]);
-  }
-  // rhog_split1, kinetic energies, total-energy advection, rhoge_split1
-  R rs1[NC_MAXK];
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    R drhog2 = fluxconv_col(c, m, k, a.hdiv[0][p], R(1.0), DV, [&](int kk) { return rws1[kk]; });
-    rs1[k] = PSk(0, k) + (a.gT[0][p] + drhog2) * dtR;
-  }
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    auto st10 = [&](int kk, int comp) -> R {
-      int q = c.at(kk);
-      return a.P[comp][q] + PSk(comp, kk);
-    };
-    auto st11 = [&](int kk, int comp) -> R {
-      int q = c.at(kk);
-      if (comp == 0) return a.P[0][q] + rs1[kk];
-      if (comp == 4) return a.P[4][q] + rws1[kk];
-      return a.P[comp][q] + a.dvh.f[comp - 1][q];
-    };
-    R kin10 = rhogkin_at(c, m, k, st10);
-    R kin11 = rhogkin_at(c, m, k, st11);
-    R drhogetot = fluxconv_col(
-        c, m, k, a.hdiv[2][p], R(1.0),
-        [&](int kk, int d) {
-          int q = c.at(kk);
-          return (a.P[1 + d][q] + a.dvh.f[d][q]) * a.ethtot0[q];
-        },
-        [&](int kk) {
-          int q = c.at(kk), qm = c.at(kk - 1);
-          return (a.P[4][q] + rws1[kk]) * (CC.afact[kk] * a.ethtot0[q] + CC.bfact[kk] * a.ethtot0[qm]);
-        });
-    R re = PSk(5, k) + (a.gT0e[p] + drhogetot) * dtR + (kin10 - kin11) + (PSk(0, k) - rs1[k]) * m.PHI[p];
-    a.dwe[0][p] = rs1[k];
-    a.dwe[1][p] = rws1[k];
-    a.dwe[2][p] = re;
-    a.PM0[p] = a.PM0[p] + rs1[k] * R(a.rweight);
-    a.PM4[p] = a.PM4[p] + rws1[k] * R(a.rweight);
+    const R re0 = __ldg(a.PS[5] + c.at(k < kmin ? kmin : (k > kmax ? kmax : k)));
+    const R pm0 = a.PM0[p], pm4 = a.PM4[p];
+    const R re = re0 + (__ldg(a.gT0e + p) + adv) * dtR + (kin10 - kin11) + (cur.r0 - cur.r1) * __ldg(m.PHI + p);
+    if (act) {
+      a.dwe[0][p] = cur.r1;
+      a.dwe[1][p] = R(wc.rws);
+      a.dwe[2][p] = re;
+      a.PM0[p] = pm0 + rs * a.rweight;
+      a.PM4[p] = pm4 + wc.rws * a.rweight;
+    }
+    rs = rsn;
+    wc = wn; wn = wnn;
+    cur = up;
+    hc = hn;
   }
 }
 
-// Regional vi_main in two column kernels (interior columns; the halo columns
-// of the outputs are replaced by the exchange that follows).
+// GU: the gamma factors are all 1 and are not loaded
+template <class R, bool GU, bool POLE>
+__global__ void __launch_bounds__(32 * VC_MAXW, NC_MINB(R, 3, 4)) k_vi_col(const __grid_constant__ VimainArgs<R> a) {
+  extern __shared__ __align__(16) double vi_sm[];
+  vi_col<R, GU, POLE>(a, (int)blockIdx.x, vi_sm);
+}
+
+// The same for more columns than fill the SMs with a thread each: two
+// kernels (interior columns).  With every SM busy the column kernel's chain is
+// hidden behind other columns and its 36 resident warps move more bytes than
+// k_vi_col's 32, whose sweeps leave seven of eight warps waiting: gl08 mixed
+// 1.15 + 0.91 ms against 2.39 ms; gl07 float64 (163,840 columns) 0.63 + 0.42 ms
+// against 0.97 ms.
 // k_vi_solve: flux convergences of diff_vh (rolling half-level fluxes), the
 // Thomas forward sweep, then the back substitution fused with rhog_split1 on
 // the way down; writes rhog_s1, rhogw_s1 and their running means.
@@ -1447,50 +1500,58 @@ __global__ void __launch_bounds__(128, NC_MINB(R, 1, NC_F32_VIENERGY)) k_vi_ener
   a.dwe[2][p] = PSk(5, k) + (a.gT0e[p] + drhogetot) * R(a.dt) + (kin10 - kin11) + (PSk(0, k) - rs1[p]) * m.PHI[p];
 }
 
-template <class R>
-__global__ void k_vimain_b(VimainArgs<R> a, int pole) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  if (!pole) vimain_column<R, false>(a, col_reg(i, j, l));
-  else vimain_column<R, true>(a, col_pl(g, lp));
-}
-
 // ---------------------------------------------------------------------------
 // elementwise helpers of the small step
 // ---------------------------------------------------------------------------
 // PROG_split = 0 (first stage) or PROG0 - PROG; PROG_mean = PROG[0:5]
 template <class R>
-__global__ void k_split_init(const R* P0a, const R* P0b, const R* P0c, const R* P0d,
-                             const R* P0e, const R* P0f, Prog<R> P, R* PS0, R* PS1, R* PS2,
-                             R* PS3, R* PS4, R* PS5, R* PM0, R* PM1, R* PM2,
-                             R* PM3, R* PM4, int n, int first) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const R* P0[6] = {P0a, P0b, P0c, P0d, P0e, P0f};
-  R* PS[6] = {PS0, PS1, PS2, PS3, PS4, PS5};
-  R* PM[5] = {PM0, PM1, PM2, PM3, PM4};
-  for (int v = 0; v < 6; ++v) PS[v][t] = first ? R(0.0) : (P0[v][t] - P.v[v][t]);
-  for (int v = 0; v < 5; ++v) PM[v][t] = P.v[v][t];
+struct SplitArgs {
+  const R *P0[6], *P[6];
+  R *PS[6], *PM[5];
+};
+template <class R>
+__global__ void k_split_init(const __grid_constant__ SplitArgs<R> a, int n, const __grid_constant__ SplitArgs<R> ap, int np, int npb, int first) {
+  const bool pole = (int)blockIdx.x < npb;
+  const int t = (int)((pole ? blockIdx.x : blockIdx.x - npb) * blockDim.x + threadIdx.x);
+  if (t >= (pole ? np : n)) return;
+  const SplitArgs<R>& s = pole ? ap : a;
+  R v[6], v0[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    v[m] = s.P[m][t];
+    v0[m] = first ? R(0.0) : s.P0[m][t];
+  }
+#pragma unroll
+  for (int m = 0; m < 6; ++m) s.PS[m][t] = first ? R(0.0) : (v0[m] - v[m]);
+#pragma unroll
+  for (int m = 0; m < 5; ++m) s.PM[m][t] = v[m];
 }
 
 // PROG += PROG_split, then horizontalize the momentum (mod_vi.py:1572-1583)
 template <class R>
-__global__ void k_post(Prog<R> P, const R* PS0, const R* PS1, const R* PS2, const R* PS3,
-                       const R* PS4, const R* PS5, int pole) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  const R* PS[6] = {PS0, PS1, PS2, PS3, PS4, PS5};
-  int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  const Col c = pole ? col_pl(g, lp) : col_reg(i, j, l);
-  const bool in = !pole && interior(i, j);
-  for (int k = 0; k < cD.KA; ++k) {
-    int p = c.at(k);
-    R v[6];
-    for (int n = 0; n < 6; ++n) v[n] = P.v[n][p] + PS[n][p];
-    if (pole) horiz_pl(g, lp, v[1], v[2], v[3]);
-    else if (in) horiz_reg(i, j, l, v[1], v[2], v[3]);
-    for (int n = 0; n < 6; ++n) P.v[n][p] = v[n];
+struct PostArgs {
+  R* P[6];
+  const R* PS[6];
+};
+template <class R>
+__device__ __forceinline__ void post_point(const PostArgs<R>& a, int p, const Pt& q, bool pole) {
+  R v[6];
+#pragma unroll
+  for (int n = 0; n < 6; ++n) v[n] = a.P[n][p] + a.PS[n][p];
+  if (pole) horiz_pl(q.g, q.lp, v[1], v[2], v[3]);
+  else if (interior(q.i, q.j)) horiz_reg(q.i, q.j, q.l, v[1], v[2], v[3]);
+#pragma unroll
+  for (int n = 0; n < 6; ++n) a.P[n][p] = v[n];
+}
+template <class R>
+__global__ void k_post(const __grid_constant__ PostArgs<R> a, const __grid_constant__ PostArgs<R> ap, int npb) {
+  Pt q;
+  if ((int)blockIdx.x < npb) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (pole_point(t, q)) post_point(ap, t, q, true);   // the pole layout is (g, k, lp), as the threads'
+  } else {
+    const int t = (int)((blockIdx.x - npb) * blockDim.x + threadIdx.x);
+    if (reg_point(t, q)) post_point(a, t, q, false);
   }
 }
 

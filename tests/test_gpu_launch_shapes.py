@@ -1,0 +1,67 @@
+"""The step on both sides of each size rule of its launches, and at the
+remainders of its splits (B200).
+
+* Numbers of layers that do not divide by the warps of the vi_main column
+  kernel, the levels per block of path 1 and the level chunks: one step at
+  gl03 equals the oracle bit for bit.
+* One gl05 grid alone (its tiles and columns do not fill the SMs: level chunks,
+  k_vi_col) against 17 of them stacked in one handle (174,080 columns, above one
+  wave of the column kernel: whole marches, k_vi_solve and k_vi_energy_p): each
+  member bit for bit, in both forms.
+"""
+import importlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _ig():
+    return importlib.import_module("pynicam-dc_b200.icogrid")
+
+
+def _perturbed(geo, s, sp, seed):
+    ens = importlib.import_module("pynicam-dc_b200.ensemble")
+    return ens.perturbed_members(geo, s, sp, 1, seed=seed, sigma=0.5, length=1500e3)[0]
+
+
+@pytest.mark.parametrize("vlayer", [5, 7, 23, 41])
+def test_odd_layers_equal_oracle(pkg, vlayer):
+    from oracle import nicam_step as O
+    g = _ig().Grid(3, vlayer=vlayer, ztop=30000.0, device="cuda")
+    geo = g.setup(dtl=600.0, gamma=7.68e17, nq=1)
+    s, sp = _perturbed(geo, *g.jw_state(nq=1), seed=3)
+    s[..., 6], sp[..., 6] = 0.01 * s[..., 0], 0.01 * sp[..., 0]
+    want, want_pl = O.dynamics_step(O.Geo(geo), s, sp)
+    c = pkg.NicamCuda(geo, graph=True)
+    try:
+        c.upload(s, sp)
+        c.step(1)
+        got, got_pl = c.download()
+    finally:
+        c.close()
+    assert np.array_equal(got, want) and np.array_equal(got_pl, want_pl)
+
+
+@pytest.mark.parametrize("prec", ["float64", "mixed"])
+def test_one_grid_equals_its_stack(pkg, prec):
+    ens = importlib.import_module("pynicam-dc_b200.ensemble")
+    g = _ig().Grid(5, vlayer=9, ztop=30000.0, device="cuda")
+    geo = g.setup(dtl=300.0, gamma=1.2e16, nq=1)
+    m, mp = _perturbed(geo, *g.jw_state(nq=1), seed=5)
+    m[..., 6], mp[..., 6] = 0.01 * m[..., 0], 0.01 * mp[..., 0]
+
+    def run(geo, s, sp):
+        c = pkg.NicamCuda(geo, graph=True, precision=prec)
+        try:
+            c.upload(s, sp)
+            c.step(2)
+            return c.download()
+        finally:
+            c.close()
+    lone, lone_pl = run(geo, m, mp)
+    n = 17
+    got = ens.unstack_states(*run(ens.stack_setup(geo, n), *ens.stack_states([(m, mp)] * n)), n)
+    for x, xp in (got[0], got[n // 2], got[-1]):
+        assert np.array_equal(x, lone) and np.array_equal(xp, lone_pl)
