@@ -47,7 +47,7 @@ static int fail(int code, const std::string& msg) {
     if (e_ != cudaSuccess) return fail(NC_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-#define NC_MAXCOMM 8
+#define NC_MAXCOMM 12
 #define NC_KNAME 48
 
 // ---------------------------------------------------------------------------
@@ -63,41 +63,29 @@ struct CommFields {
   int n;
 };
 
+// The plan in 32-bit array indices at level 0 (c_dst, c_src; see make_comm_plan):
+// entries 0..nr-1 write regional cells (a source below zero is the pole point
+// -s-1), the others pole points from regional cells.
 template <class R>
-__global__ void k_comm(CommFields<R> f, const long long* r_dst, const long long* r_src, int nr, const long long* p_dst,
-                       const long long* p_src, int np) {
+__global__ void k_comm(const __grid_constant__ CommFields<R> f, const int* c_dst, const int* c_src, int nr, int nent) {
   // consecutive threads take consecutive entries of one level: the entries are
   // sorted by destination, so a region's halo rows are read and written in
-  // contiguous runs
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int nent = nr + np;
-  long long ne = (long long)nent * cD.KA;
-  if (t >= ne) return;
-  int k = (int)(t / nent);
-  int e = (int)(t % nent);
-  const long long pl = cD.plane;
-  if (e < nr) {
-    long long d = r_dst[e];
-    long long di = ((d / pl) * cD.KA + k) * pl + d % pl;
-    long long s = r_src[e];
-    if (s >= 0) {
-      long long si = ((s / pl) * cD.KA + k) * pl + s % pl;
-      for (int n = 0; n < f.n; ++n) f.r[n][di] = f.r[n][si];
-    } else {
-      long long gp = -s - 1;   // g*LP + lp
-      int g = (int)(gp / cD.LP), lp = (int)(gp % cD.LP);
-      int pi = ipl(g, k, lp);
-      for (int n = 0; n < f.n; ++n) f.r[n][di] = f.p[n][pi];
-    }
-  } else {
-    e -= nr;
-    long long gp = p_dst[e];
-    int g = (int)(gp / cD.LP), lp = (int)(gp % cD.LP);
-    int pi = ipl(g, k, lp);
-    long long s = p_src[e];
-    long long si = ((s / pl) * cD.KA + k) * pl + s % pl;
-    for (int n = 0; n < f.n; ++n) f.p[n][pi] = f.r[n][si];
-  }
+  // contiguous runs.  Every field's value is loaded before the first is stored:
+  // one wait for memory instead of one a field.
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= nent * cD.KA) return;
+  const int k = t / nent, e = t - k * nent;
+  int d = __ldg(c_dst + e), s = __ldg(c_src + e);
+  const bool dreg = e < nr, sreg = s >= 0;
+  d += k * (dreg ? cD.planei : cD.LP);
+  s = sreg ? s + k * cD.planei : (-s - 1) + k * cD.LP;
+  R v[NC_MAXCOMM];
+#pragma unroll
+  for (int n = 0; n < NC_MAXCOMM; ++n)
+    if (n < f.n) v[n] = (sreg ? f.r[n] : f.p[n])[s];
+#pragma unroll
+  for (int n = 0; n < NC_MAXCOMM; ++n)
+    if (n < f.n) (dreg ? f.r[n] : f.p[n])[d] = v[n];
 }
 
 // ---------------------------------------------------------------------------
@@ -319,6 +307,11 @@ static const int kTuneMax[TB_N] = {128, 128, 128, NC_VP0C_BLOCK, 1024, 1024, 102
 // "no non-finite value seen": every byte 0x7f, above any variable index
 #define NC_BAD_NONE 0x7f7f7f7f
 
+// Work fields of one tracer's horizontal advection
+struct TrcWork {
+  FieldPair q, gq[3], qa[3], Qmin, Qmax;
+};
+
 struct nc_handle {
   Dims D{};
   Consts C{};
@@ -344,6 +337,7 @@ struct nc_handle {
   // halo plan
   long long *r_dst = nullptr, *r_src = nullptr, *p_dst = nullptr, *p_src = nullptr;
   int nr = 0, np = 0;
+  int *c_dst = nullptr, *c_src = nullptr;   // the same in array indices (k_comm)
   // marshal staging
   double *stage = nullptr, *stage_pl = nullptr;
   double* mass_part = nullptr;
@@ -363,7 +357,8 @@ struct nc_handle {
   FieldPair pre, tem, vx, vy, vz, w, rho, ein, eth, pregd, rhogd, vv[3];
   FieldPair gadv[4], vt[6], vt2[6], gT0[6], frhog;
   FieldPair PSa[6], PSb[6], PM[5], vtmp2[3], gT[6], Mc, Mu, Ml, ethtot0, hdiv[3];
-  FieldPair flx_v, rhog_t, flx[6], xc[9], ch[6], cm[6], q, gq[3], qa[3], Qmin, Qmax;
+  FieldPair flx_v, rhog_t, flx[6], xc[9], ch[6], cm[6];
+  TrcWork tw[TRC_NB];           // horizontal advection of a batch of tracers
   FieldPair vph[8];             // horizontal terms of vp0 (div1, div2, dd, dpg)
   const double* hs_lat = nullptr;   // Held-Suarez latitude planes (optional)
   // DCMIP forcing with Kessler microphysics (optional): full-level heights,
@@ -626,20 +621,25 @@ static cudaStream_t pole_stream(nc_handle* h) {
 }
 
 template <class R>
-static int comm(nc_handle* h, std::initializer_list<FieldPair> fl) {
-  CommFields<R> f{};
-  f.n = 0;
-  for (const FieldPair& p : fl) {
-    f.r[f.n] = RG<R>(p);
-    f.p[f.n] = PL<R>(p);
-    f.n++;
-  }
-  long long ne = (long long)(h->nr + h->np) * h->D.KA;
-  unsigned g = (unsigned)((ne + 255) / 256);
+static int comm_fields_of(nc_handle* h, const FieldPair* fl, int nf, const char* what) {
+  const long long ne = (long long)(h->nr + h->np) * h->D.KA;
+  const unsigned g = (unsigned)((ne + 255) / 256);
   TRY_(join_pl(h));
-  k_comm<<<g, 256, 0, h->stream>>>(f, h->r_dst, h->r_src, h->nr, h->p_dst, h->p_src, h->np);
-  TRY_(check_launch(h, "comm"));
+  for (int at = 0; at < nf; at += NC_MAXCOMM) {
+    CommFields<R> f{};
+    f.n = std::min(nf - at, NC_MAXCOMM);
+    for (int n = 0; n < f.n; ++n) {
+      f.r[n] = RG<R>(fl[at + n]);
+      f.p[n] = PL<R>(fl[at + n]);
+    }
+    k_comm<<<g, 256, 0, h->stream>>>(f, h->c_dst, h->c_src, h->nr, h->nr + h->np);
+    TRY_(check_launch(h, what));
+  }
   return fork_pl(h);
+}
+template <class R>
+static int comm(nc_handle* h, std::initializer_list<FieldPair> fl) {
+  return comm_fields_of<R>(h, fl.begin(), (int)fl.size(), "comm");
 }
 
 template <class R>
@@ -666,18 +666,9 @@ static Prog<R> prog_pl(nc_handle* h) {
 // halo exchange of the whole PRG_var: PROG and every tracer
 template <class R>
 static int comm_prg(nc_handle* h) {
-  const Dims& D = h->D;
-  CommFields<R> f{};
-  int n = 0;
-  for (int v = 0; v < 6; ++v) { f.r[n] = RG<R>(h->P[v]); f.p[n] = PL<R>(h->P[v]); n++; }
-  for (int iq = 0; iq < D.nq && n < NC_MAXCOMM; ++iq) { f.r[n] = RG<R>(h->Pq[iq]); f.p[n] = PL<R>(h->Pq[iq]); n++; }
-  f.n = n;
-  long long ne = (long long)(h->nr + h->np) * D.KA;
-  TRY(join_pl(h));
-  k_comm<<<(unsigned)((ne + 255) / 256), 256, 0, h->stream>>>(f, h->r_dst, h->r_src, h->nr, h->p_dst, h->p_src, h->np);
-  TRY(check_launch(h, "comm_final"));
-  for (int iq = NC_MAXCOMM - 6; iq < D.nq; ++iq) TRY(comm<R>(h, {h->Pq[iq]}));
-  return 0;
+  std::vector<FieldPair> fl(h->P, h->P + 6);
+  fl.insert(fl.end(), h->Pq, h->Pq + h->D.nq);
+  return comm_fields_of<R>(h, fl.data(), (int)fl.size(), "comm_final");
 }
 
 // ---------------------------------------------------------------------------
@@ -691,39 +682,38 @@ static int comm_prg(nc_handle* h) {
 template <class R>
 static int trc_vflux(nc_handle* h) {
   const Dims& D = h->D;
-  const cudaStream_t s = h->stream, ps = pole_stream(h);
-  const unsigned pcb = (unsigned)((6 * D.LP + 31) / 32);
-  const double dt = h->dtl;
+  TrcFluxArgs<R> ta[2];
   for (int pole = 0; pole < 2; ++pole) {
-    TrcFluxArgs<R> ta;
+    TrcFluxArgs<R>& a = ta[pole];
     auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
-    ta.rvx = F(h->PM[1]); ta.rvy = F(h->PM[2]); ta.rvz = F(h->PM[3]); ta.rw = F(h->PM[4]);
-    ta.rhog_in = F(h->P0[0]); ta.frhog = F(h->frhog); ta.flx_v = F(h->flx_v); ta.rhog_t = F(h->rhog_t);
-    ta.dt = dt;
-    if (!pole) k_trc_vflux<<<(unsigned)((D.npt2 + h->blk[TB_TRC_VFLUX] - 1) / h->blk[TB_TRC_VFLUX]), h->blk[TB_TRC_VFLUX], 0, s>>>(ta, 0);
-    else k_trc_vflux<<<pcb, 32, 0, ps>>>(ta, 1);
-    TRY(check_launch(h, pole ? "trc_vflux_pl" : "trc_vflux"));
+    a.rvx = F(h->PM[1]); a.rvy = F(h->PM[2]); a.rvz = F(h->PM[3]); a.rw = F(h->PM[4]);
+    a.rhog_in = F(h->P0[0]); a.frhog = F(h->frhog); a.flx_v = F(h->flx_v); a.rhog_t = F(h->rhog_t);
+    a.dt = h->dtl;
   }
-  return 0;
+  const int tb = h->blk[TB_TRC_VFLUX], npb = (D.npl + tb - 1) / tb;
+  TRY(join_pl(h));
+  k_trc_vflux<<<(unsigned)(npb + (D.npt + tb - 1) / tb), tb, 0, h->stream>>>(ta[0], ta[1], npb);
+  TRY(check_launch(h, "trc_vflux"));
+  return fork_pl(h);
 }
 
-// vertical advection of the tracer mass x in place: the first (second) step
-// of the tracer advection, density P0[0] (rhog_t), no clamp (clamp)
+// vertical advection of the tracer masses x[0..nx-1] in place: the first
+// (second) step of the tracer advection, density P0[0] (rhog_t), no clamp (clamp)
 template <class R>
-static int trc_vadv(nc_handle* h, FieldPair& x, bool second) {
+static int trc_vadv(nc_handle* h, FieldPair* x, int nx, bool second) {
   const Dims& D = h->D;
   const cudaStream_t s = h->stream, ps = pole_stream(h);
   const unsigned pcb = (unsigned)((6 * D.LP + 31) / 32);
-  const double dt = h->dtl;
   for (int pole = 0; pole < 2; ++pole) {
     TrcVadvArgs<R> va;
     auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
-    va.rhogq = F(x);
+    for (int n = 0; n < nx; ++n) va.rhogq_of[n] = F(x[n]);
     va.den = second ? F(h->rhog_t) : F(h->P0[0]);
     va.flx_v = F(h->flx_v); va.frhog = F(h->frhog);
-    va.dt = dt; va.bcoef = 0.0; va.clamp = second ? 1 : 0; va.dtl = dt;
-    if (!pole) k_trc_vadv<<<(unsigned)((D.npt2 + h->blk[TB_TRC_VADV] - 1) / h->blk[TB_TRC_VADV]), h->blk[TB_TRC_VADV], 0, s>>>(va, 0);
-    else k_trc_vadv<<<pcb, 32, 0, ps>>>(va, 1);
+    va.dt = h->dtl; va.bcoef = 0.0; va.clamp = second ? 1 : 0; va.dtl = h->dtl;
+    const int tb = h->blk[TB_TRC_VADV];
+    if (!pole) k_trc_vadv<<<dim3((unsigned)((D.npt2 + tb - 1) / tb), (unsigned)nx), tb, 0, s>>>(va, 0);
+    else k_trc_vadv<<<dim3(pcb, (unsigned)nx), 32, 0, ps>>>(va, 1);
     TRY(check_launch(h, pole ? "trc_vadv_pl" : "trc_vadv"));
   }
   return 0;
@@ -755,55 +745,74 @@ static int trc_hflux(nc_handle* h) {
   return 0;
 }
 
-// horizontal advection of the tracer mass x in place (gradient, exchange, face
-// values, Qout, exchange, flux update); leaves q, gq, qa, Qmin / Qmax behind
+// horizontal advection of the tracer masses x[0..nx-1] in place (gradient,
+// exchange, face values, Qout, exchange, flux update), in batches of TRC_NB
+// whose kernels read the winds' fields (centroids, masks, Courant numbers, mass
+// fluxes) once; leaves q, gq, qa, Qmin / Qmax of the last batch behind
 template <class R>
-static int trc_horizontal(nc_handle* h, FieldPair& x) {
+static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
   const Dims& D = h->D;
   const cudaStream_t s = h->stream, ps = pole_stream(h);
-  const unsigned pkb = (unsigned)((D.KA * D.LP + 127) / 128);
+  const unsigned pkb = (unsigned)((D.KA * D.LP + 31) / 32);
   const double dt = h->dtl;
-  {
+  for (int at = 0; at < nx; at += TRC_NB) {
+    const int nb = std::min(nx - at, TRC_NB);
+    FieldPair* xb = x + at;
+    const dim3 pg(pkb, (unsigned)nb);
     const dim3 gt((unsigned)D.KA, (unsigned)(((D.G - 2 + TG_DX - 1) / TG_DX) * ((D.G - 2 + TG_DY - 1) / TG_DY)),
                   (unsigned)D.L);
-    k_trc_grad_t<<<gt, TG_DX * TG_DY, 0, s>>>(RG<R>(x), RG<R>(h->rhog_t), RG<R>(h->q), RG<R>(h->gq[0]), RG<R>(h->gq[1]),
-                                              RG<R>(h->gq[2]));
+    TrcGradArgs<R> ga[2];
+    TrcRemapArgs<R> ra;
+    TrcRemapPlArgs<R> rp;
+    TrcLimArgs<R> la;
+    TrcLimPlArgs<R> lp;
+    std::vector<FieldPair> cq, cl;
+    for (int n = 0; n < nb; ++n) {
+      TrcWork& w = h->tw[n];
+      for (int pole = 0; pole < 2; ++pole) {
+        auto F = [&](FieldPair& f) { return pole ? PL<R>(f) : RG<R>(f); };
+        ga[pole].rhogq[n] = F(xb[n]); ga[pole].q[n] = F(w.q);
+        for (int d = 0; d < 3; ++d) ga[pole].gq[n][d] = F(w.gq[d]);
+      }
+      ra.q[n] = RG<R>(w.q); rp.q[n] = PL<R>(w.q);
+      for (int d = 0; d < 3; ++d) {
+        ra.gq[n][d] = RG<R>(w.gq[d]); rp.gq[n][d] = PL<R>(w.gq[d]);
+        ra.qa[n][d] = RG<R>(w.qa[d]); la.qa[n][d] = RG<R>(w.qa[d]);
+        cq.push_back(w.gq[d]);
+      }
+      rp.qa[n] = PL<R>(w.qa[0]); lp.qa[n] = PL<R>(w.qa[0]);
+      la.q[n] = RG<R>(w.q); la.Qmin[n] = RG<R>(w.Qmin); la.Qmax[n] = RG<R>(w.Qmax); la.rhogq[n] = RG<R>(xb[n]);
+      lp.q_of[n] = PL<R>(w.q); lp.Qmin[n] = PL<R>(w.Qmin); lp.Qmax[n] = PL<R>(w.Qmax); lp.rhogq[n] = PL<R>(xb[n]);
+      cl.push_back(w.Qmin); cl.push_back(w.Qmax);
+    }
+    ga[0].rhog_t = RG<R>(h->rhog_t); ga[1].rhog_t = PL<R>(h->rhog_t);
+    ga[0].nb = ga[1].nb = ra.nb = la.nb = nb;
+    for (int f = 0; f < 9; ++f) ra.xc[f] = RG<R>(h->xc[f]);
+    for (int f = 0; f < 6; ++f) { ra.cm[f] = RG<R>(h->cm[f]); la.ch[f] = RG<R>(h->ch[f]); la.cm[f] = RG<R>(h->cm[f]); la.flx[f] = RG<R>(h->flx[f]); }
+    rp.xc = PL<R>(h->xc[0]); rp.cm = PL<R>(h->cm[0]);
+    la.rhog_t = RG<R>(h->rhog_t); la.frhog = RG<R>(h->frhog); la.dt = dt;
+    lp.ch = PL<R>(h->ch[0]); lp.cm = PL<R>(h->cm[0]); lp.rhog_t = PL<R>(h->rhog_t); lp.frhog = PL<R>(h->frhog);
+    lp.flx = PL<R>(h->flx[0]); lp.dt = dt;
+    k_trc_grad_t<<<gt, TG_DX * TG_DY, 0, s>>>(ga[0]);
+    TRY(check_launch(h, "trc_grad"));
+    k_trc_grad_pl<<<pg, 32, 0, ps>>>(ga[1]);
+    TRY(check_launch(h, "trc_grad_pl"));
+    TRY(comm_fields_of<R>(h, cq.data(), (int)cq.size(), "comm"));
+    auto pts = [&](int tb) { return (unsigned)((D.npt + h->blk[tb] - 1) / h->blk[tb]); };
+    k_trc_remap<<<pts(TB_TRC_REMAP), h->blk[TB_TRC_REMAP], 0, s>>>(ra);
+    TRY(check_launch(h, "trc_remap"));
+    k_trc_remap_pl<<<pg, 32, 0, ps>>>(rp);
+    TRY(check_launch(h, "trc_remap_pl"));
+    k_trc_qout<<<pts(TB_TRC_QOUT), h->blk[TB_TRC_QOUT], 0, s>>>(la);
+    TRY(check_launch(h, "trc_qout"));
+    k_trc_qout_pl<<<pg, 32, 0, ps>>>(lp);
+    TRY(check_launch(h, "trc_qout_pl"));
+    TRY(comm_fields_of<R>(h, cl.data(), (int)cl.size(), "comm"));
+    k_trc_apply<<<pts(TB_TRC_APPLY), h->blk[TB_TRC_APPLY], 0, s>>>(la);
+    TRY(check_launch(h, "trc_apply"));
+    k_trc_apply_pl<<<pg, 32, 0, ps>>>(lp);
+    TRY(check_launch(h, "trc_apply_pl"));
   }
-  TRY(check_launch(h, "trc_grad"));
-  k_trc_grad_pl<<<pkb, 128, 0, ps>>>(PL<R>(x), PL<R>(h->rhog_t), PL<R>(h->q), PL<R>(h->gq[0]), PL<R>(h->gq[1]), PL<R>(h->gq[2]));
-  TRY(check_launch(h, "trc_grad_pl"));
-  TRY(comm<R>(h, {h->gq[0], h->gq[1], h->gq[2]}));
-  TrcRemapArgs<R> ra;
-  ra.q = RG<R>(h->q); ra.gq0 = RG<R>(h->gq[0]); ra.gq1 = RG<R>(h->gq[1]); ra.gq2 = RG<R>(h->gq[2]);
-  for (int f = 0; f < 9; ++f) ra.xc[f] = RG<R>(h->xc[f]);
-  for (int f = 0; f < 6; ++f) ra.cm[f] = RG<R>(h->cm[f]);
-  for (int f = 0; f < 3; ++f) ra.qa[f] = RG<R>(h->qa[f]);
-  k_trc_remap<<<(unsigned)((D.npt2 + h->blk[TB_TRC_REMAP] - 1) / h->blk[TB_TRC_REMAP]), h->blk[TB_TRC_REMAP], 0, s>>>(ra);
-  TRY(check_launch(h, "trc_remap"));
-  TrcRemapPlArgs<R> rp;
-  rp.q = PL<R>(h->q); rp.gq0 = PL<R>(h->gq[0]); rp.gq1 = PL<R>(h->gq[1]); rp.gq2 = PL<R>(h->gq[2]); rp.xc = PL<R>(h->xc[0]);
-  rp.cm = PL<R>(h->cm[0]); rp.qa = PL<R>(h->qa[0]);
-  k_trc_remap_pl<<<pkb, 128, 0, ps>>>(rp);
-  TRY(check_launch(h, "trc_remap_pl"));
-  TrcLimArgs<R> la;
-  la.q = RG<R>(h->q); la.rhog_t = RG<R>(h->rhog_t); la.frhog = RG<R>(h->frhog);
-  for (int f = 0; f < 6; ++f) { la.ch[f] = RG<R>(h->ch[f]); la.cm[f] = RG<R>(h->cm[f]); la.flx[f] = RG<R>(h->flx[f]); }
-  for (int f = 0; f < 3; ++f) la.qa[f] = RG<R>(h->qa[f]);
-  la.qout_min = RG<R>(h->Qmin); la.qout_max = RG<R>(h->Qmax); la.Qmin = RG<R>(h->Qmin); la.Qmax = RG<R>(h->Qmax);
-  la.rhogq = RG<R>(x); la.dt = dt;
-  TrcLimPlArgs<R> lp;
-  lp.q = PL<R>(h->q); lp.ch = PL<R>(h->ch[0]); lp.cm = PL<R>(h->cm[0]); lp.rhog_t = PL<R>(h->rhog_t); lp.frhog = PL<R>(h->frhog);
-  lp.qa = PL<R>(h->qa[0]); lp.flx = PL<R>(h->flx[0]); lp.Qmin = PL<R>(h->Qmin); lp.Qmax = PL<R>(h->Qmax);
-  lp.qout_min = PL<R>(h->Qmin); lp.qout_max = PL<R>(h->Qmax); lp.rhogq = PL<R>(x); lp.dt = dt;
-  k_trc_qout<<<(unsigned)((D.npt2 + h->blk[TB_TRC_QOUT] - 1) / h->blk[TB_TRC_QOUT]), h->blk[TB_TRC_QOUT], 0, s>>>(la);
-  TRY(check_launch(h, "trc_qout"));
-  k_trc_qout_pl<<<pkb, 128, 0, ps>>>(lp);
-  TRY(check_launch(h, "trc_qout_pl"));
-  TRY(comm<R>(h, {h->Qmin, h->Qmax}));
-  k_trc_apply<<<(unsigned)((D.npt2 + h->blk[TB_TRC_APPLY] - 1) / h->blk[TB_TRC_APPLY]), h->blk[TB_TRC_APPLY], 0, s>>>(la);
-  TRY(check_launch(h, "trc_apply"));
-  k_trc_apply_pl<<<pkb, 128, 0, ps>>>(lp);
-  TRY(check_launch(h, "trc_apply_pl"));
   return 0;
 }
 
@@ -813,7 +822,7 @@ static int trc_rhog(nc_handle* h) {
   const cudaStream_t s = h->stream;
   const double dt = h->dtl;
   TRY(join_pl(h));
-  k_trc_rhog<<<(unsigned)(((D.npt2 + (long long)D.KA * D.LP) + h->blk[TB_TRC_RHOG] - 1) / h->blk[TB_TRC_RHOG]), h->blk[TB_TRC_RHOG], 0, s>>>(RG<R>(h->rhog_t), RG<R>(h->flx[0]), RG<R>(h->flx[1]), RG<R>(h->flx[2]), RG<R>(h->flx[3]), RG<R>(h->flx[4]),
+  k_trc_rhog<<<(unsigned)(((D.npt + (long long)D.KA * D.LP) + h->blk[TB_TRC_RHOG] - 1) / h->blk[TB_TRC_RHOG]), h->blk[TB_TRC_RHOG], 0, s>>>(RG<R>(h->rhog_t), RG<R>(h->flx[0]), RG<R>(h->flx[1]), RG<R>(h->flx[2]), RG<R>(h->flx[3]), RG<R>(h->flx[4]),
                                      RG<R>(h->flx[5]), RG<R>(h->frhog), (R)dt, PL<R>(h->flx[0]), PL<R>(h->rhog_t), PL<R>(h->frhog));
   TRY(check_launch(h, "trc_rhog"));
   TRY(fork_pl(h));
@@ -1121,14 +1130,14 @@ static int run_step(nc_handle* h) {
   TRY(trc_vflux<R>(h));
   // first vertical step uses the density at the start of the step; the
   // Courant numbers of the first step are those of rhog_in
-  for (int iq = 0; iq < D.nq; ++iq) TRY(trc_vadv<R>(h, h->Pq[iq], false));
+  TRY(trc_vadv<R>(h, h->Pq, D.nq, false));
   PHASE();
   TRY(trc_hflux<R>(h));
   PHASE();
-  for (int iq = 0; iq < D.nq; ++iq) TRY(trc_horizontal<R>(h, h->Pq[iq]));
+  TRY(trc_horizontal<R>(h, h->Pq, D.nq));
   PHASE();
   TRY(trc_rhog<R>(h));
-  for (int iq = 0; iq < D.nq; ++iq) TRY(trc_vadv<R>(h, h->Pq[iq], true));
+  TRY(trc_vadv<R>(h, h->Pq, D.nq, true));
   PHASE();
   if (h->trcadv) {
     // the prescribed winds of the next time (mod_forcing.py forcing_update)
@@ -1352,11 +1361,12 @@ static int vadv_lin_launch(nc_handle* h, int mode, const FieldPair& at, const Fi
 static HLin hlin_args(nc_handle* h) {
   HLin a{};
   FieldPair* L = h->lin;
-  a.q = h->q.r; a.Qmin = h->Qmin.r; a.Qmax = h->Qmax.r; a.rhog_t = L[LN_RHO].r; a.frhog = h->frhog.r;
-  for (int f = 0; f < 3; ++f) a.qa[f] = h->qa[f].r;
+  TrcWork& w = h->tw[0];
+  a.q = w.q.r; a.Qmin = w.Qmin.r; a.Qmax = w.Qmax.r; a.rhog_t = L[LN_RHO].r; a.frhog = h->frhog.r;
+  for (int f = 0; f < 3; ++f) a.qa[f] = w.qa[f].r;
   for (int f = 0; f < 6; ++f) { a.ch[f] = h->ch[f].r; a.cm[f] = h->cm[f].r; a.flx[f] = h->flx[f].r; }
   for (int f = 0; f < 9; ++f) a.xc[f] = h->xc[f].r;
-  a.q_pl = h->q.p; a.qa_pl = h->qa[0].p; a.Qmin_pl = h->Qmin.p; a.Qmax_pl = h->Qmax.p; a.rhog_t_pl = L[LN_RHO].p;
+  a.q_pl = w.q.p; a.qa_pl = w.qa[0].p; a.Qmin_pl = w.Qmin.p; a.Qmax_pl = w.Qmax.p; a.rhog_t_pl = L[LN_RHO].p;
   a.frhog_pl = h->frhog.p; a.ch_pl = h->ch[0].p; a.cm_pl = h->cm[0].p; a.flx_pl = h->flx[0].p; a.xc_pl = h->xc[0].p;
   a.dt = h->dtl;
   a.dq = L[LN_DQ].r; a.dq_pl = L[LN_DQ].p;
@@ -1383,12 +1393,12 @@ static int trc_lin_forward(nc_handle* h, const double* x0, const double* x0_pl) 
   TRY(copy_in(h, L[LN_RHO], h->rhog_t.r, h->rhog_t.p));
   TRY(copy_in(h, L[LN_X0], x0, x0_pl));
   TRY(copy_in(h, L[LN_X1], x0, x0_pl));
-  TRY(trc_vadv<double>(h, L[LN_X1], false));
+  TRY(trc_vadv<double>(h, &L[LN_X1], 1, false));
   TRY(copy_in(h, L[LN_X2], L[LN_X1].r, L[LN_X1].p));
-  TRY(trc_horizontal<double>(h, L[LN_X2]));
+  TRY(trc_horizontal<double>(h, &L[LN_X2], 1));
   TRY(trc_rhog<double>(h));
   TRY(copy_in(h, L[LN_X3], L[LN_X2].r, L[LN_X2].p));
-  return trc_vadv<double>(h, L[LN_X3], true);
+  return trc_vadv<double>(h, &L[LN_X3], 1, true);
 }
 
 // tangent-linear of the horizontal step at X1: T2 = H'(X1) T1
@@ -1400,23 +1410,31 @@ static int hlin_tl(nc_handle* h) {
   {
     const dim3 gt((unsigned)D.KA, (unsigned)(((D.G - 2 + TG_DX - 1) / TG_DX) * ((D.G - 2 + TG_DY - 1) / TG_DY)),
                   (unsigned)D.L);
-    k_trc_grad_t<<<gt, TG_DX * TG_DY, 0, s>>>(L[LN_T1].r, L[LN_RHO].r, L[LN_DQ].r, L[LN_DG0].r, L[LN_DG1].r,
-                                              L[LN_DG2].r);
-    TRY(check_launch(h, "lin_grad"));
+    for (int pole = 0; pole < 2; ++pole) {
+      auto F = [&](int n) { return pole ? L[n].p : L[n].r; };
+      TrcGradArgs<double> ga;
+      ga.rhogq[0] = F(LN_T1); ga.rhog_t = F(LN_RHO); ga.q[0] = F(LN_DQ);
+      for (int d = 0; d < 3; ++d) ga.gq[0][d] = F(LN_DG0 + d);
+      ga.nb = 1;
+      if (!pole) k_trc_grad_t<<<gt, TG_DX * TG_DY, 0, s>>>(ga);
+      else k_trc_grad_pl<<<pkb, 128, 0, s>>>(ga);
+      TRY(check_launch(h, pole ? "lin_grad_pl" : "lin_grad"));
+    }
   }
-  k_trc_grad_pl<<<pkb, 128, 0, s>>>(L[LN_T1].p, L[LN_RHO].p, L[LN_DQ].p, L[LN_DG0].p, L[LN_DG1].p, L[LN_DG2].p);
-  TRY(check_launch(h, "lin_grad_pl"));
   TRY(comm<double>(h, {L[LN_DG0], L[LN_DG1], L[LN_DG2]}));
   TrcRemapArgs<double> ra;
-  ra.q = L[LN_DQ].r; ra.gq0 = L[LN_DG0].r; ra.gq1 = L[LN_DG1].r; ra.gq2 = L[LN_DG2].r;
+  TrcRemapPlArgs<double> rp;
+  ra.q[0] = L[LN_DQ].r; rp.q[0] = L[LN_DQ].p;
+  for (int d = 0; d < 3; ++d) {
+    ra.gq[0][d] = L[LN_DG0 + d].r; rp.gq[0][d] = L[LN_DG0 + d].p;
+    ra.qa[0][d] = L[LN_DQA0 + d].r;
+  }
+  ra.nb = 1;
   for (int f = 0; f < 9; ++f) ra.xc[f] = h->xc[f].r;
   for (int f = 0; f < 6; ++f) ra.cm[f] = h->cm[f].r;
-  for (int f = 0; f < 3; ++f) ra.qa[f] = L[LN_DQA0 + f].r;
-  k_trc_remap<<<cb, 128, 0, s>>>(ra);
+  k_trc_remap<<<(unsigned)((D.npt + 127) / 128), 128, 0, s>>>(ra);
   TRY(check_launch(h, "lin_remap"));
-  TrcRemapPlArgs<double> rp;
-  rp.q = L[LN_DQ].p; rp.gq0 = L[LN_DG0].p; rp.gq1 = L[LN_DG1].p; rp.gq2 = L[LN_DG2].p; rp.xc = h->xc[0].p;
-  rp.cm = h->cm[0].p; rp.qa = L[LN_DQA0].p;
+  rp.xc = h->xc[0].p; rp.cm = h->cm[0].p; rp.qa[0] = L[LN_DQA0].p;
   k_trc_remap_pl<<<pkb, 128, 0, s>>>(rp);
   TRY(check_launch(h, "lin_remap_pl"));
   HLin a = hlin_args(h);
@@ -1986,6 +2004,27 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
       h->allocs.push_back(*dst[n]);
       if (numel(src[n])) CU(cudaMemcpy(*dst[n], src[n]->data, numel(src[n]) * sizeof(long long), cudaMemcpyHostToDevice));
     }
+    // k_comm's form: array indices at level 0 (6 npt < 2^31 is checked above)
+    const long long pl = D.plane;
+    auto reg0 = [&](long long c) { return (int)((c / pl) * D.KA * pl + c % pl); };
+    auto pol0 = [&](long long g) { return (int)((g / D.LP) * D.KA * D.LP + g % D.LP); };
+    std::vector<int> cd, cs;
+    const long long *rd = (const long long*)a->data, *rs = (const long long*)b->data, *pd = (const long long*)c->data,
+                    *psrc = (const long long*)d->data;
+    for (int n = 0; n < h->nr; ++n) {
+      cd.push_back(reg0(rd[n]));
+      cs.push_back(rs[n] >= 0 ? reg0(rs[n]) : -pol0(-rs[n] - 1) - 1);
+    }
+    for (int n = 0; n < h->np; ++n) {
+      cd.push_back(pol0(pd[n]));
+      cs.push_back(reg0(psrc[n]));
+    }
+    for (int n = 0; n < 2; ++n) {
+      const std::vector<int>& v = n ? cs : cd;
+      int** out = n ? &h->c_src : &h->c_dst;
+      TRY(dev_alloc_bytes(h, (void**)out, std::max<size_t>(v.size(), 1) * sizeof(int)));
+      if (!v.empty()) CU(cudaMemcpy(*out, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice));
+    }
   }
   if (h->mixed) {
     if (h->hist || h->hs_lat || h->kess_zf)
@@ -2017,13 +2056,20 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
   for (int d = 0; d < 3; ++d) {
     snprintf(nm, sizeof nm, "vtmp2.%d", d); TRY(field(h, h->vtmp2[d], nm));
     snprintf(nm, sizeof nm, "hdiv.%d", d); TRY(field(h, h->hdiv[d], nm));
-    snprintf(nm, sizeof nm, "gq.%d", d); TRY(field(h, h->gq[d], nm));
-    snprintf(nm, sizeof nm, "qa.%d", d); TRY(field(h, h->qa[d], nm));
   }
   TRY(field(h, h->Mc, "Mc", true)); TRY(field(h, h->Mu, "Mu", true)); TRY(field(h, h->Ml, "Ml", true));
   TRY(field(h, h->ethtot0, "ethtot0"));
-  TRY(field(h, h->flx_v, "flx_v")); TRY(field(h, h->rhog_t, "rhog_t")); TRY(field(h, h->q, "q"));
-  TRY(field(h, h->Qmin, "Qmin")); TRY(field(h, h->Qmax, "Qmax"));
+  TRY(field(h, h->flx_v, "flx_v")); TRY(field(h, h->rhog_t, "rhog_t"));
+  for (int n = 0; n < std::min(std::max(D.nq, 1), TRC_NB); ++n) {   // named as one tracer's fields for the first of a batch
+    const std::string sfx = n ? "#" + std::to_string(n) : "";
+    TrcWork& w = h->tw[n];
+    TRY(field(h, w.q, ("q" + sfx).c_str()));
+    TRY(field(h, w.Qmin, ("Qmin" + sfx).c_str())); TRY(field(h, w.Qmax, ("Qmax" + sfx).c_str()));
+    for (int d = 0; d < 3; ++d) {
+      TRY(field(h, w.gq[d], ("gq." + std::to_string(d) + sfx).c_str()));
+      TRY(field(h, w.qa[d], ("qa." + std::to_string(d) + sfx).c_str()));
+    }
+  }
   for (int n = 0; n < 8; ++n) { snprintf(nm, sizeof nm, "vph.%d", n); TRY(field(h, h->vph[n], nm)); }
   for (int f = 0; f < 6; ++f) {
     snprintf(nm, sizeof nm, "flx.%d", f); TRY(field(h, h->flx[f], nm));
@@ -2815,7 +2861,7 @@ int nc_laplacian(nc_handle* h, int32_t transpose, const double* q, const double*
     f.p[0] = w_pl;
     f.n = 1;
     if (ne > 0) {
-      k_comm<<<gc, 256, 0, h->stream>>>(f, h->r_dst, h->r_src, h->nr, h->p_dst, h->p_src, h->np);
+      k_comm<<<gc, 256, 0, h->stream>>>(f, h->c_dst, h->c_src, h->nr, h->nr + h->np);
       TRY(check_launch(h, "lap_comm"));
     }
     k_lap_fwd<<<gr, 256, 0, h->stream>>>(w, y);
@@ -2873,7 +2919,7 @@ int nc_trc_step_lin(nc_handle* h, int32_t mode, const double* x0, const double* 
   if (mode != 2 && ne > 0) {   // the closing exchange of PRG_var
     cf.r[0] = out;
     cf.p[0] = out_pl;
-    k_comm<<<gc, 256, 0, h->stream>>>(cf, h->r_dst, h->r_src, h->nr, h->p_dst, h->p_src, h->np);
+    k_comm<<<gc, 256, 0, h->stream>>>(cf, h->c_dst, h->c_src, h->nr, h->nr + h->np);
     TRY(check_launch(h, "lin_comm"));
   }
   if (h->prof) TRY(collect_profile(h));
@@ -2927,7 +2973,7 @@ static int comm_fields(nc_handle* h, double* r, double* p, int nf, bool adjoint)
       cf.r[0] = rf;
       cf.p[0] = pf;
       cf.n = 1;
-      k_comm<<<gc, 256, 0, h->stream>>>(cf, h->r_dst, h->r_src, h->nr, h->p_dst, h->p_src, h->np);
+      k_comm<<<gc, 256, 0, h->stream>>>(cf, h->c_dst, h->c_src, h->nr, h->nr + h->np);
       TRY(check_launch(h, "op_comm"));
     } else {
       k_comm_adj_add<<<gc, 256, 0, h->stream>>>(rf, pf, h->r_dst, h->r_src, h->nr, h->p_dst, h->p_src, h->np);

@@ -233,6 +233,22 @@ struct RecipF {
 __device__ __forceinline__ RecipF recip_of(float b) { return RecipF{__frcp_rn(b)}; }
 __device__ __forceinline__ float div_by(float x, const RecipF& r) { return x * r.h; }
 
+// x / b for a divisor that several quotients share, exactly: through one
+// reciprocal in float64 (div_by), by the division itself in float32 (whose
+// div_by is not the rounded quotient)
+struct DivD {
+  Recip r;
+  __device__ __forceinline__ explicit DivD(double b) : r(recip_of(b)) {}
+  __device__ __forceinline__ double operator()(double x) const { return div_by(x, r); }
+};
+struct DivF {
+  float b;
+  __device__ __forceinline__ explicit DivF(float x) : b(x) {}
+  __device__ __forceinline__ float operator()(float x) const { return x / b; }
+};
+template <class R> struct DivOf { using type = DivD; };
+template <> struct DivOf<float> { using type = DivF; };
+
 // ---- indexing -------------------------------------------------------------
 __device__ __forceinline__ int ix(int i, int j, int k, int l) {
   return ((l * cD.KA + k) * cD.G + j) * cD.G + i;

@@ -19,43 +19,39 @@ struct TrcFluxArgs {
   R dt;
 };
 
+// flx_v at level k and the density, one thread per point (the flux above is formed again)
 template <class R>
-__device__ void trc_vflux_column(const Col c, const MetT<R> m, const TrcFluxArgs<R>& a) {
-  const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    R f = R(0.0);
-    if (k >= kmin + 1 && k <= kmax) {
-      int pm = c.at(k - 1);
-      R horiz = (mc(m.C2WGz, c, 0, 6, k) * a.rvx[p] + mc(m.C2WGz, c, 1, 6, k) * a.rvx[pm] +
-                      mc(m.C2WGz, c, 2, 6, k) * a.rvy[p] + mc(m.C2WGz, c, 3, 6, k) * a.rvy[pm] +
-                      mc(m.C2WGz, c, 4, 6, k) * a.rvz[p] + mc(m.C2WGz, c, 5, 6, k) * a.rvz[pm]) * gam_at(m.RGAMH, p);
-      R vert = a.rw[p] * m.RGSQRTH[p];
-      f = (horiz + vert) * R(0.5) * a.dt;
-    }
-    a.flx_v[p] = f;
-  }
-  for (int k = 0; k < KA; ++k) {
-    int p = c.at(k);
-    R r = R(0.0);
-    if (k >= kmin && k <= kmax) {
-      r = a.rhog_in[p] - (a.flx_v[c.at(k + 1)] - a.flx_v[p]) * CC.rdgz[k] + R(0.0) * a.frhog[p] * a.dt;
-    } else if (k == kmin - 1) {
-      r = a.rhog_in[c.at(kmin)];
-    } else if (k == kmax + 1) {
-      r = a.rhog_in[c.at(kmax)];
-    }
-    a.rhog_t[p] = r;
-  }
+__device__ __forceinline__ void trc_vflux_point(const Col c, const MetT<R> m, const TrcFluxArgs<R>& a, int k) {
+  const int kmin = cD.kmin, kmax = cD.kmax;
+  auto flux = [&](int kk) -> R {
+    if (kk < kmin + 1 || kk > kmax) return R(0.0);
+    const int p = c.at(kk), pm = c.at(kk - 1);
+    const R horiz = (mc(m.C2WGz, c, 0, 6, kk) * a.rvx[p] + mc(m.C2WGz, c, 1, 6, kk) * a.rvx[pm] +
+                     mc(m.C2WGz, c, 2, 6, kk) * a.rvy[p] + mc(m.C2WGz, c, 3, 6, kk) * a.rvy[pm] +
+                     mc(m.C2WGz, c, 4, 6, kk) * a.rvz[p] + mc(m.C2WGz, c, 5, 6, kk) * a.rvz[pm]) *
+                    gam_at(m.RGAMH, p);
+    const R vert = a.rw[p] * m.RGSQRTH[p];
+    return (horiz + vert) * R(0.5) * a.dt;
+  };
+  const int p = c.at(k);
+  const R f = flux(k);
+  R r = R(0.0);
+  if (k >= kmin && k <= kmax) r = a.rhog_in[p] - (flux(k + 1) - f) * CC.rdgz[k] + R(0.0) * a.frhog[p] * a.dt;
+  else if (k == kmin - 1) r = a.rhog_in[c.at(kmin)];
+  else if (k == kmax + 1) r = a.rhog_in[c.at(kmax)];
+  a.flx_v[p] = f;
+  a.rhog_t[p] = r;
 }
 
 template <class R>
-__global__ void k_trc_vflux(TrcFluxArgs<R> a, int pole) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  if (!pole) trc_vflux_column(col_reg(i, j, l), met_of<R>(false), a);
-  else trc_vflux_column(col_pl(g, lp), met_of<R>(true), a);
+__global__ void k_trc_vflux(const __grid_constant__ TrcFluxArgs<R> a, const __grid_constant__ TrcFluxArgs<R> ap, int npb) {
+  Pt q;
+  if ((int)blockIdx.x < npb) {
+    if (pole_point((int)(blockIdx.x * blockDim.x + threadIdx.x), q))
+      trc_vflux_point(col_pl(q.g, q.lp), met_of<R>(true), ap, q.k);
+  } else if (reg_point((int)((blockIdx.x - npb) * blockDim.x + threadIdx.x), q)) {
+    trc_vflux_point(col_reg(q.i, q.j, q.l), met_of<R>(false), a, q.k);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -64,7 +60,7 @@ __global__ void k_trc_vflux(TrcFluxArgs<R> a, int pole) {
 // ---------------------------------------------------------------------------
 template <class R>
 struct TrcVadvArgs {
-  R* rhogq;
+  R* rhogq_of[NC_MAXNQ];   // the tracers of the launch (blockIdx.y)
   const R *den, *flx_v, *frhog;
   R dt, bcoef;      // d = bcoef*frhog/den*dt
   int clamp;             // second step: zero tiny negatives, then add dt*0
@@ -78,27 +74,39 @@ struct TrcVadvArgs {
 // of the reference (q, qh and ck on every level, the limiter, the update),
 // in the same order, so the same results.
 template <class R>
-__device__ void trc_vadv_column(const Col c, const TrcVadvArgs<R>& a) {
+__device__ void trc_vadv_column(const Col c, const TrcVadvArgs<R>& a, R* rhogq) {
   const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
   const R BIG = CC.HUGE_, EPS = CC.EPS;
   auto finish = [&](int k, R x) {   // clamp and store of one updated level
     if (a.clamp && x > -R(1.0e-10) && x < R(0.0)) x = R(0.0);
     if (a.clamp) x = x + a.dtl * R(0.0);
-    a.rhogq[c.at(k)] = x;
+    rhogq[c.at(k)] = x;
   };
   // q at kmin-1 and kmin, den and flx_v at kmin (read before the ghost levels are zeroed)
   const int p = c.at(kmin);
-  R rq_m = a.rhogq[c.at(kmin - 1)], rq_k = a.rhogq[p];
-  R q_m = rq_m / __ldg(&a.den[c.at(kmin - 1)]), q_k = rq_k / __ldg(&a.den[p]);
-  R den_k = __ldg(&a.den[p]), flx_k = __ldg(&a.flx_v[p]);
+  R rq_m = rhogq[c.at(kmin - 1)], rq_k = rhogq[p];
+  using Div = typename DivOf<R>::type;
+  Div by_k(__ldg(&a.den[p]));       // the divisions by a level's density share its reciprocal
+  R q_m = rq_m / __ldg(&a.den[c.at(kmin - 1)]), q_k = by_k(rq_k);
+  R flx_k = __ldg(&a.flx_v[p]);
+  R ck0 = by_k(-flx_k) * CC.rdgz[kmin];
   R qmin_prev = R(0.0), qmax_prev = R(0.0), qh_prev = R(0.0), rq_prev = R(0.0), flx_prev = R(0.0);
+  // the loads of level k+2 are issued before level k is worked on
+  R rq_n = rhogq[c.at(kmin + 1)], den_n = __ldg(&a.den[c.at(kmin + 1)]), flx_n = __ldg(&a.flx_v[c.at(kmin + 1)]);
+  R fr_n = __ldg(&a.frhog[p]);
   for (int k = kmin; k <= kmax; ++k) {
-    const int pp = c.at(k + 1);
-    const R rq_p = a.rhogq[pp], den_p = __ldg(&a.den[pp]), flx_p = __ldg(&a.flx_v[pp]);
-    const R q_p = rq_p / den_p;
-    const R ck0 = -flx_k / den_k * CC.rdgz[k];
-    const R ck1 = flx_p / den_k * CC.rdgz[k];
-    const R ck0_p = (k + 1 <= kmax) ? -flx_p / den_p * CC.rdgz[k + 1] : R(0.0);
+    const R rq_p = rq_n, den_p = den_n, flx_p = flx_n, fr_k = fr_n;
+    if (k < kmax) {
+      const int p2 = c.at(k + 2);
+      rq_n = rhogq[p2];
+      den_n = __ldg(&a.den[p2]);
+      flx_n = __ldg(&a.flx_v[p2]);
+      fr_n = __ldg(&a.frhog[c.at(k + 1)]);
+    }
+    const Div by_p(den_p);
+    const R q_p = by_p(rq_p);
+    const R ck1 = by_k(flx_p) * CC.rdgz[k];
+    const R ck0_p = (k + 1 <= kmax) ? by_p(-flx_p) * CC.rdgz[k + 1] : R(0.0);
     const R qh_raw = CC.afact[k] * q_k + CC.bfact[k] * q_m;
     const R inL = R(0.5) - copysign(R(0.5), ck0);
     const R inU = R(0.5) + copysign(R(0.5), ck0_p);
@@ -115,9 +123,10 @@ __device__ void trc_vadv_column(const Col c, const TrcVadvArgs<R>& a) {
     const R CQmin = inL * c1 * QminL + inU * c2 * QminU;
     const R CQmax = inL * c1 * QmaxL + inU * c2 * QmaxU;
     const R zsw = R(0.5) - copysign(R(0.5), fabs(Cout) - EPS);
-    const R dk = a.bcoef * __ldg(&a.frhog[c.at(k)]) / den_k * a.dt;
-    const R qomin = ((qc - qnmax) + qnmax * (Cin + Cout - dk) - CQmax) / (Cout + zsw) * (R(1.0) - zsw) + qc * zsw;
-    const R qomax = ((qc - qnmin) + qnmin * (Cin + Cout - dk) - CQmin) / (Cout + zsw) * (R(1.0) - zsw) + qc * zsw;
+    const R dk = by_k(a.bcoef * fr_k) * a.dt;
+    const Div by_o(Cout + zsw);
+    const R qomin = by_o((qc - qnmax) + qnmax * (Cin + Cout - dk) - CQmax) * (R(1.0) - zsw) + qc * zsw;
+    const R qomax = by_o((qc - qnmin) + qnmin * (Cin + Cout - dk) - CQmin) * (R(1.0) - zsw) + qc * zsw;
     R qh = R(0.0);   // the face at kmin stays zero
     if (k > kmin)
       qh = inL * npmin(npmax(qh_raw, qmin_prev), qmax_prev) + (R(1.0) - inL) * npmin(npmax(qh_raw, qomin), qomax);
@@ -128,7 +137,8 @@ __device__ void trc_vadv_column(const Col c, const TrcVadvArgs<R>& a) {
     rq_prev = rq_k;
     flx_prev = flx_k;
     q_m = q_k; q_k = q_p; rq_k = rq_p;
-    den_k = den_p; flx_k = flx_p;
+    by_k = by_p; flx_k = flx_p;
+    ck0 = ck0_p;
   }
   // cell kmax: its upper face (kmax+1) is zero
   finish(kmax, rq_prev - (flx_k * R(0.0) - flx_prev * qh_prev) * CC.rdgz[kmax]);
@@ -136,13 +146,15 @@ __device__ void trc_vadv_column(const Col c, const TrcVadvArgs<R>& a) {
   for (int k = kmax + 1; k < KA; ++k) finish(k, R(0.0));
 }
 
+// Every tracer of the step in one launch: the sweep is a serial chain per
+// column, so one tracer's columns alone leave the SMs waiting (263 us a tracer
+// at gl07 z60 float64)
 template <class R>
-__global__ void k_trc_vadv(TrcVadvArgs<R> a, int pole) {
+__global__ void k_trc_vadv(const __grid_constant__ TrcVadvArgs<R> a, int pole) {
   int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
   int i, j, l, g, lp;
   if (!map_col(pole, t, i, j, l, g, lp)) return;
-  if (!pole) trc_vadv_column(col_reg(i, j, l), a);
-  else trc_vadv_column(col_pl(g, lp), a);
+  trc_vadv_column(pole ? col_pl(g, lp) : col_reg(i, j, l), a, a.rhogq_of[blockIdx.y]);
 }
 
 // ---------------------------------------------------------------------------
@@ -348,34 +360,48 @@ __global__ void k_trc_hflux_pl(TrcHfluxPlArgs<R> a) {
 // stencil use), then each cell's gradient is read from there.  The region's
 // halo cells get q and a zero gradient from the tile that holds their nearest
 // interior cell, so every cell is written exactly once.
+// The tracers of a batch (up to TRC_NB) share the block: each gradient
+// coefficient and each cell's density is read once for all of them.
 #define TG_DX 32
 #define TG_DY 8
+#define TRC_NB 4
 template <class R>
-__global__ void __launch_bounds__(TG_DX * TG_DY) k_trc_grad_t(const R* rhogq, const R* rhog_t, R* q,
-                                                              R* gq0, R* gq1, R* gq2) {
-  constexpr int PX = TG_DX + 2, PY = TG_DY + 2;
-  __shared__ R s_q[PY * PX];
+struct TrcGradArgs {
+  const R* rhogq[TRC_NB];
+  const R* rhog_t;
+  R *q[TRC_NB], *gq[TRC_NB][3];
+  int nb;
+};
+template <class R>
+__global__ void __launch_bounds__(TG_DX * TG_DY) k_trc_grad_t(const __grid_constant__ TrcGradArgs<R> a) {
+  constexpr int PX = TG_DX + 2, PY = TG_DY + 2, NP = PX * PY;
+  __shared__ R s_q[TRC_NB][NP];
   const TileLv tl = tile_level<TG_DX, TG_DY>(0);
   const int k = tl.k, l = tl.l, i0 = tl.i0, j0 = tl.j0;
   const int G = cD.G, gmax = cD.G - 2;
   const int tid = threadIdx.x;
-  for (int p = tid; p < PX * PY; p += blockDim.x) {
+  for (int p = tid; p < NP; p += blockDim.x) {
     const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
-    R v = R(0.0);
-    if (ii < G && jj < G) {
-      const int qq = ix(ii, jj, k, l);
-      v = rhogq[qq] / rhog_t[qq];
-      if (!interior(ii, jj)) {
-        const int ci = min(max(ii, 1), gmax), cj = min(max(jj, 1), gmax);
-        if (ci >= i0 && ci < i0 + TG_DX && cj >= j0 && cj < j0 + TG_DY) {
-          q[qq] = v;
-          gq0[qq] = R(0.0);
-          gq1[qq] = R(0.0);
-          gq2[qq] = R(0.0);
-        }
+    const bool ok = ii < G && jj < G;
+    const int qq = ok ? ix(ii, jj, k, l) : 0;
+    bool mine = false;   // a halo cell of the region that this tile writes
+    if (ok && !interior(ii, jj)) {
+      const int ci = min(max(ii, 1), gmax), cj = min(max(jj, 1), gmax);
+      mine = ci >= i0 && ci < i0 + TG_DX && cj >= j0 && cj < j0 + TG_DY;
+    }
+    const typename DivOf<R>::type den(ok ? __ldg(a.rhog_t + qq) : R(1.0));
+#pragma unroll
+    for (int n = 0; n < TRC_NB; ++n) {
+      if (n >= a.nb) break;
+      const R v = ok ? den(__ldg(a.rhogq[n] + qq)) : R(0.0);
+      s_q[n][p] = v;
+      if (mine) {
+        a.q[n][qq] = v;
+        a.gq[n][0][qq] = R(0.0);
+        a.gq[n][1][qq] = R(0.0);
+        a.gq[n][2][qq] = R(0.0);
       }
     }
-    s_q[p] = v;
   }
   __syncthreads();
   const int tx = tid % TG_DX, ty = tid / TG_DX;
@@ -383,108 +409,126 @@ __global__ void __launch_bounds__(TG_DX * TG_DY) k_trc_grad_t(const R* rhogq, co
   if (i > gmax || j > gmax) return;
   const int qq = ix(i, j, k, l);
   const int c0 = (ty + 1) * PX + (tx + 1);
-  const R s7[7] = {s_q[c0], s_q[c0 + 1], s_q[c0 + PX + 1], s_q[c0 + PX], s_q[c0 - 1], s_q[c0 - PX - 1], s_q[c0 - PX]};
-  q[qq] = s7[0];
-  R* gq[3] = {gq0, gq1, gq2};
+  const int nb[7] = {c0, c0 + 1, c0 + PX + 1, c0 + PX, c0 - 1, c0 - PX - 1, c0 - PX};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {   // grad7 (kernels/oprtgradient.py:45-70)
-    R a = P2c(CG.coef_grad, d * 7 + 0, i, j, l) * s7[0];
+    R cg[7];
 #pragma unroll
-    for (int m = 1; m < 7; ++m) a = a + P2c(CG.coef_grad, d * 7 + m, i, j, l) * s7[m];
-    gq[d][qq] = a;
+    for (int m = 0; m < 7; ++m) cg[m] = P2c(CG.coef_grad, d * 7 + m, i, j, l);
+#pragma unroll
+    for (int n = 0; n < TRC_NB; ++n) {
+      if (n >= a.nb) break;
+      R g = cg[0] * s_q[n][c0];
+#pragma unroll
+      for (int m = 1; m < 7; ++m) g = g + cg[m] * s_q[n][nb[m]];
+      a.gq[n][d][qq] = g;
+      if (d == 0) a.q[n][qq] = s_q[n][c0];
+    }
   }
 }
 
 template <class R>
-__global__ void k_trc_grad_pl(const R* rhogq, const R* rhog_t, R* q, R* gq0, R* gq1,
-                              R* gq2) {
+__global__ void k_trc_grad_pl(const __grid_constant__ TrcGradArgs<R> a) {
   int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= cD.KA * cD.LP) return;
   int k = t / cD.LP, lp = t % cD.LP;
+  const int n = (int)blockIdx.y;
   R qv[6];
   for (int v = 0; v < 6; ++v) {
     int p = ipl(v, k, lp);
-    qv[v] = rhogq[p] / rhog_t[p];
-    q[p] = qv[v];
+    qv[v] = a.rhogq[n][p] / a.rhog_t[p];
+    a.q[n][p] = qv[v];
   }
-  R* gq[3] = {gq0, gq1, gq2};
   for (int d = 0; d < 3; ++d) {
     R row = R(0.0);
     for (int v = 0; v < 6; ++v) {
       R tv = CG.coef_grad_pl[(v * cD.LP + lp) * 3 + d] * qv[v];
       row = (v == 0) ? tv : row + tv;
     }
-    gq[d][ipl(0, k, lp)] = row;
-    for (int v = 1; v < 6; ++v) gq[d][ipl(v, k, lp)] = R(0.0);
+    a.gq[n][d][ipl(0, k, lp)] = row;
+    for (int v = 1; v < 6; ++v) a.gq[n][d][ipl(v, k, lp)] = R(0.0);
   }
 }
 
 // ---------------------------------------------------------------------------
 // MIURA2004 face values of edges 0..2 (mod_src_tracer.py:1696-1787)
 // ---------------------------------------------------------------------------
+// One thread per point: the offsets of the face centroids from the two cells
+// of each face are formed once for the tracers of the batch.
 template <class R>
 struct TrcRemapArgs {
-  const R *q, *gq0, *gq1, *gq2;
+  const R *q[TRC_NB], *gq[TRC_NB][3];
   const R* xc[9];
   const R* cm[6];
-  R* qa[3];
+  R* qa[TRC_NB][3];
+  int nb;
 };
 
 template <class R>
-__device__ __forceinline__ R trc_rec(const TrcRemapArgs<R>& a, int ii, int jj, int k, int l, int pxc, int f) {
-  int q = ix(ii, jj, k, l);
-  R r = a.q[q];
-  r = r + a.gq0[q] * (a.xc[f * 3 + 0][pxc] - P2(CG.GRD_x, 0, ii, jj, l));
-  r = r + a.gq1[q] * (a.xc[f * 3 + 1][pxc] - P2(CG.GRD_x, 1, ii, jj, l));
-  r = r + a.gq2[q] * (a.xc[f * 3 + 2][pxc] - P2(CG.GRD_x, 2, ii, jj, l));
-  return r;
-}
-
-template <class R>
-__global__ void k_trc_remap(TrcRemapArgs<R> a) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l;
-  if (!col_of(t, i, j, l)) return;
+__global__ void k_trc_remap(const __grid_constant__ TrcRemapArgs<R> a) {
+  Pt c;
+  const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (!reg_point(p, c)) return;
   const int G = cD.G;
-  const bool ok = (i <= G - 2 && j <= G - 2);
-  for (int k = 0; k < cD.KA; ++k) {
-    int p = ix(i, j, k, l);
-    if (!ok) {
-      a.qa[0][p] = R(0.0); a.qa[1][p] = R(0.0); a.qa[2][p] = R(0.0);
-      continue;
+  if (c.i > G - 2 || c.j > G - 2) {
+    for (int n = 0; n < a.nb; ++n) a.qa[n][0][p] = a.qa[n][1][p] = a.qa[n][2][p] = R(0.0);
+    return;
+  }
+  const int mi[3] = {1, 1, 0}, mj[3] = {0, 1, 1};
+  const int pn[3] = {p + 1, p + G + 1, p + G};
+  R op[3][3], on[3][3], cf[3];   // offsets from the cell and from the face's other cell
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const R x = __ldg(a.xc[f * 3 + d] + p);
+      op[f][d] = x - P2c(CG.GRD_x, d, c.i, c.j, c.l);
+      on[f][d] = x - P2c(CG.GRD_x, d, c.i + mi[f], c.j + mj[f], c.l);
     }
-    const int mi[3] = {1, 1, 0}, mj[3] = {0, 1, 1};
+    cf[f] = __ldg(a.cm[f] + p);
+  }
+  for (int n = 0; n < a.nb; ++n) {
+    R v[3];
+    const R q0 = __ldg(a.q[n] + p), g0 = __ldg(a.gq[n][0] + p), g1 = __ldg(a.gq[n][1] + p), g2 = __ldg(a.gq[n][2] + p);
+#pragma unroll
     for (int f = 0; f < 3; ++f) {
-      R ap = trc_rec(a, i, j, k, l, p, f);
-      R am = trc_rec(a, i + mi[f], j + mj[f], k, l, p, f);
-      R c = a.cm[f][p];
-      a.qa[f][p] = c * am + (R(1.0) - c) * ap;
+      const int m = pn[f];
+      R ap = q0, am = __ldg(a.q[n] + m);
+      ap = ap + g0 * op[f][0];
+      ap = ap + g1 * op[f][1];
+      ap = ap + g2 * op[f][2];
+      am = am + __ldg(a.gq[n][0] + m) * on[f][0];
+      am = am + __ldg(a.gq[n][1] + m) * on[f][1];
+      am = am + __ldg(a.gq[n][2] + m) * on[f][2];
+      v[f] = cf[f] * am + (R(1.0) - cf[f]) * ap;
     }
+#pragma unroll
+    for (int f = 0; f < 3; ++f) a.qa[n][f][p] = v[f];
   }
 }
 
 template <class R>
 struct TrcRemapPlArgs {
-  const R *q, *gq0, *gq1, *gq2, *xc, *cm;
-  R* qa;
+  const R *q[TRC_NB], *gq[TRC_NB][3], *xc, *cm;
+  R* qa[TRC_NB];
 };
 
 template <class R>
-__global__ void k_trc_remap_pl(TrcRemapPlArgs<R> a) {
+__global__ void k_trc_remap_pl(const __grid_constant__ TrcRemapPlArgs<R> a) {
   int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= cD.KA * cD.LP) return;
   int k = t / cD.LP, lp = t % cD.LP;
+  const int n = (int)blockIdx.y;
   const R* X = CG.GRD_x_pl;
-  const R* gq[3] = {a.gq0, a.gq1, a.gq2};
   int p0 = ipl(0, k, lp);
   for (int v = 1; v <= 5; ++v) {
     int pv = ipl(v, k, lp);
-    R ap = a.q[p0];
-    for (int d = 0; d < 3; ++d) ap = ap + gq[d][p0] * (a.xc[pv * 3 + d] - X[(0 * cD.LP + lp) * 3 + d]);
-    R am = a.q[pv];
-    for (int d = 0; d < 3; ++d) am = am + gq[d][pv] * (a.xc[pv * 3 + d] - X[(v * cD.LP + lp) * 3 + d]);
+    R ap = a.q[n][p0];
+    for (int d = 0; d < 3; ++d) ap = ap + a.gq[n][d][p0] * (a.xc[pv * 3 + d] - X[(0 * cD.LP + lp) * 3 + d]);
+    R am = a.q[n][pv];
+    for (int d = 0; d < 3; ++d) am = am + a.gq[n][d][pv] * (a.xc[pv * 3 + d] - X[(v * cD.LP + lp) * 3 + d]);
     R c = a.cm[pv];
-    a.qa[pv] = c * am + (R(1.0) - c) * ap;
+    a.qa[n][pv] = c * am + (R(1.0) - c) * ap;
   }
 }
 
@@ -493,166 +537,169 @@ __global__ void k_trc_remap_pl(TrcRemapPlArgs<R> a) {
 // ---------------------------------------------------------------------------
 template <class R>
 struct TrcLimArgs {
-  const R *q, *rhog_t, *frhog;
+  const R *q[TRC_NB], *rhog_t, *frhog;
   const R* ch[6];
   const R* cm[6];
-  const R* qa[3];
-  const R *qout_min, *qout_max;
-  R *Qmin, *Qmax;          // Qout (output of the Qout kernel)
+  const R* qa[TRC_NB][3];
+  R *Qmin[TRC_NB], *Qmax[TRC_NB];   // Qout
   const R* flx[6];
-  R* rhogq;
+  R* rhogq[TRC_NB];
   R dt;
+  int nb;
 };
 
-// q_min / q_max over the stencil of edge f of cell (a,b) (mod_src_tracer.py:2191-2217)
+// The six faces of a cell (slots 0..2: its own faces 0..2; slots 3..5: faces
+// 0..2 of the cells behind it) touch the seven cells of its hexagon only,
+// numbered as the stencils' offsets (kNbI, kNbJ).  For each slot: the four cells
+// whose smallest and largest q bound the face, in the reference's order
+// (mod_src_tracer.py:2191-2217), the cell that owns the face and the other one.
+struct FaceCells {
+  int c[4], own, other;
+};
+__device__ __forceinline__ constexpr FaceCells face_cells(int m) {
+  return m == 0   ? FaceCells{{0, 6, 1, 2}, 0, 1}
+         : m == 1 ? FaceCells{{0, 1, 2, 3}, 0, 2}
+         : m == 2 ? FaceCells{{0, 2, 3, 4}, 0, 3}
+         : m == 3 ? FaceCells{{4, 5, 0, 3}, 4, 0}
+         : m == 4 ? FaceCells{{5, 6, 0, 4}, 5, 0}
+                  : FaceCells{{6, 1, 0, 5}, 6, 0};
+}
+// Smallest and largest q of face slot m.  sgp: the face at a singular point,
+// slot 4 of cell (1,1): np.min over [q(0,0), q(1,1), q(2,1), q(0,1)] (:2298-2323)
 template <class R>
-__device__ void trc_face_minmax(const R* q, int a, int b, int k, int l, int f, R& qn, R& qx) {
-  auto Q = [&](int ii, int jj) { return q[ix(ii, jj, k, l)]; };
-  R q0 = Q(a, b);
-  R q2 = Q(a + 1, b), q3 = Q(a + 1, b + 1), qj = Q(a, b + 1);
-  R v1, v2, v3;
-  if (f == 0) {
-    R q1 = (b > 0) ? Q(a, b - 1) : Q(0, 0);
-    v1 = q1; v2 = q2; v3 = q3;
-  } else if (f == 1) {
-    v1 = q2; v2 = q3; v3 = qj;
-  } else {
-    R q4 = (a > 0) ? Q(a - 1, b) : Q(0, 0);
-    v1 = q3; v2 = qj; v3 = q4;
-  }
+__device__ __forceinline__ void trc_face_minmax(const R q[7], int m, bool sgp, R& qn, R& qx) {
+  const FaceCells f = face_cells(m);
+  const R q0 = q[f.c[0]];
+  R v1 = q[f.c[1]], v2 = q[f.c[2]], v3 = q[f.c[3]];
+  if (m == 4 && sgp) { v1 = q[0]; v2 = q[1]; }
   qn = npmin(npmin(npmin(q0, v1), v2), v3);
   qx = npmax(npmax(npmax(q0, v1), v2), v3);
 }
-
-// Qin of slot m (0..5) of cell (i,j): slots 0..2 from the cell's own edges,
-// slots 3..5 from the neighbours' edges 0..2 (mod_src_tracer.py:2220-2234 and
-// the singular-point override :2298-2323)
+// The bounds that a face with the upwind mask c gives the cell it belongs to
+// (slots 0..2) and the cell behind it (slots 3..5) (mod_src_tracer.py:2220-2234)
 template <class R>
-__device__ void trc_qin(const TrcLimArgs<R>& a, int i, int j, int k, int l, int m, R& qin_min, R& qin_max) {
+__device__ __forceinline__ void trc_qin(R c, bool sgp, R qn, R qx, bool behind, R& qin_min, R& qin_max) {
   const R BIG = CC.HUGE_;
-  int ai = i, bj = j, f = m;
-  if (m >= 3) {
-    const int nbI[3] = {-1, -1, 0}, nbJ[3] = {0, -1, -1};
-    ai = i + nbI[m - 3];
-    bj = j + nbJ[m - 3];
-    f = m - 3;
+  if (!behind) {
+    qin_min = sgp ? ((c == R(1.0)) ? qn : BIG) : c * qn + (R(1.0) - c) * BIG;
+    qin_max = sgp ? ((c == R(1.0)) ? qx : -BIG) : c * qx + (R(1.0) - c) * (-BIG);
+  } else {
+    qin_min = sgp ? ((c == R(1.0)) ? BIG : qn) : c * BIG + (R(1.0) - c) * qn;
+    qin_max = sgp ? ((c == R(1.0)) ? -BIG : qx) : c * (-BIG) + (R(1.0) - c) * qx;
   }
-  R cmv = a.cm[f][ix(ai, bj, k, l)];
-  R qn, qx;
-  const bool sgp = CG.have_sgp[l] && ai == 0 && bj == 0 && f == 1;
-  if (sgp) {
-    auto Q = [&](int ii, int jj) { return a.q[ix(ii, jj, k, l)]; };
-    // np.min over [q(0,0), q(1,1), q(2,1), q(0,1)]
-    qn = npmin(npmin(npmin(Q(0, 0), Q(1, 1)), Q(2, 1)), Q(0, 1));
-    qx = npmax(npmax(npmax(Q(0, 0), Q(1, 1)), Q(2, 1)), Q(0, 1));
-    if (m < 3) {
-      qin_min = (cmv == R(1.0)) ? qn : BIG;
-      qin_max = (cmv == R(1.0)) ? qx : -BIG;
-    } else {
-      qin_min = (cmv == R(1.0)) ? BIG : qn;
-      qin_max = (cmv == R(1.0)) ? -BIG : qx;
-    }
+}
+// offset of cell n of the hexagon, and the owner of face slot m
+__device__ __forceinline__ int hex_off(int n) { return kNbI[n] + kNbJ[n] * cD.G; }
+
+// Outflow bounds, one thread per point; the Courant numbers and masks are read
+// once for the tracers of the batch.
+template <class R>
+__global__ void k_trc_qout(const __grid_constant__ TrcLimArgs<R> a) {
+  Pt t;
+  const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (!reg_point(p, t)) return;
+  if (!interior(t.i, t.j)) {
+    for (int n = 0; n < a.nb; ++n) a.Qmin[n][p] = a.Qmax[n][p] = a.q[n][p];
     return;
   }
-  trc_face_minmax(a.q, ai, bj, k, l, f, qn, qx);
-  if (m < 3) {
-    qin_min = cmv * qn + (R(1.0) - cmv) * BIG;
-    qin_max = cmv * qx + (R(1.0) - cmv) * (-BIG);
-  } else {
-    qin_min = cmv * BIG + (R(1.0) - cmv) * qn;
-    qin_max = cmv * (-BIG) + (R(1.0) - cmv) * qx;
-  }
-}
-
-template <class R>
-__global__ void k_trc_qout(TrcLimArgs<R> a) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l;
-  if (!col_of(t, i, j, l)) return;
-  const bool in = interior(i, j);
   const R EPS = CC.EPS;
-  for (int k = 0; k < cD.KA; ++k) {
-    int p = ix(i, j, k, l);
-    R qc = a.q[p];
-    if (!in) {
-      a.Qmin[p] = qc;
-      a.Qmax[p] = qc;
-      continue;
-    }
+  R ch[6], cm[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    ch[m] = __ldg(a.ch[m] + p);
+    cm[m] = __ldg(a.cm[m % 3] + p + hex_off(face_cells(m).own));
+  }
+  const bool sgp = CG.have_sgp[t.l] && t.i == 1 && t.j == 1;
+  const R d = R(1.0) * __ldg(a.frhog + p) / __ldg(a.rhog_t + p) * a.dt;
+  for (int n = 0; n < a.nb; ++n) {
+    R q[7];
+#pragma unroll
+    for (int m = 0; m < 7; ++m) q[m] = __ldg(a.q[n] + p + hex_off(m));
+    const R qc = q[0];
     R qnmin = qc, qnmax = qc;
     R Cin = R(0.0), Cout = R(0.0), CQmin = R(0.0), CQmax = R(0.0);
+#pragma unroll
     for (int m = 0; m < 6; ++m) {
-      R qi, qx;
-      trc_qin(a, i, j, k, l, m, qi, qx);
+      R qn, qx, qi, qxi;
+      const bool s = m == 4 && sgp;
+      trc_face_minmax(q, m, s, qn, qx);
+      trc_qin(cm[m], s, qn, qx, m >= 3, qi, qxi);
       qnmin = npmin(qnmin, qi);
-      qnmax = npmax(qnmax, qx);
-      R chv = a.ch[m][p];
-      R chm = npmin(chv, R(0.0));
+      qnmax = npmax(qnmax, qxi);
+      const R chm = npmin(ch[m], R(0.0));
       if (m == 0) {
-        Cin = chm; Cout = chv - chm; CQmin = chm * qi; CQmax = chm * qx;
+        Cin = chm; Cout = ch[m] - chm; CQmin = chm * qi; CQmax = chm * qxi;
       } else {
-        Cin = Cin + chm; Cout = Cout + (chv - chm); CQmin = CQmin + chm * qi; CQmax = CQmax + chm * qx;
+        Cin = Cin + chm; Cout = Cout + (ch[m] - chm); CQmin = CQmin + chm * qi; CQmax = CQmax + chm * qxi;
       }
     }
-    R zsw = R(0.5) - copysign(R(0.5), fabs(Cout) - EPS);
-    R d = R(1.0) * a.frhog[p] / a.rhog_t[p] * a.dt;
-    a.Qmin[p] = (qc - CQmax - qnmax * (R(1.0) - Cin - Cout + d)) / (Cout + zsw) * (R(1.0) - zsw) + qc * zsw;
-    a.Qmax[p] = (qc - CQmin - qnmin * (R(1.0) - Cin - Cout + d)) / (Cout + zsw) * (R(1.0) - zsw) + qc * zsw;
+    const R zsw = R(0.5) - copysign(R(0.5), fabs(Cout) - EPS);
+    const typename DivOf<R>::type den(Cout + zsw);
+    a.Qmin[n][p] = den(qc - CQmax - qnmax * (R(1.0) - Cin - Cout + d)) * (R(1.0) - zsw) + qc * zsw;
+    a.Qmax[n][p] = den(qc - CQmin - qnmin * (R(1.0) - Cin - Cout + d)) * (R(1.0) - zsw) + qc * zsw;
   }
 }
 
-// limited value of edge f in {0,1,2} of cell (ai,bj) (mod_src_tracer.py:2545-2605)
+// Limited face values (mod_src_tracer.py:2545-2605) and the flux update, one
+// thread per point: the cell limits its six faces from the q and outflow bounds
+// of its hexagon, each face's extremes formed once for both cells' bounds.
+// (A tile that shares the faces through shared memory was slower for one tracer,
+// 0.94 against 0.62 ms at gl08 mixed: two barriers and 22 KB a block.)
 template <class R>
-__device__ R trc_limited_face(const TrcLimArgs<R>& a, int ai, int bj, int k, int l, int f) {
-  const int mi[3] = {1, 1, 0}, mj[3] = {0, 1, 1};
-  int ni = ai + mi[f], nj = bj + mj[f];
-  int p = ix(ai, bj, k, l), pn = ix(ni, nj, k, l);
-  R c = a.cm[f][p];
-  R qa = a.qa[f][p];
-  R qi0, qx0, qi1, qx1;
-  trc_qin(a, ai, bj, k, l, f, qi0, qx0);
-  trc_qin(a, ni, nj, k, l, 3 + f, qi1, qx1);
-  qa = c * npmin(npmax(qa, qi0), qx0) + (R(1.0) - c) * npmin(npmax(qa, qi1), qx1);
-  qa = c * npmax(npmin(qa, a.qout_max[pn]), a.qout_min[pn]) + (R(1.0) - c) * npmax(npmin(qa, a.qout_max[p]), a.qout_min[p]);
-  return qa;
-}
-
-template <class R>
-__global__ void k_trc_apply(TrcLimArgs<R> a) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l;
-  if (!col_of(t, i, j, l)) return;
-  if (!interior(i, j)) return;
-  for (int k = 0; k < cD.KA; ++k) {
-    int p = ix(i, j, k, l);
-    R q0 = trc_limited_face(a, i, j, k, l, 0);
-    R q1 = trc_limited_face(a, i, j, k, l, 1);
-    R q2 = trc_limited_face(a, i, j, k, l, 2);
-    R q3 = trc_limited_face(a, i - 1, j, k, l, 0);
-    R q4 = trc_limited_face(a, i - 1, j - 1, k, l, 1);
-    R q5 = trc_limited_face(a, i, j - 1, k, l, 2);
-    R upd = a.flx[0][p] * q0 + a.flx[1][p] * q1 + a.flx[2][p] * q2 + a.flx[3][p] * q3 + a.flx[4][p] * q4 +
-                 a.flx[5][p] * q5;
-    a.rhogq[p] = a.rhogq[p] - upd;
+__global__ void k_trc_apply(const __grid_constant__ TrcLimArgs<R> a) {
+  Pt t;
+  const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (!reg_point(p, t) || !interior(t.i, t.j)) return;
+  const bool sgp = CG.have_sgp[t.l] && t.i == 1 && t.j == 1;
+  R fl[6], cm[6];
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    fl[m] = __ldg(a.flx[m] + p);
+    cm[m] = __ldg(a.cm[m % 3] + p + hex_off(face_cells(m).own));
+  }
+  for (int n = 0; n < a.nb; ++n) {
+    R q[7], lo[7], hi[7], v[6];
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {
+      q[m] = __ldg(a.q[n] + p + hex_off(m));
+      lo[m] = __ldg(a.Qmin[n] + p + hex_off(m));
+      hi[m] = __ldg(a.Qmax[n] + p + hex_off(m));
+    }
+#pragma unroll
+    for (int m = 0; m < 6; ++m) v[m] = __ldg(a.qa[n][m % 3] + p + hex_off(face_cells(m).own));
+    R upd = R(0.0);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+      const FaceCells f = face_cells(m);
+      const bool s = m == 4 && sgp;
+      R qn, qx, i0n, i0x, i1n, i1x;
+      trc_face_minmax(q, m, s, qn, qx);
+      const R c = cm[m];
+      trc_qin(c, s, qn, qx, false, i0n, i0x);
+      trc_qin(c, s, qn, qx, true, i1n, i1x);
+      R x = c * npmin(npmax(v[m], i0n), i0x) + (R(1.0) - c) * npmin(npmax(v[m], i1n), i1x);
+      x = c * npmax(npmin(x, hi[f.other]), lo[f.other]) + (R(1.0) - c) * npmax(npmin(x, hi[f.own]), lo[f.own]);
+      upd = m ? upd + fl[m] * x : fl[m] * x;
+    }
+    a.rhogq[n][p] = a.rhogq[n][p] - upd;
   }
 }
 
 // pole Qout (mod_src_tracer.py:2437-2495) at g = 0
 template <class R>
 struct TrcLimPlArgs {
-  const R *q, *ch, *cm, *rhog_t, *frhog, *qa, *flx;
-  R *Qmin, *Qmax;
-  const R *qout_min, *qout_max;
-  R* rhogq;
+  const R *q_of[TRC_NB], *ch, *cm, *rhog_t, *frhog, *qa[TRC_NB], *flx;
+  R *Qmin[TRC_NB], *Qmax[TRC_NB];
+  R* rhogq[TRC_NB];
   R dt;
 };
 
 template <class R>
-__device__ void trc_qin_pl(const TrcLimPlArgs<R>& a, int v, int k, int lp, R& in0n, R& in1n, R& in0x,
+__device__ void trc_qin_pl(const TrcLimPlArgs<R>& a, const R* q, int v, int k, int lp, R& in0n, R& in1n, R& in0x,
                            R& in1x) {
   const R BIG = CC.HUGE_;
   int vp1 = (v + 1 > 5) ? 1 : v + 1, vm1 = (v - 1 < 1) ? 5 : v - 1;
-  R q0 = a.q[ipl(0, k, lp)], qv = a.q[ipl(v, k, lp)], qm = a.q[ipl(vm1, k, lp)], qp = a.q[ipl(vp1, k, lp)];
+  R q0 = q[ipl(0, k, lp)], qv = q[ipl(v, k, lp)], qm = q[ipl(vm1, k, lp)], qp = q[ipl(vp1, k, lp)];
   R qn = pymin(pymin(pymin(q0, qv), qm), qp);
   R qx = pymax(pymax(pymax(q0, qv), qm), qp);
   R c = a.cm[ipl(v, k, lp)];
@@ -663,15 +710,17 @@ __device__ void trc_qin_pl(const TrcLimPlArgs<R>& a, int v, int k, int lp, R& in
 }
 
 template <class R>
-__global__ void k_trc_qout_pl(TrcLimPlArgs<R> a) {
+__global__ void k_trc_qout_pl(const __grid_constant__ TrcLimPlArgs<R> a) {
   int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= cD.KA * cD.LP) return;
   int k = t / cD.LP, lp = t % cD.LP;
   int p0 = ipl(0, k, lp);
-  R qnm = a.q[p0], qnx = a.q[p0];
+  const int n = (int)blockIdx.y;   // the tracer of the batch
+  const R* q = a.q_of[n];
+  R qnm = q[p0], qnx = q[p0];
   R in0n[6], in0x[6], d1, d2;
   for (int v = 1; v <= 5; ++v) {
-    trc_qin_pl(a, v, k, lp, in0n[v], d1, in0x[v], d2);
+    trc_qin_pl(a, q, v, k, lp, in0n[v], d1, in0x[v], d2);
     qnm = pymin(qnm, in0n[v]);
     qnx = pymax(qnx, in0x[v]);
   }
@@ -687,34 +736,36 @@ __global__ void k_trc_qout_pl(TrcLimPlArgs<R> a) {
   R zs = R(0.5) - copysign(R(0.5), fabs(Co) - CC.EPS);
   R den = Co + zs;
   R fac = R(1.0) - zs;
-  R q0 = a.q[p0];
+  R q0 = q[p0];
   R dv = R(1.0) * a.frhog[p0] / a.rhog_t[p0] * a.dt;
-  a.Qmin[p0] = (q0 - CQx - qnx * (R(1.0) - Ci - Co + dv)) / den * fac + q0 * zs;
-  a.Qmax[p0] = (q0 - CQn - qnm * (R(1.0) - Ci - Co + dv)) / den * fac + q0 * zs;
+  a.Qmin[n][p0] = (q0 - CQx - qnx * (R(1.0) - Ci - Co + dv)) / den * fac + q0 * zs;
+  a.Qmax[n][p0] = (q0 - CQn - qnm * (R(1.0) - Ci - Co + dv)) / den * fac + q0 * zs;
 }
 
 template <class R>
-__global__ void k_trc_apply_pl(TrcLimPlArgs<R> a) {
+__global__ void k_trc_apply_pl(const __grid_constant__ TrcLimPlArgs<R> a) {
   int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= cD.KA * cD.LP) return;
   int k = t / cD.LP, lp = t % cD.LP;
   int p0 = ipl(0, k, lp);
-  R acc = a.rhogq[p0];
+  const int n = (int)blockIdx.y;   // the tracer of the batch
+  const R* q = a.q_of[n];
+  R acc = a.rhogq[n][p0];
   for (int v = 1; v <= 5; ++v) {
     int pv = ipl(v, k, lp);
     R in0n, in1n, in0x, in1x;
-    trc_qin_pl(a, v, k, lp, in0n, in1n, in0x, in1x);
+    trc_qin_pl(a, q, v, k, lp, in0n, in1n, in0x, in1x);
     R c = a.cm[pv];
-    R x = a.qa[pv];
+    R x = a.qa[n][pv];
     R a0 = npmin(npmax(x, in0n), in0x);
     R a1 = npmin(npmax(x, in1n), in1x);
     x = c * a0 + (R(1.0) - c) * a1;
-    R a2 = npmax(npmin(x, a.qout_max[pv]), a.qout_min[pv]);
-    R a3 = npmax(npmin(x, a.qout_max[p0]), a.qout_min[p0]);
+    R a2 = npmax(npmin(x, a.Qmax[n][pv]), a.Qmin[n][pv]);
+    R a3 = npmax(npmin(x, a.Qmax[n][p0]), a.Qmin[n][p0]);
     x = c * a2 + (R(1.0) - c) * a3;
     acc = acc - a.flx[pv] * x;
   }
-  a.rhogq[p0] = acc;
+  a.rhogq[n][p0] = acc;
 }
 
 // density after the horizontal step (mod_src_tracer.py:890-916)
@@ -722,17 +773,14 @@ template <class R>
 __global__ void k_trc_rhog(R* rhog_t, const R* f0, const R* f1, const R* f2, const R* f3,
                            const R* f4, const R* f5, const R* frhog, R dt, const R* flx_pl,
                            R* rhog_t_pl, const R* frhog_pl) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l;
-  if (col_of(t, i, j, l)) {
-    if (!interior(i, j)) return;
-    for (int k = 0; k < cD.KA; ++k) {
-      int p = ix(i, j, k, l);
-      R s = f0[p] + f1[p] + f2[p] + f3[p] + f4[p] + f5[p];
-      rhog_t[p] = rhog_t[p] - (s - (R(1.0) * frhog[p] * dt));
-    }
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  Pt q;
+  if (reg_point(t, q)) {
+    if (!interior(q.i, q.j)) return;
+    const R s = __ldg(f0 + t) + __ldg(f1 + t) + __ldg(f2 + t) + __ldg(f3 + t) + __ldg(f4 + t) + __ldg(f5 + t);
+    rhog_t[t] = rhog_t[t] - (s - (R(1.0) * __ldg(frhog + t) * dt));
   } else {
-    int tp = t - cD.npt2i;
+    int tp = t - cD.npti;
     if (tp < cD.KA * cD.LP) {
       int k = (int)(tp / cD.LP), lp = (int)(tp % cD.LP);
       int p0 = ipl(0, k, lp);

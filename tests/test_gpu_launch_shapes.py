@@ -8,6 +8,8 @@ remainders of its splits (B200).
   k_vi_col) against 17 of them stacked in one handle (174,080 columns, above one
   wave of the column kernel: whole marches, k_vi_solve and k_vi_energy_p): each
   member bit for bit, in both forms.
+* Tracers in batches: every tracer of 6 (batches of 4 and 2) equals the same
+  tracer carried alone, bit for bit.
 """
 import importlib
 
@@ -65,3 +67,35 @@ def test_one_grid_equals_its_stack(pkg, prec):
     got = ens.unstack_states(*run(ens.stack_setup(geo, n), *ens.stack_states([(m, mp)] * n)), n)
     for x, xp in (got[0], got[n // 2], got[-1]):
         assert np.array_equal(x, lone) and np.array_equal(xp, lone_pl)
+
+
+@pytest.mark.parametrize("prec", ["float64", "mixed"])
+def test_tracer_batches_equal_lone_tracers(pkg, prec):
+    g = _ig().Grid(4, vlayer=11, ztop=12000.0, device="cuda", layer="EVEN", topo="NONE")
+    rng = np.random.default_rng(8)
+    amp, lon0 = rng.uniform(0.2, 1.0, 6), rng.uniform(0.0, 6.0, 6)
+
+    def fields(which):
+        def f(lon, lat, z):
+            lo, la = lon[..., None], lat[..., None]
+            q = [np.zeros(z.shape)]
+            for n in which:
+                r = np.arccos(np.clip(np.cos(la) * np.cos(lo - lon0[n]), -1.0, 1.0))
+                q.append(np.where(r < 0.6, amp[n], 0.1) * (1.0 + 0.1 * np.sin(z / 3000.0)))
+            return np.stack(q, axis=-1)
+        return f
+
+    def run(which):
+        geo = g.setup(dtl=600.0, gamma=9.6e16, nq=1 + len(which), trcadv=True)
+        s, sp = g.trcadv_state(fields(which))
+        c = pkg.NicamCuda(geo, graph=True, precision=prec)
+        try:
+            c.upload(s, sp)
+            c.step(2)
+            return c.download()
+        finally:
+            c.close()
+    s, sp = run(range(5))          # 6 with the vapour slot
+    for n in range(5):
+        a, ap = run([n])
+        assert np.array_equal(s[..., 7 + n], a[..., 7]) and np.array_equal(sp[..., 7 + n], ap[..., 7]), n
