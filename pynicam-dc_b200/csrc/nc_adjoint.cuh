@@ -501,91 +501,93 @@ __device__ void qout_lin(const HLin& a, int i, int j, int k, int l, QoutLin& o) 
   o.fz = o.f + zsw;
 }
 
-__global__ void k_hlin_qout(HLin a, int adjoint) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  int i, j, l;
-  if (!col_of(t, i, j, l)) return;
-  const bool in = interior(i, j);
-  for (int k = 0; k < cD.KA; ++k) {
-    const int p = ix(i, j, k, l);
-    if (!in) {   // Qmin = Qmax = q
-      if (adjoint) atomicAdd(&a.gq[p], a.gQmin[p] + a.gQmax[p]);
-      else { a.oQmin[p] = a.dq[p]; a.oQmax[p] = a.dq[p]; }
-      continue;
+// One thread per point (as the two kernels that follow): nothing links the levels.
+__global__ void k_hlin_qout(const __grid_constant__ HLin a, int adjoint) {
+  const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  Pt c;
+  if (!reg_point(p, c)) return;
+  if (!interior(c.i, c.j)) {   // Qmin = Qmax = q
+    if (adjoint) atomicAdd(&a.gq[p], a.gQmin[p] + a.gQmax[p]);
+    else { a.oQmin[p] = a.dq[p]; a.oQmax[p] = a.dq[p]; }
+    return;
+  }
+  QoutLin o;
+  qout_lin(a, c.i, c.j, c.k, c.l, o);
+  if (!adjoint) {
+    double cqmin = 0.0, cqmax = 0.0;
+    for (int m = 0; m < 6; ++m) {
+      cqmin += o.chm[m] * src_tl(a, o.imin[m]);
+      cqmax += o.chm[m] * src_tl(a, o.imax[m]);
     }
-    QoutLin o;
-    qout_lin(a, i, j, k, l, o);
-    if (!adjoint) {
-      double cqmin = 0.0, cqmax = 0.0;
-      for (int m = 0; m < 6; ++m) {
-        cqmin += o.chm[m] * src_tl(a, o.imin[m]);
-        cqmax += o.chm[m] * src_tl(a, o.imax[m]);
-      }
-      a.oQmin[p] = o.fz * a.dq[p] - o.f * cqmax - o.f * o.B * src_tl(a, o.nmax);
-      a.oQmax[p] = o.fz * a.dq[p] - o.f * cqmin - o.f * o.B * src_tl(a, o.nmin);
-    } else {
-      const double gn = a.gQmin[p], gx = a.gQmax[p];
-      atomicAdd(&a.gq[p], o.fz * (gn + gx));
-      for (int m = 0; m < 6; ++m) {
-        src_ad(a, o.imax[m], -o.f * o.chm[m] * gn);
-        src_ad(a, o.imin[m], -o.f * o.chm[m] * gx);
-      }
-      src_ad(a, o.nmax, -o.f * o.B * gn);
-      src_ad(a, o.nmin, -o.f * o.B * gx);
+    a.oQmin[p] = o.fz * a.dq[p] - o.f * cqmax - o.f * o.B * src_tl(a, o.nmax);
+    a.oQmax[p] = o.fz * a.dq[p] - o.f * cqmin - o.f * o.B * src_tl(a, o.nmin);
+  } else {
+    const double gn = a.gQmin[p], gx = a.gQmax[p];
+    if (gn == 0.0 && gx == 0.0) return;   // no limited face takes this cell's bounds: it adds zeros
+    atomicAdd(&a.gq[p], o.fz * (gn + gx));
+    for (int m = 0; m < 6; ++m) {
+      src_ad(a, o.imax[m], -o.f * o.chm[m] * gn);
+      src_ad(a, o.imin[m], -o.f * o.chm[m] * gx);
     }
+    src_ad(a, o.nmax, -o.f * o.B * gn);
+    src_ad(a, o.nmin, -o.f * o.B * gx);
   }
 }
 
 // the flux update of the interior cells (k_trc_apply): y = x - sum flx_f v_f
-__global__ void k_hlin_apply(HLin a, int adjoint) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  int i, j, l;
-  if (!col_of(t, i, j, l)) return;
-  const bool in = interior(i, j);
-  for (int k = 0; k < cD.KA; ++k) {
-    const int p = ix(i, j, k, l);
-    if (!in) {
-      if (!adjoint) a.y[p] = a.x[p];
-      continue;
-    }
-    const Src s[6] = {limited_face_src(a, i, j, k, l, 0),     limited_face_src(a, i, j, k, l, 1),
-                      limited_face_src(a, i, j, k, l, 2),     limited_face_src(a, i - 1, j, k, l, 0),
-                      limited_face_src(a, i - 1, j - 1, k, l, 1), limited_face_src(a, i, j - 1, k, l, 2)};
-    if (!adjoint) {
-      double upd = 0.0;
-      for (int f = 0; f < 6; ++f) upd += a.flx[f][p] * src_tl(a, s[f]);
-      a.y[p] = a.x[p] - upd;
-    } else {
-      const double g = a.x[p];
-      for (int f = 0; f < 6; ++f) src_ad(a, s[f], -a.flx[f][p] * g);
-    }
+__global__ void k_hlin_apply(const __grid_constant__ HLin a, int adjoint) {
+  const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  Pt t;
+  if (!reg_point(p, t)) return;
+  if (!interior(t.i, t.j)) {
+    if (!adjoint) a.y[p] = a.x[p];
+    return;
+  }
+  const int i = t.i, j = t.j, k = t.k, l = t.l;
+  const Src s[6] = {limited_face_src(a, i, j, k, l, 0),     limited_face_src(a, i, j, k, l, 1),
+                    limited_face_src(a, i, j, k, l, 2),     limited_face_src(a, i - 1, j, k, l, 0),
+                    limited_face_src(a, i - 1, j - 1, k, l, 1), limited_face_src(a, i, j - 1, k, l, 2)};
+  if (!adjoint) {
+    double upd = 0.0;
+    for (int f = 0; f < 6; ++f) upd += a.flx[f][p] * src_tl(a, s[f]);
+    a.y[p] = a.x[p] - upd;
+  } else {
+    const double g = a.x[p];
+    for (int f = 0; f < 6; ++f) src_ad(a, s[f], -a.flx[f][p] * g);
   }
 }
 
-// MIURA2004 face values (k_trc_remap), adjoint: scatter into gq and the gradient cotangents
-__global__ void k_hlin_remap_ad(HLin a) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  int i, j, l;
-  if (!col_of(t, i, j, l)) return;
+// MIURA2004 face values (k_trc_remap), adjoint: each cell gathers from its
+// three faces and from the three whose other cell it is, so the gradient
+// cotangents are written, not accumulated
+__global__ void k_hlin_remap_ad(const __grid_constant__ HLin a) {
+  const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  Pt t;
+  if (!reg_point(p, t)) return;
   const int G = cD.G;
-  if (i > G - 2 || j > G - 2) return;
   const int mi[3] = {1, 1, 0}, mj[3] = {0, 1, 1};
-  for (int k = 0; k < cD.KA; ++k) {
-    const int p = ix(i, j, k, l);
-    for (int f = 0; f < 3; ++f) {
-      const double g = a.gqa[f][p];
-      if (g == 0.0) continue;
-      const double c = a.cm[f][p];
-      const int ni = i + mi[f], nj = j + mj[f], pn = ix(ni, nj, k, l);
-      atomicAdd(&a.gq[p], (1.0 - c) * g);
-      atomicAdd(&a.gq[pn], c * g);
-      for (int d = 0; d < 3; ++d) {
-        const double xcv = a.xc[f * 3 + d][p];
-        atomicAdd(&a.gg[d][p], (1.0 - c) * g * (xcv - P2(cG.GRD_x, d, i, j, l)));
-        atomicAdd(&a.gg[d][pn], c * g * (xcv - P2(cG.GRD_x, d, ni, nj, l)));
-      }
-    }
+  const double X[3] = {P2(cG.GRD_x, 0, t.i, t.j, t.l), P2(cG.GRD_x, 1, t.i, t.j, t.l), P2(cG.GRD_x, 2, t.i, t.j, t.l)};
+  double gq = 0.0, gg[3] = {0.0, 0.0, 0.0};
+  auto take = [&](int pf, int f, bool behind) {   // face f of cell pf
+    const double g = a.gqa[f][pf], c = a.cm[f][pf];
+    const double w = behind ? c * g : (1.0 - c) * g;
+    if (w == 0.0) return;
+    gq += w;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) gg[d] += w * (a.xc[f * 3 + d][pf] - X[d]);
+  };
+  if (t.i <= G - 2 && t.j <= G - 2) {
+#pragma unroll
+    for (int f = 0; f < 3; ++f) take(p, f, false);
   }
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+    const int bi = t.i - mi[f], bj = t.j - mj[f];
+    if (bi >= 0 && bj >= 0 && bi <= G - 2 && bj <= G - 2) take(p - mi[f] - mj[f] * G, f, true);
+  }
+  a.gq[p] += gq;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) a.gg[d][p] = gg[d];
 }
 
 // gradient (k_trc_grad_t) adjoint on the interior cells, then x-bar +=

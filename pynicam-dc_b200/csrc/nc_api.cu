@@ -1406,7 +1406,7 @@ static int hlin_tl(nc_handle* h) {
   const Dims& D = h->D;
   FieldPair* L = h->lin;
   const cudaStream_t s = h->stream;
-  const unsigned pkb = (unsigned)((D.KA * D.LP + 127) / 128), cb = (unsigned)((D.npt2 + 127) / 128);
+  const unsigned pkb = (unsigned)((D.KA * D.LP + 127) / 128), cb = (unsigned)((D.npt + 127) / 128);
   {
     const dim3 gt((unsigned)D.KA, (unsigned)(((D.G - 2 + TG_DX - 1) / TG_DX) * ((D.G - 2 + TG_DY - 1) / TG_DY)),
                   (unsigned)D.L);
@@ -1455,8 +1455,10 @@ static int hlin_ad(nc_handle* h) {
   const Dims& D = h->D;
   FieldPair* L = h->lin;
   const cudaStream_t s = h->stream;
-  const unsigned pkb = (unsigned)((D.KA * D.LP + 127) / 128), cb = (unsigned)((D.npt2 + 127) / 128);
-  for (int n : {LN_DQ, LN_DG0, LN_DG1, LN_DG2, LN_DQA0, LN_DQA1, LN_DQA2, LN_DQN, LN_DQX}) TRY(zero_pair(h, L[n]));
+  const unsigned pkb = (unsigned)((D.KA * D.LP + 127) / 128), cb = (unsigned)((D.npt + 127) / 128);
+  for (int n : {LN_DQ, LN_DQA0, LN_DQA1, LN_DQA2, LN_DQN, LN_DQX}) TRY(zero_pair(h, L[n]));
+  for (int d = 0; d < 3; ++d)   // the regional part is written by k_hlin_remap_ad
+    CU(cudaMemsetAsync(L[LN_DG0 + d].p, 0, D.npl * sizeof(double), s));
   TRY(copy_in(h, L[LN_T2], L[LN_T1].r, L[LN_T1].p));   // y = x - ...: the direct part
   HLin a = hlin_args(h);
   a.x = L[LN_T1].r; a.x_pl = L[LN_T1].p;
