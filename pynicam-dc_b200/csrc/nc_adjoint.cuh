@@ -27,7 +27,12 @@ namespace nc {
 #define NC_ADJ_K 64
 
 // ---------------------------------------------------------------------------
-// tridiagonal solve and its transpose, one thread per regional column
+// tridiagonal solve and its transpose: a block takes 32 columns (a lane each),
+// its warps read the operands of the levels into shared memory (four doubles a
+// level and column, 43 KB at 42 levels), warp 0 walks the two sweeps, and the
+// warps write the solution and the matrix cotangents.  (A thread per column
+// waited for memory at every level and kept the sweep's factors in local
+// memory.)
 // ---------------------------------------------------------------------------
 struct TriArgs {
   const double *Mc, *Mu, *Ml, *b;
@@ -40,41 +45,71 @@ struct TriArgs {
   int transpose;
 };
 
-__device__ void tri_column(const Col c, const TriArgs& a) {
-  const int k0 = cD.kmin + 1, N = cD.kmax - cD.kmin, KA = cD.KA;
-  // row n: lo(n) x[n-1] + Mc[n] x[n] + up(n) x[n+1] = b[n]
-  auto lo = [&](int n) { return a.transpose ? a.Mu[c.at(k0 + n - 1)] : a.Ml[c.at(k0 + n)]; };
-  auto up = [&](int n) { return a.transpose ? a.Ml[c.at(k0 + n + 1)] : a.Mu[c.at(k0 + n)]; };
-  double u[NC_ADJ_K], gam[NC_ADJ_K];
-  double beta = a.Mc[c.at(k0)];
-  u[0] = a.b[c.at(k0)] / beta;
-  for (int n = 1; n < N; ++n) {
-    gam[n] = up(n - 1) / beta;
-    beta = a.Mc[c.at(k0 + n)] - lo(n) * gam[n];
-    u[n] = (a.b[c.at(k0 + n)] - lo(n) * u[n - 1]) / beta;
-  }
-  for (int n = N - 2; n >= 0; --n) u[n] = u[n] - gam[n + 1] * u[n + 1];
-  for (int k = 0; k < KA; ++k) a.x[c.at(k)] = (k >= k0 && k < k0 + N) ? u[k - k0] : 0.0;
-  if (!a.x_fwd) return;
-  for (int k = 0; k < KA; ++k) {
-    const int n = k - k0;
-    double gc = 0.0, gu = 0.0, gl = 0.0;
-    if (n >= 0 && n < N) {
-      gc = -u[n] * a.x_fwd[c.at(k)];
-      if (n + 1 < N) gu = -u[n] * a.x_fwd[c.at(k + 1)];
-      if (n > 0) gl = -u[n] * a.x_fwd[c.at(k - 1)];
-    }
-    a.gMc[c.at(k)] = gc;
-    a.gMu[c.at(k)] = gu;
-    a.gMl[c.at(k)] = gl;
-  }
-}
+#define TRI_W 8
+static inline size_t tri_smem(int rows) { return (size_t)4 * rows * 32 * sizeof(double); }
 
-__global__ void k_tri_solve(TriArgs a, int pole) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(32 * TRI_W) k_tri_solve(const __grid_constant__ TriArgs a, int pole) {
+  extern __shared__ __align__(16) double tri_sm[];
+  const int k0 = cD.kmin + 1, N = cD.kmax - cD.kmin, KA = cD.KA;
+  const int lane = (int)(threadIdx.x % 32), w = (int)(threadIdx.x / 32);
+  const int ncol = pole ? 6 * cD.LP : cD.npt2i;
+  const int t0 = (int)blockIdx.x * 32 + lane;
+  const bool act = t0 < ncol;     // surplus lanes repeat the last column and store nothing
   int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  tri_column(pole ? col_pl(g, lp) : col_reg(i, j, l), a);
+  map_col(pole, act ? t0 : ncol - 1, i, j, l, g, lp);
+  const Col c = pole ? col_pl(g, lp) : col_reg(i, j, l);
+  double* s_lo = tri_sm + lane;            // sub-diagonal, then gamma
+  double* s_mc = s_lo + N * 32;
+  double* s_up = s_mc + N * 32;
+  double* s_u = s_up + N * 32;             // right-hand side, then the solution
+  // row n: lo(n) x[n-1] + Mc[n] x[n] + up(n) x[n+1] = b[n]
+  for (int n = w; n < N; n += TRI_W) {
+    const int p = c.at(k0 + n);
+    s_lo[n * 32] = n ? (a.transpose ? __ldg(a.Mu + c.at(k0 + n - 1)) : __ldg(a.Ml + p)) : 0.0;
+    s_mc[n * 32] = __ldg(a.Mc + p);
+    s_up[n * 32] = n + 1 < N ? (a.transpose ? __ldg(a.Ml + c.at(k0 + n + 1)) : __ldg(a.Mu + p)) : 0.0;
+    s_u[n * 32] = __ldg(a.b + p);
+  }
+  __syncthreads();
+  if (w == 0) {
+    double beta = s_mc[0], up = s_up[0], u = s_u[0] / beta;
+    s_u[0] = u;
+    double lo = s_lo[min(1, N - 1) * 32], mc_ = s_mc[min(1, N - 1) * 32], b = s_u[min(1, N - 1) * 32];
+    double upn = s_up[min(1, N - 1) * 32];
+    for (int n = 1; n < N; ++n) {          // the operands of row n+1 are read before row n is stored
+      const int m = min(n + 1, N - 1) * 32;
+      const double lo1 = s_lo[m], mc1 = s_mc[m], b1 = s_u[m], up1 = s_up[m];
+      const double gam = up / beta;
+      beta = mc_ - lo * gam;
+      u = (b - lo * u) / beta;
+      s_lo[n * 32] = gam;
+      s_u[n * 32] = u;
+      up = upn; upn = up1; lo = lo1; mc_ = mc1; b = b1;
+    }
+    for (int n = N - 2; n >= 0; --n) {
+      u = s_u[n * 32] - s_lo[(n + 1) * 32] * u;
+      s_u[n * 32] = u;
+    }
+  }
+  __syncthreads();
+  if (!act) return;
+  for (int k = w; k < KA; k += TRI_W) {
+    const int n = k - k0, p = c.at(k);
+    const bool in = n >= 0 && n < N;
+    const double u = in ? s_u[n * 32] : 0.0;
+    if (a.x_fwd) {
+      double gc = 0.0, gu = 0.0, gl = 0.0;
+      if (in) {
+        gc = -u * __ldg(a.x_fwd + p);
+        if (n + 1 < N) gu = -u * __ldg(a.x_fwd + c.at(k + 1));
+        if (n > 0) gl = -u * __ldg(a.x_fwd + c.at(k - 1));
+      }
+      a.gMc[p] = gc;
+      a.gMu[p] = gu;
+      a.gMl[p] = gl;
+    }
+    a.x[p] = u;
+  }
 }
 
 // ---------------------------------------------------------------------------

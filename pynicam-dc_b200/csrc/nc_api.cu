@@ -1684,6 +1684,7 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
                         (const void*)k_vi_col<double, false, true>, (const void*)k_vi_col<float, true, false>,
                         (const void*)k_vi_col<float, false, false>, (const void*)k_vi_col<float, false, true>})
     CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vi_col_smem(NC_MAXK)));
+  CU(cudaFuncSetAttribute(k_tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem(NC_ADJ_K)));
   ArrTab T;
   for (int n = 0; n < narrays; ++n) {
     if (!arrays[n].name || !arrays[n].data) return fail(NC_ERR_ARG, "null array entry");
@@ -2824,7 +2825,7 @@ int nc_vsolve(nc_handle* h, int32_t pole, int32_t transpose, const double* Mc, c
     return fail(NC_ERR_ARG, "nc_vsolve: the matrix cotangents need transpose = 1 and gMc, gMu, gMl");
   TriArgs a{Mc, Mu, Ml, b, x, x_fwd, gMc, gMu, gMl, transpose ? 1 : 0};
   TRY(after_caller(h, stream));
-  k_tri_solve<<<col_blocks(h, pole, 128), 128, 0, h->stream>>>(a, pole ? 1 : 0);
+  k_tri_solve<<<col_blocks(h, pole, 32), 32 * TRI_W, tri_smem(h->D.kmax - h->D.kmin), h->stream>>>(a, pole ? 1 : 0);
   TRY(check_launch(h, "vsolve"));
   return before_caller(h, stream);
 }
