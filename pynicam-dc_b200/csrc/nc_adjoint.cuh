@@ -285,52 +285,195 @@ __global__ void k_vadv_lin(VadvLin a, int pole) {
 }
 
 // ---------------------------------------------------------------------------
-// horizontal Laplacian and its adjoint (the exchange first / its adjoint last)
+// The linear stencil operators after the halo exchange, y = L(C(x)), and their
+// adjoints x = C^T L^T y: the Laplacian (kernels/oprtlaplacian.py:41-70), the
+// divergence (kernels/fluxconv.py:52-108) and the gradient
+// (kernels/oprtgradient.py:45-88).  Fields of several components are stored one
+// component after the other (npt regional, npl pole values each).
+//
+// Forward: one launch.  A halo cell is read at its exchange source (hsrc, one
+// int a cell; hsrc_pl for the pole neighbours), so the input is neither copied
+// nor exchanged (copying, exchanging and the pole launch took six more).
+// Adjoint: one launch writes L^T y on the interior cells and the pole points
+// and clears the halo, a second forms L^T y at the halo entries and adds it to
+// their sources (atomically: several may share one), instead of writing the
+// halo, adding it up from there and clearing it in launches of their own.
 // ---------------------------------------------------------------------------
-// y = L(q) on interior cells (halo cells 0); pole point row g = 0, neighbours 0
-__global__ void k_lap_fwd(const double* q, double* y) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.npti) return;
-  const int G = cD.G, KA = cD.KA;
-  const int i = t % G, j = (t / G) % G, k = (t / (G * G)) % KA, l = t / (G * G * KA);
-  double v = 0.0;
-  if (interior(i, j)) v = lap7<double>(i, j, k, l, [&](int ii, int jj, int kk) { return q[ix(ii, jj, kk, l)]; });
-  y[t] = v;
+enum { LOP_LAP, LOP_DIV, LOP_GRAD };
+__host__ __device__ constexpr int lop_in(int op) { return op == LOP_DIV ? 3 : 1; }
+__host__ __device__ constexpr int lop_out(int op) { return op == LOP_GRAD ? 3 : 1; }
+template <int OP>
+__device__ __forceinline__ const double* lop_coef() {
+  return OP == LOP_LAP ? cG.coef_lap : (OP == LOP_DIV ? cG.coef_div : cG.coef_grad);
 }
-__global__ void k_lap_fwd_pl(const double* q, double* y) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  const int k = t / cD.LP, lp = t % cD.LP;
-  double row = 0.0;
-  for (int v = 0; v < 6; ++v) {
-    const double tv = cG.coef_lap_pl[v * cD.LP + lp] * q[ipl(v, k, lp)];
-    row = (v == 0) ? tv : row + tv;
+template <int OP>
+__device__ __forceinline__ const double* lop_coef_pl(int g, int lp) {   // of pole row g: one value, or one a direction
+  return OP == LOP_LAP ? cG.coef_lap_pl + (g * cD.LP + lp)
+                       : (OP == LOP_DIV ? cG.coef_div_pl : cG.coef_grad_pl) + (g * cD.LP + lp) * 3;
+}
+
+template <int OP>
+__global__ void k_lop_fwd(const double* x, const double* x_pl, const int* hsrc, const int* hsrc_pl, double* y,
+                          double* y_pl, int npb) {
+  const int n = cD.npti, np = cD.npl;
+  if ((int)blockIdx.x < npb) {   // pole rows: a thread per (level, pole)
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t >= cD.KA * cD.LP) return;
+    const int k = t / cD.LP, lp = t % cD.LP;
+    double row[lop_out(OP)];
+    for (int g = 0; g < 6; ++g) {
+      const int s = __ldg(hsrc_pl + g * cD.LP + lp);
+      auto in = [&](int c) { return s >= 0 ? x[c * n + s + k * cD.planei] : x_pl[c * np + (-s - 1) + k * cD.LP]; };
+      const double* cf = lop_coef_pl<OP>(g, lp);
+      if (OP == LOP_DIV) {
+        const double pv = cf[0] * in(0) + cf[1] * in(1) + cf[2] * in(2);
+        row[0] = (g == 0) ? pv : row[0] + pv;
+      } else {
+        const double v = in(0);
+#pragma unroll
+        for (int d = 0; d < lop_out(OP); ++d) row[d] = (g == 0) ? cf[d] * v : row[d] + cf[d] * v;
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < lop_out(OP); ++d) {
+      y_pl[d * np + ipl(0, k, lp)] = row[d];
+      for (int g = 1; g < 6; ++g) y_pl[d * np + ipl(g, k, lp)] = 0.0;
+    }
+    return;
   }
-  y[ipl(0, k, lp)] = row;
-  for (int g = 1; g < 6; ++g) y[ipl(g, k, lp)] = 0.0;
+  const int p = (int)((blockIdx.x - npb) * blockDim.x + threadIdx.x);
+  Pt c;
+  if (!reg_point(p, c)) return;
+  double o[lop_out(OP)];
+#pragma unroll
+  for (int d = 0; d < lop_out(OP); ++d) o[d] = 0.0;
+  if (interior(c.i, c.j)) {
+    const int G = cD.G, c2 = (c.l * G + c.j) * G + c.i;
+    const double* cf = lop_coef<OP>();
+    const bool edge = c.i == 1 || c.j == 1 || c.i == G - 2 || c.j == G - 2;
+    double v[lop_in(OP)][7];
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {
+      const int off = kNbI[m] + kNbJ[m] * G;
+      int s = p + off;
+      bool pole = false;
+      if (edge && !interior(c.i + kNbI[m], c.j + kNbJ[m])) {
+        const int h = __ldg(hsrc + c2 + off);
+        pole = h < 0;
+        s = pole ? (-h - 1) + c.k * cD.LP : h + c.k * cD.planei;
+      }
+#pragma unroll
+      for (int d = 0; d < lop_in(OP); ++d) v[d][m] = pole ? __ldg(x_pl + d * np + s) : __ldg(x + d * n + s);
+    }
+    if (OP == LOP_DIV) {   // per direction left to right, then x + y + z
+      double acc[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        double r = __ldg(cf + d * 7 * cD.npt2i + c2) * v[d % lop_in(OP)][0];
+#pragma unroll
+        for (int m = 1; m < 7; ++m) r = r + __ldg(cf + (d * 7 + m) * cD.npt2i + c2) * v[d % lop_in(OP)][m];
+        acc[d] = r;
+      }
+      o[0] = acc[0] + acc[1] + acc[2];
+    } else {
+#pragma unroll
+      for (int d = 0; d < lop_out(OP); ++d) {
+        double r = __ldg(cf + d * 7 * cD.npt2i + c2) * v[0][0];
+#pragma unroll
+        for (int m = 1; m < 7; ++m) r = r + __ldg(cf + (d * 7 + m) * cD.npt2i + c2) * v[0][m];
+        o[d] = r;
+      }
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < lop_out(OP); ++d) y[d * n + p] = o[d];
 }
-// the transposed stencil: every cell gathers coef_lap[m](i) y(i) from the
-// interior cells i whose stencil point m it is
-__global__ void k_lap_adj(const double* y, double* g) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.npti) return;
-  const int G = cD.G, KA = cD.KA;
-  const int i = t % G, j = (t / G) % G, k = (t / (G * G)) % KA, l = t / (G * G * KA);
-  double s = 0.0;
+
+// L^T y at regional cell (i, j): gathered from the interior cells whose stencil point m it is
+template <int OP>
+__device__ __forceinline__ void lop_gather(const double* y, int i, int j, int k, int l, double o[lop_in(OP)]) {
+  const int G = cD.G, n = cD.npti;
+  const double* cf = lop_coef<OP>();
+#pragma unroll
+  for (int d = 0; d < lop_in(OP); ++d) o[d] = 0.0;
+#pragma unroll
   for (int m = 0; m < 7; ++m) {
     const int si = i - kNbI[m], sj = j - kNbJ[m];
-    if (si >= 0 && sj >= 0 && si < G && sj < G && interior(si, sj))
-      s += P2(cG.coef_lap, m, si, sj, l) * y[ix(si, sj, k, l)];
+    if (si >= 1 && sj >= 1 && si <= G - 2 && sj <= G - 2) {
+      const int s2 = (l * G + sj) * G + si, s = ix(si, sj, k, l);
+      if (OP == LOP_DIV) {
+        const double ys = __ldg(y + s);
+#pragma unroll
+        for (int d = 0; d < lop_in(OP); ++d) o[d] += __ldg(cf + (d * 7 + m) * cD.npt2i + s2) * ys;
+      } else {
+#pragma unroll
+        for (int d = 0; d < lop_out(OP); ++d) o[0] += __ldg(cf + (d * 7 + m) * cD.npt2i + s2) * __ldg(y + d * n + s);
+      }
+    }
   }
-  g[t] = s;
 }
-__global__ void k_lap_adj_pl(const double* y, double* g) {
+// ... and at pole row g of (k, lp)
+template <int OP>
+__device__ __forceinline__ void lop_gather_pl(const double* y_pl, int g, int k, int lp, double o[lop_in(OP)]) {
+  const double* cf = lop_coef_pl<OP>(g, lp);
+  const int p0 = ipl(0, k, lp);
+  if (OP == LOP_DIV) {
+#pragma unroll
+    for (int d = 0; d < lop_in(OP); ++d) o[d] = cf[d] * y_pl[p0];
+  } else {
+    double acc = 0.0;
+#pragma unroll
+    for (int d = 0; d < lop_out(OP); ++d) acc += cf[d] * y_pl[d * cD.npl + p0];
+    o[0] = acc;
+  }
+}
+
+template <int OP>
+__global__ void k_lop_adj(const double* y, const double* y_pl, const int* hsrc, const int* hsrc_pl, double* x,
+                          double* x_pl, int npb) {
+  double o[lop_in(OP)];
+  if ((int)blockIdx.x < npb) {
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    Pt q;
+    if (!pole_point(t, q)) return;
+    // a pole point that is a destination of the exchange is cleared
+    const bool own = __ldg(hsrc_pl + q.g * cD.LP + q.lp) == -(q.g * cD.KA * cD.LP + q.lp) - 1;
+    lop_gather_pl<OP>(y_pl, q.g, q.k, q.lp, o);
+#pragma unroll
+    for (int d = 0; d < lop_in(OP); ++d) x_pl[d * cD.npl + t] = own ? o[d] : 0.0;
+    return;
+  }
+  const int p = (int)((blockIdx.x - npb) * blockDim.x + threadIdx.x);
+  Pt c;
+  if (!reg_point(p, c)) return;
+  const int G = cD.G;
+  const bool own = interior(c.i, c.j) || __ldg(hsrc + (c.l * G + c.j) * G + c.i) == ix(c.i, c.j, 0, c.l);
+  if (own) lop_gather<OP>(y, c.i, c.j, c.k, c.l, o);
+#pragma unroll
+  for (int d = 0; d < lop_in(OP); ++d) x[d * cD.npti + p] = own ? o[d] : 0.0;
+}
+// the destinations' share of L^T y, added to their sources (c_dst, c_src: k_comm's plan)
+template <int OP>
+__global__ void k_lop_adj_halo(const double* y, const double* y_pl, const int* c_dst, const int* c_src, int nr, int nent,
+                               double* x, double* x_pl) {
   const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  const int k = t / cD.LP, lp = t % cD.LP;
-  const double y0 = y[ipl(0, k, lp)];
-  for (int v = 0; v < 6; ++v) g[ipl(v, k, lp)] = cG.coef_lap_pl[v * cD.LP + lp] * y0;
+  if (t >= nent * cD.KA) return;
+  const int k = t / nent, e = t - k * nent;
+  const int d0 = __ldg(c_dst + e), s0 = __ldg(c_src + e);
+  double o[lop_in(OP)];
+  if (e < nr) {   // regional destination, level-0 index ((l * KA) * G + j) * G + i
+    const int G = cD.G, i = d0 % G, j = (d0 / G) % G, l = d0 / (cD.planei * cD.KA);
+    lop_gather<OP>(y, i, j, k, l, o);
+  } else {
+    lop_gather_pl<OP>(y_pl, d0 / (cD.KA * cD.LP), k, d0 % cD.LP, o);
+  }
+#pragma unroll
+  for (int d = 0; d < lop_in(OP); ++d) {
+    if (s0 >= 0) atomicAdd(x + d * cD.npti + s0 + k * cD.planei, o[d]);
+    else atomicAdd(x_pl + d * cD.npl + (-s0 - 1) + k * cD.LP, o[d]);
+  }
 }
+
 // adjoint of the halo exchange on one field: each destination's value is added
 // to its source (atomically: several destinations may share a source), then
 // the destinations are cleared by k_comm_adj_clear
@@ -789,113 +932,6 @@ __global__ void k_hlin_pole_grad_ad(HLin a) {
   for (int v = 0; v < 6; ++v) {
     const int pv = ipl(v, k, lp);
     a.gx_pl[pv] += a.gq_pl[pv] / a.rhog_t_pl[pv];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// divergence (kernels/fluxconv.py:52-108) and gradient
-// (kernels/oprtgradient.py:45-88) after the halo exchange, and their
-// adjoints.  Three-component fields are stored one component after the other
-// (3 x npt regional, 3 x npl pole values).
-// ---------------------------------------------------------------------------
-__global__ void k_div_fwd(const double* v, double* y) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.npti) return;
-  const int G = cD.G, KA = cD.KA, n = cD.npti;
-  const int i = t % G, j = (t / G) % G, k = (t / (G * G)) % KA, l = t / (G * G * KA);
-  double r = 0.0;
-  if (interior(i, j))
-    r = div7<double>(i, j, k, l, [&](int ii, int jj, int kk, int d) { return v[d * n + ix(ii, jj, kk, l)]; });
-  y[t] = r;
-}
-__global__ void k_div_fwd_pl(const double* v, double* y) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  const int k = t / cD.LP, lp = t % cD.LP, np = cD.npl;
-  double row = 0.0;
-  for (int g = 0; g < 6; ++g) {
-    const int q = ipl(g, k, lp);
-    const double* cd = cG.coef_div_pl + (g * cD.LP + lp) * 3;
-    const double pv = cd[0] * v[q] + cd[1] * v[np + q] + cd[2] * v[2 * np + q];
-    row = (g == 0) ? pv : row + pv;
-  }
-  y[ipl(0, k, lp)] = row;
-  for (int g = 1; g < 6; ++g) y[ipl(g, k, lp)] = 0.0;
-}
-// v-bar_d at every cell: the interior cells s whose stencil point m it is
-__global__ void k_div_adj(const double* y, double* v) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.npti) return;
-  const int G = cD.G, KA = cD.KA, n = cD.npti;
-  const int i = t % G, j = (t / G) % G, k = (t / (G * G)) % KA, l = t / (G * G * KA);
-  double acc[3] = {0.0, 0.0, 0.0};
-  for (int m = 0; m < 7; ++m) {
-    const int si = i - kNbI[m], sj = j - kNbJ[m];
-    if (si >= 1 && sj >= 1 && si <= G - 2 && sj <= G - 2) {
-      const double ys = y[ix(si, sj, k, l)];
-      for (int d = 0; d < 3; ++d) acc[d] += P2(cG.coef_div, d * 7 + m, si, sj, l) * ys;
-    }
-  }
-  for (int d = 0; d < 3; ++d) v[d * n + t] = acc[d];
-}
-__global__ void k_div_adj_pl(const double* y, double* v) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  const int k = t / cD.LP, lp = t % cD.LP, np = cD.npl;
-  const double y0 = y[ipl(0, k, lp)];
-  for (int g = 0; g < 6; ++g) {
-    const int q = ipl(g, k, lp);
-    const double* cd = cG.coef_div_pl + (g * cD.LP + lp) * 3;
-    for (int d = 0; d < 3; ++d) v[d * np + q] = cd[d] * y0;
-  }
-}
-__global__ void k_grad_fwd(const double* q, double* gr) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.npti) return;
-  const int G = cD.G, KA = cD.KA, n = cD.npti;
-  const int i = t % G, j = (t / G) % G, k = (t / (G * G)) % KA, l = t / (G * G * KA);
-  double o[3] = {0.0, 0.0, 0.0};
-  if (interior(i, j)) grad7<double>(i, j, k, l, [&](int ii, int jj, int kk) { return q[ix(ii, jj, kk, l)]; }, o);
-  for (int d = 0; d < 3; ++d) gr[d * n + t] = o[d];
-}
-__global__ void k_grad_fwd_pl(const double* q, double* gr) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  const int k = t / cD.LP, lp = t % cD.LP, np = cD.npl;
-  for (int d = 0; d < 3; ++d) {
-    double row = 0.0;
-    for (int g = 0; g < 6; ++g) {
-      const double tv = cG.coef_grad_pl[(g * cD.LP + lp) * 3 + d] * q[ipl(g, k, lp)];
-      row = (g == 0) ? tv : row + tv;
-    }
-    gr[d * np + ipl(0, k, lp)] = row;
-    for (int g = 1; g < 6; ++g) gr[d * np + ipl(g, k, lp)] = 0.0;
-  }
-}
-__global__ void k_grad_adj(const double* gr, double* q) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.npti) return;
-  const int G = cD.G, KA = cD.KA, n = cD.npti;
-  const int i = t % G, j = (t / G) % G, k = (t / (G * G)) % KA, l = t / (G * G * KA);
-  double acc = 0.0;
-  for (int m = 0; m < 7; ++m) {
-    const int si = i - kNbI[m], sj = j - kNbJ[m];
-    if (si >= 1 && sj >= 1 && si <= G - 2 && sj <= G - 2) {
-      const int ps = ix(si, sj, k, l);
-      for (int d = 0; d < 3; ++d) acc += P2(cG.coef_grad, d * 7 + m, si, sj, l) * gr[d * n + ps];
-    }
-  }
-  q[t] = acc;
-}
-__global__ void k_grad_adj_pl(const double* gr, double* q) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  const int k = t / cD.LP, lp = t % cD.LP, np = cD.npl;
-  const int p0 = ipl(0, k, lp);
-  for (int g = 0; g < 6; ++g) {
-    double acc = 0.0;
-    for (int d = 0; d < 3; ++d) acc += cG.coef_grad_pl[(g * cD.LP + lp) * 3 + d] * gr[d * np + p0];
-    q[ipl(g, k, lp)] = acc;
   }
 }
 

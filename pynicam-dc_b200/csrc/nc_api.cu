@@ -338,6 +338,7 @@ struct nc_handle {
   long long *r_dst = nullptr, *r_src = nullptr, *p_dst = nullptr, *p_src = nullptr;
   int nr = 0, np = 0;
   int *c_dst = nullptr, *c_src = nullptr;   // the same in array indices (k_comm)
+  int *hsrc = nullptr, *hsrc_pl = nullptr;  // the exchange source of every cell and pole point (itself where none)
   // marshal staging
   double *stage = nullptr, *stage_pl = nullptr;
   double* mass_part = nullptr;
@@ -1511,6 +1512,41 @@ static HsParams hs_params(const nc_handle* h, bool moist = false) {
   return hp;
 }
 
+// A linear operator of nc_adjoint.cuh on x (transposed: its adjoint) into y.
+// The kernels read neighbours of x while y is written, so an input that
+// overlaps its output is copied first.
+template <int OP>
+static int linear_op(nc_handle* h, int transpose, const double* x, const double* x_pl, double* y, double* y_pl) {
+  const Dims& D = h->D;
+  const cudaStream_t s = h->stream;
+  const int ni = transpose ? lop_out(OP) : lop_in(OP), no = transpose ? lop_in(OP) : lop_out(OP);
+  auto meet = [](const double* a, size_t n, const double* b, size_t m) { return a < b + m && b < a + n; };
+  const size_t xr = (size_t)ni * D.npt, xp = (size_t)ni * D.npl, yr = (size_t)no * D.npt, yp = (size_t)no * D.npl;
+  if (meet(x, xr, y, yr) || meet(x_pl, xp, y_pl, yp) || meet(x, xr, y_pl, yp) || meet(x_pl, xp, y, yr)) {
+    if (!h->adj_work3) TRY(dev_alloc(h, &h->adj_work3, 3 * ((size_t)D.npt + D.npl)));
+    CU(cudaMemcpyAsync(h->adj_work3, x, xr * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    CU(cudaMemcpyAsync(h->adj_work3 + xr, x_pl, xp * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    x = h->adj_work3;
+    x_pl = h->adj_work3 + xr;
+  }
+  const int tb = 128, nreg = (int)((D.npt + tb - 1) / tb);
+  if (!transpose) {
+    const int npb = (D.KA * D.LP + tb - 1) / tb;
+    k_lop_fwd<OP><<<(unsigned)(npb + nreg), tb, 0, s>>>(x, x_pl, h->hsrc, h->hsrc_pl, y, y_pl, npb);
+    return check_launch(h, "lop_fwd");
+  }
+  const int npb = (D.npl + tb - 1) / tb;
+  k_lop_adj<OP><<<(unsigned)(npb + nreg), tb, 0, s>>>(x, x_pl, h->hsrc, h->hsrc_pl, y, y_pl, npb);
+  TRY(check_launch(h, "lop_adj"));
+  const int nent = h->nr + h->np;
+  if (nent > 0) {
+    k_lop_adj_halo<OP><<<(unsigned)(((long long)nent * D.KA + tb - 1) / tb), tb, 0, s>>>(x, x_pl, h->c_dst, h->c_src, h->nr,
+                                                                                        nent, y, y_pl);
+    TRY(check_launch(h, "lop_adj_halo"));
+  }
+  return 0;
+}
+
 extern "C" {
 
 int nc_forcing_step(nc_handle* h) {
@@ -2022,9 +2058,16 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
       cd.push_back(pol0(pd[n]));
       cs.push_back(reg0(psrc[n]));
     }
-    for (int n = 0; n < 2; ++n) {
-      const std::vector<int>& v = n ? cs : cd;
-      int** out = n ? &h->c_src : &h->c_dst;
+    std::vector<int> hs((size_t)D.npt2), hp((size_t)6 * D.LP);
+    for (int n = 0; n < (int)hs.size(); ++n) hs[n] = reg0(n);
+    for (int n = 0; n < (int)hp.size(); ++n) hp[n] = -pol0(n) - 1;
+    for (int n = 0; n < h->nr; ++n) hs[rd[n]] = cs[n];
+    for (int n = 0; n < h->np; ++n) hp[pd[n]] = cs[h->nr + n];
+    const std::vector<int>* vs[4] = {&cd, &cs, &hs, &hp};
+    int** outs[4] = {&h->c_dst, &h->c_src, &h->hsrc, &h->hsrc_pl};
+    for (int n = 0; n < 4; ++n) {
+      const std::vector<int>& v = *vs[n];
+      int** out = outs[n];
       TRY(dev_alloc_bytes(h, (void**)out, std::max<size_t>(v.size(), 1) * sizeof(int)));
       if (!v.empty()) CU(cudaMemcpy(*out, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice));
     }
@@ -2848,41 +2891,8 @@ int nc_laplacian(nc_handle* h, int32_t transpose, const double* q, const double*
   TRY(adj_ready(h, "nc_laplacian"));
   if (!q || !q_pl || !y || !y_pl) return fail(NC_ERR_ARG, "nc_laplacian: null pointer");
   if (q == y || q_pl == y_pl) return fail(NC_ERR_ARG, "nc_laplacian: input and output must not alias");
-  const Dims& D = h->D;
-  const long long ne = (long long)(h->nr + h->np) * D.KA;
-  const unsigned gc = (unsigned)((ne + 255) / 256);
-  const unsigned gr = (unsigned)((D.npt + 255) / 256), gp = (unsigned)((D.KA * D.LP + 127) / 128);
   TRY(after_caller(h, stream));
-  if (!transpose) {
-    if (!h->adj_work) TRY(dev_alloc(h, &h->adj_work, (size_t)D.npt + D.npl));
-    double* w = h->adj_work;
-    double* w_pl = h->adj_work + D.npt;
-    CU(cudaMemcpyAsync(w, q, (size_t)D.npt * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    CU(cudaMemcpyAsync(w_pl, q_pl, (size_t)D.npl * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    CommFields<double> f{};
-    f.r[0] = w;
-    f.p[0] = w_pl;
-    f.n = 1;
-    if (ne > 0) {
-      k_comm<<<gc, 256, 0, h->stream>>>(f, h->c_dst, h->c_src, h->nr, h->nr + h->np);
-      TRY(check_launch(h, "lap_comm"));
-    }
-    k_lap_fwd<<<gr, 256, 0, h->stream>>>(w, y);
-    TRY(check_launch(h, "lap"));
-    k_lap_fwd_pl<<<gp, 128, 0, h->stream>>>(w_pl, y_pl);
-    TRY(check_launch(h, "lap_pl"));
-  } else {
-    k_lap_adj<<<gr, 256, 0, h->stream>>>(q, y);
-    TRY(check_launch(h, "lap_adj"));
-    k_lap_adj_pl<<<gp, 128, 0, h->stream>>>(q_pl, y_pl);
-    TRY(check_launch(h, "lap_adj_pl"));
-    if (ne > 0) {
-      k_comm_adj_add<<<gc, 256, 0, h->stream>>>(y, y_pl, h->r_dst, h->r_src, h->nr, h->p_dst, h->p_src, h->np);
-      TRY(check_launch(h, "comm_adj"));
-      k_comm_adj_clear<<<gc, 256, 0, h->stream>>>(y, y_pl, h->r_dst, h->nr, h->p_dst, h->np);
-      TRY(check_launch(h, "comm_adj_clear"));
-    }
-  }
+  TRY(linear_op<LOP_LAP>(h, transpose, q, q_pl, y, y_pl));
   return before_caller(h, stream);
 }
 
@@ -3000,27 +3010,9 @@ int nc_exchange(nc_handle* h, int32_t transpose, double* x, double* x_pl, int32_
 int nc_divergence(nc_handle* h, int32_t transpose, double* v, double* v_pl, double* y, double* y_pl, void* stream) {
   TRY(adj_ready(h, "nc_divergence"));
   if (!v || !v_pl || !y || !y_pl) return fail(NC_ERR_ARG, "nc_divergence: null pointer");
-  const Dims& D = h->D;
-  const unsigned gr = (unsigned)((D.npt + 255) / 256), gp = (unsigned)((D.KA * D.LP + 127) / 128);
   TRY(after_caller(h, stream));
-  if (!transpose) {
-    if (!h->adj_work3) TRY(dev_alloc(h, &h->adj_work3, 3 * ((size_t)D.npt + D.npl)));
-    double* w = h->adj_work3;
-    double* w_pl = w + 3 * (size_t)D.npt;
-    CU(cudaMemcpyAsync(w, v, 3 * D.npt * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    CU(cudaMemcpyAsync(w_pl, v_pl, 3 * (size_t)D.npl * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    TRY(comm_fields(h, w, w_pl, 3, false));
-    k_div_fwd<<<gr, 256, 0, h->stream>>>(w, y);
-    TRY(check_launch(h, "div"));
-    k_div_fwd_pl<<<gp, 128, 0, h->stream>>>(w_pl, y_pl);
-    TRY(check_launch(h, "div_pl"));
-  } else {
-    k_div_adj<<<gr, 256, 0, h->stream>>>(y, v);
-    TRY(check_launch(h, "div_adj"));
-    k_div_adj_pl<<<gp, 128, 0, h->stream>>>(y_pl, v_pl);
-    TRY(check_launch(h, "div_adj_pl"));
-    TRY(comm_fields(h, v, v_pl, 3, true));
-  }
+  if (!transpose) TRY(linear_op<LOP_DIV>(h, 0, v, v_pl, y, y_pl));
+  else TRY(linear_op<LOP_DIV>(h, 1, y, y_pl, v, v_pl));
   return before_caller(h, stream);
 }
 
@@ -3123,27 +3115,9 @@ int nc_divdamp2d(nc_handle* h, int32_t transpose, double* v, double* v_pl, doubl
 int nc_gradient(nc_handle* h, int32_t transpose, double* q, double* q_pl, double* g, double* g_pl, void* stream) {
   TRY(adj_ready(h, "nc_gradient"));
   if (!q || !q_pl || !g || !g_pl) return fail(NC_ERR_ARG, "nc_gradient: null pointer");
-  const Dims& D = h->D;
-  const unsigned gr = (unsigned)((D.npt + 255) / 256), gp = (unsigned)((D.KA * D.LP + 127) / 128);
   TRY(after_caller(h, stream));
-  if (!transpose) {
-    if (!h->adj_work) TRY(dev_alloc(h, &h->adj_work, (size_t)D.npt + D.npl));
-    double* w = h->adj_work;
-    double* w_pl = w + D.npt;
-    CU(cudaMemcpyAsync(w, q, D.npt * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    CU(cudaMemcpyAsync(w_pl, q_pl, (size_t)D.npl * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    TRY(comm_fields(h, w, w_pl, 1, false));
-    k_grad_fwd<<<gr, 256, 0, h->stream>>>(w, g);
-    TRY(check_launch(h, "grad"));
-    k_grad_fwd_pl<<<gp, 128, 0, h->stream>>>(w_pl, g_pl);
-    TRY(check_launch(h, "grad_pl"));
-  } else {
-    k_grad_adj<<<gr, 256, 0, h->stream>>>(g, q);
-    TRY(check_launch(h, "grad_adj"));
-    k_grad_adj_pl<<<gp, 128, 0, h->stream>>>(g_pl, q_pl);
-    TRY(check_launch(h, "grad_adj_pl"));
-    TRY(comm_fields(h, q, q_pl, 1, true));
-  }
+  if (!transpose) TRY(linear_op<LOP_GRAD>(h, 0, q, q_pl, g, g_pl));
+  else TRY(linear_op<LOP_GRAD>(h, 1, g, g_pl, q, q_pl));
   return before_caller(h, stream);
 }
 

@@ -10,6 +10,7 @@ remainders of its splits (B200).
   member bit for bit, in both forms.
 * Tracers in batches: every tracer of 6 (batches of 4 and 2) equals the same
   tracer carried alone, bit for bit.
+* The linear operators on an input that overlaps the output.
 """
 import importlib
 
@@ -99,3 +100,35 @@ def test_tracer_batches_equal_lone_tracers(pkg, prec):
     for n in range(5):
         a, ap = run([n])
         assert np.array_equal(s[..., 7 + n], a[..., 7]) and np.array_equal(sp[..., 7 + n], ap[..., 7]), n
+
+
+def test_linear_operators_in_place(pkg):
+    import torch
+    g = _ig().Grid(4, vlayer=5, ztop=30000.0, device="cuda")
+    geo = g.setup(dtl=600.0, gamma=9.6e16, nq=1)
+    c = pkg.NicamCuda(geo, graph=False)
+    try:
+        gen = torch.Generator(device="cuda").manual_seed(4)
+        F, P = c.field_shape, c.field_shape_pl
+        rand = lambda n, f: torch.randn((n,) + tuple(f), generator=gen, dtype=torch.float64, device="cuda")
+        for op, ni, no in ((c.gradient, 1, 3), (c.divergence, 3, 1)):
+            for transpose in (False, True):
+                x, x_pl, y, y_pl = rand(ni, F), rand(ni, P), rand(no, F), rand(no, P)
+                one = lambda t: t[0] if t.shape[0] == 1 else t
+                want = [t.clone() for t in (x, x_pl, y, y_pl)]
+                op(*[one(t) for t in want], transpose=transpose)
+                out = want[:2] if transpose else want[2:]
+                # the single component shares its memory with the first of the three
+                big, big_pl = (y, y_pl) if no == 3 else (x, x_pl)
+                small, small_pl = (x, x_pl) if no == 3 else (y, y_pl)
+                three_in = (no == 3) == transpose
+                if not three_in:
+                    big[0].copy_(small[0])
+                    big_pl[0].copy_(small_pl[0])
+                args = ((big[0], big_pl[0], big, big_pl) if no == 3 else (big, big_pl, big[0], big_pl[0]))
+                op(*args, transpose=transpose)
+                got = (big[:1], big_pl[:1]) if three_in else (big, big_pl)
+                for a, b in zip(got, out):
+                    assert float((a - b).abs().max()) <= 1e-15 * float(b.abs().max()) + 0.0, (op.__name__, transpose)
+    finally:
+        c.close()
