@@ -1015,7 +1015,8 @@ static int run_step(nc_handle* h) {
       }
       Vp0H<R> vh;
       for (int n = 0; n < 8; ++n) vh.out[n] = RG<R>(h->vph[n]);
-      k_vp0_hl<<<lvgrid_vp, VP_DX * VP_DY, 0, s>>>(v0[0], vh);
+      const dim3 hgrid((lvgrid_vp.x + VP_NK<R> - 1) / VP_NK<R>, lvgrid_vp.y, lvgrid_vp.z);
+      k_vp0_hl<R, VP_NK<R>><<<hgrid, VP_DX * VP_DY, 0, s>>>(v0[0], vh);
       TRY(check_launch(h, "vp0_h"));
       const int tb = h->blk[TB_VP0C];
       const int nk = column_chunks(h, D.KA);
@@ -1047,7 +1048,8 @@ static int run_step(nc_handle* h) {
           for (int n = 0; n < 5; ++n) pa.PM[n] = F(h->PM[n]);
           pa.dt = h->dts; pa.rweight = rweight; pa.RovCV = RovCV;
         }
-        k_path1_l<<<lvgrid, DD_DX * DD_DY, 0, s>>>(p1[0]);
+        const dim3 pgrid((lvgrid.x + P1_NK<R> - 1) / P1_NK<R>, lvgrid.y, lvgrid.z);
+        k_path1_l<R, P1_NK<R>, P1_MINB<R>><<<pgrid, DD_DX * DD_DY, 0, s>>>(p1[0]);
         TRY(check_launch(h, "path1"));
         k_path1_pl<<<ppb, 32, 0, ps>>>(p1[1]);
         TRY(check_launch(h, "path1_pl"));

@@ -175,6 +175,11 @@ template <> __device__ __forceinline__ const GeomT<float>& geom<float>() { retur
 #define NC_F32_VIENERGY 12
 #endif
 
+// a * b + c: two roundings in the float64 form (the reference's), one in the
+// float32 form, whose stencils are bound by the instructions they issue
+__device__ __forceinline__ double mad(double a, double b, double c) { return a * b + c; }
+__device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
 // The gamma factors of the vertical metrics: RGAM, RGAMH, GAM2H (regional or
 // pole) at index p.  With a shallow atmosphere every value is exactly 1 (the
 // host checks each element at set-up and sets gam_unit); the factor is then

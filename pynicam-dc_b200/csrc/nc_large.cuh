@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(256, NC_MINB(R, 2, NC_F32_ADVMOM)) k_advmom_t(
 #pragma unroll
           for (int m = 0; m < 7; ++m) {
             const R v = (s_rv[d][nb[m]] * s_vv[s][nb[m]]) * s_rg[nb[m]];
-            const R t = P2(CG.coef_div, d * 7 + m, i, j, l) * v;
-            sm = (m == 0) ? t : sm + t;
+            const R cf = P2(CG.coef_div, d * 7 + m, i, j, l);
+            sm = (m == 0) ? cf * v : mad(cf, v, sm);
           }
           acc[d] = sm;
         }
@@ -397,7 +397,7 @@ __global__ void k_hdiff1(Six<R> src, SixOut<R> out) {
     auto scl = [&](int m) { return (n >= 4) ? __ldg(s + nb[m]) - __ldg(bs + nb[m]) : __ldg(s + nb[m]); };
     v[n] = cl[0] * scl(0);
 #pragma unroll
-    for (int m = 1; m < 7; ++m) v[n] = v[n] + cl[m] * scl(m);
+    for (int m = 1; m < 7; ++m) v[n] = mad(cl[m], scl(m), v[n]);
   }
 #pragma unroll
   for (int n = 0; n < 6; ++n) out.f[n][p] = -v[n];
@@ -560,8 +560,8 @@ __global__ void __launch_bounds__(HD_DX * HD_DY, NC_MINB(R, 2, 4)) k_hdiff2_m(Si
             const R w1i = s_w[((d * 3 + 0) * 2 + 0) * NT + p], w2i = s_w[((d * 3 + 1) * 2 + 0) * NT + p];
             const R w3i = s_w[((d * 3 + 2) * 2 + 0) * NT + p], w1j = s_w[((d * 3 + 0) * 2 + 1) * NT + p];
             const R w2j = s_w[((d * 3 + 1) * 2 + 1) * NT + p], w3j = s_w[((d * 3 + 2) * 2 + 1) * NT + p];
-            ti = div3(w1i * s0 + w2i * sip + w3i * sd);
-            tj = div3(w1j * s0 + w2j * sd + w3j * sjp);
+            ti = div3(mad(w3i, sd, mad(w2i, sip, w1i * s0)));
+            tj = div3(mad(w3j, sjp, mad(w2j, sd, w1j * s0)));
           }
           s_t[(f * 6 + d) * NT + p] = ti;
           s_t[(f * 6 + 3 + d) * NT + p] = tj;
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(HD_DX * HD_DY, NC_MINB(R, 2, 4)) k_hdiff2_m(Si
         const R* sf = s_f + n * NP;
         R v = cl[0] * sf[nb[0]];
 #pragma unroll
-        for (int m = 1; m < 7; ++m) v = v + cl[m] * sf[nb[m]];
+        for (int m = 1; m < 7; ++m) v = mad(cl[m], sf[nb[m]], v);
         out.f[n][q] = -v;
       }
       const int ta = (ty + 1) * TX + (tx + 1), tb = ta - 1, tc = ta - TX - 1, td = ta - TX;
@@ -601,9 +601,12 @@ __global__ void __launch_bounds__(HD_DX * HD_DY, NC_MINB(R, 2, 4)) k_hdiff2_m(Si
           const R* tj = s_t + (f * 6 + 3 + d) * NT;
           const R aTI = ti[ta], aTJ = tj[ta], bTI = ti[tb];
           const R cTI = ti[tc], cTJ = tj[tc], dTJ = tj[td];
-          const R blk = kf1 * cd[d * 6 + 0] * (aTI + aTJ) + kf2 * cd[d * 6 + 1] * (aTJ + bTI) +
-                        kf3 * cd[d * 6 + 2] * (bTI + cTJ) + kf4 * cd[d * 6 + 3] * (cTJ + cTI) +
-                        kf5 * cd[d * 6 + 4] * (cTI + dTJ) + kf6 * cd[d * 6 + 5] * (dTJ + aTI);
+          R blk = kf1 * cd[d * 6 + 0] * (aTI + aTJ);
+          blk = mad(kf2 * cd[d * 6 + 1], aTJ + bTI, blk);
+          blk = mad(kf3 * cd[d * 6 + 2], bTI + cTJ, blk);
+          blk = mad(kf4 * cd[d * 6 + 3], cTJ + cTI, blk);
+          blk = mad(kf5 * cd[d * 6 + 4], cTI + dTJ, blk);
+          blk = mad(kf6 * cd[d * 6 + 5], dTJ + aTI, blk);
           inner = (d == 0) ? blk : inner + blk;
         }
         out.f[4 + f][q] = -inner;

@@ -141,8 +141,8 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4
   // vertical mass flux at half level k (q: the point at k)
   auto rwv = [&](int q) -> R {
     const int qm = q - cD.planei;
-    const R h = cz[q] * v.f[0][q] + cz[n + q] * v.f[0][qm] + cz[2 * n + q] * v.f[1][q] + cz[3 * n + q] * v.f[1][qm] +
-                cz[4 * n + q] * v.f[2][q] + cz[5 * n + q] * v.f[2][qm];
+    const R h = mad(cz[5 * n + q], v.f[2][qm], mad(cz[4 * n + q], v.f[2][q], mad(cz[3 * n + q], v.f[1][qm],
+                mad(cz[2 * n + q], v.f[1][q], mad(cz[n + q], v.f[0][qm], cz[q] * v.f[0][q])))));
     return h * gam_at(CG.RGAMH, q) + v.f[3][q] * CG.RGSQRTH[q];
   };
   for (int p = tid; p < NP; p += blockDim.x) {   // at the chunk's first level (zero at kmin)
@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4
         c = f2 * rg;
         if (up) {
           const int qp = q + cD.planei;   // level k+1
-          const R h = cz[qp] * v.f[0][qp] + cz[n + qp] * f0 + cz[2 * n + qp] * v.f[1][qp] +
-                      cz[3 * n + qp] * f1 + cz[4 * n + qp] * v.f[2][qp] + cz[5 * n + qp] * f2;
+          const R h = mad(cz[5 * n + qp], f2, mad(cz[4 * n + qp], v.f[2][qp], mad(cz[3 * n + qp], f1,
+                      mad(cz[2 * n + qp], v.f[1][qp], mad(cz[n + qp], f0, cz[qp] * v.f[0][qp])))));
           r = h * gam_at(CG.RGAMH, qp) + v.f[3][qp] * CG.RGSQRTH[qp];
         }
       }
@@ -187,12 +187,17 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4
       const R* v0 = s_vm;
       const R* v1 = s_vm + NP;
       const R* v2 = s_vm + 2 * NP;
-      R sTI = C(0, 0, 0) * v0[a] + C(0, 1, 0) * v0[b] + C(0, 2, 0) * v0[c] + C(1, 0, 0) * v1[a] +
-              C(1, 1, 0) * v1[b] + C(1, 2, 0) * v1[c] + C(2, 0, 0) * v2[a] + C(2, 1, 0) * v2[b] +
-              C(2, 2, 0) * v2[c] + wTI;
-      R sTJ = C(0, 0, 1) * v0[a] + C(0, 1, 1) * v0[c] + C(0, 2, 1) * v0[d] + C(1, 0, 1) * v1[a] +
-              C(1, 1, 1) * v1[c] + C(1, 2, 1) * v1[d] + C(2, 0, 1) * v2[a] + C(2, 1, 1) * v2[c] +
-              C(2, 2, 1) * v2[d] + wTJ;
+      R sTI = C(0, 0, 0) * v0[a], sTJ = C(0, 0, 1) * v0[a];
+      sTI = mad(C(0, 1, 0), v0[b], sTI); sTJ = mad(C(0, 1, 1), v0[c], sTJ);
+      sTI = mad(C(0, 2, 0), v0[c], sTI); sTJ = mad(C(0, 2, 1), v0[d], sTJ);
+      sTI = mad(C(1, 0, 0), v1[a], sTI); sTJ = mad(C(1, 0, 1), v1[a], sTJ);
+      sTI = mad(C(1, 1, 0), v1[b], sTI); sTJ = mad(C(1, 1, 1), v1[c], sTJ);
+      sTI = mad(C(1, 2, 0), v1[c], sTI); sTJ = mad(C(1, 2, 1), v1[d], sTJ);
+      sTI = mad(C(2, 0, 0), v2[a], sTI); sTJ = mad(C(2, 0, 1), v2[a], sTJ);
+      sTI = mad(C(2, 1, 0), v2[b], sTI); sTJ = mad(C(2, 1, 1), v2[c], sTJ);
+      sTI = mad(C(2, 2, 0), v2[c], sTI); sTJ = mad(C(2, 2, 1), v2[d], sTJ);
+      sTI = sTI + wTI;
+      sTJ = sTJ + wTJ;
       const int ii = i0 - 1 + px, jj = j0 - 1 + py;
       if (!(ii <= G - 2 && jj <= G - 2)) sTI = sTJ = R(0.0);
       s_ti[p] = sTI;
@@ -213,8 +218,8 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4
       auto D = [&](int m) { return CDR ? cd[CDR ? m : 0] : P2c(CG.coef_diff, m, i, j, l); };
 #pragma unroll
       for (int d = 0; d < 3; ++d)
-        out.f[d][q] = D(d * 6 + 0) * (aTI + aTJ) + D(d * 6 + 1) * (aTJ + bTI) + D(d * 6 + 2) * (bTI + cTJ) +
-                      D(d * 6 + 3) * (cTJ + cTI) + D(d * 6 + 4) * (cTI + dTJ) + D(d * 6 + 5) * (dTJ + aTI);
+        out.f[d][q] = mad(D(d * 6 + 5), dTJ + aTI, mad(D(d * 6 + 4), cTI + dTJ, mad(D(d * 6 + 3), cTJ + cTI,
+                      mad(D(d * 6 + 2), bTI + cTJ, mad(D(d * 6 + 1), aTJ + bTI, D(d * 6 + 0) * (aTI + aTJ))))));
     }
     cur ^= 1;
   }
@@ -459,44 +464,39 @@ struct Vp0H {
   R* out[8];               // div1, div2, dd x/y/z, dpg x/y/z
 };
 
-// vp0 horizontal terms, one block per (level, tile).
-// vp0 keeps a 32x8 tile: its staged fields need more than the 48 KB of
-// static shared memory at larger tiles
+// vp0 horizontal terms, one block per (NK levels, tile): like k_path1_l, each of
+// the 78 coefficients is loaded once and applied to the block's NK levels (the
+// float32 instance; two float64 levels do not leave room for four blocks of
+// shared memory).  vp0 keeps a 32x8 tile: its staged fields need more than the
+// 48 KB of static shared memory at larger tiles.
 #define VP_DX 32
 #define VP_DY 8
-template <class R>
+template <class R> constexpr int VP_NK = sizeof(R) == 8 ? 1 : 2;
+template <class R, int NK>
 __global__ void __launch_bounds__(VP_DX * VP_DY, NC_MINB(R, 4, NC_F32_VP0H)) k_vp0_hl(Vp0Args<R> a, Vp0H<R> h) {
-  constexpr int PX = VP_DX + 2, PY = VP_DY + 2, TX = VP_DX + 1, TY = VP_DY + 1;
-  __shared__ R s_m[3][PY * PX];    // RGAM * rhogv
-  __shared__ R s_e[3][PY * PX];    // RGAM * rhogv * eth
-  __shared__ R s_v[3][PY * PX];    // -vtmp2
-  __shared__ R s_p[PY * PX];       // RGAM * pregd at the gradient level
-  __shared__ R s_ti[TY * TX], s_tj[TY * TX];
-  const TileLv tl = tile_level<VP_DX, VP_DY>(cD.kmin);
+  constexpr int PX = VP_DX + 2, PY = VP_DY + 2, TX = VP_DX + 1, TY = VP_DY + 1, NP = PX * PY, NT = TX * TY;
+  __shared__ R s_m[NK][3][NP];    // RGAM * rhogv
+  __shared__ R s_e[NK][3][NP];    // RGAM * rhogv * eth
+  __shared__ R s_v[NK][3][NP];    // -vtmp2
+  __shared__ R s_p[NK][NP];       // RGAM * pregd at the gradient level
+  __shared__ R s_ti[NK][NT], s_tj[NK][NT];
+  const TileLv tl = tile_level<VP_DX, VP_DY>(0);
   const int l = tl.l, i0 = tl.i0, j0 = tl.j0;
-  const int G = cD.G, gmax = cD.G - 2, kmin = cD.kmin;
+  const int G = cD.G, gmax = cD.G - 2, kmin = cD.kmin, kmax = cD.kmax;
+  const int ka = kmin + tl.k * NK;
   const int tid = threadIdx.x, tx = tid % VP_DX, ty = tid / VP_DX;
-  const int i = i0 + tx, j = j0 + ty;
-  const bool own = (i <= gmax) && (j <= gmax);
-  const R ddc = CC.divdamp_coef;
-  const int n = cD.npti;
   const R* cz = CG.C2WGz;
   const R* const* P = a.P.v;
-  R gxyz[3] = {R(0.0), R(0.0), R(0.0)};
-  int q0 = 0;
-  if (own) {
+  for (int p = tid; p < NP; p += blockDim.x) {
+    const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
+    const bool ok = ii < G && jj < G;
+    const int q0 = ok ? ix(ii, jj, 0, l) : 0;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) gxyz[d] = P2(CG.GRD_x, d, i, j, l);
-    q0 = ix(i, j, 0, l);
-  }
-  {
-    const int k = tl.k;
-    const int kk = (k == kmin) ? kmin + 1 : k;
-    for (int p = tid; p < PX * PY; p += blockDim.x) {
-      const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
+    for (int n = 0; n < NK; ++n) {
+      const int k = min(ka + n, kmax), kk = (k == kmin) ? kmin + 1 : k;   // a level past kmax repeats it
       R mv[3] = {R(0.0), R(0.0), R(0.0)}, ev[3] = {R(0.0), R(0.0), R(0.0)}, vv[3] = {R(0.0), R(0.0), R(0.0)}, pp = R(0.0);
-      if (ii < G && jj < G) {
-        const int q = ix(ii, jj, k, l);
+      if (ok) {
+        const int q = q0 + k * cD.planei, qk = q0 + kk * cD.planei;
         const R rg = CG.RGAM[q], e = a.eth[q];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -505,103 +505,140 @@ __global__ void __launch_bounds__(VP_DX * VP_DY, NC_MINB(R, 4, NC_F32_VP0H)) k_v
           ev[d] = (pv * e) * rg;
           vv[d] = -a.vt.f[d][q];
         }
-        const int qk = ix(ii, jj, kk, l);
         pp = a.pregd[qk] * CG.RGAM[qk];
       }
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        s_m[d][p] = mv[d];
-        s_e[d][p] = ev[d];
-        s_v[d][p] = vv[d];
+        s_m[n][d][p] = mv[d];
+        s_e[n][d][p] = ev[d];
+        s_v[n][d][p] = vv[d];
       }
-      s_p[p] = pp;
+      s_p[n][p] = pp;
     }
-    __syncthreads();
-    for (int p = tid; p < TX * TY; p += blockDim.x) {
-      const int px = p % TX, py = p / TX;
-      const int ii = i0 - 1 + px, jj = j0 - 1 + py;
-      R sTI = R(0.0), sTJ = R(0.0);
-      if (ii <= G - 2 && jj <= G - 2) {
-        const int ia = py * PX + px, ib = ia + 1, ic = ia + PX + 1, id = ia + PX;
-        auto C = [&](int dir, int pt, int t) { return P2(CG.coef_intp, (dir * 3 + pt) * 2 + t, ii, jj, l); };
-        sTI = C(0, 0, 0) * s_v[0][ia] + C(0, 1, 0) * s_v[0][ib] + C(0, 2, 0) * s_v[0][ic] +
-              C(1, 0, 0) * s_v[1][ia] + C(1, 1, 0) * s_v[1][ib] + C(1, 2, 0) * s_v[1][ic] +
-              C(2, 0, 0) * s_v[2][ia] + C(2, 1, 0) * s_v[2][ib] + C(2, 2, 0) * s_v[2][ic];
-        sTJ = C(0, 0, 1) * s_v[0][ia] + C(0, 1, 1) * s_v[0][ic] + C(0, 2, 1) * s_v[0][id] +
-              C(1, 0, 1) * s_v[1][ia] + C(1, 1, 1) * s_v[1][ic] + C(1, 2, 1) * s_v[1][id] +
-              C(2, 0, 1) * s_v[2][ia] + C(2, 1, 1) * s_v[2][ic] + C(2, 2, 1) * s_v[2][id];
-      }
-      s_ti[p] = sTI;
-      s_tj[p] = sTJ;
-    }
-    __syncthreads();
-    if (own) {
-      const int c0 = (ty + 1) * PX + (tx + 1);
-      const int nb[7] = {c0, c0 + 1, c0 + PX + 1, c0 + PX, c0 - 1, c0 - PX - 1, c0 - PX};
-      const int q = q0 + (int)k * cD.planei;
-      // divergences (div7: per direction left to right, then x + y + z)
-      R acc1[3], acc2[3];
+  }
+  __syncthreads();
+  for (int p = tid; p < NT; p += blockDim.x) {
+    const int px = p % TX, py = p / TX;
+    const int ii = i0 - 1 + px, jj = j0 - 1 + py;
+    R sI[NK], sJ[NK];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        R s1 = R(0.0), s2 = R(0.0);
+    for (int n = 0; n < NK; ++n) sI[n] = sJ[n] = R(0.0);
+    if (ii <= G - 2 && jj <= G - 2) {
+      const int ia = py * PX + px;
+      const int vI[3] = {ia, ia + 1, ia + PX + 1}, vJ[3] = {ia, ia + PX + 1, ia + PX};
 #pragma unroll
-        for (int m = 0; m < 7; ++m) {
-          const R cdv = P2(CG.coef_div, d * 7 + m, i, j, l);
-          const R t1 = cdv * s_m[d][nb[m]], t2 = cdv * s_e[d][nb[m]];
-          s1 = (m == 0) ? t1 : s1 + t1;
-          s2 = (m == 0) ? t2 : s2 + t2;
+      for (int m = 0; m < 9; ++m) {   // direction m / 3, vertex m % 3, left to right
+        const R cI = P2(CG.coef_intp, m * 2, ii, jj, l), cJ = P2(CG.coef_intp, m * 2 + 1, ii, jj, l);
+#pragma unroll
+        for (int n = 0; n < NK; ++n) {
+          const R xI = s_v[n][m / 3][vI[m % 3]], xJ = s_v[n][m / 3][vJ[m % 3]];
+          sI[n] = m ? mad(cI, xI, sI[n]) : cI * xI;
+          sJ[n] = m ? mad(cJ, xJ, sJ[n]) : cJ * xJ;
         }
-        acc1[d] = s1;
-        acc2[d] = s2;
-      }
-      h.out[0][q] = acc1[0] + acc1[1] + acc1[2];
-      h.out[1][q] = acc2[0] + acc2[1] + acc2[2];
-      // 2-D divergence damping, projected
-      const int ta = (ty + 1) * TX + (tx + 1);
-      const R aTI = s_ti[ta], aTJ = s_tj[ta], bTI = s_ti[ta - 1];
-      const R cTI = s_ti[ta - TX - 1], cTJ = s_tj[ta - TX - 1], dTJ = s_tj[ta - TX];
-      R dd[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d)
-        dd[d] = ddc * (P2(CG.coef_diff, d * 6 + 0, i, j, l) * (aTI + aTJ) +
-                       P2(CG.coef_diff, d * 6 + 1, i, j, l) * (aTJ + bTI) +
-                       P2(CG.coef_diff, d * 6 + 2, i, j, l) * (bTI + cTJ) +
-                       P2(CG.coef_diff, d * 6 + 3, i, j, l) * (cTJ + cTI) +
-                       P2(CG.coef_diff, d * 6 + 4, i, j, l) * (cTI + dTJ) +
-                       P2(CG.coef_diff, d * 6 + 5, i, j, l) * (dTJ + aTI));
-      {
-        const R prd = div_r(dd[0] * gxyz[0] + dd[1] * gxyz[1] + dd[2] * gxyz[2]);
-        dd[0] = dd[0] - div_r(prd * gxyz[0]);
-        dd[1] = dd[1] - div_r(prd * gxyz[1]);
-        dd[2] = dd[2] - div_r(prd * gxyz[2]);
-      }
-      // pressure gradient of pregd at level kk
-      const int qkk = q0 + (int)kk * cD.planei, qk1 = qkk + cD.planei, qkm = qkk - cD.planei;
-      const R P_k1 = a.pregd[qk1], P_k = a.pregd[qkk], P_km = a.pregd[qkm];
-      const R rgh1 = CG.RGAMH[qk1], rgh0 = CG.RGAMH[qkk];
-      R pg[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        R g = P2(CG.coef_grad, d * 7 + 0, i, j, l) * s_p[nb[0]];
-#pragma unroll
-        for (int m = 1; m < 7; ++m) g = g + P2(CG.coef_grad, d * 7 + m, i, j, l) * s_p[nb[m]];
-        const R up = (cz[(2 * d) * n + qk1] * P_k1 + cz[(2 * d + 1) * n + qk1] * P_k) * rgh1;
-        const R dn = (cz[(2 * d) * n + qkk] * P_k + cz[(2 * d + 1) * n + qkk] * P_km) * rgh0;
-        pg[d] = g + (up - dn) * CC.rdgz[kk];
-      }
-      {
-        const R prd = div_r(pg[0] * gxyz[0] + pg[1] * gxyz[1] + pg[2] * gxyz[2]);
-        pg[0] = pg[0] - div_r(prd * gxyz[0]);
-        pg[1] = pg[1] - div_r(prd * gxyz[1]);
-        pg[2] = pg[2] - div_r(prd * gxyz[2]);
-      }
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        h.out[2 + d][q] = dd[d];
-        h.out[5 + d][q] = pg[d];
       }
     }
-    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < NK; ++n) {
+      s_ti[n][p] = sI[n];
+      s_tj[n][p] = sJ[n];
+    }
+  }
+  __syncthreads();
+  const int i = i0 + tx, j = j0 + ty;
+  if (i > gmax || j > gmax) return;
+  const R ddc = CC.divdamp_coef;
+  const int npt = cD.npti;
+  const R gx = P2(CG.GRD_x, 0, i, j, l), gy = P2(CG.GRD_x, 1, i, j, l), gz = P2(CG.GRD_x, 2, i, j, l);
+  const int q0 = ix(i, j, 0, l);
+  const int ta = (ty + 1) * TX + (tx + 1), c0 = (ty + 1) * PX + (tx + 1);
+  const int nb[7] = {c0, c0 + 1, c0 + PX + 1, c0 + PX, c0 - 1, c0 - PX - 1, c0 - PX};
+  {
+    // divergences (div7: per direction left to right, then x + y + z)
+    R d1[NK], d2[NK];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      R s1[NK], s2[NK];
+#pragma unroll
+      for (int m = 0; m < 7; ++m) {
+        const R cf = P2(CG.coef_div, d * 7 + m, i, j, l);
+#pragma unroll
+        for (int n = 0; n < NK; ++n) {
+          s1[n] = m ? mad(cf, s_m[n][d][nb[m]], s1[n]) : cf * s_m[n][d][nb[m]];
+          s2[n] = m ? mad(cf, s_e[n][d][nb[m]], s2[n]) : cf * s_e[n][d][nb[m]];
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < NK; ++n) {
+        d1[n] = d ? d1[n] + s1[n] : s1[n];
+        d2[n] = d ? d2[n] + s2[n] : s2[n];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < NK; ++n)
+      if (ka + n <= kmax) {
+        h.out[0][q0 + (ka + n) * cD.planei] = d1[n];
+        h.out[1][q0 + (ka + n) * cD.planei] = d2[n];
+      }
+  }
+  auto flat = [&](R* x) {   // tangent-plane projection
+    const R prd = div_r(x[0] * gx + x[1] * gy + x[2] * gz);
+    x[0] = x[0] - div_r(prd * gx);
+    x[1] = x[1] - div_r(prd * gy);
+    x[2] = x[2] - div_r(prd * gz);
+  };
+  R x[NK][3];
+  // 2-D divergence damping
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      const R cf = P2(CG.coef_diff, d * 6 + e, i, j, l);
+#pragma unroll
+      for (int n = 0; n < NK; ++n) {
+        const R* I = s_ti[n];
+        const R* J = s_tj[n];
+        const R t = e == 0 ? I[ta] + J[ta] : e == 1 ? J[ta] + I[ta - 1] : e == 2 ? I[ta - 1] + J[ta - TX - 1]
+                  : e == 3 ? J[ta - TX - 1] + I[ta - TX - 1] : e == 4 ? I[ta - TX - 1] + J[ta - TX] : J[ta - TX] + I[ta];
+        x[n][d] = e ? mad(cf, t, x[n][d]) : cf * t;
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < NK; ++n) {
+    if (ka + n > kmax) break;
+    const int q = q0 + (ka + n) * cD.planei;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) x[n][d] = ddc * x[n][d];
+    flat(x[n]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) h.out[2 + d][q] = x[n][d];
+  }
+  // pressure gradient of pregd
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {
+      const R cf = P2(CG.coef_grad, d * 7 + m, i, j, l);
+#pragma unroll
+      for (int n = 0; n < NK; ++n) x[n][d] = m ? mad(cf, s_p[n][nb[m]], x[n][d]) : cf * s_p[n][nb[m]];
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < NK; ++n) {
+    const int k = ka + n, kk = (k == kmin) ? kmin + 1 : k;
+    if (k > kmax) break;
+    const int q = q0 + k * cD.planei, qkk = q0 + kk * cD.planei, qk1 = qkk + cD.planei, qkm = qkk - cD.planei;
+    const R P_k1 = a.pregd[qk1], P_k = a.pregd[qkk], P_km = a.pregd[qkm];
+    const R rgh1 = CG.RGAMH[qk1], rgh0 = CG.RGAMH[qkk];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const R up = (cz[(2 * d) * npt + qk1] * P_k1 + cz[(2 * d + 1) * npt + qk1] * P_k) * rgh1;
+      const R dn = (cz[(2 * d) * npt + qkk] * P_k + cz[(2 * d + 1) * npt + qkk] * P_km) * rgh0;
+      x[n][d] = x[n][d] + (up - dn) * CC.rdgz[kk];
+    }
+    flat(x[n]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) h.out[5 + d][q] = x[n][d];
   }
 }
 
@@ -790,128 +827,167 @@ __global__ void k_path1_pl(const __grid_constant__ Path1Args<R> a) {
   }
 }
 
-// Regional path 1, one block per (level, tile): same stencils and
-// arithmetic as k_path1_pl.  The blocks at kmin and kmax also write the
-// boundary rows kmin-1 and kmax+1 from the values they computed.
-template <class R>
-__global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, 6, NC_F32_PATH1))) k_path1_l(Path1Args<R> a) {
-  constexpr int PX = DD_DX + 2, PY = DD_DY + 2, TX = DD_DX + 1, TY = DD_DY + 1;
-  __shared__ R s_v[3][PY * PX];
-  __shared__ R s_p[PY * PX];
-  __shared__ R s_ti[TY * TX], s_tj[TY * TX];
-  const TileLv tl = tile_level<DD_DX, DD_DY>(cD.kmin);
-  const int k = tl.k, l = tl.l, i0 = tl.i0, j0 = tl.j0;
+// Regional path 1, one block per (NK levels, tile): same stencils and
+// arithmetic as k_path1_pl.  The kernel is bound by the instructions it issues
+// (920 a point for one level per block, a third of them the addresses and
+// loads of the 60 coefficient planes), so each coefficient is loaded once and
+// applied to the block's NK levels, whose sums run side by side.  The levels
+// kmin and kmax also write the boundary rows kmin-1 and kmax+1 from the values
+// they computed.
+#ifndef P1_NK_F32
+#define P1_NK_F32 4
+#define P1_MINB_F32 3
+#endif
+#ifndef P1_NK_F64
+#define P1_NK_F64 2
+#define P1_MINB_F64 4
+#endif
+template <class R> constexpr int P1_NK = sizeof(R) == 8 ? P1_NK_F64 : P1_NK_F32;
+template <class R> constexpr int P1_MINB = sizeof(R) == 8 ? P1_MINB_F64 : P1_MINB_F32;
+template <class R, int NK, int MINB>
+__global__ void __launch_bounds__(DD_DX * DD_DY, MINB) k_path1_l(Path1Args<R> a) {
+  constexpr int PX = DD_DX + 2, PY = DD_DY + 2, TX = DD_DX + 1, TY = DD_DY + 1, NP = PX * PY, NT = TX * TY;
+  __shared__ R s_v[NK][3][NP];
+  __shared__ R s_p[NK][NP];
+  __shared__ R s_ti[NK][NT], s_tj[NK][NT];
+  const TileLv tl = tile_level<DD_DX, DD_DY>(0);
+  const int l = tl.l, i0 = tl.i0, j0 = tl.j0;
   const int G = cD.G, gmax = cD.G - 2, kmin = cD.kmin, kmax = cD.kmax;
-  const int kk = (k == kmin) ? kmin + 1 : k;
+  const int ka = kmin + tl.k * NK;
   const int tid = threadIdx.x, tx = tid % DD_DX, ty = tid / DD_DX;
   const R RovCV = a.RovCV;
-  for (int p = tid; p < PX * PY; p += blockDim.x) {
+  for (int p = tid; p < NP; p += blockDim.x) {
     const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
-    R x = R(0.0), y = R(0.0), z = R(0.0), pp = R(0.0);
-    if (ii < G && jj < G) {
-      const int q = ix(ii, jj, k, l);
-      x = -__ldg(&a.vt.f[0][q]);
-      y = -__ldg(&a.vt.f[1][q]);
-      z = -__ldg(&a.vt.f[2][q]);
-      const int qk = ix(ii, jj, kk, l);
-      pp = __ldg(&a.PS[5][qk]) * RovCV * __ldg(&CG.RGAM[qk]);
+    const bool ok = ii < G && jj < G;
+    const int q0 = ok ? ix(ii, jj, 0, l) : 0;
+#pragma unroll
+    for (int n = 0; n < NK; ++n) {
+      const int k = min(ka + n, kmax), kk = (k == kmin) ? kmin + 1 : k;   // a level past kmax repeats it
+      const int q = q0 + k * cD.planei, qk = q0 + kk * cD.planei;
+      s_v[n][0][p] = ok ? -__ldg(&a.vt.f[0][q]) : R(0.0);
+      s_v[n][1][p] = ok ? -__ldg(&a.vt.f[1][q]) : R(0.0);
+      s_v[n][2][p] = ok ? -__ldg(&a.vt.f[2][q]) : R(0.0);
+      s_p[n][p] = ok ? __ldg(&a.PS[5][qk]) * RovCV * __ldg(&CG.RGAM[qk]) : R(0.0);
     }
-    s_v[0][p] = x;
-    s_v[1][p] = y;
-    s_v[2][p] = z;
-    s_p[p] = pp;
   }
   __syncthreads();
-  for (int p = tid; p < TX * TY; p += blockDim.x) {
+  for (int p = tid; p < NT; p += blockDim.x) {
     const int px = p % TX, py = p / TX;
     const int ii = i0 - 1 + px, jj = j0 - 1 + py;
-    R sTI = R(0.0), sTJ = R(0.0);
+    R sI[NK], sJ[NK];
+#pragma unroll
+    for (int n = 0; n < NK; ++n) sI[n] = sJ[n] = R(0.0);
     if (ii <= G - 2 && jj <= G - 2) {
-      const int ia = py * PX + px, ib = ia + 1, ic = ia + PX + 1, id = ia + PX;
-      auto C = [&](int dir, int pt, int t) { return P2c(CG.coef_intp, (dir * 3 + pt) * 2 + t, ii, jj, l); };
-      sTI = C(0, 0, 0) * s_v[0][ia] + C(0, 1, 0) * s_v[0][ib] + C(0, 2, 0) * s_v[0][ic] +
-            C(1, 0, 0) * s_v[1][ia] + C(1, 1, 0) * s_v[1][ib] + C(1, 2, 0) * s_v[1][ic] +
-            C(2, 0, 0) * s_v[2][ia] + C(2, 1, 0) * s_v[2][ib] + C(2, 2, 0) * s_v[2][ic];
-      sTJ = C(0, 0, 1) * s_v[0][ia] + C(0, 1, 1) * s_v[0][ic] + C(0, 2, 1) * s_v[0][id] +
-            C(1, 0, 1) * s_v[1][ia] + C(1, 1, 1) * s_v[1][ic] + C(1, 2, 1) * s_v[1][id] +
-            C(2, 0, 1) * s_v[2][ia] + C(2, 1, 1) * s_v[2][ic] + C(2, 2, 1) * s_v[2][id];
+      const int ia = py * PX + px;
+      const int vI[3] = {ia, ia + 1, ia + PX + 1}, vJ[3] = {ia, ia + PX + 1, ia + PX};
+#pragma unroll
+      for (int m = 0; m < 9; ++m) {   // direction m / 3, vertex m % 3, left to right
+        const R cI = P2c(CG.coef_intp, m * 2, ii, jj, l), cJ = P2c(CG.coef_intp, m * 2 + 1, ii, jj, l);
+#pragma unroll
+        for (int n = 0; n < NK; ++n) {
+          const R xI = s_v[n][m / 3][vI[m % 3]], xJ = s_v[n][m / 3][vJ[m % 3]];
+          sI[n] = m ? mad(cI, xI, sI[n]) : cI * xI;
+          sJ[n] = m ? mad(cJ, xJ, sJ[n]) : cJ * xJ;
+        }
+      }
     }
-    s_ti[p] = sTI;
-    s_tj[p] = sTJ;
+#pragma unroll
+    for (int n = 0; n < NK; ++n) {
+      s_ti[n][p] = sI[n];
+      s_tj[n][p] = sJ[n];
+    }
   }
   __syncthreads();
   const int i = i0 + tx, j = j0 + ty;
   if (i > gmax || j > gmax) return;
   const R ddc = CC.divdamp_coef, dt = a.dt, rweight = a.rweight;
-  const int n = cD.npti;
+  const int npt = cD.npti;
   const R* cz = CG.C2WGz;
   const R gx = P2c(CG.GRD_x, 0, i, j, l), gy = P2c(CG.GRD_x, 1, i, j, l), gz = P2c(CG.GRD_x, 2, i, j, l);
   const int q0 = ix(i, j, 0, l);
-  auto Pown = [&](int k2) {
-    const int kc = k2 < kmin ? kmin : (k2 > kmax ? kmax : k2);
-    return __ldg(&a.PS[5][q0 + (int)kc * cD.planei]) * RovCV;
-  };
-  const int ta = (ty + 1) * TX + (tx + 1);
-  const R aTI = s_ti[ta], aTJ = s_tj[ta], bTI = s_ti[ta - 1];
-  const R cTI = s_ti[ta - TX - 1], cTJ = s_tj[ta - TX - 1], dTJ = s_tj[ta - TX];
-  R dd[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-    dd[d] = ddc * (P2c(CG.coef_diff, d * 6 + 0, i, j, l) * (aTI + aTJ) + P2c(CG.coef_diff, d * 6 + 1, i, j, l) * (aTJ + bTI) +
-                   P2c(CG.coef_diff, d * 6 + 2, i, j, l) * (bTI + cTJ) + P2c(CG.coef_diff, d * 6 + 3, i, j, l) * (cTJ + cTI) +
-                   P2c(CG.coef_diff, d * 6 + 4, i, j, l) * (cTI + dTJ) + P2c(CG.coef_diff, d * 6 + 5, i, j, l) * (dTJ + aTI));
-  {
-    const R prd = div_r(dd[0] * gx + dd[1] * gy + dd[2] * gz);
-    dd[0] = dd[0] - div_r(prd * gx);
-    dd[1] = dd[1] - div_r(prd * gy);
-    dd[2] = dd[2] - div_r(prd * gz);
-  }
-  const int c0 = (ty + 1) * PX + (tx + 1);
-  const R s7[7] = {s_p[c0], s_p[c0 + 1], s_p[c0 + PX + 1], s_p[c0 + PX], s_p[c0 - 1], s_p[c0 - PX - 1], s_p[c0 - PX]};
-  const int qkk = q0 + (int)kk * cD.planei, qk1 = qkk + cD.planei;
-  const R P_k1 = Pown(kk + 1), P_k = Pown(kk), P_km = Pown(kk - 1);
-  const R rgh1 = __ldg(&CG.RGAMH[qk1]), rgh0 = __ldg(&CG.RGAMH[qkk]);
-  R pg[3];
+  const int ta = (ty + 1) * TX + (tx + 1), c0 = (ty + 1) * PX + (tx + 1);
+  R dd[NK][3], pg[NK][3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    R g = P2c(CG.coef_grad, d * 7 + 0, i, j, l) * s7[0];
 #pragma unroll
-    for (int m = 1; m < 7; ++m) g = g + P2c(CG.coef_grad, d * 7 + m, i, j, l) * s7[m];
-    const R up = (__ldg(&cz[(2 * d) * n + qk1]) * P_k1 + __ldg(&cz[(2 * d + 1) * n + qk1]) * P_k) * rgh1;
-    const R dn = (__ldg(&cz[(2 * d) * n + qkk]) * P_k + __ldg(&cz[(2 * d + 1) * n + qkk]) * P_km) * rgh0;
-    pg[d] = g + (up - dn) * CC.rdgz[kk];
-  }
-  {
-    const R prd = div_r(pg[0] * gx + pg[1] * gy + pg[2] * gz);
-    pg[0] = pg[0] - div_r(prd * gx);
-    pg[1] = pg[1] - div_r(prd * gy);
-    pg[2] = pg[2] - div_r(prd * gz);
-  }
-  const int q = q0 + (int)k * cD.planei;
-  R v[3];
+    for (int e = 0; e < 6; ++e) {
+      const R cf = P2c(CG.coef_diff, d * 6 + e, i, j, l);
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const R drv = __ldg(&a.gT[1 + d][q]) - pg[d] + dd[d] + R(0.0);
-    v[d] = __ldg(&a.PS[1 + d][q]) + drv * dt;
-    a.dvh[d][q] = v[d];
-    a.PM[1 + d][q] = a.PM[1 + d][q] + v[d] * rweight;
-  }
-  if (k == kmin) {
-    const int pB = q - cD.planei;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const R vB = -R(1.0) * (v[d] / __ldg(&a.rhog[q])) * __ldg(&a.rhog[pB]);
-      a.dvh[d][pB] = vB;
-      a.PM[1 + d][pB] = a.PM[1 + d][pB] + vB * rweight;
+      for (int n = 0; n < NK; ++n) {
+        const R* I = s_ti[n];
+        const R* J = s_tj[n];
+        const R x = e == 0 ? I[ta] + J[ta] : e == 1 ? J[ta] + I[ta - 1] : e == 2 ? I[ta - 1] + J[ta - TX - 1]
+                  : e == 3 ? J[ta - TX - 1] + I[ta - TX - 1] : e == 4 ? I[ta - TX - 1] + J[ta - TX] : J[ta - TX] + I[ta];
+        dd[n][d] = e ? mad(cf, x, dd[n][d]) : cf * x;
+      }
     }
   }
-  if (k == kmax) {
-    const int pT = q + cD.planei;
+  const int nb[7] = {c0, c0 + 1, c0 + PX + 1, c0 + PX, c0 - 1, c0 - PX - 1, c0 - PX};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {
+      const R cf = P2c(CG.coef_grad, d * 7 + m, i, j, l);
+#pragma unroll
+      for (int n = 0; n < NK; ++n) pg[n][d] = m ? mad(cf, s_p[n][nb[m]], pg[n][d]) : cf * s_p[n][nb[m]];
+    }
+  }
+  auto flat = [&](R* x) {   // tangent-plane projection
+    const R prd = div_r(x[0] * gx + x[1] * gy + x[2] * gz);
+    x[0] = x[0] - div_r(prd * gx);
+    x[1] = x[1] - div_r(prd * gy);
+    x[2] = x[2] - div_r(prd * gz);
+  };
+  auto Pown = [&](int k2) {
+    const int kc = k2 < kmin ? kmin : (k2 > kmax ? kmax : k2);
+    return __ldg(&a.PS[5][q0 + kc * cD.planei]) * RovCV;
+  };
+#pragma unroll
+  for (int n = 0; n < NK; ++n) {
+    const int k = ka + n, kk = (k == kmin) ? kmin + 1 : k;
+    if (k > kmax) return;
+    const int qkk = q0 + kk * cD.planei, qk1 = qkk + cD.planei;
+    const R P_k1 = Pown(kk + 1), P_k = Pown(kk), P_km = Pown(kk - 1);
+    const R rgh1 = __ldg(&CG.RGAMH[qk1]), rgh0 = __ldg(&CG.RGAMH[qkk]);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const R vT = R(1.0) * (v[d] / __ldg(&a.rhog[q])) * __ldg(&a.rhog[pT]);
-      a.dvh[d][pT] = vT;
-      a.PM[1 + d][pT] = a.PM[1 + d][pT] + vT * rweight;
+      dd[n][d] = ddc * dd[n][d];
+      const R up = mad(__ldg(&cz[(2 * d + 1) * npt + qk1]), P_k, __ldg(&cz[(2 * d) * npt + qk1]) * P_k1) * rgh1;
+      const R dn = mad(__ldg(&cz[(2 * d + 1) * npt + qkk]), P_km, __ldg(&cz[(2 * d) * npt + qkk]) * P_k) * rgh0;
+      pg[n][d] = pg[n][d] + (up - dn) * CC.rdgz[kk];
+    }
+    flat(dd[n]);
+    flat(pg[n]);
+    const int q = q0 + k * cD.planei;
+    R v[3], pm[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const R drv = __ldg(&a.gT[1 + d][q]) - pg[n][d] + dd[n][d] + R(0.0);
+      v[d] = __ldg(&a.PS[1 + d][q]) + drv * dt;
+      pm[d] = a.PM[1 + d][q];
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      a.dvh[d][q] = v[d];
+      a.PM[1 + d][q] = pm[d] + v[d] * rweight;
+    }
+    if (k == kmin) {
+      const int pB = q - cD.planei;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const R vB = -R(1.0) * (v[d] / __ldg(&a.rhog[q])) * __ldg(&a.rhog[pB]);
+        a.dvh[d][pB] = vB;
+        a.PM[1 + d][pB] = a.PM[1 + d][pB] + vB * rweight;
+      }
+    }
+    if (k == kmax) {
+      const int pT = q + cD.planei;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const R vT = R(1.0) * (v[d] / __ldg(&a.rhog[q])) * __ldg(&a.rhog[pT]);
+        a.dvh[d][pT] = vT;
+        a.PM[1 + d][pT] = a.PM[1 + d][pT] + vT * rweight;
+      }
     }
   }
 }
@@ -1075,8 +1151,8 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, 4, 5))) k_vi
         for (int m = 0; m < 7; ++m) {
 #pragma unroll
           for (int f = 0; f < 3; ++f) {
-            const R t = cdv[d * 7 + m] * s_h[f][d][nb[m]];
-            sv[f] = (m == 0) ? t : sv[f] + t;
+            const R x = s_h[f][d][nb[m]];
+            sv[f] = (m == 0) ? cdv[d * 7 + m] * x : mad(cdv[d * 7 + m], x, sv[f]);
           }
         }
 #pragma unroll

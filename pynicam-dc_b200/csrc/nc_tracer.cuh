@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(TG_DX * TG_DY) k_trc_grad_t(const __grid_const
       if (n >= a.nb) break;
       R g = cg[0] * s_q[n][c0];
 #pragma unroll
-      for (int m = 1; m < 7; ++m) g = g + cg[m] * s_q[n][nb[m]];
+      for (int m = 1; m < 7; ++m) g = mad(cg[m], s_q[n][nb[m]], g);
       a.gq[n][d][qq] = g;
       if (d == 0) a.q[n][qq] = s_q[n][c0];
     }
