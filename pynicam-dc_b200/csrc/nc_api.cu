@@ -621,6 +621,11 @@ static cudaStream_t pole_stream(nc_handle* h) {
   return (h->prof || h->single || !h->stream2) ? h->stream : h->stream2;
 }
 
+// tiles per region, and the regions that take the 16-wide tile
+template <class T>
+static int tiles_of(const Dims& D) { return ((D.G - 2 + T::X - 1) / T::X) * ((D.G - 2 + T::Y - 1) / T::Y); }
+static bool narrow(const Dims& D) { return D.G - 2 <= Tile16::X; }
+
 template <class R>
 static int comm_fields_of(nc_handle* h, const FieldPair* fl, int nf, const char* what) {
   const long long ne = (long long)(h->nr + h->np) * h->D.KA;
@@ -760,8 +765,7 @@ static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
     const int nb = std::min(nx - at, TRC_NB);
     FieldPair* xb = x + at;
     const dim3 pg(pkb, (unsigned)nb);
-    const dim3 gt((unsigned)D.KA, (unsigned)(((D.G - 2 + TG_DX - 1) / TG_DX) * ((D.G - 2 + TG_DY - 1) / TG_DY)),
-                  (unsigned)D.L);
+    const dim3 gt((unsigned)D.KA, (unsigned)(narrow(D) ? tiles_of<Tile16>(D) : tiles_of<Tile32>(D)), (unsigned)D.L);
     TrcGradArgs<R> ga[2];
     TrcRemapArgs<R> ra;
     TrcRemapPlArgs<R> rp;
@@ -794,7 +798,8 @@ static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
     la.rhog_t = RG<R>(h->rhog_t); la.frhog = RG<R>(h->frhog); la.dt = dt;
     lp.ch = PL<R>(h->ch[0]); lp.cm = PL<R>(h->cm[0]); lp.rhog_t = PL<R>(h->rhog_t); lp.frhog = PL<R>(h->frhog);
     lp.flx = PL<R>(h->flx[0]); lp.dt = dt;
-    k_trc_grad_t<<<gt, TG_DX * TG_DY, 0, s>>>(ga[0]);
+    if (narrow(D)) k_trc_grad_t<R, Tile16><<<gt, TILE_THREADS, 0, s>>>(ga[0]);
+    else k_trc_grad_t<R, Tile32><<<gt, TILE_THREADS, 0, s>>>(ga[0]);
     TRY(check_launch(h, "trc_grad"));
     k_trc_grad_pl<<<pg, 32, 0, ps>>>(ga[1]);
     TRY(check_launch(h, "trc_grad_pl"));
@@ -846,7 +851,7 @@ static int column_chunks(const nc_handle* h, int levels) {
   return (int)((levels + n - 1) / n);
 }
 
-template <class R>
+template <class R, class T>
 static int run_step(nc_handle* h) {
   cudaStream_t s = h->stream;
   const cudaStream_t ps = pole_stream(h);
@@ -866,12 +871,8 @@ static int run_step(nc_handle* h) {
   auto pblk = [&](int tb) { return (int)((D.npl + h->blk[tb] - 1) / h->blk[tb]); };
   auto rblk = [&](int tb) { return (int)((D.npt + h->blk[tb] - 1) / h->blk[tb]); };
   // per-level tiled kernels: (levels kmin..kmax, tiles, regions)
-  const dim3 vagrid((unsigned)((D.kmax - D.kmin + VA_NK) / VA_NK),
-                    (unsigned)(((D.G - 2 + DD_DX - 1) / DD_DX) * ((D.G - 2 + DD_DY - 1) / DD_DY)), (unsigned)D.L);
-  const dim3 lvgrid((unsigned)(D.kmax - D.kmin + 1),
-                    (unsigned)(((D.G - 2 + DD_DX - 1) / DD_DX) * ((D.G - 2 + DD_DY - 1) / DD_DY)), (unsigned)D.L);
-  const dim3 lvgrid_vp((unsigned)(D.kmax - D.kmin + 1),
-                       (unsigned)(((D.G - 2 + VP_DX - 1) / VP_DX) * ((D.G - 2 + VP_DY - 1) / VP_DY)), (unsigned)D.L);
+  const int levels = D.kmax - D.kmin + 1, tiles = tiles_of<T>(D);
+  auto lvgrid = [&](int nk) { return dim3((unsigned)((levels + nk - 1) / nk), (unsigned)tiles, (unsigned)D.L); };
   // PROG0 = PROG at the start of the step (mod_dynamics.py:1939-1968)
   for (int v = 0; v < 6; ++v) {
     CU(cudaMemcpyAsync(RG<R>(h->P0[v]), RG<R>(h->P[v]), D.npt * sizeof(R), cudaMemcpyDeviceToDevice, s));
@@ -909,11 +910,10 @@ static int run_step(nc_handle* h) {
     }
     {
       // interior cells, levels kmin..kmax (see k_advmom_t)
-      const int tiles = ((D.G - 2 + 31) / 32) * ((D.G - 2 + 7) / 8);
-      const int nk = tile_chunks(h, tiles * D.L, D.kmax - D.kmin + 1);
-      const dim3 gt((unsigned)tiles, (unsigned)((D.kmax - D.kmin + nk) / nk), (unsigned)D.L);
-      if (gt.y > 1) k_advmom_t<R, true><<<gt, 256, 0, s>>>(am, nk);
-      else k_advmom_t<R, false><<<gt, 256, 0, s>>>(am, nk);
+      const int nk = tile_chunks(h, tiles * D.L, levels);
+      const dim3 gt((unsigned)tiles, (unsigned)((levels + nk - 1) / nk), (unsigned)D.L);
+      if (gt.y > 1) k_advmom_t<R, T, true><<<gt, TILE_THREADS, 0, s>>>(am, nk);
+      else k_advmom_t<R, T, false><<<gt, TILE_THREADS, 0, s>>>(am, nk);
     }
     TRY(check_launch(h, "advmom"));
     k_advmom_pl<<<ppb, 32, 0, ps>>>(amp);
@@ -941,9 +941,8 @@ static int run_step(nc_handle* h) {
     }
     {
       // interior cells; the exchange below fills the halo rows
-      const int tiles = ((D.G - 2 + HD_DX - 1) / HD_DX) * ((D.G - 2 + HD_DY - 1) / HD_DY);
       const dim3 gl2((unsigned)((D.KA + HD_NK - 1) / HD_NK), (unsigned)tiles, (unsigned)D.L);
-      k_hdiff2_m<<<gl2, HD_DX * HD_DY, hdiff2_m_smem<R>(), s>>>(vin, RG<R>(h->P[0]), o2);
+      k_hdiff2_m<R, T><<<gl2, TILE_THREADS, hdiff2_m_smem<R, T>(), s>>>(vin, RG<R>(h->P[0]), o2);
       TRY(check_launch(h, "hdiff2"));
     }
     k_hdiff2_pl<<<pkb, 32, 0, ps>>>(vinp, PL<R>(h->P[0]), o2p);
@@ -985,10 +984,10 @@ static int run_step(nc_handle* h) {
       for (int d = 0; d < 3; ++d) { o.f[d] = RG<R>(h->vtmp2[d]); op.f[d] = PL<R>(h->vtmp2[d]); }
       // interior cells only: halo rows are filled by the exchange below and the
       // boundary levels of vtmp2 stay zero from allocation
-      const unsigned tx = (unsigned)((D.G - 2 + DD_DX - 1) / DD_DX), ty = (unsigned)((D.G - 2 + DD_DY - 1) / DD_DY);
-      const int nk = tile_chunks(h, (int)(tx * ty) * D.L, D.kmax - D.kmin + 1);
-      const dim3 gt(tx, ty, (unsigned)(D.L * ((D.kmax - D.kmin + nk) / nk)));
-      k_dd3d_m<R, true><<<gt, DD_DX * DD_DY, dd3d_m_smem<R>(), s>>>(v, o, nk);
+      const unsigned tx = (unsigned)((D.G - 2 + T::X - 1) / T::X), ty = (unsigned)((D.G - 2 + T::Y - 1) / T::Y);
+      const int nk = tile_chunks(h, tiles * D.L, levels);
+      const dim3 gt(tx, ty, (unsigned)(D.L * ((levels + nk - 1) / nk)));
+      k_dd3d_m<R, T, true><<<gt, TILE_THREADS, dd3d_m_smem<R, T>(), s>>>(v, o, nk);
       TRY(check_launch(h, "dd3d"));
       k_dd3d_pl<<<pkb, 32, 0, ps>>>(vp, op);
       TRY(check_launch(h, "dd3d_pl"));
@@ -1015,8 +1014,7 @@ static int run_step(nc_handle* h) {
       }
       Vp0H<R> vh;
       for (int n = 0; n < 8; ++n) vh.out[n] = RG<R>(h->vph[n]);
-      const dim3 hgrid((lvgrid_vp.x + VP_NK<R> - 1) / VP_NK<R>, lvgrid_vp.y, lvgrid_vp.z);
-      k_vp0_hl<R, VP_NK<R>><<<hgrid, VP_DX * VP_DY, 0, s>>>(v0[0], vh);
+      k_vp0_hl<R, T, VP_NK<R>><<<lvgrid(VP_NK<R>), TILE_THREADS, 0, s>>>(v0[0], vh);
       TRY(check_launch(h, "vp0_h"));
       const int tb = h->blk[TB_VP0C];
       const int nk = column_chunks(h, D.KA);
@@ -1048,8 +1046,7 @@ static int run_step(nc_handle* h) {
           for (int n = 0; n < 5; ++n) pa.PM[n] = F(h->PM[n]);
           pa.dt = h->dts; pa.rweight = rweight; pa.RovCV = RovCV;
         }
-        const dim3 pgrid((lvgrid.x + P1_NK<R> - 1) / P1_NK<R>, lvgrid.y, lvgrid.z);
-        k_path1_l<R, P1_NK<R>, P1_MINB<R>><<<pgrid, DD_DX * DD_DY, 0, s>>>(p1[0]);
+        k_path1_l<R, T, P1_NK<R>, P1_MINB<R>><<<lvgrid(P1_NK<R>), TILE_THREADS, 0, s>>>(p1[0]);
         TRY(check_launch(h, "path1"));
         k_path1_pl<<<ppb, 32, 0, ps>>>(p1[1]);
         TRY(check_launch(h, "path1_pl"));
@@ -1069,8 +1066,8 @@ static int run_step(nc_handle* h) {
         va.PM0 = F(h->PM[0]); va.PM4 = F(h->PM[4]);
         va.dt = h->dts; va.rweight = rweight; va.RovCV = RovCV;
       }
-      if constexpr (std::is_same<R, float>::value) k_vimain_a_m<<<vagrid, DD_DX * DD_DY, 0, s>>>(vi[0]);
-      else k_vimain_a_l<<<lvgrid, DD_DX * DD_DY, 0, s>>>(vi[0]);
+      if constexpr (std::is_same<R, float>::value) k_vimain_a_m<R, T><<<lvgrid(VA_NK), TILE_THREADS, 0, s>>>(vi[0]);
+      else k_vimain_a_l<R, T><<<lvgrid(1), TILE_THREADS, 0, s>>>(vi[0]);
       TRY(check_launch(h, "vimain_a"));
       {
         const int ncol = D.L * (D.G - 2) * (D.G - 2);
@@ -1294,7 +1291,9 @@ static int mass_sum(nc_handle* h, int n) {
                                                 h->mass_part);
   return check_launch(h, "mass");
 }
-static int step_once(nc_handle* h) { return h->mixed ? run_step<float>(h) : run_step<double>(h); }
+template <class T>
+static int step_tiled(nc_handle* h) { return h->mixed ? run_step<float, T>(h) : run_step<double, T>(h); }
+static int step_once(nc_handle* h) { return narrow(h->D) ? step_tiled<Tile16>(h) : step_tiled<Tile32>(h); }
 // forget the captured step (the next nc_step captures it again)
 static int drop_graph(nc_handle* h) {
   if (h->gexec || h->graph) CU(cudaStreamSynchronize(h->stream));
@@ -1411,15 +1410,15 @@ static int hlin_tl(nc_handle* h) {
   const cudaStream_t s = h->stream;
   const unsigned pkb = (unsigned)((D.KA * D.LP + 127) / 128), cb = (unsigned)((D.npt + 127) / 128);
   {
-    const dim3 gt((unsigned)D.KA, (unsigned)(((D.G - 2 + TG_DX - 1) / TG_DX) * ((D.G - 2 + TG_DY - 1) / TG_DY)),
-                  (unsigned)D.L);
+    const dim3 gt((unsigned)D.KA, (unsigned)(narrow(D) ? tiles_of<Tile16>(D) : tiles_of<Tile32>(D)), (unsigned)D.L);
     for (int pole = 0; pole < 2; ++pole) {
       auto F = [&](int n) { return pole ? L[n].p : L[n].r; };
       TrcGradArgs<double> ga;
       ga.rhogq[0] = F(LN_T1); ga.rhog_t = F(LN_RHO); ga.q[0] = F(LN_DQ);
       for (int d = 0; d < 3; ++d) ga.gq[0][d] = F(LN_DG0 + d);
       ga.nb = 1;
-      if (!pole) k_trc_grad_t<<<gt, TG_DX * TG_DY, 0, s>>>(ga);
+      if (!pole && narrow(D)) k_trc_grad_t<double, Tile16><<<gt, TILE_THREADS, 0, s>>>(ga);
+      else if (!pole) k_trc_grad_t<double, Tile32><<<gt, TILE_THREADS, 0, s>>>(ga);
       else k_trc_grad_pl<<<pkb, 128, 0, s>>>(ga);
       TRY(check_launch(h, pole ? "lin_grad_pl" : "lin_grad"));
     }
@@ -1713,10 +1712,14 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
   }
   // the multi-level hyperdiffusion kernel takes more than the default 48 KB of
   // dynamic shared memory in its float64 instance
-  CU(cudaFuncSetAttribute(k_hdiff2_m<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<double>()));
-  CU(cudaFuncSetAttribute(k_hdiff2_m<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<float>()));
-  CU(cudaFuncSetAttribute(k_dd3d_m<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double>()));
-  CU(cudaFuncSetAttribute(k_dd3d_m<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float>()));
+  CU(cudaFuncSetAttribute(k_hdiff2_m<double, Tile32>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<double, Tile32>()));
+  CU(cudaFuncSetAttribute(k_hdiff2_m<double, Tile16>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<double, Tile16>()));
+  CU(cudaFuncSetAttribute(k_hdiff2_m<float, Tile32>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<float, Tile32>()));
+  CU(cudaFuncSetAttribute(k_hdiff2_m<float, Tile16>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<float, Tile16>()));
+  CU(cudaFuncSetAttribute(k_dd3d_m<double, Tile32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double, Tile32>()));
+  CU(cudaFuncSetAttribute(k_dd3d_m<double, Tile16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double, Tile16>()));
+  CU(cudaFuncSetAttribute(k_dd3d_m<float, Tile32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float, Tile32>()));
+  CU(cudaFuncSetAttribute(k_dd3d_m<float, Tile16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float, Tile16>()));
   // the column kernel of vi_main: five doubles per level of 32 columns (164 KB at NC_MAXK levels)
   for (const void* f : {(const void*)k_vi_col<double, true, false>, (const void*)k_vi_col<double, false, false>,
                         (const void*)k_vi_col<double, false, true>, (const void*)k_vi_col<float, true, false>,

@@ -168,7 +168,7 @@ struct AdvMomArgs {
   R *gvx, *gvy, *gvz, *gw;               // out
 };
 
-// Tiled momentum advection for interior cells: one block per 32x8 tile of a
+// Tiled momentum advection for interior cells: one block per tile of a
 // region, marching upward over kmin..kmax (the vertical-momentum tendency at k
 // needs the projection at k-1, and the half-level flux at k is reused from the
 // level below).  Per level the haloed tile of rhogv, the merged velocity and
@@ -181,9 +181,9 @@ struct AdvMomArgs {
 // SMs idle (see tile_chunks); a chunk walks two levels below its first
 // without storing them, for the projection and the flux that its first needs.
 // (SPLIT; the unsplit instance keeps the registers of the chunk's bounds)
-template <class R, bool SPLIT>
-__global__ void __launch_bounds__(256, NC_MINB(R, 2, NC_F32_ADVMOM)) k_advmom_t(AdvMomArgs<R> a, int nk) {
-  constexpr int TXD = 32, TYD = 8;
+template <class R, class T, bool SPLIT>
+__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, NC_F32_ADVMOM)) k_advmom_t(AdvMomArgs<R> a, int nk) {
+  constexpr int TXD = T::X, TYD = T::Y;
   constexpr int PX = TXD + 2, PY = TYD + 2;
   __shared__ R s_rv[3][PY * PX], s_vv[3][PY * PX], s_rg[PY * PX];
   const int ntx = (cD.G - 2 + TXD - 1) / TXD;
@@ -421,8 +421,6 @@ __global__ void k_intp_weights(const double* ci, double* w, int npt2) {
     }
 }
 
-#define HD_DX 32
-#define HD_DY 8
 
 // Kh of the hyperdiffusion at level k: the uniform DIRECT coefficient, or for
 // NONLINEAR1 (mod_numfilter.py:1153-1184) the coefficient from the
@@ -435,7 +433,7 @@ __device__ __forceinline__ R hdiff_kh(R lapT, int k) {
   return fmin(fmax(c, CC.nl_min), CC.nl_khmax[k]);
 }
 
-// Second hyperdiffusion pass, one block per (HD_NK levels, HD_DX x HD_DY tile)
+// Second hyperdiffusion pass, one block per (HD_NK levels, tile)
 // of interior cells: the haloed tile of the six Laplacians and of rhog is
 // staged in shared memory per level, the triangle gradients of the
 // temperature and density Laplacians are formed once (with the singular-point
@@ -446,14 +444,14 @@ __device__ __forceinline__ R hdiff_kh(R lapT, int k) {
 // staged in shared memory and the cell's Laplacian and diffusion coefficients
 // (coef_lap 7, coef_diff 18) held in registers once for all of the block's
 // levels, instead of re-read from L2 at every level.  Dynamic shared memory:
-// hdiff2_m_smem<R>() bytes (45 KB float, 90 KB double).  Kh per cell from
+// hdiff2_m_smem<R, T>() bytes (45 KB float, 90 KB double).  Kh per cell from
 // hdiff_kh (the first pass's temperature Laplacian is the staged field 4).
 #ifndef HD_NK
 #define HD_NK 6
 #endif
-template <class R>
+template <class R, class T>
 constexpr int hdiff2_m_smem() {
-  return ((18 + 12) * (HD_DX + 1) * (HD_DY + 1) + 7 * (HD_DX + 2) * (HD_DY + 2)) * (int)sizeof(R);
+  return ((18 + 12) * (T::X + 1) * (T::Y + 1) + 7 * (T::X + 2) * (T::Y + 2)) * (int)sizeof(R);
 }
 template <class R>
 __global__ void k_hdiff2_pl(const __grid_constant__ Six<R> vt, const R* rhog, const __grid_constant__ SixOut<R> out) {
@@ -502,21 +500,21 @@ __global__ void k_hdiff2_pl(const __grid_constant__ Six<R> vt, const R* rhog, co
   }
 }
 
-template <class R>
-__global__ void __launch_bounds__(HD_DX * HD_DY, NC_MINB(R, 2, 4)) k_hdiff2_m(Six<R> vt, const R* rhog,
+template <class R, class T>
+__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, 4)) k_hdiff2_m(Six<R> vt, const R* rhog,
                                                                             SixOut<R> out) {
-  constexpr int PX = HD_DX + 2, PY = HD_DY + 2, NP = PX * PY, TX = HD_DX + 1, TY = HD_DY + 1, NT = TX * TY;
+  constexpr int PX = T::X + 2, PY = T::Y + 2, NP = PX * PY, TX = T::X + 1, TY = T::Y + 1, NT = TX * TY;
   extern __shared__ __align__(16) unsigned char hd_smem[];
   R* s_w = reinterpret_cast<R*>(hd_smem);   // [18][NT] triangle weights
   R* s_f = s_w + 18 * NT;                     // [6][NP] the six Laplacians
   R* s_r = s_f + 6 * NP;                      // [NP] rhog
   R* s_t = s_r + NP;                          // [2][6][NT] triangle values of fields 4 and 5
   const int l = (int)blockIdx.z;
-  const int ntx = (cD.G - 2 + HD_DX - 1) / HD_DX;
-  const int i0 = 1 + ((int)blockIdx.y % ntx) * HD_DX, j0 = 1 + ((int)blockIdx.y / ntx) * HD_DY;
+  const int ntx = (cD.G - 2 + T::X - 1) / T::X;
+  const int i0 = 1 + ((int)blockIdx.y % ntx) * T::X, j0 = 1 + ((int)blockIdx.y / ntx) * T::Y;
   const int k0 = (int)blockIdx.x * HD_NK, k1 = min(k0 + HD_NK, cD.KA);
   const int G = cD.G, gmax = cD.G - 2;
-  const int tid = threadIdx.x, tx = tid % HD_DX, ty = tid / HD_DX;
+  const int tid = threadIdx.x, tx = tid % T::X, ty = tid / T::X;
   const int i = i0 + tx, j = j0 + ty;
   const bool own = (i <= gmax) && (j <= gmax);
   const R kfac[2] = {CC.CVdry, CC.hdiff_fact_rho};

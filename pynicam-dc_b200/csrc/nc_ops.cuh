@@ -52,6 +52,13 @@ __device__ __forceinline__ bool map_col(int pole, int t, int& i, int& j, int& l,
   return true;
 }
 
+// Tile shapes (cells of a region along i and j; 256 threads): 32 x 8, or 16 x 16
+// for regions of at most 16 cells a side (gl05 and coarser at 40 regions), of
+// which a 32-wide tile leaves half the lanes idle.
+struct Tile32 { static constexpr int X = 32, Y = 8; };
+struct Tile16 { static constexpr int X = 16, Y = 16; };
+#define TILE_THREADS 256
+
 // Thread -> grid point of a launch whose first npb blocks (along x) take the
 // pole points and the others the regional points, halo ring included.  A
 // thread per point: where a level needs its neighbours' half-level values it

@@ -26,7 +26,7 @@ __device__ __forceinline__ R ddivd(int i, int j, int l, int d, const R aTI, cons
          P2(CG.coef_diff, d * 6 + 4, i, j, l) * (cTI + dTJ) + P2(CG.coef_diff, d * 6 + 5, i, j, l) * (dTJ + aTI);
 }
 
-// Tiled 3-D divergence damping: one block per DD_DX x DD_DY tile of output
+// Tiled 3-D divergence damping: one block per T::X x T::Y tile of output
 // cells of one region, marching upward in k.  Per level the block stages the
 // haloed tile of RGAM-scaled momentum and the vertical mass flux rwv(k+1) in
 // shared memory (rwv(k) is kept from the level below), evaluates every
@@ -36,22 +36,13 @@ __device__ __forceinline__ R ddivd(int i, int j, int l, int d, const R aTI, cons
 // ((rwv(k+1) summed over the vertices) - (rwv(k) summed)) / 3 * rdgz(k)
 // (kernels/oprt3ddivdamp.py:50-173); the rwv sums and coefficient products
 // are added left to right in the reference's order.
-#ifndef DD_DX
-#define DD_DX 32
-#endif
-#ifndef DD_DY
-#define DD_DY 8
-#endif
-// resident blocks per SM for a register budget of n blocks of 256 threads
-#define DD_MINB(n) ((n) * 256 / (DD_DX * DD_DY) > 0 ? (n) * 256 / (DD_DX * DD_DY) : 1)
 // The tile's k-invariant coefficients are read once per block instead of
 // once per level: the triangle weights coef_intp (18 planes) staged in shared
 // memory, the cell's coef_diff (18) held in registers (CDR) or read per
-// level.  Dynamic shared memory dd3d_m_smem<R>().
-template <class R>
+// level.  Dynamic shared memory dd3d_m_smem<R, T>().
+template <class R, class T>
 constexpr int dd3d_m_smem() {
-  return (18 * (DD_DX + 1) * (DD_DY + 1) + 5 * (DD_DX + 2) * (DD_DY + 2) + 2 * (DD_DX + 1) * (DD_DY + 1)) *
-         (int)sizeof(R);
+  return (18 * (T::X + 1) * (T::Y + 1) + 5 * (T::X + 2) * (T::Y + 2) + 2 * (T::X + 1) * (T::Y + 1)) * (int)sizeof(R);
 }
 #ifndef DD_M_MINB
 #define DD_M_MINB 2
@@ -107,11 +98,11 @@ __global__ void k_dd3d_pl(const __grid_constant__ Four<R> v, const __grid_consta
 
 // The levels are split into chunks of nk where the tiles alone leave SMs idle
 // (see tile_chunks); blockIdx.z counts (region, chunk).
-template <class R, bool CDR>
-__global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4))) k_dd3d_m(Four<R> v, Three<R> out,
+template <class R, class T, bool CDR>
+__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, DD_M_MINB, 4)) k_dd3d_m(Four<R> v, Three<R> out,
                                                                                            int nk) {
-  constexpr int PX = DD_DX + 2, PY = DD_DY + 2, NP = PX * PY;
-  constexpr int TX = DD_DX + 1, TY = DD_DY + 1, NT = TX * TY;
+  constexpr int PX = T::X + 2, PY = T::Y + 2, NP = PX * PY;
+  constexpr int TX = T::X + 1, TY = T::Y + 1, NT = TX * TY;
   extern __shared__ __align__(16) unsigned char dd_smem[];
   R* s_ci = reinterpret_cast<R*>(dd_smem);   // [18][NT] coef_intp of each triangle
   R* s_vm = s_ci + 18 * NT;                    // [3][NP]
@@ -120,9 +111,9 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4
   R* s_tj = s_ti + NT;                         // [NT]
   const int l = (int)blockIdx.z % cD.L;
   const int ka = cD.kmin + (int)blockIdx.z / cD.L * nk, kb = min(ka + nk - 1, cD.kmax);
-  const int i0 = 1 + blockIdx.x * DD_DX, j0 = 1 + blockIdx.y * DD_DY;
+  const int i0 = 1 + blockIdx.x * T::X, j0 = 1 + blockIdx.y * T::Y;
   const int G = cD.G, gmax = cD.G - 2;
-  const int tid = threadIdx.x, tx = tid % DD_DX, ty = tid / DD_DX;
+  const int tid = threadIdx.x, tx = tid % T::X, ty = tid / T::X;
   const int i = i0 + tx, j = j0 + ty;
   const bool own = (i <= gmax) && (j <= gmax);
   const int n = cD.npti;
@@ -231,8 +222,9 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, DD_M_MINB, 4
 struct TileLv {
   int k, l, i0, j0;
 };
-template <int TDX, int TDY>
+template <class T>
 __device__ __forceinline__ TileLv tile_level(int kbase) {
+  constexpr int TDX = T::X, TDY = T::Y;
   const int ntx = (cD.G - 2 + TDX - 1) / TDX;
   TileLv t;
   t.k = kbase + (int)blockIdx.x;
@@ -467,24 +459,21 @@ struct Vp0H {
 // vp0 horizontal terms, one block per (NK levels, tile): like k_path1_l, each of
 // the 78 coefficients is loaded once and applied to the block's NK levels (the
 // float32 instance; two float64 levels do not leave room for four blocks of
-// shared memory).  vp0 keeps a 32x8 tile: its staged fields need more than the
-// 48 KB of static shared memory at larger tiles.
-#define VP_DX 32
-#define VP_DY 8
+// shared memory). 
 template <class R> constexpr int VP_NK = sizeof(R) == 8 ? 1 : 2;
-template <class R, int NK>
-__global__ void __launch_bounds__(VP_DX * VP_DY, NC_MINB(R, 4, NC_F32_VP0H)) k_vp0_hl(Vp0Args<R> a, Vp0H<R> h) {
-  constexpr int PX = VP_DX + 2, PY = VP_DY + 2, TX = VP_DX + 1, TY = VP_DY + 1, NP = PX * PY, NT = TX * TY;
+template <class R, class T, int NK>
+__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 4, NC_F32_VP0H)) k_vp0_hl(Vp0Args<R> a, Vp0H<R> h) {
+  constexpr int PX = T::X + 2, PY = T::Y + 2, TX = T::X + 1, TY = T::Y + 1, NP = PX * PY, NT = TX * TY;
   __shared__ R s_m[NK][3][NP];    // RGAM * rhogv
   __shared__ R s_e[NK][3][NP];    // RGAM * rhogv * eth
   __shared__ R s_v[NK][3][NP];    // -vtmp2
   __shared__ R s_p[NK][NP];       // RGAM * pregd at the gradient level
   __shared__ R s_ti[NK][NT], s_tj[NK][NT];
-  const TileLv tl = tile_level<VP_DX, VP_DY>(0);
+  const TileLv tl = tile_level<T>(0);
   const int l = tl.l, i0 = tl.i0, j0 = tl.j0;
   const int G = cD.G, gmax = cD.G - 2, kmin = cD.kmin, kmax = cD.kmax;
   const int ka = kmin + tl.k * NK;
-  const int tid = threadIdx.x, tx = tid % VP_DX, ty = tid / VP_DX;
+  const int tid = threadIdx.x, tx = tid % T::X, ty = tid / T::X;
   const R* cz = CG.C2WGz;
   const R* const* P = a.P.v;
   for (int p = tid; p < NP; p += blockDim.x) {
@@ -844,17 +833,17 @@ __global__ void k_path1_pl(const __grid_constant__ Path1Args<R> a) {
 #endif
 template <class R> constexpr int P1_NK = sizeof(R) == 8 ? P1_NK_F64 : P1_NK_F32;
 template <class R> constexpr int P1_MINB = sizeof(R) == 8 ? P1_MINB_F64 : P1_MINB_F32;
-template <class R, int NK, int MINB>
-__global__ void __launch_bounds__(DD_DX * DD_DY, MINB) k_path1_l(Path1Args<R> a) {
-  constexpr int PX = DD_DX + 2, PY = DD_DY + 2, TX = DD_DX + 1, TY = DD_DY + 1, NP = PX * PY, NT = TX * TY;
+template <class R, class T, int NK, int MINB>
+__global__ void __launch_bounds__(TILE_THREADS, MINB) k_path1_l(Path1Args<R> a) {
+  constexpr int PX = T::X + 2, PY = T::Y + 2, TX = T::X + 1, TY = T::Y + 1, NP = PX * PY, NT = TX * TY;
   __shared__ R s_v[NK][3][NP];
   __shared__ R s_p[NK][NP];
   __shared__ R s_ti[NK][NT], s_tj[NK][NT];
-  const TileLv tl = tile_level<DD_DX, DD_DY>(0);
+  const TileLv tl = tile_level<T>(0);
   const int l = tl.l, i0 = tl.i0, j0 = tl.j0;
   const int G = cD.G, gmax = cD.G - 2, kmin = cD.kmin, kmax = cD.kmax;
   const int ka = kmin + tl.k * NK;
-  const int tid = threadIdx.x, tx = tid % DD_DX, ty = tid / DD_DX;
+  const int tid = threadIdx.x, tx = tid % T::X, ty = tid / T::X;
   const R RovCV = a.RovCV;
   for (int p = tid; p < NP; p += blockDim.x) {
     const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
@@ -1033,14 +1022,14 @@ __global__ void k_vimain_a_pl(const __grid_constant__ VimainArgs<R> a) {
 
 // vi_main kernel A, one block per (level, tile): the horizontal divergences
 // of RGAM*diff_vh, RGAM*diff_vh*eth and RGAM*(rhogv + diff_vh)*ethtot0.
-template <class R>
-__global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, 6, NC_F32_VIMAINA))) k_vimain_a_l(VimainArgs<R> a) {
-  constexpr int PX = DD_DX + 2, PY = DD_DY + 2;
+template <class R, class T>
+__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 6, NC_F32_VIMAINA)) k_vimain_a_l(VimainArgs<R> a) {
+  constexpr int PX = T::X + 2, PY = T::Y + 2;
   __shared__ R s_h[3][3][PY * PX];
-  const TileLv tl = tile_level<DD_DX, DD_DY>(cD.kmin);
+  const TileLv tl = tile_level<T>(cD.kmin);
   const int l = tl.l, i0 = tl.i0, j0 = tl.j0;
   const int G = cD.G, gmax = cD.G - 2;
-  const int tid = threadIdx.x, tx = tid % DD_DX, ty = tid / DD_DX;
+  const int tid = threadIdx.x, tx = tid % T::X, ty = tid / T::X;
   const int i = i0 + tx, j = j0 + ty;
   const bool own = (i <= gmax) && (j <= gmax);
   {
@@ -1101,16 +1090,16 @@ __global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, 6, NC_F32_VI
 #ifndef VA_NK
 #define VA_NK 5
 #endif
-template <class R>
-__global__ void __launch_bounds__(DD_DX * DD_DY, DD_MINB(NC_MINB(R, 4, 5))) k_vimain_a_m(VimainArgs<R> a) {
-  constexpr int PX = DD_DX + 2, PY = DD_DY + 2;
+template <class R, class T>
+__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 4, 5)) k_vimain_a_m(VimainArgs<R> a) {
+  constexpr int PX = T::X + 2, PY = T::Y + 2;
   __shared__ R s_h[3][3][PY * PX];
-  const int ntx = (cD.G - 2 + DD_DX - 1) / DD_DX;
+  const int ntx = (cD.G - 2 + T::X - 1) / T::X;
   const int l = (int)blockIdx.z;
-  const int i0 = 1 + ((int)blockIdx.y % ntx) * DD_DX, j0 = 1 + ((int)blockIdx.y / ntx) * DD_DY;
+  const int i0 = 1 + ((int)blockIdx.y % ntx) * T::X, j0 = 1 + ((int)blockIdx.y / ntx) * T::Y;
   const int ka = cD.kmin + (int)blockIdx.x * VA_NK, kb = min(ka + VA_NK - 1, cD.kmax);
   const int G = cD.G, gmax = cD.G - 2;
-  const int tid = threadIdx.x, tx = tid % DD_DX, ty = tid / DD_DX;
+  const int tid = threadIdx.x, tx = tid % T::X, ty = tid / T::X;
   const int i = i0 + tx, j = j0 + ty;
   const bool own = (i <= gmax) && (j <= gmax);
   R cdv[21];

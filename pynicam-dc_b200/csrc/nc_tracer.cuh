@@ -355,15 +355,13 @@ __global__ void k_trc_hflux_pl(TrcHfluxPlArgs<R> a) {
 // ---------------------------------------------------------------------------
 // per tracer: q and its gradient (mod_src_tracer.py:758-771, 1634-1640)
 // ---------------------------------------------------------------------------
-// One block per (level, 32 x 8 tile of interior cells): q of the haloed tile
+// One block per (level, tile of interior cells): q of the haloed tile
 // is formed once into shared memory (one division per cell instead of one per
 // stencil use), then each cell's gradient is read from there.  The region's
 // halo cells get q and a zero gradient from the tile that holds their nearest
 // interior cell, so every cell is written exactly once.
 // The tracers of a batch (up to TRC_NB) share the block: each gradient
 // coefficient and each cell's density is read once for all of them.
-#define TG_DX 32
-#define TG_DY 8
 #define TRC_NB 4
 template <class R>
 struct TrcGradArgs {
@@ -372,11 +370,11 @@ struct TrcGradArgs {
   R *q[TRC_NB], *gq[TRC_NB][3];
   int nb;
 };
-template <class R>
-__global__ void __launch_bounds__(TG_DX * TG_DY) k_trc_grad_t(const __grid_constant__ TrcGradArgs<R> a) {
-  constexpr int PX = TG_DX + 2, PY = TG_DY + 2, NP = PX * PY;
+template <class R, class T>
+__global__ void __launch_bounds__(TILE_THREADS) k_trc_grad_t(const __grid_constant__ TrcGradArgs<R> a) {
+  constexpr int PX = T::X + 2, PY = T::Y + 2, NP = PX * PY;
   __shared__ R s_q[TRC_NB][NP];
-  const TileLv tl = tile_level<TG_DX, TG_DY>(0);
+  const TileLv tl = tile_level<T>(0);
   const int k = tl.k, l = tl.l, i0 = tl.i0, j0 = tl.j0;
   const int G = cD.G, gmax = cD.G - 2;
   const int tid = threadIdx.x;
@@ -387,7 +385,7 @@ __global__ void __launch_bounds__(TG_DX * TG_DY) k_trc_grad_t(const __grid_const
     bool mine = false;   // a halo cell of the region that this tile writes
     if (ok && !interior(ii, jj)) {
       const int ci = min(max(ii, 1), gmax), cj = min(max(jj, 1), gmax);
-      mine = ci >= i0 && ci < i0 + TG_DX && cj >= j0 && cj < j0 + TG_DY;
+      mine = ci >= i0 && ci < i0 + T::X && cj >= j0 && cj < j0 + T::Y;
     }
     const typename DivOf<R>::type den(ok ? __ldg(a.rhog_t + qq) : R(1.0));
 #pragma unroll
@@ -404,7 +402,7 @@ __global__ void __launch_bounds__(TG_DX * TG_DY) k_trc_grad_t(const __grid_const
     }
   }
   __syncthreads();
-  const int tx = tid % TG_DX, ty = tid / TG_DX;
+  const int tx = tid % T::X, ty = tid / T::X;
   const int i = i0 + tx, j = j0 + ty;
   if (i > gmax || j > gmax) return;
   const int qq = ix(i, j, k, l);
