@@ -128,160 +128,172 @@ struct VadvLin {
 __device__ __forceinline__ int amin2(double a, double b) { return (a < b) ? 0 : 1; }
 __device__ __forceinline__ int amax2(double a, double b) { return (a > b) ? 0 : 1; }
 
-__device__ void vadv_lin_column(const Col c, const VadvLin& a) {
+// One thread per level and column: a block takes VL_COLS columns and their kall
+// levels (at most NC_ADJ_K), and the levels hand each other q, the outflow
+// bounds, the limited faces and the cotangents through shared memory (nothing
+// here is a recurrence: every quantity takes its neighbours' values of the
+// stage before).  A column per thread kept twenty per-level arrays in local
+// memory (0.9 ms a call at gl06 z60).
+#define VL_COLS 16
+static inline size_t vadv_lin_smem(int KA) { return (size_t)7 * (KA + 2) * VL_COLS * sizeof(double); }
+
+__global__ void __launch_bounds__(VL_COLS * NC_ADJ_K) k_vadv_lin(const __grid_constant__ VadvLin a, int pole) {
+  extern __shared__ __align__(16) double vl_sm[];
   const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
   const double BIG = cC.HUGE_, EPS = cC.EPS;
-  double q[NC_ADJ_K], raw[NC_ADJ_K], omin[NC_ADJ_K], omax[NC_ADJ_K];
-  double fk[NC_ADJ_K], zk[NC_ADJ_K], Ak[NC_ADJ_K], c1v[NC_ADJ_K], c2v[NC_ADJ_K];
-  // branch record per level: upwind sides; argument of the Q bounds (0 qc, 1 neighbour);
-  // qnmin / qnmax (0 QL, 1 QU, 2 qc); limited face (0 raw, 1 lower bound, 2 upper bound)
-  signed char inL[NC_ADJ_K], inU[NC_ADJ_K], sminL[NC_ADJ_K], sminU[NC_ADJ_K], smaxL[NC_ADJ_K], smaxU[NC_ADJ_K];
-  signed char snmin[NC_ADJ_K], snmax[NC_ADJ_K], sh[NC_ADJ_K];
-  bool clamped[NC_ADJ_K];
-  for (int k = 0; k < KA; ++k) q[k] = a.rhogq[c.at(k)] / a.den[c.at(k)];
-  for (int k = kmin; k <= kmax + 1; ++k) raw[k] = cC.afact[k] * q[k] + cC.bfact[k] * q[k - 1];
-  for (int k = kmin; k <= kmax; ++k) {
-    const int p = c.at(k);
-    const double denk = a.den[p];
-    const double ck0 = -a.flx_v[p] / denk * cC.rdgz[k];
-    const double ck1 = a.flx_v[c.at(k + 1)] / denk * cC.rdgz[k];
-    const double ck0p = (k + 1 <= kmax) ? -a.flx_v[c.at(k + 1)] / a.den[c.at(k + 1)] * cC.rdgz[k + 1] : 0.0;
+  const int lane = (int)(threadIdx.x % VL_COLS), k = (int)(threadIdx.x / VL_COLS);   // blockDim.x = VL_COLS * KA
+  const int ncol = pole ? 6 * cD.LP : cD.npt2i;
+  const int t0 = (int)blockIdx.x * VL_COLS + lane;
+  const bool act = t0 < ncol;              // surplus lanes repeat the last column and store nothing
+  int i, j, l, g, lp;
+  map_col(pole, act ? t0 : ncol - 1, i, j, l, g, lp);
+  const Col c = pole ? col_pl(g, lp) : col_reg(i, j, l);
+  // rows -1 .. KA of each array; the rows beyond the column stay zero
+  const int st = (KA + 2) * VL_COLS, at = (k + 1) * VL_COLS + lane;
+  double* s_q = vl_sm + at;
+  double* s_d = s_q + st;       // perturbation of q (TL)
+  double* s_n = s_d + st;       // lower bound
+  double* s_x = s_n + st;       // upper bound
+  double* s_h = s_x + st;       // limited face
+  double* s_a = s_h + st;       // TL: face; AD: contribution to the level above, ...
+  double* s_b = s_a + st;       // ... and below
+  if (k == 0 || k == KA - 1) {
+    const int o = k == 0 ? -VL_COLS : VL_COLS;
+    s_q[o] = s_d[o] = s_n[o] = s_x[o] = s_h[o] = s_a[o] = s_b[o] = 0.0;
+    if (KA == 1) s_q[VL_COLS] = s_d[VL_COLS] = s_n[VL_COLS] = s_x[VL_COLS] = s_h[VL_COLS] = s_a[VL_COLS] = s_b[VL_COLS] = 0.0;
+  }
+  const int p = c.at(k);
+  const bool in = k >= kmin && k <= kmax;
+  const double den = __ldg(a.den + p), rq = __ldg(a.rhogq + p), q0 = rq / den;
+  const double flx = __ldg(a.flx_v + p), flxu = in ? __ldg(a.flx_v + c.at(k + 1)) : 0.0;
+  const double inv = a.mode ? __ldg(a.in + p) : 0.0;
+  const double rdz = cC.rdgz[k];
+  s_q[0] = q0;
+  s_d[0] = a.mode == 1 ? inv / den : 0.0;
+  s_n[0] = s_x[0] = s_h[0] = s_a[0] = s_b[0] = 0.0;
+  __syncthreads();
+  const double qb = s_q[-VL_COLS], qa = s_q[VL_COLS];
+  const double raw = cC.afact[k] * q0 + cC.bfact[k] * qb;      // k = kmin .. kmax + 1
+  // branches of level k: upwind sides; argument of the Q bounds (0 qc, 1 neighbour);
+  // qnmin / qnmax (0 QL, 1 QU, 2 qc)
+  bool inL = false, inU = false;
+  int sminL = 0, sminU = 0, smaxL = 0, smaxU = 0, snmin = 0, snmax = 0;
+  double fk = 0.0, zk = 0.0, Ak = 0.0, c1 = 0.0, c2 = 0.0;
+  if (in) {
+    const double ck0 = -flx / den * rdz, ck1 = flxu / den * rdz;
+    const double ck0p = (k + 1 <= kmax) ? -flxu / __ldg(a.den + c.at(k + 1)) * cC.rdgz[k + 1] : 0.0;
     const double L = 0.5 - copysign(0.5, ck0), U = 0.5 + copysign(0.5, ck0p);
-    inL[k] = (L == 1.0);
-    inU[k] = (U == 1.0);
-    const double qc = q[k], qb = q[k - 1], qa = q[k + 1];
-    sminL[k] = amin2(qc, qb); smaxL[k] = amax2(qc, qb);
-    sminU[k] = amin2(qc, qa); smaxU[k] = amax2(qc, qa);
-    const double QminL = inL[k] ? (sminL[k] ? qb : qc) : BIG, QmaxL = inL[k] ? (smaxL[k] ? qb : qc) : -BIG;
-    const double QminU = inU[k] ? (sminU[k] ? qa : qc) : BIG, QmaxU = inU[k] ? (smaxU[k] ? qa : qc) : -BIG;
-    const int s1 = amin2(QminL, QminU);
-    const double m1 = s1 ? QminU : QminL;
-    snmin[k] = amin2(m1, qc) ? 2 : s1;
-    const double qnmin = (snmin[k] == 2) ? qc : m1;
-    const int s2 = amax2(QmaxL, QmaxU);
-    const double x1 = s2 ? QmaxU : QmaxL;
-    snmax[k] = amax2(x1, qc) ? 2 : s2;
-    const double qnmax = (snmax[k] == 2) ? qc : x1;
+    inL = (L == 1.0);
+    inU = (U == 1.0);
+    sminL = amin2(q0, qb); smaxL = amax2(q0, qb);
+    sminU = amin2(q0, qa); smaxU = amax2(q0, qa);
+    const double QminL = inL ? (sminL ? qb : q0) : BIG, QmaxL = inL ? (smaxL ? qb : q0) : -BIG;
+    const double QminU = inU ? (sminU ? qa : q0) : BIG, QmaxU = inU ? (smaxU ? qa : q0) : -BIG;
+    const int s1 = amin2(QminL, QminU), s2 = amax2(QmaxL, QmaxU);
+    const double m1 = s1 ? QminU : QminL, x1 = s2 ? QmaxU : QmaxL;
+    snmin = amin2(m1, q0) ? 2 : s1;
+    snmax = amax2(x1, q0) ? 2 : s2;
+    const double qnmin = (snmin == 2) ? q0 : m1, qnmax = (snmax == 2) ? q0 : x1;
     const double Cin = L * ck0 + U * ck1, Cout = (1.0 - L) * ck0 + (1.0 - U) * ck1;
     const double CQmin = L * ck0 * QminL + U * ck1 * QminU, CQmax = L * ck0 * QmaxL + U * ck1 * QmaxU;
     const double zsw = 0.5 - copysign(0.5, fabs(Cout) - EPS);
-    const double dk = a.bcoef * a.frhog[p] / denk * a.dt;
-    const double A = Cin + Cout - dk;
-    omin[k] = ((qc - qnmax) + qnmax * A - CQmax) / (Cout + zsw) * (1.0 - zsw) + qc * zsw;
-    omax[k] = ((qc - qnmin) + qnmin * A - CQmin) / (Cout + zsw) * (1.0 - zsw) + qc * zsw;
-    fk[k] = (1.0 - zsw) / (Cout + zsw);
-    zk[k] = zsw;
-    Ak[k] = A;
-    c1v[k] = L * ck0;
-    c2v[k] = U * ck1;
+    const double dk = a.bcoef * __ldg(a.frhog + p) / den * a.dt;
+    Ak = Cin + Cout - dk;
+    s_n[0] = ((q0 - qnmax) + qnmax * Ak - CQmax) / (Cout + zsw) * (1.0 - zsw) + q0 * zsw;
+    s_x[0] = ((q0 - qnmin) + qnmin * Ak - CQmin) / (Cout + zsw) * (1.0 - zsw) + q0 * zsw;
+    fk = (1.0 - zsw) / (Cout + zsw);
+    zk = zsw;
+    c1 = L * ck0;
+    c2 = U * ck1;
   }
-  // limited faces qh[k] on k = kmin+1..kmax, zero at kmin and kmax+1: the
-  // bounds of the upwind cell, k-1 when inflow comes from below (inL)
-  double qh[NC_ADJ_K];
-  for (int k = 0; k < KA; ++k) qh[k] = 0.0;
-  for (int k = kmin + 1; k <= kmax; ++k) {
-    const int jb = inL[k] ? k - 1 : k;
-    const double lo = omin[jb], hi = omax[jb];
-    const int s_lo = amax2(raw[k], lo);            // np.maximum(raw, lo)
-    const double mx = s_lo ? lo : raw[k];
+  __syncthreads();
+  // the limited face at k (kmin+1..kmax, zero elsewhere): the bounds of the
+  // upwind cell, k-1 when inflow comes from below; sh 0 raw, 1 lower, 2 upper bound
+  int sh = 0;
+  const bool face = k > kmin && k <= kmax;
+  if (face) {
+    const int o = inL ? -VL_COLS : 0;
+    const double lo = s_n[o], hi = s_x[o];
+    const int s_lo = amax2(raw, lo);               // np.maximum(raw, lo)
+    const double mx = s_lo ? lo : raw;
     const int s_hi = amin2(mx, hi);                // np.minimum(mx, hi)
-    sh[k] = s_hi ? 2 : (s_lo ? 1 : 0);
-    qh[k] = s_hi ? hi : mx;
+    sh = s_hi ? 2 : (s_lo ? 1 : 0);
+    s_h[0] = s_hi ? hi : mx;
   }
-  for (int k = 0; k < KA; ++k) clamped[k] = false;
+  __syncthreads();
+  const double x = in ? rq - (flxu * s_h[VL_COLS] - flx * s_h[0]) * rdz : 0.0;
+  const bool clamped = in && a.clamp && x > -1.0e-10 && x < 0.0;
   if (a.mode == 0) {
-    for (int k = 0; k < KA; ++k) a.out[c.at(k)] = 0.0;
-    for (int k = kmin; k <= kmax; ++k) {
-      double x = a.rhogq[c.at(k)] - (a.flx_v[c.at(k + 1)] * qh[k + 1] - a.flx_v[c.at(k)] * qh[k]) * cC.rdgz[k];
-      if (a.clamp && x > -1.0e-10 && x < 0.0) x = 0.0;
-      a.out[c.at(k)] = x;
-    }
+    if (act) a.out[p] = clamped ? 0.0 : x;
     return;
   }
-  for (int k = kmin; k <= kmax; ++k) {
-    const double x = a.rhogq[c.at(k)] - (a.flx_v[c.at(k + 1)] * qh[k + 1] - a.flx_v[c.at(k)] * qh[k]) * cC.rdgz[k];
-    clamped[k] = a.clamp && x > -1.0e-10 && x < 0.0;
-  }
+  __syncthreads();   // the bounds and faces are read; their rows take the derivatives
   if (a.mode == 1) {
     // tangent-linear: the same sequence on perturbations
-    double dq[NC_ADJ_K], draw[NC_ADJ_K], dmin[NC_ADJ_K], dmax[NC_ADJ_K], dqh[NC_ADJ_K];
-    for (int k = 0; k < KA; ++k) {
-      dq[k] = a.in[c.at(k)] / a.den[c.at(k)];
-      dqh[k] = 0.0;
-    }
-    for (int k = kmin; k <= kmax + 1; ++k) draw[k] = cC.afact[k] * dq[k] + cC.bfact[k] * dq[k - 1];
-    for (int k = kmin; k <= kmax; ++k) {
-      const double dc = dq[k];
-      const double dminL = inL[k] ? (sminL[k] ? dq[k - 1] : dc) : 0.0, dmaxL = inL[k] ? (smaxL[k] ? dq[k - 1] : dc) : 0.0;
-      const double dminU = inU[k] ? (sminU[k] ? dq[k + 1] : dc) : 0.0, dmaxU = inU[k] ? (smaxU[k] ? dq[k + 1] : dc) : 0.0;
-      const double dnmin = (snmin[k] == 2) ? dc : (snmin[k] == 1 ? dminU : dminL);
-      const double dnmax = (snmax[k] == 2) ? dc : (snmax[k] == 1 ? dmaxU : dmaxL);
-      const double dCQmin = c1v[k] * dminL + c2v[k] * dminU, dCQmax = c1v[k] * dmaxL + c2v[k] * dmaxU;
+    const double dc = s_d[0], db = s_d[-VL_COLS], da = s_d[VL_COLS];
+    s_n[0] = s_x[0] = 0.0;
+    if (in) {
+      const double dminL = inL ? (sminL ? db : dc) : 0.0, dmaxL = inL ? (smaxL ? db : dc) : 0.0;
+      const double dminU = inU ? (sminU ? da : dc) : 0.0, dmaxU = inU ? (smaxU ? da : dc) : 0.0;
+      const double dnmin = (snmin == 2) ? dc : (snmin == 1 ? dminU : dminL);
+      const double dnmax = (snmax == 2) ? dc : (snmax == 1 ? dmaxU : dmaxL);
+      const double dCQmin = c1 * dminL + c2 * dminU, dCQmax = c1 * dmaxL + c2 * dmaxU;
       // qomin = f (qc - qnmax + A qnmax - CQmax) + zsw qc
-      dmin[k] = fk[k] * (dc + (Ak[k] - 1.0) * dnmax - dCQmax) + zk[k] * dc;
-      dmax[k] = fk[k] * (dc + (Ak[k] - 1.0) * dnmin - dCQmin) + zk[k] * dc;
+      s_n[0] = fk * (dc + (Ak - 1.0) * dnmax - dCQmax) + zk * dc;
+      s_x[0] = fk * (dc + (Ak - 1.0) * dnmin - dCQmin) + zk * dc;
     }
-    for (int k = kmin + 1; k <= kmax; ++k) {
-      const int jb = inL[k] ? k - 1 : k;
-      dqh[k] = (sh[k] == 0) ? draw[k] : (sh[k] == 1 ? dmin[jb] : dmax[jb]);
+    __syncthreads();
+    if (face) {
+      const int o = inL ? -VL_COLS : 0;
+      s_a[0] = (sh == 0) ? cC.afact[k] * dc + cC.bfact[k] * db : (sh == 1 ? s_n[o] : s_x[o]);
     }
-    for (int k = 0; k < KA; ++k) a.out[c.at(k)] = 0.0;
-    for (int k = kmin; k <= kmax; ++k) {
-      const double d = a.in[c.at(k)] - (a.flx_v[c.at(k + 1)] * dqh[k + 1] - a.flx_v[c.at(k)] * dqh[k]) * cC.rdgz[k];
-      a.out[c.at(k)] = clamped[k] ? 0.0 : d;
-    }
+    __syncthreads();
+    const double d = inv - (flxu * s_a[VL_COLS] - flx * s_a[0]) * rdz;
+    if (act) a.out[p] = (in && !clamped) ? d : 0.0;
     return;
   }
   // adjoint: the tangent-linear steps transposed, in reverse order
-  double gy[NC_ADJ_K], gqh[NC_ADJ_K], graw[NC_ADJ_K], gmin[NC_ADJ_K], gmax[NC_ADJ_K], gq[NC_ADJ_K], gr[NC_ADJ_K];
-  for (int k = 0; k < KA; ++k) {
-    gy[k] = (k >= kmin && k <= kmax && !clamped[k]) ? a.in[c.at(k)] : 0.0;
-    gqh[k] = graw[k] = gmin[k] = gmax[k] = gq[k] = gr[k] = 0.0;
-  }
-  for (int k = kmin; k <= kmax; ++k) {   // out_k = in_k - (flx_{k+1} qh_{k+1} - flx_k qh_k) rdgz_k
-    gr[k] += gy[k];
-    gqh[k + 1] -= a.flx_v[c.at(k + 1)] * cC.rdgz[k] * gy[k];
-    gqh[k] += a.flx_v[c.at(k)] * cC.rdgz[k] * gy[k];
-  }
-  for (int k = kmin + 1; k <= kmax; ++k) {
-    const int jb = inL[k] ? k - 1 : k;
-    if (sh[k] == 0) graw[k] += gqh[k];
-    else if (sh[k] == 1) gmin[jb] += gqh[k];
-    else gmax[jb] += gqh[k];
-  }
-  for (int k = kmin; k <= kmax; ++k) {
+  const double gy = (in && !clamped) ? inv : 0.0;
+  s_h[0] = gy * rdz;          // out_k = in_k - (flx_{k+1} qh_{k+1} - flx_k qh_k) rdgz_k
+  __syncthreads();
+  const double gqh = flx * (s_h[0] - s_h[-VL_COLS]);
+  // the face's cotangent: to raw_k, or to a bound of cell k or k-1
+  const double graw = (face && sh == 0) ? gqh : 0.0;
+  const double gn = (face && sh == 1) ? gqh : 0.0, gx = (face && sh == 2) ? gqh : 0.0;
+  s_n[0] = inL ? gn : 0.0;    // handed to the cell below
+  s_x[0] = inL ? gx : 0.0;
+  s_d[0] = graw;
+  __syncthreads();
+  double gq = 0.0, up = 0.0, dn = 0.0;   // cotangents of q at k, k+1 and k-1
+  if (in) {
+    const double gmin = (inL ? 0.0 : gn) + s_n[VL_COLS], gmax = (inL ? 0.0 : gx) + s_x[VL_COLS];
     // dmin = (f + zsw) dc + f (A - 1) dnmax - f dCQmax, and the same for dmax with qnmin / CQmin
-    gq[k] += (fk[k] + zk[k]) * (gmin[k] + gmax[k]);
-    const double gnmax = fk[k] * (Ak[k] - 1.0) * gmin[k], gCQmax = -fk[k] * gmin[k];
-    const double gnmin = fk[k] * (Ak[k] - 1.0) * gmax[k], gCQmin = -fk[k] * gmax[k];
-    double gminL = c1v[k] * gCQmin, gminU = c2v[k] * gCQmin, gmaxL = c1v[k] * gCQmax, gmaxU = c2v[k] * gCQmax;
-    if (snmin[k] == 2) gq[k] += gnmin;
-    else if (snmin[k] == 1) gminU += gnmin;
+    gq = (fk + zk) * (gmin + gmax);
+    const double gnmax = fk * (Ak - 1.0) * gmin, gCQmax = -fk * gmin;
+    const double gnmin = fk * (Ak - 1.0) * gmax, gCQmin = -fk * gmax;
+    double gminL = c1 * gCQmin, gminU = c2 * gCQmin, gmaxL = c1 * gCQmax, gmaxU = c2 * gCQmax;
+    if (snmin == 2) gq += gnmin;
+    else if (snmin == 1) gminU += gnmin;
     else gminL += gnmin;
-    if (snmax[k] == 2) gq[k] += gnmax;
-    else if (snmax[k] == 1) gmaxU += gnmax;
+    if (snmax == 2) gq += gnmax;
+    else if (snmax == 1) gmaxU += gnmax;
     else gmaxL += gnmax;
-    if (inL[k]) {
-      gq[sminL[k] ? k - 1 : k] += gminL;
-      gq[smaxL[k] ? k - 1 : k] += gmaxL;
+    if (inL) {
+      (sminL ? dn : gq) += gminL;
+      (smaxL ? dn : gq) += gmaxL;
     }
-    if (inU[k]) {
-      gq[sminU[k] ? k + 1 : k] += gminU;
-      gq[smaxU[k] ? k + 1 : k] += gmaxU;
+    if (inU) {
+      (sminU ? up : gq) += gminU;
+      (smaxU ? up : gq) += gmaxU;
     }
   }
-  for (int k = kmin; k <= kmax + 1; ++k) {   // raw_k = afact_k q_k + bfact_k q_{k-1}
-    gq[k] += cC.afact[k] * graw[k];
-    gq[k - 1] += cC.bfact[k] * graw[k];
-  }
-  for (int k = 0; k < KA; ++k) a.out[c.at(k)] = gr[k] + gq[k] / a.den[c.at(k)];
-}
-
-__global__ void k_vadv_lin(VadvLin a, int pole) {
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  int i, j, l, g, lp;
-  if (!map_col(pole, t, i, j, l, g, lp)) return;
-  vadv_lin_column(pole ? col_pl(g, lp) : col_reg(i, j, l), a);
+  s_a[0] = up;
+  s_b[0] = dn;
+  __syncthreads();
+  // raw_k = afact_k q_k + bfact_k q_{k-1}
+  gq += s_a[-VL_COLS] + s_b[VL_COLS] + cC.afact[k] * graw;
+  if (k + 1 < KA) gq += cC.bfact[k + 1] * s_d[VL_COLS];
+  if (act) a.out[p] = gy + gq / den;
 }
 
 // ---------------------------------------------------------------------------

@@ -1348,14 +1348,17 @@ static int comm_adj(nc_handle* h, FieldPair& f) {
   k_comm_adj_clear<<<g, 256, 0, h->stream>>>(f.r, f.p, h->r_dst, h->nr, h->p_dst, h->np);
   return check_launch(h, "comm_adj_clear");
 }
+static unsigned col_blocks(const nc_handle* h, int pole, int tpb) {
+  const long long n = pole ? 6LL * h->D.LP : h->D.npt2;
+  return (unsigned)((n + tpb - 1) / tpb);
+}
 static int vadv_lin_launch(nc_handle* h, int mode, const FieldPair& at, const FieldPair& den, const double* in_r,
                            const double* in_p, double* out_r, double* out_p, bool second) {
   for (int pole = 0; pole < 2; ++pole) {
     VadvLin a{pole ? at.p : at.r, pole ? den.p : den.r, pole ? h->flx_v.p : h->flx_v.r,
               pole ? h->frhog.p : h->frhog.r, pole ? in_p : in_r, pole ? out_p : out_r, h->dtl, 0.0,
               second ? 1 : 0, mode};
-    const long long n = pole ? 6LL * h->D.LP : h->D.npt2;
-    k_vadv_lin<<<(unsigned)((n + 63) / 64), 64, 0, h->stream>>>(a, pole);
+    k_vadv_lin<<<col_blocks(h, pole, VL_COLS), VL_COLS * h->D.KA, vadv_lin_smem(h->D.KA), h->stream>>>(a, pole);
     TRY(check_launch(h, mode == 1 ? "vadv_tl" : "vadv_ad"));
   }
   return 0;
@@ -1725,6 +1728,7 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
                         (const void*)k_vi_col<double, false, true>, (const void*)k_vi_col<float, true, false>,
                         (const void*)k_vi_col<float, false, false>, (const void*)k_vi_col<float, false, true>})
     CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vi_col_smem(NC_MAXK)));
+  CU(cudaFuncSetAttribute(k_vadv_lin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vadv_lin_smem(NC_ADJ_K)));
   CU(cudaFuncSetAttribute(k_tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem(NC_ADJ_K)));
   ArrTab T;
   for (int n = 0; n < narrays; ++n) {
@@ -2859,10 +2863,6 @@ static int adj_ready(nc_handle* h, const char* what) {
     return fail(NC_ERR_ARG, std::string(what) + ": needs 1 <= kmin < kmax <= kall - 2");
   return load_consts(h);
 }
-static unsigned col_blocks(const nc_handle* h, int pole, int tpb) {
-  const long long n = pole ? 6LL * h->D.LP : h->D.npt2;
-  return (unsigned)((n + tpb - 1) / tpb);
-}
 
 int nc_vsolve(nc_handle* h, int32_t pole, int32_t transpose, const double* Mc, const double* Mu, const double* Ml,
               const double* b, double* x, const double* x_fwd, double* gMc, double* gMu, double* gMl,
@@ -2886,7 +2886,7 @@ int nc_vadv_lin(nc_handle* h, int32_t pole, int32_t mode, const double* rhogq, c
   if (!rhogq || !den || !flx_v || !frhog || !out || (mode && !in)) return fail(NC_ERR_ARG, "nc_vadv_lin: null pointer");
   VadvLin a{rhogq, den, flx_v, frhog, in, out, dt, bcoef, clamp ? 1 : 0, mode};
   TRY(after_caller(h, stream));
-  k_vadv_lin<<<col_blocks(h, pole, 64), 64, 0, h->stream>>>(a, pole ? 1 : 0);
+  k_vadv_lin<<<col_blocks(h, pole, VL_COLS), VL_COLS * h->D.KA, vadv_lin_smem(h->D.KA), h->stream>>>(a, pole ? 1 : 0);
   TRY(check_launch(h, "vadv_lin"));
   return before_caller(h, stream);
 }
