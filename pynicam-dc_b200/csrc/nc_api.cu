@@ -1072,20 +1072,10 @@ static int run_step(nc_handle* h) {
       {
         const int ncol = D.L * (D.G - 2) * (D.G - 2);
         const size_t sm = vi_col_smem(D.KA);
-        if (ncol <= h->sms * 9 * 128) {   // one wave of the column kernel's nine 128-thread blocks per SM
-          const unsigned nb = (unsigned)((ncol + VC_COLS - 1) / VC_COLS);
-          if (h->C.gam_unit) k_vi_col<R, true, false><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
-          else k_vi_col<R, false, false><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
-          TRY(check_launch(h, "vi_solve"));
-        } else {
-          const int tb = h->blk[TB_VISOLVE];
-          const unsigned nb = (unsigned)((D.npt2 + tb - 1) / tb);
-          if (h->C.gam_unit) k_vi_solve<R, true><<<nb, tb, 0, s>>>(vi[0]);
-          else k_vi_solve<R, false><<<nb, tb, 0, s>>>(vi[0]);
-          TRY(check_launch(h, "vi_solve"));
-          k_vi_energy_p<<<(unsigned)((D.npt + h->blk[TB_VIENERGY] - 1) / h->blk[TB_VIENERGY]), h->blk[TB_VIENERGY], 0, s>>>(vi[0]);
-          TRY(check_launch(h, "vi_energy"));
-        }
+        const unsigned nb = (unsigned)((ncol + VC_COLS - 1) / VC_COLS);
+        if (h->C.gam_unit) k_vi_col<R, true, false><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
+        else k_vi_col<R, false, false><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
+        TRY(check_launch(h, "vi_solve"));
         k_vimain_a_pl<<<pkb, 32, 0, ps>>>(vi[1]);
         TRY(check_launch(h, "vimain_a_pl"));
         k_vi_col<R, false, true><<<(6 * D.LP + VC_COLS - 1) / VC_COLS, 32 * VC_MAXW, sm, ps>>>(vi[1]);

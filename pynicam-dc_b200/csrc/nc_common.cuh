@@ -153,26 +153,14 @@ template <> __device__ __forceinline__ const GeomT<float>& geom<float>() { retur
 #ifndef NC_F32_ADVMOM
 #define NC_F32_ADVMOM 4
 #endif
-#ifndef NC_F32_HDIFF2
-#define NC_F32_HDIFF2 4
-#endif
 #ifndef NC_F32_VP0H
 #define NC_F32_VP0H 5
 #endif
 #ifndef NC_F32_VP0C
 #define NC_F32_VP0C 3
 #endif
-#ifndef NC_F32_PATH1
-#define NC_F32_PATH1 6
-#endif
 #ifndef NC_F32_VIMAINA
 #define NC_F32_VIMAINA 6
-#endif
-#ifndef NC_F32_VISOLVE
-#define NC_F32_VISOLVE 9
-#endif
-#ifndef NC_F32_VIENERGY
-#define NC_F32_VIENERGY 12
 #endif
 
 // a * b + c: two roundings in the float64 form (the reference's), one in the

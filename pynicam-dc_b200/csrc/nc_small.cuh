@@ -1165,10 +1165,18 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 4, 5)) k_vimain_a_m(V
 // (five doubles per level and column: 54 KB at 42 levels), then each warp
 // finishes its levels, again marching upward; a part of the column repeats one
 // level (assembly) or two (finish) of its neighbour instead of exchanging them.
-// A column per thread was bound by its chain of loads and divisions (gl05 z40
-// float64: 6 us a level, whatever the number of columns) and kept the sweep's
-// factors in local memory; the finish in the same launch finds the fields that
-// both parts read in L2.
+// Bound by memory latency: a warp waits for each level's loads, and a column per
+// thread (a kernel for the solve and a point kernel for the energies) was bound
+// by its chain of loads and divisions besides (6 us a level on small grids) and
+// kept the sweep's factors in local memory.  So every level's loads stand before
+// its arithmetic, under no condition and as read-only loads, which the stores of
+// the level below cannot hold up; the finish finds what both parts read in L2.
+// Launch bounds: two blocks an SM in double (128 registers; three: spills, 1.12
+// against 0.71 ms at gl07 z40), three in float (two: 1.87, four: 2.89 against
+// 1.63 ms at gl08 z40).
+// One layer of 40 levels, solve and energies, two kernels -> this one: gl05
+// float64 287 -> 83 us, gl06 mixed 307 -> 125 us, gl07 float64 1049 -> 705 us,
+// gl08 mixed 2065 -> 1627 us.
 // Slots, by level (kmin..kmax+1) and lane:
 //   0 horizontal part of the half-level mass flux
 //   1 the right-hand side, then the solution
@@ -1207,44 +1215,55 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
   auto cz = [&](int comp, int q) -> R { return __ldg(POLE ? m.C2WGz + q * 6 + comp : m.C2WGz + comp * cD.npti + q); };
   auto two = [&](const R* w, int comp, int q) -> R { return __ldg(POLE ? w + q * 2 + comp : w + comp * cD.npti + q); };
   int lo, hi;
-  // ---- right-hand side on kmin+1..kmax
+  // ---- right-hand side on kmin+1..kmax.  Every level's loads stand before its
+  // arithmetic and under no condition (indices clamped to the column), so that
+  // a level waits for memory once.
   warp_levels(kmin + 1, kmax, lo, hi);
   if (lo < hi) {
     const double CVovRt2 = CVdry / Rdry / (dt * dt);
-    double f0m, f1m, f2m, em;             // diff_vh and eth one level below
-    auto flux = [&](int k, double& hd, double& he) {   // half-level fluxes at k; level k becomes the one below
-      const int p = c.at(k);
-      const double f0 = __ldg(DV[0] + p), f1 = __ldg(DV[1] + p), f2 = __ldg(DV[2] + p), e = __ldg(a.eth + p);
-      const double z0 = cz(0, p), z1 = cz(1, p), z2 = cz(2, p), z3 = cz(3, p), z4 = cz(4, p), z5 = cz(5, p);
-      const double g = GU ? 1.0 : (double)__ldg(m.RGAMH + p);
-      hd = (z0 * f0 + z1 * f0m + z2 * f1 + z3 * f1m + z4 * f2 + z5 * f2m) * g;
-      he = (z0 * (f0 * e) + z1 * (f0m * em) + z2 * (f1 * e) + z3 * (f1m * em) + z4 * (f2 * e) + z5 * (f2m * em)) * g;
-      f0m = f0; f1m = f1; f2m = f2; em = e;
-    };
-    double hD = 0.0, hE = 0.0;            // zero at kmin (and at kmax+1)
-    {
-      const int k = (lo - 1 > kmin) ? lo - 2 : lo - 1;
+    R m0, m1, m2, me;                     // diff_vh and eth one level below
+    R f0, f1, f2, fe, z0, z1, z2, z3, z4, z5, gh;
+    auto load = [&](int k) {
       const int q = c.at(k);
-      f0m = __ldg(DV[0] + q); f1m = __ldg(DV[1] + q); f2m = __ldg(DV[2] + q); em = __ldg(a.eth + q);
-      if (lo - 1 > kmin) flux(lo - 1, hD, hE);
+      f0 = __ldg(DV[0] + q); f1 = __ldg(DV[1] + q); f2 = __ldg(DV[2] + q); fe = __ldg(a.eth + q);
+      z0 = cz(0, q); z1 = cz(1, q); z2 = cz(2, q); z3 = cz(3, q); z4 = cz(4, q); z5 = cz(5, q);
+      gh = GU ? R(1.0) : __ldg(m.RGAMH + q);
+    };
+    auto flux = [&](double& hd, double& he) {   // half-level fluxes at the loaded level
+      const double a0 = f0, a1 = f1, a2 = f2, e = fe, b0 = m0, b1 = m1, b2 = m2, em = me;
+      hd = (z0 * a0 + z1 * b0 + z2 * a1 + z3 * b1 + z4 * a2 + z5 * b2) * (double)gh;
+      he = (z0 * (a0 * e) + z1 * (b0 * em) + z2 * (a1 * e) + z3 * (b1 * em) + z4 * (a2 * e) + z5 * (b2 * em)) * (double)gh;
+    };
+    {
+      const int q = c.at(lo - 2);
+      m0 = __ldg(DV[0] + q); m1 = __ldg(DV[1] + q); m2 = __ldg(DV[2] + q); me = __ldg(a.eth + q);
     }
+    load(lo - 1);
+    double hD, hE;
+    flux(hD, hE);
+    if (lo - 1 == kmin) hD = hE = 0.0;    // zero at kmin and at kmax+1
+    m0 = f0; m1 = f1; m2 = f2; me = fe;
     double T1m = 0.0, T2m = 0.0;
     for (int k = lo - 1; k < hi; ++k) {
       const int p = c.at(k);
-      double hDn = 0.0, hEn = 0.0;
-      if (k < kmax) flux(k + 1, hDn, hEn);
-      const double drhog = -__ldg(a.hdiv[0] + p) - (hDn - hD) * cC.rdgz[k];
-      const double drhoge = -__ldg(a.hdiv[1] + p) - (hEn - hE) * cC.rdgz[k];
-      const double g1 = __ldg(a.gT[0] + p) + drhog;
-      const double gp = (__ldg(a.gT[5] + p) + drhoge) * Rdry / CVdry;
-      const double rgm = GU ? 1.0 : (double)__ldg(m.RGAM + p);
-      const double T1 = (__ldg(a.PS[5] + p) * RovCV + dt * gp) * __ldg(m.RGSGAM2 + p);
-      const double T2 = (__ldg(a.PS[0] + p) + dt * g1) * (rgm * rgm);
+      load(k + 1);
+      const R hd0 = __ldg(a.hdiv[0] + p), hd1 = __ldg(a.hdiv[1] + p), g0 = __ldg(a.gT[0] + p), g5 = __ldg(a.gT[5] + p);
+      const R ps5 = __ldg(a.PS[5] + p), ps0 = __ldg(a.PS[0] + p), rs2 = __ldg(m.RGSGAM2 + p);
+      const R g4 = __ldg(a.gT[4] + p), ps4 = __ldg(a.PS[4] + p);
+      const double mu = __ldg(a.Mu + p), ml = __ldg(a.Ml + p), mcc = __ldg(a.Mc + p);
+      const double rgm = GU ? 1.0 : (double)__ldg(m.RGAM + p), rgh = GU ? 1.0 : (double)__ldg(m.RGAMH + p);
+      double hDn, hEn;
+      flux(hDn, hEn);
+      if (k == kmax) hDn = hEn = 0.0;
+      const double drhog = -hd0 - (hDn - hD) * cC.rdgz[k];
+      const double drhoge = -hd1 - (hEn - hE) * cC.rdgz[k];
+      const double g1 = g0 + drhog;
+      const double gp = (g5 + drhoge) * Rdry / CVdry;
+      const double T1 = (ps5 * RovCV + dt * gp) * rs2;
+      const double T2 = (ps0 + dt * g1) * (rgm * rgm);
       if (k >= lo) {
-        const double rgh = GU ? 1.0 : (double)__ldg(m.RGAMH + p);
-        const double Sw = __ldg(a.gT[4] + p) + 0.0 * cC.alpha;
-        const double mu = __ldg(a.Mu + p), ml = __ldg(a.Ml + p);
-        double b = ((__ldg(a.PS[4] + p) * cC.alpha + dt * Sw) * (rgh * rgh) - (T1 - T1m) * dt * cC.rdgzh[k] -
+        const double Sw = g4 + 0.0 * cC.alpha;
+        double b = ((ps4 * cC.alpha + dt * Sw) * (rgh * rgh) - (T1 - T1m) * dt * cC.rdgzh[k] -
                     (T2 * cC.afact[k] + T2m * cC.bfact[k]) * dt * cC.GRAV) *
                    CVovRt2;
         if (k == kmin + 1) {
@@ -1252,11 +1271,9 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
           b = b - ml * rw_kmin;
           S(s1, kmin) = rw_kmin;
         }
-        if (k == kmax) {
-          const int pT = c.at(kT);
-          const double top = -(cz(0, pT) * __ldg(DV[0] + pT) + cz(1, pT) * __ldg(DV[0] + p) + cz(2, pT) * __ldg(DV[1] + pT) +
-                               cz(3, pT) * __ldg(DV[1] + p) + cz(4, pT) * __ldg(DV[2] + pT) + cz(5, pT) * __ldg(DV[2] + p));
-          const double rw_top = top * __ldg(m.RGSGAM2H + pT);
+        if (k == kmax) {   // the loaded level is kmax+1
+          const double top = -(z0 * f0 + z1 * m0 + z2 * f1 + z3 * m1 + z4 * f2 + z5 * m2);
+          const double rw_top = top * __ldg(m.RGSGAM2H + c.at(kT));
           b = b - mu * rw_top;
           S(s1, kT) = rw_top;
         }
@@ -1264,9 +1281,10 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
         S(s1, k) = b;
         S(s2, k) = mu;
         S(s3, k) = ml;
-        S(s4, k) = __ldg(a.Mc + p);
+        S(s4, k) = mcc;
       }
       T1m = T1; T2m = T2; hD = hDn; hE = hEn;
+      m0 = f0; m1 = f1; m2 = f2; me = fe;
     }
   }
   __syncthreads();
@@ -1300,269 +1318,78 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
   }
   __syncthreads();
   // ---- rhogw_split1, rhog_split1, the kinetic energies before and after, the
-  // total-energy advection and rhoge_split1 on every level
+  // total-energy advection and rhoge_split1 on every level: the march reads level
+  // kk, forms its half-level terms with the level below and writes level kk-1
   warp_levels(0, KA - 1, lo, hi);
   if (lo >= hi) return;
   const R dtR = R(dt);
-  struct W { double rws, v2; };          // rhogw_split1 and its mass flux at half level k
-  auto wat = [&](int k) -> W {
-    W w{0.0, 0.0};
-    if (k < kmin || k > kT) return w;
-    const int p = c.at(k);
-    w.rws = S(s1, k) * __ldg(m.GSGAM2H + p);
-    if (k > kmin && k <= kmax) w.v2 = S(s0, k) + 1.0 * w.rws * __ldg(m.RGSQRTH + p);
-    return w;
-  };
-  auto rsat = [&](int k, double v2, double v2n) -> double {   // rhog_split1 at level k
-    const int p = c.at(k);
-    double drhog2 = 0.0;
-    if (k >= kmin && k <= kmax) drhog2 = -__ldg(a.hdiv[0] + p) - (v2n - v2) * cC.rdgz[k];
-    return __ldg(a.PS[0] + p) + (__ldg(a.gT[0] + p) + drhog2) * dt;
-  };
-  struct L { R rg, r0, r1, vx, vy, vz, x1, y1, z1, et; };   // the values of one level
-  auto lat = [&](int k, double rs) -> L {
-    const int p = c.at(k);
-    L q;
-    q.rg = __ldg(a.P[0] + p);
-    q.r0 = __ldg(a.PS[0] + p);
-    q.r1 = R(rs);
-    q.vx = __ldg(a.P[1] + p); q.vy = __ldg(a.P[2] + p); q.vz = __ldg(a.P[3] + p);
-    q.x1 = q.vx + __ldg(DV[0] + p); q.y1 = q.vy + __ldg(DV[1] + p); q.z1 = q.vz + __ldg(DV[2] + p);
-    q.et = __ldg(a.ethtot0 + p);
-    return q;
-  };
-  struct H { R k10, k11, fl; };          // half-level kinetic energies and total-energy flux
-  auto half = [&](int k, const L& u, const L& d, double rws) -> H {   // between the levels k (u) and k-1 (d)
-    const int p = c.at(k);
-    H h;
-    const R c0 = two(m.C2W, 0, p), c1 = two(m.C2W, 1, p), w = __ldg(a.P[4] + p);
-    const R w0 = w + __ldg(a.PS[4] + p), w1 = w + R(rws);
-    h.k10 = R(0.5) * (w0 * w0) / (c0 * (u.rg + u.r0) + c1 * (d.rg + d.r0));
-    h.k11 = R(0.5) * (w1 * w1) / (c0 * (u.rg + u.r1) + c1 * (d.rg + d.r1));
-    const R f = cz(0, p) * (u.x1 * u.et) + cz(1, p) * (d.x1 * d.et) + cz(2, p) * (u.y1 * u.et) +
-                cz(3, p) * (d.y1 * d.et) + cz(4, p) * (u.z1 * u.et) + cz(5, p) * (d.z1 * d.et);
-    h.fl = f * (GU && !POLE ? R(1.0) : gam_at(m.RGAMH, p)) +
-           R(1.0) * (w1 * (CC.afact[k] * u.et + CC.bfact[k] * d.et)) * __ldg(m.RGSQRTH + p);
-    return h;
-  };
-  W wc = wat(lo), wn = wat(lo + 1);
-  double rs = rsat(lo, wc.v2, wn.v2);
-  L cur = lat(lo, rs);
-  H hc{R(0.0), R(0.0), R(0.0)};
-  if (lo > kmin && lo <= kmax) {
-    const L below = lat(lo - 1, rsat(lo - 1, wat(lo - 1).v2, wc.v2));
-    hc = half(lo, cur, below, wc.rws);
-  }
-  for (int k = lo; k < hi; ++k) {
-    const int p = c.at(k);
-    const W wnn = wat(k + 2);
-    double rsn = 0.0;
-    L up = cur;
-    H hn{R(0.0), R(0.0), R(0.0)};
-    if (k + 1 < KA) {
-      rsn = rsat(k + 1, wn.v2, wnn.v2);
-      up = lat(k + 1, rsn);
-      if (k + 1 > kmin && k < kmax) hn = half(k + 1, up, cur, wn.rws);
+  const int kk0 = max(lo - 1, 0);
+  R gs = __ldg(m.GSGAM2H + c.at(kk0)), rq = __ldg(m.RGSQRTH + c.at(kk0));
+  // values of level kk-1 (d...) and its half-level terms (h...)
+  R drg = R(0.0), dr0 = R(0.0), dr1 = R(0.0), dvx = R(0.0), dvy = R(0.0), dvz = R(0.0), dx = R(0.0), dy = R(0.0),
+    dz = R(0.0), det = R(0.0), h10 = R(0.0), h11 = R(0.0), hfl = R(0.0);
+  double drs = 0.0, drw = 0.0;
+  for (int kk = kk0; kk <= hi; ++kk) {
+    const int ke = min(kk, KA - 1), kn = min(kk + 1, KA - 1), ko = max(kk - 1, 0);
+    const int p = c.at(ke), pn = c.at(kn), po = c.at(ko);
+    const R gsn = __ldg(m.GSGAM2H + pn), rqn = __ldg(m.RGSQRTH + pn);
+    const R rg = __ldg(a.P[0] + p), vx = __ldg(a.P[1] + p), vy = __ldg(a.P[2] + p), vz = __ldg(a.P[3] + p),
+            w = __ldg(a.P[4] + p), r0 = __ldg(a.PS[0] + p), ps4 = __ldg(a.PS[4] + p), et = __ldg(a.ethtot0 + p),
+            u0 = __ldg(DV[0] + p), u1 = __ldg(DV[1] + p), u2 = __ldg(DV[2] + p), hd0 = __ldg(a.hdiv[0] + p),
+            g0 = __ldg(a.gT[0] + p), c0 = two(m.C2W, 0, p), c1 = two(m.C2W, 1, p), z0 = cz(0, p), z1 = cz(1, p),
+            z2 = cz(2, p), z3 = cz(3, p), z4 = cz(4, p), z5 = cz(5, p);
+    const R ps1 = __ldg(a.PS[1] + po), ps2 = __ldg(a.PS[2] + po), ps3 = __ldg(a.PS[3] + po), w2c0 = two(m.W2C, 0, po),
+            w2c1 = two(m.W2C, 1, po), hd2 = __ldg(a.hdiv[2] + po), g0e = __ldg(a.gT0e + po), phi = __ldg(m.PHI + po),
+            re0 = __ldg(a.PS[5] + c.at(min(max(ko, kmin), kmax))), pm0 = a.PM0[po], pm4 = a.PM4[po];
+    const R ghh = GU && !POLE ? R(1.0) : gam_at(m.RGAMH, p);
+    // rhogw_split1 and its mass flux at the half levels kk and kk+1
+    auto rws_at = [&](int k, R g) -> double { return (k >= kmin && k <= kT) ? S(s1, k) * g : 0.0; };
+    auto v2_at = [&](int k, double r, R q) -> double { return (k > kmin && k <= kmax) ? S(s0, k) + 1.0 * r * q : 0.0; };
+    const double rws = rws_at(ke, gs), rwn = rws_at(kn, gsn);
+    const double v2 = v2_at(ke, rws, rq), v2n = v2_at(kn, rwn, rqn);
+    const bool in = kk >= kmin && kk <= kmax;
+    const double drhog2 = in ? -hd0 - (v2n - v2) * cC.rdgz[ke] : 0.0;
+    const double rs = r0 + (g0 + drhog2) * dt;
+    const R r1 = R(rs);
+    const R x1 = vx + u0, y1 = vy + u1, z1v = vz + u2;
+    // between the levels kk and kk-1
+    R k10 = R(0.0), k11 = R(0.0), fl = R(0.0);
+    if (kk > kmin && kk <= kmax) {
+      const R w0 = w + ps4, w1 = w + R(rws);
+      k10 = R(0.5) * (w0 * w0) / (c0 * (rg + r0) + c1 * (drg + dr0));
+      k11 = R(0.5) * (w1 * w1) / (c0 * (rg + r1) + c1 * (drg + dr1));
+      const R f = z0 * (x1 * et) + z1 * (dx * det) + z2 * (y1 * et) + z3 * (dy * det) + z4 * (z1v * et) + z5 * (dz * det);
+      fl = f * ghh + R(1.0) * (w1 * (CC.afact[ke] * et + CC.bfact[ke] * det)) * rq;
     }
-    R kin10 = R(0.0), kin11 = R(0.0), adv = R(0.0);
-    if (k >= kmin && k <= kmax) {
-      const R x0 = cur.vx + __ldg(a.PS[1] + p), y0 = cur.vy + __ldg(a.PS[2] + p), z0 = cur.vz + __ldg(a.PS[3] + p);
-      const R w0 = two(m.W2C, 0, p), w1 = two(m.W2C, 1, p);
-      kin10 = R(0.5) * (x0 * x0 + y0 * y0 + z0 * z0) / (cur.rg + cur.r0) + w0 * hn.k10 + w1 * hc.k10;
-      kin11 = R(0.5) * (cur.x1 * cur.x1 + cur.y1 * cur.y1 + cur.z1 * cur.z1) / (cur.rg + cur.r1) + w0 * hn.k11 +
-              w1 * hc.k11;
-      adv = -__ldg(a.hdiv[2] + p) - (hn.fl - hc.fl) * CC.rdgz[k];
+    if (kk > lo) {   // level kk-1
+      R kin10 = R(0.0), kin11 = R(0.0), adv = R(0.0);
+      if (ko >= kmin && ko <= kmax) {
+        const R x0 = dvx + ps1, y0 = dvy + ps2, z0v = dvz + ps3;
+        kin10 = R(0.5) * (x0 * x0 + y0 * y0 + z0v * z0v) / (drg + dr0) + w2c0 * k10 + w2c1 * h10;
+        kin11 = R(0.5) * (dx * dx + dy * dy + dz * dz) / (drg + dr1) + w2c0 * k11 + w2c1 * h11;
+        adv = -hd2 - (fl - hfl) * CC.rdgz[ko];
+      }
+      const R re = re0 + (g0e + adv) * dtR + (kin10 - kin11) + (dr0 - dr1) * phi;
+      if (act) {
+        a.dwe[0][po] = dr1;
+        a.dwe[1][po] = R(drw);
+        a.dwe[2][po] = re;
+        a.PM0[po] = pm0 + drs * a.rweight;
+        a.PM4[po] = pm4 + drw * a.rweight;
+      }
     }
-    const R re0 = __ldg(a.PS[5] + c.at(k < kmin ? kmin : (k > kmax ? kmax : k)));
-    const R pm0 = a.PM0[p], pm4 = a.PM4[p];
-    const R re = re0 + (__ldg(a.gT0e + p) + adv) * dtR + (kin10 - kin11) + (cur.r0 - cur.r1) * __ldg(m.PHI + p);
-    if (act) {
-      a.dwe[0][p] = cur.r1;
-      a.dwe[1][p] = R(wc.rws);
-      a.dwe[2][p] = re;
-      a.PM0[p] = pm0 + rs * a.rweight;
-      a.PM4[p] = pm4 + wc.rws * a.rweight;
-    }
-    rs = rsn;
-    wc = wn; wn = wnn;
-    cur = up;
-    hc = hn;
+    drg = rg; dr0 = r0; dr1 = r1; dvx = vx; dvy = vy; dvz = vz; dx = x1; dy = y1; dz = z1v; det = et;
+    h10 = k10; h11 = k11; hfl = fl;
+    drs = rs; drw = rws;
+    gs = gsn; rq = rqn;
   }
 }
 
 // GU: the gamma factors are all 1 and are not loaded
 template <class R, bool GU, bool POLE>
-__global__ void __launch_bounds__(32 * VC_MAXW, NC_MINB(R, 3, 4)) k_vi_col(const __grid_constant__ VimainArgs<R> a) {
+__global__ void __launch_bounds__(32 * VC_MAXW, NC_MINB(R, 2, 3)) k_vi_col(const __grid_constant__ VimainArgs<R> a) {
   extern __shared__ __align__(16) double vi_sm[];
   vi_col<R, GU, POLE>(a, (int)blockIdx.x, vi_sm);
-}
-
-// The same for more columns than fill the SMs with a thread each: two
-// kernels (interior columns).  With every SM busy the column kernel's chain is
-// hidden behind other columns and its 36 resident warps move more bytes than
-// k_vi_col's 32, whose sweeps leave seven of eight warps waiting: gl08 mixed
-// 1.15 + 0.91 ms against 2.39 ms; gl07 float64 (163,840 columns) 0.63 + 0.42 ms
-// against 0.97 ms.
-// k_vi_solve: flux convergences of diff_vh (rolling half-level fluxes), the
-// Thomas forward sweep, then the back substitution fused with rhog_split1 on
-// the way down; writes rhog_s1, rhogw_s1 and their running means.
-// nine 128-thread blocks per SM (56 registers): the 655,360 interior columns
-// of gl08 fill 3.84 waves of the 148 SMs instead of 4.32 at eight
-// GU: the gamma factors are all 1 and are not loaded; the other instance loads them
-template <class R, bool GU>
-__global__ void __launch_bounds__(128, NC_MINB(R, 9, NC_F32_VISOLVE)) k_vi_solve(VimainArgs<R> a) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, l;
-  if (!col_of(t, i, j, l) || !interior(i, j)) return;
-  const Col c = col_reg(i, j, l);
-  const MetT<R> m = met_of<R>(false);
-  const int kmin = cD.kmin, kmax = cD.kmax, kT = kmax + 1;
-  const double dt = a.dt, Rdry = cC.Rdry, CVdry = cC.CVdry, RovCV = a.RovCV;
-  const int n = cD.npti;
-  const R* cz = CG.C2WGz;
-  const R* const* DVp = a.dvh.f;
-  auto preg0 = [&](int k) -> double {
-    const int k2 = k < kmin ? kmin : (k > kmax ? kmax : k);
-    return a.PS[5][c.at(k2)] * RovCV;
-  };
-  // horizontal part of the half-level flux of diff_vh (and of diff_vh*eth) at kk
-  auto hflux = [&](int kk, bool withe) -> double {
-    const int q = c.at(kk), qm = c.at(kk - 1);
-    const double e = withe ? a.eth[q] : 1.0, em = withe ? a.eth[qm] : 1.0;
-    double f0 = DVp[0][q], f0m = DVp[0][qm], f1 = DVp[1][q], f1m = DVp[1][qm], f2 = DVp[2][q], f2m = DVp[2][qm];
-    if (withe) {
-      f0 = f0 * e; f0m = f0m * em; f1 = f1 * e; f1m = f1m * em; f2 = f2 * e; f2m = f2m * em;
-    }
-    const double h = cz[q] * f0 + cz[n + q] * f0m + cz[2 * n + q] * f1 + cz[3 * n + q] * f1m + cz[4 * n + q] * f2 +
-                     cz[5 * n + q] * f2m;
-    return h * (GU ? 1.0 : m.RGAMH[q]);
-  };
-  double hD[NC_MAXK];
-  const int pT = c.at(kT), pK = c.at(kmax);
-  const double rw_top = -(cz[pT] * DVp[0][pT] + cz[n + pT] * DVp[0][pK] + cz[2 * n + pT] * DVp[1][pT] +
-                          cz[3 * n + pT] * DVp[1][pK] + cz[4 * n + pT] * DVp[2][pT] + cz[5 * n + pT] * DVp[2][pK]);
-  const double CVovRt2 = CVdry / Rdry / (dt * dt);
-  const double rw_kmin = 0.0 * m.RGSGAM2H[c.at(kmin)];
-  const double rw_kmaxp1 = rw_top * m.RGSGAM2H[pT];
-  const int N = kmax - kmin;
-  double u[NC_MAXK], gam[NC_MAXK];
-  double vD_lo = 0.0, vE_lo = 0.0, g1_prev = 0.0, gp_prev = 0.0, beta = 0.0;
-  for (int k = kmin; k <= kmax; ++k) {
-    const int p = c.at(k);
-    const int kk = k + 1;
-    double vD_hi = 0.0, vE_hi = 0.0;
-    if (kk <= kmax) {
-      const double hd = hflux(kk, false);
-      hD[kk] = hd;
-      const double rq = m.RGSQRTH[c.at(kk)];
-      vD_hi = hd + 0.0 * a.PS[4][c.at(kk)] * rq;
-      vE_hi = hflux(kk, true) + 0.0 * 0.0 * rq;
-    }
-    const double drhog = -a.hdiv[0][p] - (vD_hi - vD_lo) * cC.rdgz[k];
-    const double drhoge = -a.hdiv[1][p] - (vE_hi - vE_lo) * cC.rdgz[k];
-    const double g1 = a.gT[0][p] + drhog;
-    const double gp = (a.gT[5][p] + drhoge) * Rdry / CVdry;
-    if (k >= kmin + 1) {
-      const int nn = k - kmin - 1;
-      const int pm = c.at(k - 1);
-      const double rgh = GU ? 1.0 : m.RGAMH[p], rgm = GU ? 1.0 : m.RGAM[p], rgmm = GU ? 1.0 : m.RGAM[pm];
-      const double rg2 = rgh * rgh;
-      const double rgam2 = rgm * rgm, rgam2m = rgmm * rgmm;
-      const double Sw = a.gT[4][p] + 0.0 * cC.alpha;
-      double S = ((a.PS[4][p] * cC.alpha + dt * Sw) * rg2 -
-                  ((preg0(k) + dt * gp) * m.RGSGAM2[p] - (preg0(k - 1) + dt * gp_prev) * m.RGSGAM2[pm]) * dt *
-                      cC.rdgzh[k] -
-                  ((a.PS[0][p] + dt * g1) * rgam2 * cC.afact[k] + (a.PS[0][pm] + dt * g1_prev) * rgam2m * cC.bfact[k]) *
-                      dt * cC.GRAV) *
-                 CVovRt2;
-      if (nn == 0) S = S - a.Ml[c.at(kmin + 1)] * rw_kmin;
-      if (nn == N - 1) S = S - a.Mu[c.at(kmax)] * rw_kmaxp1;
-      const double Mc = a.Mc[p], Ml = a.Ml[p];
-      if (nn == 0) {
-        beta = Mc;
-        u[0] = S / beta;
-      } else {
-        const double gg = a.Mu[pm] / beta;
-        beta = Mc - Ml * gg;
-        u[nn] = (S - Ml * u[nn - 1]) / beta;
-        gam[nn] = gg;
-      }
-    }
-    g1_prev = g1;
-    gp_prev = gp;
-    vD_lo = vD_hi;
-    vE_lo = vE_hi;
-  }
-  // back substitution (downward) fused with rhog_split1
-  double x = 0.0, v2_hi = 0.0;
-  for (int k = kT; k >= 0; --k) {
-    const int p = c.at(k);
-    double rws;
-    if (k == kT) {
-      rws = rw_kmaxp1 * m.GSGAM2H[p];
-    } else if (k >= kmin + 1) {
-      const int nn = k - kmin - 1;
-      x = (nn == N - 1) ? u[N - 1] : u[nn] - gam[nn + 1] * x;
-      rws = x * m.GSGAM2H[p];
-    } else if (k == kmin) {
-      rws = rw_kmin * m.GSGAM2H[p];
-    } else {
-      rws = 0.0;
-    }
-    const double v2 = (k > kmin && k <= kmax) ? hD[k] + 1.0 * rws * m.RGSQRTH[p] : 0.0;
-    double drhog2 = 0.0;
-    if (k >= kmin && k <= kmax) drhog2 = -a.hdiv[0][p] - (v2_hi - v2) * cC.rdgz[k];
-    const double rs = a.PS[0][p] + (a.gT[0][p] + drhog2) * dt;
-    a.dwe[0][p] = rs;
-    a.dwe[1][p] = rws;
-    a.PM0[p] = a.PM0[p] + rs * a.rweight;
-    a.PM4[p] = a.PM4[p] + rws * a.rweight;
-    v2_hi = v2;
-  }
-}
-
-// vi_main energy update with one thread per interior grid point: kinetic
-// energies, total-energy advection and rhoge_split1 from the rhog_s1 /
-// rhogw_s1 written by k_vi_solve (no vertical recurrence; neighbouring levels
-// are read through the cache).
-template <class R>
-__global__ void __launch_bounds__(128, NC_MINB(R, 1, NC_F32_VIENERGY)) k_vi_energy_p(VimainArgs<R> a) {
-  int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= cD.npti) return;
-  const int G = cD.G, KA = cD.KA;
-  const int i = (int)(t % G), j = (int)((t / G) % G), k = (int)((t / ((int)G * G)) % KA);
-  const int l = (int)(t / ((int)G * G * KA));
-  if (!interior(i, j)) return;
-  const Col c = col_reg(i, j, l);
-  const MetT<R> m = met_of<R>(false);
-  const int kmin = cD.kmin, kmax = cD.kmax;
-  const R* rs1 = a.dwe[0];
-  const R* rws1 = a.dwe[1];
-  auto PSk = [&](int comp, int kk) -> R {
-    if (comp == 5) kk = kk < kmin ? kmin : (kk > kmax ? kmax : kk);
-    return a.PS[comp][c.at(kk)];
-  };
-  const int p = c.at(k);
-  auto st10 = [&](int kk, int comp) -> R { return a.P[comp][c.at(kk)] + PSk(comp, kk); };
-  auto st11 = [&](int kk, int comp) -> R {
-    const int q = c.at(kk);
-    if (comp == 0) return a.P[0][q] + rs1[q];
-    if (comp == 4) return a.P[4][q] + rws1[q];
-    return a.P[comp][q] + a.dvh.f[comp - 1][q];
-  };
-  const R kin10 = rhogkin_at(c, m, k, st10);
-  const R kin11 = rhogkin_at(c, m, k, st11);
-  const R drhogetot = fluxconv_col(
-      c, m, k, a.hdiv[2][p], R(1.0),
-      [&](int kk, int d) {
-        const int q = c.at(kk);
-        return (a.P[1 + d][q] + a.dvh.f[d][q]) * a.ethtot0[q];
-      },
-      [&](int kk) {
-        const int q = c.at(kk), qm = c.at(kk - 1);
-        return (a.P[4][q] + rws1[q]) * (CC.afact[kk] * a.ethtot0[q] + CC.bfact[kk] * a.ethtot0[qm]);
-      });
-  a.dwe[2][p] = PSk(5, k) + (a.gT0e[p] + drhogetot) * R(a.dt) + (kin10 - kin11) + (PSk(0, k) - rs1[p]) * m.PHI[p];
 }
 
 // ---------------------------------------------------------------------------

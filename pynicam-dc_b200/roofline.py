@@ -78,19 +78,17 @@ KERNELS = {
               _m("RGSQRTH", "C2W.0", "C2W.1", "W2C.0", "W2C.1", "RGSGAM2", "PHI") + C2WGZ,
               _f(*_n("gT.", 6), "ethtot0") + _f64("Mc", "Mu", "Ml"), ()),
     # acoustic loop: path 1 (k_path1_l), vi_main horizontal divergences (k_vimain_a_l),
-    # Thomas solve (k_vi_solve) and energy update (k_vi_energy_p)
+    # Thomas solve and energy update (k_vi_col)
     "path1": (_f(*_n("vtmp2.", 3), "PS.5", "PS.1", "PS.2", "PS.3", "gT.1", "gT.2", "gT.3", "PM.1", "PM.2", "PM.3") +
               _m("RGAM", "RGAMH") + C2WGZ,
               _f("dvh.0", "dvh.1", "dvh.2", "PM.1", "PM.2", "PM.3"),
               _n("GRD_x.", 3) + _n("coef_intp.", 18) + _n("coef_diff.", 18) + _n("coef_grad.", 21)),
     "vimain_a": (_f("eth", "ethtot0", "dvh.0", "dvh.1", "dvh.2", "RHOGVX", "RHOGVY", "RHOGVZ"),
                  _f("hdiv.0", "hdiv.1", "hdiv.2"), _n("coef_div.", 21)),
-    "vi_solve": (_f("dvh.0", "dvh.1", "dvh.2", "eth", "PS.0", "PS.4", "PS.5", "hdiv.0", "hdiv.1", "gT.0", "gT.4", "gT.5",
-                    "PM.0", "PM.4") + _f64("Mc", "Mu", "Ml") + C2WGZ + _m("RGSQRTH", "RGSGAM2", "GSGAM2H"),
-                 _f("dwe.0", "dwe.1", "PM.0", "PM.4"), ()),
-    "vi_energy": (_f(*PROG[:5], "PS.0", "PS.1", "PS.2", "PS.3", "PS.4", "PS.5", "dwe.0", "dwe.1", "dvh.0", "dvh.1", "dvh.2",
-                     "hdiv.2", "ethtot0", "gT0.5") + _m("C2W.0", "C2W.1", "W2C.0", "W2C.1", "RGSQRTH", "PHI") + C2WGZ,
-                  _f("dwe.2"), ()),
+    "vi_solve": (_f("dvh.0", "dvh.1", "dvh.2", "eth", *_n("PS.", 6), "hdiv.0", "hdiv.1", "hdiv.2", "gT.0", "gT.4", "gT.5",
+                    "PM.0", "PM.4", *PROG[:5], "ethtot0", "gT0.5") + _f64("Mc", "Mu", "Ml") + C2WGZ +
+                 _m("RGSQRTH", "RGSGAM2", "GSGAM2H", "C2W.0", "C2W.1", "W2C.0", "W2C.1", "PHI"),
+                 _f("dwe.0", "dwe.1", "dwe.2", "PM.0", "PM.4"), ()),
     # PROG += PROG_split with the projection (k_post)
     "post": (_f(*PROG, *_n("PS.", 6)), _f(*PROG), _n("GRD_x.", 3)),
     # tracer advection (nc_tracer.cuh)
@@ -136,7 +134,7 @@ def step_launches(sstep=(2, 3, 6), nq: int = 1) -> dict:
     nst = len(sstep)
     return {"diag": nst, "advmom": nst, "hdiff1": nst, "hdiff2": nst, "gtend": nst, "split_init": nst - 1,
             "split_init_first": 1, "dd3d": nst + ns, "vp0_h": nst, "vp0_c": nst, "path1": ns, "vimain_a": ns,
-            "vi_solve": ns, "vi_energy": ns, "post": nst, "trc_vflux": 1, "trc_vadv": 2 * nq, "trc_hflux": 1,
+            "vi_solve": ns, "post": nst, "trc_vflux": 1, "trc_vadv": 2 * nq, "trc_hflux": 1,
             "trc_grad": nq, "trc_remap": nq, "trc_qout": nq, "trc_apply": nq, "trc_rhog": 1}
 
 

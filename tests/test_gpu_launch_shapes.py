@@ -4,10 +4,9 @@ remainders of its splits (B200).
 * Numbers of layers that do not divide by the warps of the vi_main column
   kernel, the levels per block of path 1 and the level chunks: one step at
   gl03 equals the oracle bit for bit.
-* One gl05 grid alone (its tiles and columns do not fill the SMs: level chunks,
-  k_vi_col) against 17 of them stacked in one handle (174,080 columns, above one
-  wave of the column kernel: whole marches, k_vi_solve and k_vi_energy_p): each
-  member bit for bit, in both forms.
+* One gl05 grid alone (its tiles and columns do not fill the SMs: level chunks)
+  against 17 of them stacked in one handle (whole marches): each member bit for
+  bit, in both forms.
 * Tracers in batches: every tracer of 6 (batches of 4 and 2) equals the same
   tracer carried alone, bit for bit.
 * The linear operators on an input that overlaps the output.
