@@ -989,7 +989,7 @@ static int run_step(nc_handle* h) {
       const dim3 gt(tx, ty, (unsigned)(D.L * ((levels + nk - 1) / nk)));
       k_dd3d_m<R, T, true><<<gt, TILE_THREADS, dd3d_m_smem<R, T>(), s>>>(v, o, nk);
       TRY(check_launch(h, "dd3d"));
-      k_dd3d_pl<<<pkb, 32, 0, ps>>>(vp, op);
+      k_dd3d_pl<<<(unsigned)((D.KA * D.LP * 8 + 31) / 32), 32, 0, ps>>>(vp, op);
       TRY(check_launch(h, "dd3d_pl"));
       return comm<R>(h, {h->vtmp2[0], h->vtmp2[1], h->vtmp2[2]});
     };

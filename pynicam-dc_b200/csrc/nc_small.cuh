@@ -54,45 +54,68 @@ constexpr int dd3d_m_smem() {
 // barrier is needed at the end of a level, and the corner tile alone waits
 // for its singular-point fix.
 
-// pole 3-D divergence damping (kernels/oprt3ddivdamp.py:176-237)
+// pole 3-D divergence damping (kernels/oprt3ddivdamp.py:176-237): eight lanes
+// per (level, pole), a lane for each pole point's momenta and half-level fluxes
+// and for each triangle between them (one thread formed every flux up to six
+// times over: 22 us a call, longer than the regional kernel on small grids)
 template <class R>
 __global__ void k_dd3d_pl(const __grid_constant__ Four<R> v, const __grid_constant__ Three<R> out) {
   const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= cD.KA * cD.LP) return;
-  int k = t / cD.LP, lp = t % cD.LP;
-  for (int g = 0; g < 6; ++g)
-    for (int d = 0; d < 3; ++d) out.f[d][ipl(g, k, lp)] = R(0.0);
-  if (k < cD.kmin || k > cD.kmax) return;
-  auto rw = [&](int g, int kk) -> R {
-    if (kk <= cD.kmin || kk > cD.kmax) return R(0.0);
-    int q = ipl(g, kk, lp), qm = ipl(g, kk - 1, lp);
-    const R* cz = CG.C2WGz_pl;
-    R h = cz[q * 6 + 0] * v.f[0][q] + cz[q * 6 + 1] * v.f[0][qm] + cz[q * 6 + 2] * v.f[1][q] +
-               cz[q * 6 + 3] * v.f[1][qm] + cz[q * 6 + 4] * v.f[2][q] + cz[q * 6 + 5] * v.f[2][qm];
-    return h * gam_at(CG.RGAMH_pl, q) + v.f[3][q] * CG.RGSQRTH_pl[q];
-  };
-  R vm[6][3];
-  for (int g = 0; g < 6; ++g) {
-    int q = ipl(g, k, lp);
-    for (int d = 0; d < 3; ++d) vm[g][d] = v.f[d][q] * gam_at(CG.RGAM_pl, q);
+  const int g = t % 8, np = cD.KA * cD.LP;
+  const bool live = t / 8 < np;
+  const int e = live ? t / 8 : np - 1;
+  const int k = e / cD.LP, lp = e % cD.LP;
+  const bool in = k >= cD.kmin && k <= cD.kmax;
+  R r0 = R(0.0), r1 = R(0.0), vm[3] = {R(0.0), R(0.0), R(0.0)};
+  if (g < 6 && in) {
+    auto rw = [&](int kk) -> R {
+      if (kk <= cD.kmin || kk > cD.kmax) return R(0.0);
+      const int q = ipl(g, kk, lp), qm = ipl(g, kk - 1, lp);
+      const R* cz = CG.C2WGz_pl;
+      const R h = cz[q * 6 + 0] * v.f[0][q] + cz[q * 6 + 1] * v.f[0][qm] + cz[q * 6 + 2] * v.f[1][q] +
+                  cz[q * 6 + 3] * v.f[1][qm] + cz[q * 6 + 4] * v.f[2][q] + cz[q * 6 + 5] * v.f[2][qm];
+      return h * gam_at(CG.RGAMH_pl, q) + v.f[3][q] * CG.RGSQRTH_pl[q];
+    };
+    r0 = rw(k);
+    r1 = rw(k + 1);
+    const int q = ipl(g, k, lp);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) vm[d] = v.f[d][q] * gam_at(CG.RGAM_pl, q);
   }
-  R sclt[5];
-  for (int v_ = 1; v_ <= 5; ++v_) {
-    int vp1 = (v_ == 5) ? 1 : v_ + 1;
-    R sw = div3((rw(0, k + 1) + rw(v_, k + 1) + rw(vp1, k + 1)) - (rw(0, k) + rw(v_, k) + rw(vp1, k))) * CC.rdgz[k];
-    const R* cI = CG.coef_intp_pl + (v_ * cD.LP + lp) * 9;
-    sclt[v_ - 1] = cI[0] * vm[0][0] + cI[1] * vm[v_][0] + cI[2] * vm[vp1][0] + cI[3] * vm[0][1] + cI[4] * vm[v_][1] +
-                   cI[5] * vm[vp1][1] + cI[6] * vm[0][2] + cI[7] * vm[v_][2] + cI[8] * vm[vp1][2] + sw;
-  }
+  // lane g = 1..5: the triangle of the pole, point g and the next point
+  const int gn = (g >= 5) ? 1 : g + 1;
+  auto of = [&](R x, int lane) { return __shfl_sync(0xffffffffu, x, lane, 8); };
+  const R u0 = of(r1, 0), un = of(r1, gn), d0 = of(r0, 0), dn = of(r0, gn);
+  R a[3], n[3];
+#pragma unroll
   for (int d = 0; d < 3; ++d) {
-    R row = R(0.0);
-    for (int v_ = 1; v_ <= 5; ++v_) {
-      int vm1 = (v_ == 1) ? 5 : v_ - 1;
-      R pair = sclt[vm1 - 1] + sclt[v_ - 1];
-      R tv = CG.coef_diff_pl[(v_ * cD.LP + lp) * 3 + d] * pair;
-      row = (v_ == 1) ? tv : row + tv;
+    a[d] = of(vm[d], 0);
+    n[d] = of(vm[d], gn);
+  }
+  R sclt = R(0.0);
+  if (g >= 1 && g <= 5 && in) {
+    const R sw = div3((u0 + r1 + un) - (d0 + r0 + dn)) * CC.rdgz[k];
+    const R* cI = CG.coef_intp_pl + (g * cD.LP + lp) * 9;
+    sclt = cI[0] * a[0] + cI[1] * vm[0] + cI[2] * n[0] + cI[3] * a[1] + cI[4] * vm[1] + cI[5] * n[1] + cI[6] * a[2] +
+           cI[7] * vm[2] + cI[8] * n[2] + sw;
+  }
+  R s[6];
+#pragma unroll
+  for (int m = 1; m <= 5; ++m) s[m] = of(sclt, m);
+  // lane g = 0..2: component g of the pole row; the other rows are zero
+  R row = R(0.0);
+  if (g < 3 && in) {
+#pragma unroll
+    for (int m = 1; m <= 5; ++m) {
+      const R tv = CG.coef_diff_pl[(m * cD.LP + lp) * 3 + g] * (s[m == 1 ? 5 : m - 1] + s[m]);
+      row = (m == 1) ? tv : row + tv;
     }
-    out.f[d][ipl(0, k, lp)] = row;
+  }
+  if (live && g < 3) {
+    R* o = out.f[g];
+    o[ipl(0, k, lp)] = row;
+#pragma unroll
+    for (int m = 1; m <= 5; ++m) o[ipl(m, k, lp)] = R(0.0);
   }
 }
 
