@@ -42,17 +42,22 @@ __device__ __forceinline__ R ddivd(int i, int j, int l, int d, const R aTI, cons
 // level.  Dynamic shared memory dd3d_m_smem<R, T>().
 template <class R, class T>
 constexpr int dd3d_m_smem() {
-  return (18 * (T::X + 1) * (T::Y + 1) + 5 * (T::X + 2) * (T::Y + 2) + 2 * (T::X + 1) * (T::Y + 1)) * (int)sizeof(R);
+  return (18 * (T::X + 1) * (T::Y + 1) + 9 * (T::X + 2) * (T::Y + 2) + 4 * (T::X + 1) * (T::Y + 1)) * (int)sizeof(R);
 }
 #ifndef DD_M_MINB
 #define DD_M_MINB 2
 #endif
-// The next level's staging writes s_vm and the rwv buffer of the level below,
-// which only this level's triangle pass reads (done before its second
-// barrier), and the next level's triangle pass writes s_ti / s_tj only after
-// the next first barrier, which every thread reaches after its cell pass: no
-// barrier is needed at the end of a level, and the corner tile alone waits
-// for its singular-point fix.
+// The march takes two levels at a time: a triangle's coefficients are read once
+// for both, and a pair of levels costs two barriers.  Bound by shared-memory
+// reads and barriers: gl08 mixed 636 -> 509 us, gl06 mixed 66 -> 58 us, gl07
+// float64 385 -> 362 us, gl05 float64 42 -> 41 us against one level at a time
+// (z40); with three float blocks an SM instead of four 546 us at gl08.
+// The next pair's staging writes s_vm and the rwv buffers of this pair's lower
+// half levels, which only this pair's triangle pass reads (done before its
+// second barrier), and the next triangle pass writes s_ti / s_tj only after the
+// next first barrier, which every thread reaches after its cell pass: no barrier
+// is needed at the end of a pair, and the corner tile alone waits for its
+// singular-point fix.
 
 // pole 3-D divergence damping (kernels/oprt3ddivdamp.py:176-237): eight lanes
 // per (level, pole), a lane for each pole point's momenta and half-level fluxes
@@ -128,14 +133,14 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, DD_M_MINB, 4)) k_dd3d
   constexpr int TX = T::X + 1, TY = T::Y + 1, NT = TX * TY;
   extern __shared__ __align__(16) unsigned char dd_smem[];
   R* s_ci = reinterpret_cast<R*>(dd_smem);   // [18][NT] coef_intp of each triangle
-  R* s_vm = s_ci + 18 * NT;                    // [3][NP]
-  R* s_rw = s_vm + 3 * NP;                     // [2][NP]
-  R* s_ti = s_rw + 2 * NP;                     // [NT]
-  R* s_tj = s_ti + NT;                         // [NT]
+  R* s_vm = s_ci + 18 * NT;                    // [2][3][NP] of the pair's levels
+  R* s_rw = s_vm + 6 * NP;                     // [3][NP] half levels k, k+1, k+2
+  R* s_ti = s_rw + 3 * NP;                     // [2][NT]
+  R* s_tj = s_ti + 2 * NT;                     // [2][NT]
   const int l = (int)blockIdx.z % cD.L;
   const int ka = cD.kmin + (int)blockIdx.z / cD.L * nk, kb = min(ka + nk - 1, cD.kmax);
   const int i0 = 1 + blockIdx.x * T::X, j0 = 1 + blockIdx.y * T::Y;
-  const int G = cD.G, gmax = cD.G - 2;
+  const int G = cD.G, gmax = cD.G - 2, kmax = cD.kmax;
   const int tid = threadIdx.x, tx = tid % T::X, ty = tid / T::X;
   const int i = i0 + tx, j = j0 + ty;
   const bool own = (i <= gmax) && (j <= gmax);
@@ -152,90 +157,113 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, DD_M_MINB, 4)) k_dd3d
 #pragma unroll
     for (int m = 0; m < (CDR ? 18 : 1); ++m) cd[m] = P2c(CG.coef_diff, m, i, j, l);
   }
-  // vertical mass flux at half level k (q: the point at k)
-  auto rwv = [&](int q) -> R {
-    const int qm = q - cD.planei;
-    const R h = mad(cz[5 * n + q], v.f[2][qm], mad(cz[4 * n + q], v.f[2][q], mad(cz[3 * n + q], v.f[1][qm],
-                mad(cz[2 * n + q], v.f[1][q], mad(cz[n + q], v.f[0][qm], cz[q] * v.f[0][q])))));
-    return h * gam_at(CG.RGAMH, q) + v.f[3][q] * CG.RGSQRTH[q];
+  // vertical mass flux at the half level of q from the momenta at q (u) and below (d)
+  auto rwv = [&](int q, const R* u, const R* d, R w) -> R {
+    const R h = mad(cz[5 * n + q], d[2], mad(cz[4 * n + q], u[2], mad(cz[3 * n + q], d[1],
+                mad(cz[2 * n + q], u[1], mad(cz[n + q], d[0], cz[q] * u[0])))));
+    return h * gam_at(CG.RGAMH, q) + w * CG.RGSQRTH[q];
   };
   for (int p = tid; p < NP; p += blockDim.x) {   // at the chunk's first level (zero at kmin)
     const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
-    s_rw[p] = (ka > cD.kmin && ii < G && jj < G) ? rwv(ix(ii, jj, ka, l)) : R(0.0);
+    R r = R(0.0);
+    if (ka > cD.kmin && ii < G && jj < G) {
+      const int q = ix(ii, jj, ka, l), qm = q - cD.planei;
+      const R u[3] = {v.f[0][q], v.f[1][q], v.f[2][q]}, d[3] = {v.f[0][qm], v.f[1][qm], v.f[2][qm]};
+      r = rwv(q, u, d, v.f[3][q]);
+    }
+    s_rw[p] = r;
   }
-  int cur = 0;
-  for (int k = ka; k <= kb; ++k) {
-    const bool up = (k + 1 <= cD.kmax);   // rwv(k+1) = 0 above kmax
+  int c0 = 0;   // slot of half level k
+  for (int k = ka; k <= kb; k += 2) {
+    const int c1 = (c0 + 1) % 3, c2 = (c0 + 2) % 3;
     for (int p = tid; p < NP; p += blockDim.x) {
       const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
-      R a = R(0.0), b = R(0.0), c = R(0.0), r = R(0.0);
+      R f[3][3], r1 = R(0.0), r2 = R(0.0), rg0 = R(0.0), rg1 = R(0.0);
+#pragma unroll
+      for (int m = 0; m < 9; ++m) f[m / 3][m % 3] = R(0.0);
       if (ii < G && jj < G) {
         const int q = ix(ii, jj, k, l);
-        const R f0 = v.f[0][q], f1 = v.f[1][q], f2 = v.f[2][q];
-        const R rg = gam_at(CG.RGAM, q);
-        a = f0 * rg;
-        b = f1 * rg;
-        c = f2 * rg;
-        if (up) {
-          const int qp = q + cD.planei;   // level k+1
-          const R h = mad(cz[5 * n + qp], f2, mad(cz[4 * n + qp], v.f[2][qp], mad(cz[3 * n + qp], f1,
-                      mad(cz[2 * n + qp], v.f[1][qp], mad(cz[n + qp], f0, cz[qp] * v.f[0][qp])))));
-          r = h * gam_at(CG.RGAMH, qp) + v.f[3][qp] * CG.RGSQRTH[qp];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) f[0][d] = v.f[d][q];
+        rg0 = gam_at(CG.RGAM, q);
+        if (k + 1 <= kmax) {          // rwv is zero above kmax
+          const int q1 = q + cD.planei;
+#pragma unroll
+          for (int d = 0; d < 3; ++d) f[1][d] = v.f[d][q1];
+          rg1 = gam_at(CG.RGAM, q1);
+          r1 = rwv(q1, f[1], f[0], v.f[3][q1]);
+          if (k + 2 <= kmax) {
+            const int q2 = q1 + cD.planei;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) f[2][d] = v.f[d][q2];
+            r2 = rwv(q2, f[2], f[1], v.f[3][q2]);
+          }
         }
       }
-      s_vm[p] = a;
-      s_vm[NP + p] = b;
-      s_vm[2 * NP + p] = c;
-      s_rw[(cur ^ 1) * NP + p] = r;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        s_vm[d * NP + p] = f[0][d] * rg0;
+        s_vm[(3 + d) * NP + p] = f[1][d] * rg1;
+      }
+      s_rw[c1 * NP + p] = r1;
+      s_rw[c2 * NP + p] = r2;
     }
     __syncthreads();
-    const R rdz = CC.rdgz[k];
-    const R* rU = s_rw + (cur ^ 1) * NP;
-    const R* rD = s_rw + cur * NP;
+    const R* rw[3] = {s_rw + c0 * NP, s_rw + c1 * NP, s_rw + c2 * NP};
     for (int p = tid; p < NT; p += blockDim.x) {
       const int px = p % TX, py = p / TX;
       const int a = py * PX + px, b = a + 1, c = a + PX + 1, d = a + PX;
-      auto C = [&](int dir, int pt, int t) { return s_ci[((dir * 3 + pt) * 2 + t) * NT + p]; };
-      const R wTI = div3((rU[a] + rU[b] + rU[c]) - (rD[a] + rD[b] + rD[c])) * rdz;
-      const R wTJ = div3((rU[a] + rU[c] + rU[d]) - (rD[a] + rD[c] + rD[d])) * rdz;
-      const R* v0 = s_vm;
-      const R* v1 = s_vm + NP;
-      const R* v2 = s_vm + 2 * NP;
-      R sTI = C(0, 0, 0) * v0[a], sTJ = C(0, 0, 1) * v0[a];
-      sTI = mad(C(0, 1, 0), v0[b], sTI); sTJ = mad(C(0, 1, 1), v0[c], sTJ);
-      sTI = mad(C(0, 2, 0), v0[c], sTI); sTJ = mad(C(0, 2, 1), v0[d], sTJ);
-      sTI = mad(C(1, 0, 0), v1[a], sTI); sTJ = mad(C(1, 0, 1), v1[a], sTJ);
-      sTI = mad(C(1, 1, 0), v1[b], sTI); sTJ = mad(C(1, 1, 1), v1[c], sTJ);
-      sTI = mad(C(1, 2, 0), v1[c], sTI); sTJ = mad(C(1, 2, 1), v1[d], sTJ);
-      sTI = mad(C(2, 0, 0), v2[a], sTI); sTJ = mad(C(2, 0, 1), v2[a], sTJ);
-      sTI = mad(C(2, 1, 0), v2[b], sTI); sTJ = mad(C(2, 1, 1), v2[c], sTJ);
-      sTI = mad(C(2, 2, 0), v2[c], sTI); sTJ = mad(C(2, 2, 1), v2[d], sTJ);
-      sTI = sTI + wTI;
-      sTJ = sTJ + wTJ;
+      const int vI[3] = {a, b, c}, vJ[3] = {a, c, d};
+      R sI[2], sJ[2];
+#pragma unroll
+      for (int m = 0; m < 9; ++m) {   // direction m / 3, vertex m % 3, left to right
+        const R cI = s_ci[(m * 2) * NT + p], cJ = s_ci[(m * 2 + 1) * NT + p];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const R* x = s_vm + (3 * e + m / 3) * NP;
+          sI[e] = m ? mad(cI, x[vI[m % 3]], sI[e]) : cI * x[vI[0]];
+          sJ[e] = m ? mad(cJ, x[vJ[m % 3]], sJ[e]) : cJ * x[vJ[0]];
+        }
+      }
       const int ii = i0 - 1 + px, jj = j0 - 1 + py;
-      if (!(ii <= G - 2 && jj <= G - 2)) sTI = sTJ = R(0.0);
-      s_ti[p] = sTI;
-      s_tj[p] = sTJ;
+      const bool ok = ii <= G - 2 && jj <= G - 2;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const R* rU = rw[e + 1];
+        const R* rD = rw[e];
+        const R rdz = CC.rdgz[k + e];
+        const R wI = div3((rU[a] + rU[b] + rU[c]) - (rD[a] + rD[b] + rD[c])) * rdz;
+        const R wJ = div3((rU[a] + rU[c] + rU[d]) - (rD[a] + rD[c] + rD[d])) * rdz;
+        s_ti[e * NT + p] = ok ? sI[e] + wI : R(0.0);
+        s_tj[e * NT + p] = ok ? sJ[e] + wJ : R(0.0);
+      }
     }
     __syncthreads();
     if (i0 == 1 && j0 == 1) {   // singular-point fix at the (0,0) triangle (block-uniform branch)
-      if (tid == 0) s_ti[0] = s_ti[0] * (R)CG.pntmask[l * 2 + 0] + s_tj[1] * (R)CG.pntmask[l * 2 + 1];
+      if (tid < 2)
+        s_ti[tid * NT] = s_ti[tid * NT] * (R)CG.pntmask[l * 2 + 0] + s_tj[tid * NT + 1] * (R)CG.pntmask[l * 2 + 1];
       __syncthreads();
     }
     if (own) {
       const int ta = (ty + 1) * TX + (tx + 1);   // triangle (i, j)
-      const R aTI = s_ti[ta], aTJ = s_tj[ta];
-      const R bTI = s_ti[ta - 1];            // (i-1, j)
-      const R cTI = s_ti[ta - TX - 1], cTJ = s_tj[ta - TX - 1];   // (i-1, j-1)
-      const R dTJ = s_tj[ta - TX];           // (i, j-1)
-      const int q = ix(i, j, k, l);
       auto D = [&](int m) { return CDR ? cd[CDR ? m : 0] : P2c(CG.coef_diff, m, i, j, l); };
 #pragma unroll
-      for (int d = 0; d < 3; ++d)
-        out.f[d][q] = mad(D(d * 6 + 5), dTJ + aTI, mad(D(d * 6 + 4), cTI + dTJ, mad(D(d * 6 + 3), cTJ + cTI,
-                      mad(D(d * 6 + 2), bTI + cTJ, mad(D(d * 6 + 1), aTJ + bTI, D(d * 6 + 0) * (aTI + aTJ))))));
+      for (int e = 0; e < 2; ++e) {
+        if (k + e > kb) break;
+        const R* I = s_ti + e * NT;
+        const R* J = s_tj + e * NT;
+        const R aTI = I[ta], aTJ = J[ta];
+        const R bTI = I[ta - 1];                                // (i-1, j)
+        const R cTI = I[ta - TX - 1], cTJ = J[ta - TX - 1];     // (i-1, j-1)
+        const R dTJ = J[ta - TX];                               // (i, j-1)
+        const int q = ix(i, j, k + e, l);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          out.f[d][q] = mad(D(d * 6 + 5), dTJ + aTI, mad(D(d * 6 + 4), cTI + dTJ, mad(D(d * 6 + 3), cTJ + cTI,
+                        mad(D(d * 6 + 2), bTI + cTJ, mad(D(d * 6 + 1), aTJ + bTI, D(d * 6 + 0) * (aTI + aTJ))))));
+      }
     }
-    cur ^= 1;
+    c0 = c2;
   }
 }
 
