@@ -725,6 +725,16 @@ static int trc_vadv(nc_handle* h, FieldPair* x, int nx, bool second) {
   return 0;
 }
 
+// Levels per chunk of a kernel whose blocks march over the levels of a tile:
+// all of them where the tiles fill the SMs (4 blocks each; a chunk repeats its
+// first half level and re-reads the tile's coefficients), else enough chunks
+// for that, of at least 4 levels.
+static int tile_chunks(const nc_handle* h, int blocks, int levels) {
+  const int want = 4 * h->sms;
+  const int n = std::max(1, std::min((want + blocks - 1) / blocks, levels / 4));
+  return (levels + n - 1) / n;
+}
+
 template <class R>
 static int trc_hflux(nc_handle* h) {
   const Dims& D = h->D;
@@ -738,8 +748,13 @@ static int trc_hflux(nc_handle* h) {
     for (int f = 0; f < 9; ++f) ha.xc[f] = RG<R>(h->xc[f]);
     ha.dt = dt;
     {
-      const dim3 gt((unsigned)D.KA, (unsigned)(((D.G + TH_DX - 1) / TH_DX) * ((D.G + TH_DY - 1) / TH_DY)), (unsigned)D.L);
-      k_trc_hflux_t<<<gt, TH_DX * TH_DY, 0, s>>>(ha);
+      const int tiles = ((D.G + TH_DX - 1) / TH_DX) * ((D.G + TH_DY - 1) / TH_DY);
+      if constexpr (std::is_same<R, float>::value) {
+        const int nk = tile_chunks(h, tiles * D.L, D.KA);
+        k_trc_hflux_m<<<dim3((unsigned)((D.KA + nk - 1) / nk), (unsigned)tiles, (unsigned)D.L), TH_DX * TH_DY, 0, s>>>(ha, nk);
+      } else {
+        k_trc_hflux_t<<<dim3((unsigned)D.KA, (unsigned)tiles, (unsigned)D.L), TH_DX * TH_DY, 0, s>>>(ha);
+      }
     }
     TRY(check_launch(h, "trc_hflux"));
     TrcHfluxPlArgs<R> hp;
@@ -835,15 +850,6 @@ static int trc_rhog(nc_handle* h) {
   return 0;
 }
 
-// Levels per chunk of a kernel whose blocks march over the levels of a tile:
-// all of them where the tiles fill the SMs (4 blocks each; a chunk repeats its
-// first half level and re-reads the tile's coefficients), else enough chunks
-// for that, of at least 4 levels.
-static int tile_chunks(const nc_handle* h, int blocks, int levels) {
-  const int want = 4 * h->sms;
-  const int n = std::max(1, std::min((want + blocks - 1) / blocks, levels / 4));
-  return (levels + n - 1) / n;
-}
 // Levels per thread of a column kernel split along the levels
 static int column_chunks(const nc_handle* h, int levels) {
   const long long want = 4LL * 1024 * h->sms;

@@ -306,6 +306,132 @@ __global__ void __launch_bounds__(TH_DX * TH_DY) k_trc_hflux_t(TrcHfluxArgs<R> a
   }
 }
 
+// The same with a march over nk levels in each block, the float form: the vertex
+// weights GMTR_t in shared memory, the coefficients of the cell's own faces and
+// of its neighbours' in registers once for the block's levels.  Bound by
+// instructions, of which the 33 reads of coefficients a cell and level were the
+// largest part; three blocks an SM (80 registers; four spill: 1.33 ms).
+// gl08 z40 1.56 -> 1.20 ms, gl06 z40 164 -> 131 us, 12 x gl05 z40 518 -> 449 us.
+// The double form stays with a block per level: the coefficients take 56 more
+// registers (two blocks an SM: gl07 z40 0.62 -> 0.70 ms; read per level in the
+// march instead: 0.79 ms).
+// The next level's staging writes s_f, read before this level's last barrier,
+// and its vertex pass writes s_ti / s_tj after the next barrier, which every
+// thread reaches after its faces: two barriers a level.
+template <class R>
+__global__ void __launch_bounds__(TH_DX * TH_DY, 3) k_trc_hflux_m(const __grid_constant__ TrcHfluxArgs<R> a, int nk) {
+  constexpr int PX = TH_DX + 2, PY = TH_DY + 2, TX = TH_DX + 1, TY = TH_DY + 1, NT = TX * TY;
+  __shared__ R s_f[4][PY * PX];
+  __shared__ R s_w[6][NT];
+  __shared__ R s_ti[4][NT], s_tj[4][NT];
+  const int G = cD.G, l = (int)blockIdx.z;
+  const int ntx = (G + TH_DX - 1) / TH_DX;
+  const int i0 = ((int)blockIdx.y % ntx) * TH_DX, j0 = ((int)blockIdx.y / ntx) * TH_DY;
+  const int ka = (int)blockIdx.x * nk, kb = min(ka + nk, cD.KA);
+  const int tid = threadIdx.x;
+  for (int p = tid; p < NT; p += blockDim.x) {   // weights of the vertices (i0-1.., j0-1..)
+    const int vi = i0 - 1 + p % TX, vj = j0 - 1 + p / TX;
+    const bool ok = vi >= 0 && vj >= 0 && vi <= G - 2 && vj <= G - 2;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) s_w[m][p] = ok ? P2c(CG.GMTR_t, m, vi, vj, l) : R(0.0);
+  }
+  const int i = i0 + tid % TH_DX, j = j0 + tid / TH_DX;
+  const bool own = i < G && j < G;
+  const bool hi = i <= G - 2, hj = j <= G - 2;
+  // which of the cell's faces exist, and the owner cell of each
+  const bool on[6] = {own && hi && hj && j >= 1, own && hi && hj, own && hi && hj && i >= 1,
+                      own && i >= 1 && hj && j >= 1, own && i >= 1 && j >= 1, own && i >= 1 && hi && j >= 1};
+  R ga[6][3], xr[9];
+#pragma unroll
+  for (int f = 0; f < 6; ++f) {
+    const int ci = (f == 3 || f == 4) ? i - 1 : i, cj = f >= 4 ? j - 1 : j;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) ga[f][d] = on[f] ? P2c(CG.GMTR_a, (f % 3) * 3 + d, ci, cj, l) : R(0.0);
+  }
+#pragma unroll
+  for (int m = 0; m < 9; ++m) xr[m] = on[m / 3] ? P2c(CG.GRD_xr, m, i, j, l) : R(0.0);
+  const R PR = own ? P2c(CG.GMTR_p, 0, i, j, l) : R(0.0);
+  const R m0 = (R)CG.pntmask[l * 2 + 0], m1 = (R)CG.pntmask[l * 2 + 1];
+  const R dt = a.dt;
+  const bool corner = i == 1 && j == 1;
+  // vertices (i, j), (i-1, j), (i, j-1) and (i-1, j-1)
+  const int vc = (j - j0 + 1) * TX + (i - i0 + 1), vw = vc - 1, vs = vc - TX, vsw = vc - TX - 1;
+  for (int k = ka; k < kb; ++k) {
+    for (int p = tid; p < PX * PY; p += blockDim.x) {
+      const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
+      R f0 = R(0.0), f1 = R(0.0), f2 = R(0.0), f3 = R(0.0);
+      if (ii >= 0 && jj >= 0 && ii < G && jj < G) {
+        const int q = ix(ii, jj, k, l);
+        const R rg = CG.RGAM[q];
+        f0 = a.rho[q];
+        f1 = a.rvx[q] * rg;
+        f2 = a.rvy[q] * rg;
+        f3 = a.rvz[q] * rg;
+      }
+      s_f[0][p] = f0; s_f[1][p] = f1; s_f[2][p] = f2; s_f[3][p] = f3;
+    }
+    const int p = own ? ix(i, j, k, l) : 0;
+    const R rgt = a.rhog_t[p];
+    __syncthreads();
+    for (int v = tid; v < NT; v += blockDim.x) {
+      const int ia = (v / TX) * PX + v % TX, ib = ia + 1, ic = ia + PX + 1, id = ia + PX;
+      const int vi = i0 - 1 + v % TX, vj = j0 - 1 + v / TX;
+      const bool ok = vi >= 0 && vj >= 0 && vi <= G - 2 && vj <= G - 2;
+      R w[6];
+#pragma unroll
+      for (int m = 0; m < 6; ++m) w[m] = s_w[m][v];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const R f0 = s_f[n][ia], fi = s_f[n][ib], fd = s_f[n][ic], fj = s_f[n][id];
+        const R ti = mad(fd, w[2], mad(fi, w[1], f0 * w[0]));
+        const R tj = mad(f0, w[3], mad(fj, w[5], fd * w[4]));
+        s_ti[n][v] = ok ? ti : R(0.0);
+        s_tj[n][v] = ok ? tj : R(0.0);
+      }
+    }
+    __syncthreads();
+    if (i0 == 0 && j0 == 0) {   // singular-point fix of vertex (0,0) (mod_src_tracer.py:1409-1412)
+      const int v00 = 1 * TX + 1, v10 = 1 * TX + 2;
+      if (tid < 4) s_ti[tid][v00] = s_ti[tid][v00] * m0 + s_tj[tid][v10] * m1;
+      __syncthreads();
+    }
+    if (!own) continue;
+    // sum n of the two vertex values of face f (mod_src_tracer.py:1414-1484)
+    auto S = [&](int f, int n) -> R {
+      switch (f) {
+        case 0: return s_tj[n][vs] + s_ti[n][vc];     // TJ(i, j-1) + TI(i, j)
+        case 1: return s_ti[n][vc] + s_tj[n][vc];     // TI(i, j) + TJ(i, j)
+        case 2: return s_tj[n][vc] + s_ti[n][vw];     // TJ(i, j) + TI(i-1, j)
+        case 3: return s_tj[n][vsw] + s_ti[n][vw];    // face 0 of (i-1, j)
+        case 4: return s_ti[n][vsw] + s_tj[n][vsw];   // face 1 of (i-1, j-1)
+        default: return s_tj[n][vs] + s_ti[n][vsw];   // face 2 of (i, j-1)
+      }
+    };
+    const auto rg = recip_of(rgt);   // six quotients by rhog_t
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      const R s1 = S(f, 1), s2 = S(f, 2), s3 = S(f, 3);
+      const R flux = R(0.5) * mad(s3, ga[f][2], mad(s2, ga[f][1], s1 * ga[f][0]));
+      R fl = (f < 3 ? flux : -flux) * PR * dt;
+      fl = on[f] ? fl : R(0.0);
+      if (f == 5 && corner) fl *= m0;
+      a.flx[f][p] = fl;
+      const R chv = div_by(fl, rg);
+      a.ch[f][p] = chv;
+      a.cm[f][p] = R(0.5) - copysign(R(0.5), chv - CC.EPS);
+      if (f < 3) {
+        const R rr2 = R(1.0) / npmax(S(f, 0), CC.EPS);
+        const R sd[3] = {s1, s2, s3};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const R x = xr[f * 3 + d] - sd[d] * rr2 * dt * R(0.5);
+          a.xc[f * 3 + d][p] = on[f] ? x : R(0.0);
+        }
+      }
+    }
+  }
+}
+
 // pole edges (mod_src_tracer.py:1487-1531) and Courant numbers
 template <class R>
 struct TrcHfluxPlArgs {
