@@ -444,14 +444,17 @@ __device__ __forceinline__ R hdiff_kh(R lapT, int k) {
 // staged in shared memory and the cell's Laplacian and diffusion coefficients
 // (coef_lap 7, coef_diff 18) held in registers once for all of the block's
 // levels, instead of re-read from L2 at every level.  Dynamic shared memory:
-// hdiff2_m_smem<R, T>() bytes (45 KB float, 90 KB double).  Kh per cell from
-// hdiff_kh (the first pass's temperature Laplacian is the staged field 4).
+// hdiff2_m_smem<R, T>() bytes (46 KB float, 93 KB double).  rhog * Kh of the two
+// diffusions, from hdiff_kh (the first pass's temperature Laplacian is the staged
+// field 4), is formed where a point is staged; a cell formed the fourteen values
+// that it reads.  gl08 mixed 889 -> 844 us, gl06 mixed 69 -> 65 us, gl07 float64
+// 495 -> 490 us (constant Kh, z40; the nonlinear Kh costs a division besides).
 #ifndef HD_NK
 #define HD_NK 6
 #endif
 template <class R, class T>
 constexpr int hdiff2_m_smem() {
-  return ((18 + 12) * (T::X + 1) * (T::Y + 1) + 7 * (T::X + 2) * (T::Y + 2)) * (int)sizeof(R);
+  return ((18 + 12) * (T::X + 1) * (T::Y + 1) + 8 * (T::X + 2) * (T::Y + 2)) * (int)sizeof(R);
 }
 template <class R>
 __global__ void k_hdiff2_pl(const __grid_constant__ Six<R> vt, const R* rhog, const __grid_constant__ SixOut<R> out) {
@@ -507,8 +510,8 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, 4)) k_hdiff2_m(Six
   extern __shared__ __align__(16) unsigned char hd_smem[];
   R* s_w = reinterpret_cast<R*>(hd_smem);   // [18][NT] triangle weights
   R* s_f = s_w + 18 * NT;                     // [6][NP] the six Laplacians
-  R* s_r = s_f + 6 * NP;                      // [NP] rhog
-  R* s_t = s_r + NP;                          // [2][6][NT] triangle values of fields 4 and 5
+  R* s_k = s_f + 6 * NP;                      // [2][NP] rhog * factor * Kh of fields 4 and 5
+  R* s_t = s_k + 2 * NP;                      // [2][6][NT] triangle values of fields 4 and 5
   const int l = (int)blockIdx.z;
   const int ntx = (cD.G - 2 + T::X - 1) / T::X;
   const int i0 = 1 + ((int)blockIdx.y % ntx) * T::X, j0 = 1 + ((int)blockIdx.y / ntx) * T::Y;
@@ -538,7 +541,9 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, 4)) k_hdiff2_m(Six
       const int q = ok ? ix(ii, jj, k, l) : 0;
 #pragma unroll
       for (int n = 0; n < 6; ++n) s_f[n * NP + p] = ok ? vt.f[n][q] : R(0.0);
-      s_r[p] = ok ? rhog[q] : R(0.0);
+      const R rg = ok ? rhog[q] : R(0.0), kh = hdiff_kh<R>(s_f[4 * NP + p], k);
+      s_k[p] = rg * kfac[0] * kh;
+      s_k[NP + p] = rg * kfac[1] * kh;
     }
     __syncthreads();
     for (int p = tid; p < NT; p += blockDim.x) {
@@ -567,12 +572,14 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, 4)) k_hdiff2_m(Six
       }
     }
     __syncthreads();
-    if (i0 == 1 && j0 == 1 && tid < 6) {   // singular-point fix of the (0,0) triangle, fields 4 and 5
-      const int f = tid / 3, d = tid % 3;
-      const R m0 = (R)CG.pntmask[l * 2 + 0], m1 = (R)CG.pntmask[l * 2 + 1];
-      s_t[(f * 6 + d) * NT] = s_t[(f * 6 + d) * NT] * m0 + s_t[(f * 6 + 3 + d) * NT + 1] * m1;
+    if (i0 == 1 && j0 == 1) {   // singular-point fix of the (0,0) triangle, fields 4 and 5 (block-uniform branch)
+      if (tid < 6) {
+        const int f = tid / 3, d = tid % 3;
+        const R m0 = (R)CG.pntmask[l * 2 + 0], m1 = (R)CG.pntmask[l * 2 + 1];
+        s_t[(f * 6 + d) * NT] = s_t[(f * 6 + d) * NT] * m0 + s_t[(f * 6 + 3 + d) * NT + 1] * m1;
+      }
+      __syncthreads();
     }
-    __syncthreads();
     if (own) {
       const int q = ix(i, j, k, l);
       const int c0 = (ty + 1) * PX + (tx + 1);
@@ -588,7 +595,7 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, 4)) k_hdiff2_m(Six
       const int ta = (ty + 1) * TX + (tx + 1), tb = ta - 1, tc = ta - TX - 1, td = ta - TX;
 #pragma unroll
       for (int f = 0; f < 2; ++f) {
-        auto kh = [&](int pt) { return s_r[pt] * kfac[f] * hdiff_kh<R>(s_f[4 * NP + pt], k); };
+        auto kh = [&](int pt) { return s_k[f * NP + pt]; };
         const R kh0 = kh(nb[0]);
         const R kf1 = R(0.5) * (kh0 + kh(nb[2])), kf2 = R(0.5) * (kh0 + kh(nb[3])), kf3 = R(0.5) * (kh0 + kh(nb[4]));
         const R kf4 = R(0.5) * (kh0 + kh(nb[5])), kf5 = R(0.5) * (kh0 + kh(nb[6])), kf6 = R(0.5) * (kh0 + kh(nb[1]));
