@@ -171,8 +171,8 @@ struct AdvMomArgs {
 // Tiled momentum advection for interior cells: one block per tile of a
 // region, marching upward over kmin..kmax (the vertical-momentum tendency at k
 // needs the projection at k-1, and the half-level flux at k is reused from the
-// level below).  Per level the haloed tile of rhogv, the merged velocity and
-// RGAM is staged in shared memory for the three 7-point divergences.  Halo
+// level below).  Per level the products of rhogv, the merged velocity and
+// RGAM on the haloed tile are staged in shared memory for the 7-point divergences.  Halo
 // cells and boundary levels are not written (their values are never read:
 // the large-step tendencies derived from them are replaced by the exchanges).
 // Arithmetic and association order are those of the reference's expressions
@@ -181,11 +181,18 @@ struct AdvMomArgs {
 // SMs idle (see tile_chunks); a chunk walks two levels below its first
 // without storing them, for the projection and the flux that its first needs.
 // (SPLIT; the unsplit instance keeps the registers of the chunk's bounds)
+// Bound by shared-memory reads and, on small grids, by the latency of a level's
+// staging.  So the nine products rhogv_d * vv_s * RGAM of a point are formed once
+// where it is staged (each was formed for seven cells, from three reads), each
+// coefficient is read once for the three velocities, and the next level's loads
+// are in flight while this level is worked on (two levels in shared memory, one
+// barrier a level).  At z40, before and now: gl05 float64 92 -> 59 us, gl06 mixed
+// 153 -> 91 us, gl07 float64 611 -> 561 us, gl08 mixed 989 -> 820 us.
 template <class R, class T, bool SPLIT>
 __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, NC_F32_ADVMOM)) k_advmom_t(AdvMomArgs<R> a, int nk) {
   constexpr int TXD = T::X, TYD = T::Y;
-  constexpr int PX = TXD + 2, PY = TYD + 2;
-  __shared__ R s_rv[3][PY * PX], s_vv[3][PY * PX], s_rg[PY * PX];
+  constexpr int PX = TXD + 2, PY = TYD + 2, NP = PX * PY, PT = (NP + TILE_THREADS - 1) / TILE_THREADS;
+  __shared__ R s_p[2][9][NP];   // (rhogv_d * vv_s) * RGAM at [d * 3 + s], two levels
   const int ntx = (cD.G - 2 + TXD - 1) / TXD;
   const int l = (int)blockIdx.z;
   const int i0 = 1 + ((int)blockIdx.x % ntx) * TXD, j0 = 1 + ((int)blockIdx.x / ntx) * TYD;
@@ -197,30 +204,53 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, NC_F32_ADVMOM)) k_
   const R* vv[3] = {a.vvx, a.vvy, a.vvz};
   const R* cz = CG.C2WGz;
   const int n = cD.npti;
+  R f[PT][7];   // a level's staged points of the thread on their way to shared memory
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int e = 0; e < PT; ++e) {
+      const int p = tid + e * TILE_THREADS;
+      const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
+      const bool ok = p < NP && ii < G && jj < G;
+      const int q = ok ? ix(ii, jj, k, l) : 0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        f[e][d] = ok ? __ldg(rv[d] + q) : R(0.0);
+        f[e][3 + d] = ok ? __ldg(vv[d] + q) : R(0.0);
+      }
+      f[e][6] = ok ? gam_at(CG.RGAM, q) : R(0.0);
+    }
+  };
+  auto put = [&](int b) {
+#pragma unroll
+    for (int e = 0; e < PT; ++e) {
+      const int p = tid + e * TILE_THREADS;
+      if (p < NP) {
+#pragma unroll
+        for (int m = 0; m < 9; ++m) s_p[b][m][p] = (f[e][m / 3] * f[e][3 + m % 3]) * f[e][6];
+      }
+    }
+  };
+  const int ka = SPLIT ? kmin + (int)blockIdx.y * nk : kmin, kb = SPLIT ? min(ka + nk - 1, kmax) : kmax;
+  const int k0 = SPLIT ? max(ka - 2, kmin) : kmin;
   R gx = R(0.0), gy = R(0.0), gz = R(0.0);
   int q0 = 0;
+  R r0[3] = {R(0.0), R(0.0), R(0.0)}, v0[3] = {R(0.0), R(0.0), R(0.0)};   // the own column's rhogv and vv at level k
   if (own) {
     gx = div_r(P2(CG.GRD_x, 0, i, j, l));
     gy = div_r(P2(CG.GRD_x, 1, i, j, l));
     gz = div_r(P2(CG.GRD_x, 2, i, j, l));
     q0 = ix(i, j, 0, l);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) { r0[d] = __ldg(rv[d] + q0 + k0 * cD.planei); v0[d] = __ldg(vv[d] + q0 + k0 * cD.planei); }
   }
   R vmh_lo[3] = {R(0.0), R(0.0), R(0.0)};
   R gwc_prev = R(0.0);
-  const int ka = SPLIT ? kmin + (int)blockIdx.y * nk : kmin, kb = SPLIT ? min(ka + nk - 1, kmax) : kmax;
-  for (int k = SPLIT ? max(ka - 2, kmin) : kmin; k <= kb; ++k) {
-    for (int p = tid; p < PX * PY; p += blockDim.x) {
-      const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
-      const bool ok = ii < G && jj < G;
-      const int q = ok ? ix(ii, jj, k, l) : 0;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        s_rv[d][p] = ok ? rv[d][q] : R(0.0);
-        s_vv[d][p] = ok ? vv[d][q] : R(0.0);
-      }
-      s_rg[p] = ok ? gam_at(CG.RGAM, q) : R(0.0);
-    }
-    __syncthreads();
+  int b = 0;
+  fetch(k0);
+  put(0);
+  __syncthreads();
+  for (int k = k0; k <= kb; ++k, b ^= 1) {
+    if (k < kb) fetch(k + 1);
     if (own) {
       const int c0 = (ty + 1) * PX + (tx + 1);
       const int nb[7] = {c0, c0 + 1, c0 + PX + 1, c0 + PX, c0 - 1, c0 - PX - 1, c0 - PX};
@@ -228,37 +258,48 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, NC_F32_ADVMOM)) k_
       const int kk = k + 1;
       const bool hv = (kk > kmin && kk <= kmax);
       const int qh = p + cD.planei;   // level k+1 of the own column
+      R div[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        R sm[3];
+#pragma unroll
+        for (int m = 0; m < 7; ++m) {
+          const R cf = P2(CG.coef_div, d * 7 + m, i, j, l);
+#pragma unroll
+          for (int s = 0; s < 3; ++s) {
+            const R v = s_p[b][d * 3 + s][nb[m]];
+            sm[s] = (m == 0) ? cf * v : mad(cf, v, sm[s]);
+          }
+        }
+#pragma unroll
+        for (int s = 0; s < 3; ++s) div[s] = (d == 0) ? sm[s] : div[s] + sm[s];
+      }
+      R vmh[3] = {R(0.0), R(0.0), R(0.0)}, r1[3] = {R(0.0), R(0.0), R(0.0)}, v1[3] = {R(0.0), R(0.0), R(0.0)};
+      if (hv) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) { r1[d] = __ldg(rv[d] + qh); v1[d] = __ldg(vv[d] + qh); }
+        R z[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) z[m] = cz[m * n + qh];
+        const R rw = a.rw[qh], gh = gam_at(CG.RGAMH, qh), rgs = CG.RGSQRTH[qh];
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+          const R sh = v1[s], sl = v0[s];
+          const R h = z[0] * (r1[0] * sh) + z[1] * (r0[0] * sl) + z[2] * (r1[1] * sh) + z[3] * (r0[1] * sl) +
+                      z[4] * (r1[2] * sh) + z[5] * (r0[2] * sl);
+          const R sw = rw * (CC.afact[kk] * sh + CC.bfact[kk] * sl);
+          vmh[s] = h * gh + R(1.0) * sw * rgs;
+        }
+      }
       R dv[3];
 #pragma unroll
       for (int s = 0; s < 3; ++s) {
-        R acc[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          R sm = R(0.0);
-#pragma unroll
-          for (int m = 0; m < 7; ++m) {
-            const R v = (s_rv[d][nb[m]] * s_vv[s][nb[m]]) * s_rg[nb[m]];
-            const R cf = P2(CG.coef_div, d * 7 + m, i, j, l);
-            sm = (m == 0) ? cf * v : mad(cf, v, sm);
-          }
-          acc[d] = sm;
-        }
-        const R div = acc[0] + acc[1] + acc[2];
-        R vmh_hi = R(0.0);
-        if (hv) {
-          const R sh = vv[s][qh], sl = s_vv[s][c0];
-          const R h = cz[qh] * (rv[0][qh] * sh) + cz[n + qh] * (s_rv[0][c0] * sl) +
-                           cz[2 * n + qh] * (rv[1][qh] * sh) + cz[3 * n + qh] * (s_rv[1][c0] * sl) +
-                           cz[4 * n + qh] * (rv[2][qh] * sh) + cz[5 * n + qh] * (s_rv[2][c0] * sl);
-          const R sw = a.rw[qh] * (CC.afact[kk] * sh + CC.bfact[kk] * sl);
-          vmh_hi = h * gam_at(CG.RGAMH, qh) + R(1.0) * sw * CG.RGSQRTH[qh];
-        }
-        dv[s] = -div - (vmh_hi - vmh_lo[s]) * CC.rdgz[k];
-        vmh_lo[s] = vmh_hi;
+        dv[s] = -div[s] - (vmh[s] - vmh_lo[s]) * CC.rdgz[k];
+        vmh_lo[s] = vmh[s];
       }
       const R rh = a.rg[p];
-      const R dvx = dv[0] - (-R(2.0) * rh * (CC.OHM * s_vv[1][c0]));
-      const R dvy = dv[1] - (R(2.0) * rh * (CC.OHM * s_vv[0][c0]));
+      const R dvx = dv[0] - (-R(2.0) * rh * (CC.OHM * v0[1]));
+      const R dvy = dv[1] - (R(2.0) * rh * (CC.OHM * v0[0]));
       const R dvz = dv[2];
       const R prd = dvx * gx + dvy * gy + dvz * gz;
       const R gwc = prd * CC.alpha;
@@ -269,7 +310,10 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, NC_F32_ADVMOM)) k_
         a.gw[p] = (k >= kmin + 1) ? (CG.C2W[p] * gwc + CG.C2W[n + p] * gwc_prev) : R(0.0);
       }
       gwc_prev = gwc;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) { r0[d] = r1[d]; v0[d] = v1[d]; }
     }
+    if (k < kb) put(b ^ 1);
     __syncthreads();
   }
 }
