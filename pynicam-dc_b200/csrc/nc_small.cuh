@@ -1132,19 +1132,21 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 6, NC_F32_VIMAINA)) k
   }
 }
 
-// vi_main A with VA_NK levels per block: the cell's divergence coefficients
-// (coef_div, 21 planes) are held in registers once for all of the block's
-// levels instead of re-read from L2 at every level.  Same expressions in the
-// same order as k_vimain_a_l (same results).  Used by the float instance
-// (gl08: 6.0 -> 5.5 ms per step); the double one stays on k_vimain_a_l, which
-// is faster there (9.9 against 11.6 ms: 42 more registers cost residency).
-#ifndef VA_NK
+// vi_main A with VA_NK levels per block, the float form: the cell's divergence
+// coefficients (coef_div, 21 planes) are held in registers once for the block's
+// levels, and the next level's loads are in flight while this level is worked on
+// (two levels of products in shared memory, one barrier a level).  Same
+// expressions in the same order as k_vimain_a_l.
+// Bound by the latency of a level's staging: gl08 z40 489 -> 387 us, gl06 z40
+// 41 -> 33 us, 12 x gl05 129 -> 109 us against the march that staged a level
+// between two barriers.  Ten levels a block: 400 us at gl08, 37 at gl06; five
+// blocks an SM instead of four (spills): 460 us.  The double form stays on
+// k_vimain_a_l: 224 against 221 us at gl07 z40, 25 against 23 at gl05.
 #define VA_NK 5
-#endif
 template <class R, class T>
-__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 4, 5)) k_vimain_a_m(VimainArgs<R> a) {
-  constexpr int PX = T::X + 2, PY = T::Y + 2;
-  __shared__ R s_h[3][3][PY * PX];
+__global__ void __launch_bounds__(TILE_THREADS, 4) k_vimain_a_m(const __grid_constant__ VimainArgs<R> a) {
+  constexpr int PX = T::X + 2, PY = T::Y + 2, NP = PX * PY, PT = (NP + TILE_THREADS - 1) / TILE_THREADS;
+  __shared__ R s_h[2][9][NP];   // [field * 3 + direction], two levels
   const int ntx = (cD.G - 2 + T::X - 1) / T::X;
   const int l = (int)blockIdx.z;
   const int i0 = 1 + ((int)blockIdx.y % ntx) * T::X, j0 = 1 + ((int)blockIdx.y / ntx) * T::Y;
@@ -1153,54 +1155,73 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 4, 5)) k_vimain_a_m(V
   const int tid = threadIdx.x, tx = tid % T::X, ty = tid / T::X;
   const int i = i0 + tx, j = j0 + ty;
   const bool own = (i <= gmax) && (j <= gmax);
+  R w[PT][9];   // a level's staged points of the thread on their way to shared memory
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int e = 0; e < PT; ++e) {
+      const int p = tid + e * TILE_THREADS;
+      const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
+      const bool ok = p < NP && ii < G && jj < G;
+      const int q = ok ? ix(ii, jj, k, l) : 0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        w[e][d] = ok ? __ldg(&a.dvh.f[d][q]) : R(0.0);
+        w[e][3 + d] = ok ? __ldg(&a.P[1 + d][q]) : R(0.0);
+      }
+      w[e][6] = ok ? __ldg(&a.eth[q]) : R(0.0);
+      w[e][7] = ok ? __ldg(&a.ethtot0[q]) : R(0.0);
+      w[e][8] = ok ? gam_at_ldg(CG.RGAM, q) : R(0.0);
+    }
+  };
+  auto put = [&](int b) {
+#pragma unroll
+    for (int e = 0; e < PT; ++e) {
+      const int p = tid + e * TILE_THREADS;
+      if (p < NP) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const R dv = w[e][d], rg = w[e][8];
+          s_h[b][d][p] = dv * rg;
+          s_h[b][3 + d][p] = (dv * w[e][6]) * rg;
+          s_h[b][6 + d][p] = ((w[e][3 + d] + dv) * w[e][7]) * rg;
+        }
+      }
+    }
+  };
   R cdv[21];
   if (own) {
 #pragma unroll
     for (int m = 0; m < 21; ++m) cdv[m] = P2c(CG.coef_div, m, i, j, l);
   }
-  for (int k = ka; k <= kb; ++k) {
-    for (int p = tid; p < PX * PY; p += blockDim.x) {
-      const int ii = i0 - 1 + p % PX, jj = j0 - 1 + p / PX;
-      if (ii < G && jj < G) {
-        const int q = ix(ii, jj, k, l);
-        const R rg = gam_at_ldg(CG.RGAM, q), e = __ldg(&a.eth[q]), et = __ldg(&a.ethtot0[q]);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const R dv = __ldg(&a.dvh.f[d][q]);
-          s_h[0][d][p] = dv * rg;
-          s_h[1][d][p] = (dv * e) * rg;
-          s_h[2][d][p] = ((__ldg(&a.P[1 + d][q]) + dv) * et) * rg;
-        }
-      } else {
-#pragma unroll
-        for (int f = 0; f < 3; ++f)
-#pragma unroll
-          for (int d = 0; d < 3; ++d) s_h[f][d][p] = R(0.0);
-      }
-    }
-    __syncthreads();
+  int b = 0;
+  fetch(ka);
+  put(0);
+  __syncthreads();
+  for (int k = ka; k <= kb; ++k, b ^= 1) {
+    if (k < kb) fetch(k + 1);
     if (own) {
       const int c0 = (ty + 1) * PX + (tx + 1);
       const int nb[7] = {c0, c0 + 1, c0 + PX + 1, c0 + PX, c0 - 1, c0 - PX - 1, c0 - PX};
       const int q = ix(i, j, k, l);
-      R acc[3][3];
+      R acc[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        R sv[3] = {R(0.0), R(0.0), R(0.0)};
+        R sv[3];
 #pragma unroll
         for (int m = 0; m < 7; ++m) {
 #pragma unroll
           for (int f = 0; f < 3; ++f) {
-            const R x = s_h[f][d][nb[m]];
+            const R x = s_h[b][f * 3 + d][nb[m]];
             sv[f] = (m == 0) ? cdv[d * 7 + m] * x : mad(cdv[d * 7 + m], x, sv[f]);
           }
         }
 #pragma unroll
-        for (int f = 0; f < 3; ++f) acc[f][d] = sv[f];
+        for (int f = 0; f < 3; ++f) acc[f] = (d == 0) ? sv[f] : acc[f] + sv[f];
       }
 #pragma unroll
-      for (int f = 0; f < 3; ++f) a.hdiv[f][q] = acc[f][0] + acc[f][1] + acc[f][2];
+      for (int f = 0; f < 3; ++f) a.hdiv[f][q] = acc[f];
     }
+    if (k < kb) put(b ^ 1);
     __syncthreads();
   }
 }
