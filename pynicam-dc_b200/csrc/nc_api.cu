@@ -717,9 +717,11 @@ static int trc_vadv(nc_handle* h, FieldPair* x, int nx, bool second) {
     va.den = second ? F(h->rhog_t) : F(h->P0[0]);
     va.flx_v = F(h->flx_v); va.frhog = F(h->frhog);
     va.dt = h->dtl; va.bcoef = 0.0; va.clamp = second ? 1 : 0; va.dtl = h->dtl;
-    const int tb = h->blk[TB_TRC_VADV];
-    if (!pole) k_trc_vadv<<<dim3((unsigned)((D.npt2 + tb - 1) / tb), (unsigned)nx), tb, 0, s>>>(va, 0);
-    else k_trc_vadv<<<dim3(pcb, (unsigned)nx), 32, 0, ps>>>(va, 1);
+    const int tb = std::min(h->blk[TB_TRC_VADV], TV_THREADS);
+    const unsigned cb = (unsigned)((D.npt2 + tb - 1) / tb);
+    if (pole) k_trc_vadv<R, 1><<<dim3(pcb, (unsigned)nx), 32, 0, ps>>>(va, 1, nx);
+    else if (nx == 1 || (long long)D.npt2 * nx < 256LL * h->sms) k_trc_vadv<R, 1><<<dim3(cb, (unsigned)nx), tb, 0, s>>>(va, 0, nx);
+    else k_trc_vadv<R, TV_NT><<<dim3(cb, (unsigned)((nx + TV_NT - 1) / TV_NT)), tb, 0, s>>>(va, 0, nx);
     TRY(check_launch(h, pole ? "trc_vadv_pl" : "trc_vadv"));
   }
   return 0;

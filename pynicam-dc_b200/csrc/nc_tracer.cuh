@@ -72,89 +72,125 @@ struct TrcVadvArgs {
 // limited with the bounds of cells k-1 and k, and cell k-1, whose two faces
 // are then final, is updated.  The same expressions as the three-pass form
 // of the reference (q, qh and ck on every level, the limiter, the update),
-// in the same order, so the same results.
-template <class R>
-__device__ void trc_vadv_column(const Col c, const TrcVadvArgs<R>& a, R* rhogq) {
+// in the same order, so the same results.  NT tracers of the column (the nt
+// first of rq) at once: the Courant numbers, the upwind masks and the
+// reciprocals of a level are formed once for all of them.
+template <class R, int NT>
+__device__ __forceinline__ void trc_vadv_column(const Col c, const TrcVadvArgs<R>& a, R* const* rhogq, int nt) {
   const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax;
   const R BIG = CC.HUGE_, EPS = CC.EPS;
-  auto finish = [&](int k, R x) {   // clamp and store of one updated level
+  auto finish = [&](int m, int k, R x) {   // clamp and store of one updated level
     if (a.clamp && x > -R(1.0e-10) && x < R(0.0)) x = R(0.0);
     if (a.clamp) x = x + a.dtl * R(0.0);
-    rhogq[c.at(k)] = x;
+    if (m < nt) rhogq[m][c.at(k)] = x;
   };
+  R* rp[NT];
+#pragma unroll
+  for (int m = 0; m < NT; ++m) rp[m] = rhogq[min(m, nt - 1)];   // a surplus tracer repeats the last and stores nothing
   // q at kmin-1 and kmin, den and flx_v at kmin (read before the ghost levels are zeroed)
   const int p = c.at(kmin);
-  R rq_m = rhogq[c.at(kmin - 1)], rq_k = rhogq[p];
   using Div = typename DivOf<R>::type;
   Div by_k(__ldg(&a.den[p]));       // the divisions by a level's density share its reciprocal
-  R q_m = rq_m / __ldg(&a.den[c.at(kmin - 1)]), q_k = by_k(rq_k);
+  const R den_m = __ldg(&a.den[c.at(kmin - 1)]);
+  R rq_k[NT], q_m[NT], q_k[NT], rq_n[NT], qmin_prev[NT], qmax_prev[NT], qh_prev[NT], rq_prev[NT];
+#pragma unroll
+  for (int m = 0; m < NT; ++m) {
+    q_m[m] = rp[m][c.at(kmin - 1)] / den_m;
+    rq_k[m] = rp[m][p];
+    rq_n[m] = rp[m][c.at(kmin + 1)];
+  }
+#pragma unroll
+  for (int m = 0; m < NT; ++m) {
+    q_k[m] = by_k(rq_k[m]);
+    qmin_prev[m] = qmax_prev[m] = qh_prev[m] = rq_prev[m] = R(0.0);
+  }
   R flx_k = __ldg(&a.flx_v[p]);
   R ck0 = by_k(-flx_k) * CC.rdgz[kmin];
-  R qmin_prev = R(0.0), qmax_prev = R(0.0), qh_prev = R(0.0), rq_prev = R(0.0), flx_prev = R(0.0);
+  R flx_prev = R(0.0);
   // the loads of level k+2 are issued before level k is worked on
-  R rq_n = rhogq[c.at(kmin + 1)], den_n = __ldg(&a.den[c.at(kmin + 1)]), flx_n = __ldg(&a.flx_v[c.at(kmin + 1)]);
+  R den_n = __ldg(&a.den[c.at(kmin + 1)]), flx_n = __ldg(&a.flx_v[c.at(kmin + 1)]);
   R fr_n = __ldg(&a.frhog[p]);
   for (int k = kmin; k <= kmax; ++k) {
-    const R rq_p = rq_n, den_p = den_n, flx_p = flx_n, fr_k = fr_n;
+    const R den_p = den_n, flx_p = flx_n, fr_k = fr_n;
+    R rq_p[NT];
+#pragma unroll
+    for (int m = 0; m < NT; ++m) rq_p[m] = rq_n[m];
     if (k < kmax) {
       const int p2 = c.at(k + 2);
-      rq_n = rhogq[p2];
+#pragma unroll
+      for (int m = 0; m < NT; ++m) rq_n[m] = rp[m][p2];
       den_n = __ldg(&a.den[p2]);
       flx_n = __ldg(&a.flx_v[p2]);
       fr_n = __ldg(&a.frhog[c.at(k + 1)]);
     }
     const Div by_p(den_p);
-    const R q_p = by_p(rq_p);
     const R ck1 = by_k(flx_p) * CC.rdgz[k];
     const R ck0_p = (k + 1 <= kmax) ? by_p(-flx_p) * CC.rdgz[k + 1] : R(0.0);
-    const R qh_raw = CC.afact[k] * q_k + CC.bfact[k] * q_m;
     const R inL = R(0.5) - copysign(R(0.5), ck0);
     const R inU = R(0.5) + copysign(R(0.5), ck0_p);
-    const R qc = q_k, qb = q_m, qa = q_p;
-    const R QminL = (inL == R(1.0)) ? npmin(qc, qb) : BIG;
-    const R QminU = (inU == R(1.0)) ? npmin(qc, qa) : BIG;
-    const R QmaxL = (inL == R(1.0)) ? npmax(qc, qb) : -BIG;
-    const R QmaxU = (inU == R(1.0)) ? npmax(qc, qa) : -BIG;
-    const R qnmin = npmin(npmin(QminL, QminU), qc);
-    const R qnmax = npmax(npmax(QmaxL, QmaxU), qc);
     const R c1 = ck0, c2 = ck1;
     const R Cin = inL * c1 + inU * c2;
     const R Cout = (R(1.0) - inL) * c1 + (R(1.0) - inU) * c2;
-    const R CQmin = inL * c1 * QminL + inU * c2 * QminU;
-    const R CQmax = inL * c1 * QmaxL + inU * c2 * QmaxU;
     const R zsw = R(0.5) - copysign(R(0.5), fabs(Cout) - EPS);
     const R dk = by_k(a.bcoef * fr_k) * a.dt;
     const Div by_o(Cout + zsw);
-    const R qomin = by_o((qc - qnmax) + qnmax * (Cin + Cout - dk) - CQmax) * (R(1.0) - zsw) + qc * zsw;
-    const R qomax = by_o((qc - qnmin) + qnmin * (Cin + Cout - dk) - CQmin) * (R(1.0) - zsw) + qc * zsw;
-    R qh = R(0.0);   // the face at kmin stays zero
-    if (k > kmin)
-      qh = inL * npmin(npmax(qh_raw, qmin_prev), qmax_prev) + (R(1.0) - inL) * npmin(npmax(qh_raw, qomin), qomax);
-    if (k > kmin) finish(k - 1, rq_prev - (flx_k * qh - flx_prev * qh_prev) * CC.rdgz[k - 1]);
-    qmin_prev = qomin;
-    qmax_prev = qomax;
-    qh_prev = qh;
-    rq_prev = rq_k;
+#pragma unroll
+    for (int m = 0; m < NT; ++m) {
+      const R q_p = by_p(rq_p[m]);
+      const R qh_raw = CC.afact[k] * q_k[m] + CC.bfact[k] * q_m[m];
+      const R qc = q_k[m], qb = q_m[m], qa = q_p;
+      const R QminL = (inL == R(1.0)) ? npmin(qc, qb) : BIG;
+      const R QminU = (inU == R(1.0)) ? npmin(qc, qa) : BIG;
+      const R QmaxL = (inL == R(1.0)) ? npmax(qc, qb) : -BIG;
+      const R QmaxU = (inU == R(1.0)) ? npmax(qc, qa) : -BIG;
+      const R qnmin = npmin(npmin(QminL, QminU), qc);
+      const R qnmax = npmax(npmax(QmaxL, QmaxU), qc);
+      const R CQmin = inL * c1 * QminL + inU * c2 * QminU;
+      const R CQmax = inL * c1 * QmaxL + inU * c2 * QmaxU;
+      const R qomin = by_o((qc - qnmax) + qnmax * (Cin + Cout - dk) - CQmax) * (R(1.0) - zsw) + qc * zsw;
+      const R qomax = by_o((qc - qnmin) + qnmin * (Cin + Cout - dk) - CQmin) * (R(1.0) - zsw) + qc * zsw;
+      R qh = R(0.0);   // the face at kmin stays zero
+      if (k > kmin) {
+        qh = inL * npmin(npmax(qh_raw, qmin_prev[m]), qmax_prev[m]) + (R(1.0) - inL) * npmin(npmax(qh_raw, qomin), qomax);
+        finish(m, k - 1, rq_prev[m] - (flx_k * qh - flx_prev * qh_prev[m]) * CC.rdgz[k - 1]);
+      }
+      qmin_prev[m] = qomin;
+      qmax_prev[m] = qomax;
+      qh_prev[m] = qh;
+      rq_prev[m] = rq_k[m];
+      q_m[m] = q_k[m]; q_k[m] = q_p; rq_k[m] = rq_p[m];
+    }
     flx_prev = flx_k;
-    q_m = q_k; q_k = q_p; rq_k = rq_p;
     by_k = by_p; flx_k = flx_p;
     ck0 = ck0_p;
   }
   // cell kmax: its upper face (kmax+1) is zero
-  finish(kmax, rq_prev - (flx_k * R(0.0) - flx_prev * qh_prev) * CC.rdgz[kmax]);
-  for (int k = 0; k < kmin; ++k) finish(k, R(0.0));
-  for (int k = kmax + 1; k < KA; ++k) finish(k, R(0.0));
+#pragma unroll
+  for (int m = 0; m < NT; ++m) {
+    finish(m, kmax, rq_prev[m] - (flx_k * R(0.0) - flx_prev * qh_prev[m]) * CC.rdgz[kmax]);
+    for (int k = 0; k < kmin; ++k) finish(m, k, R(0.0));
+    for (int k = kmax + 1; k < KA; ++k) finish(m, k, R(0.0));
+  }
 }
 
 // Every tracer of the step in one launch: the sweep is a serial chain per
 // column, so one tracer's columns alone leave the SMs waiting (263 us a tracer
-// at gl07 z60 float64)
-template <class R>
-__global__ void k_trc_vadv(const __grid_constant__ TrcVadvArgs<R> a, int pole) {
+// at gl07 z60 float64).  A thread takes NT tracers of its column: bound by
+// memory (density, fluxes and tendency re-read for each tracer) and by the
+// divisions.  17 tracers at gl07 z60 float64: one a thread 1.87 ms, two 1.54,
+// three 1.47, four 1.64 (166 registers); 6 at gl06 z40 132, 113, 110, 134 us; 6 at
+// gl05 z40 53, 51, 52, 62 us; 6 at gl04 z40 30, 32, 42, 49 us.  Two, where the
+// columns of all tracers are at least 256 for each SM; fewer are bound by the
+// chain and take a tracer a thread.
+#define TV_THREADS 256
+#define TV_NT 2
+template <class R, int NT>
+__global__ void __launch_bounds__(TV_THREADS) k_trc_vadv(const __grid_constant__ TrcVadvArgs<R> a, int pole, int nx) {
   int t = (int)blockIdx.x * blockDim.x + threadIdx.x;
   int i, j, l, g, lp;
   if (!map_col(pole, t, i, j, l, g, lp)) return;
-  trc_vadv_column(pole ? col_pl(g, lp) : col_reg(i, j, l), a, a.rhogq_of[blockIdx.y]);
+  const int first = (int)blockIdx.y * NT;
+  trc_vadv_column<R, NT>(pole ? col_pl(g, lp) : col_reg(i, j, l), a, a.rhogq_of + first, min(NT, nx - first));
 }
 
 // ---------------------------------------------------------------------------

@@ -7,8 +7,9 @@ remainders of its splits (B200).
 * One gl05 grid alone (its tiles and columns do not fill the SMs: level chunks)
   against 17 of them stacked in one handle (whole marches): each member bit for
   bit, in both forms.
-* Tracers in batches: every tracer of 6 (batches of 4 and 2) equals the same
-  tracer carried alone, bit for bit.
+* Tracers in batches: every tracer of 6 (batches of 4 and 2, a thread of the
+  vertical sweep for each) and of 7 (batches of 4 and 3, two tracers a thread,
+  the last alone) equals the same tracer carried alone, bit for bit.
 * The linear operators on an input that overlaps the output.
 """
 import importlib
@@ -69,9 +70,10 @@ def test_one_grid_equals_its_stack(pkg, prec):
         assert np.array_equal(x, lone) and np.array_equal(xp, lone_pl)
 
 
+@pytest.mark.parametrize("glevel, lone", [(4, 5), (5, 6)])
 @pytest.mark.parametrize("prec", ["float64", "mixed"])
-def test_tracer_batches_equal_lone_tracers(pkg, prec):
-    g = _ig().Grid(4, vlayer=11, ztop=12000.0, device="cuda", layer="EVEN", topo="NONE")
+def test_tracer_batches_equal_lone_tracers(pkg, prec, glevel, lone):
+    g = _ig().Grid(glevel, vlayer=11, ztop=12000.0, device="cuda", layer="EVEN", topo="NONE")
     rng = np.random.default_rng(8)
     amp, lon0 = rng.uniform(0.2, 1.0, 6), rng.uniform(0.0, 6.0, 6)
 
@@ -86,7 +88,7 @@ def test_tracer_batches_equal_lone_tracers(pkg, prec):
         return f
 
     def run(which):
-        geo = g.setup(dtl=600.0, gamma=9.6e16, nq=1 + len(which), trcadv=True)
+        geo = g.setup(dtl=600.0, gamma={4: 9.6e16, 5: 1.2e16}[glevel], nq=1 + len(which), trcadv=True)
         s, sp = g.trcadv_state(fields(which))
         c = pkg.NicamCuda(geo, graph=True, precision=prec)
         try:
@@ -95,8 +97,8 @@ def test_tracer_batches_equal_lone_tracers(pkg, prec):
             return c.download()
         finally:
             c.close()
-    s, sp = run(range(5))          # 6 with the vapour slot
-    for n in range(5):
+    s, sp = run(range(lone))       # with the vapour slot one more
+    for n in range(lone):
         a, ap = run([n])
         assert np.array_equal(s[..., 7 + n], a[..., 7]) and np.array_equal(sp[..., 7 + n], ap[..., 7]), n
 
