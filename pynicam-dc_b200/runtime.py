@@ -353,6 +353,25 @@ def setup_table(geo: dict) -> dict:
 
 PRECISIONS = ("float64", "mixed")
 
+_FLOAT64 = None
+
+
+def _f64():
+    """torch.float64 (torch is imported by the first tensor call)"""
+    global _FLOAT64
+    if _FLOAT64 is None:
+        import torch
+        _FLOAT64 = torch.float64
+    return _FLOAT64
+
+
+def _stream(t) -> int:
+    """cudaStream_t of torch's current stream on the tensor's device"""
+    import torch
+    if not t.is_cuda:
+        raise ValueError(f"expected a CUDA tensor, got one on {t.device}")
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
 
 class NicamCuda:
     """One device-resident NICAM-DC dynamical core (one C-ABI handle).
@@ -394,6 +413,7 @@ class NicamCuda:
         LP = 2 * (int(_scalar(self._tab["members"])) if "members" in self._tab else 1)
         self.shape_pl = (6, K, LP, 6 + nq)
         self.kmin, self.kmax = int(_scalar(self._tab["kmin"])), int(_scalar(self._tab["kmax"]))
+        self._fshape, self._fshape_pl = (L, K, G, G), (6, K, LP)
 
     # ---- state marshal (host arrays in the reference layout)
     def upload(self, prg: np.ndarray, prg_pl: np.ndarray):
@@ -453,21 +473,21 @@ class NicamCuda:
     # [g][k][lp] = shape (6, kall, 2); float64 handles only)
     @property
     def field_shape(self):
-        G, K, L = self.shape[0], self.shape[2], self.shape[3]
-        return (L, K, G, G)
+        return self._fshape
 
     @property
     def field_shape_pl(self):
-        return (6, self.shape[2], self.shape_pl[2])
+        return self._fshape_pl
 
     def _dev(self, t, pole: bool = False, comps: int = 0):
-        import torch
-        shp = self.field_shape_pl if pole else self.field_shape
-        if comps:
-            shp = (comps,) + shp
+        # called for every tensor of an operator that takes tens of microseconds: compares
+        # shapes and types without building any
         if t is None:
             return None
-        if not t.is_cuda or t.dtype != torch.float64 or tuple(t.shape) != shp or not t.is_contiguous():
+        shp = self._fshape_pl if pole else self._fshape
+        if comps:
+            shp = (comps,) + shp
+        if t.shape != shp or not t.is_cuda or t.dtype is not _f64() or not t.is_contiguous():
             raise ValueError(f"expected a contiguous float64 CUDA tensor of shape {shp}, got "
                              f"{t.dtype} {tuple(t.shape)} on {t.device}")
         return t.data_ptr()
@@ -475,8 +495,7 @@ class NicamCuda:
     def vsolve(self, Mc, Mu, Ml, b, x, pole: bool = False, transpose: bool = False, x_fwd=None, gM=None):
         """nc_vsolve: x = M^-1 b (M^-T b with transpose); with x_fwd and
         gM = (gMc, gMu, gMl) also the matrix cotangents"""
-        import torch
-        st = torch.cuda.current_stream(b.device).cuda_stream
+        st = _stream(b)
         g = gM if gM is not None else (None, None, None)
         _check(self._lib.nc_vsolve(self._h, int(pole), int(transpose), *(self._dev(t, pole) for t in (Mc, Mu, Ml, b, x)),
                                    self._dev(x_fwd, pole), *(self._dev(t, pole) for t in g), st))
@@ -484,16 +503,14 @@ class NicamCuda:
     def vadv_lin(self, mode: int, rhogq, den, flx_v, frhog, inp, out, dt: float, bcoef: float = 0.0,
                  clamp: bool = True, pole: bool = False):
         """nc_vadv_lin: mode 0 F(rhogq), 1 dF(inp), 2 dF^T(inp) into out"""
-        import torch
-        st = torch.cuda.current_stream(out.device).cuda_stream
+        st = _stream(out)
         _check(self._lib.nc_vadv_lin(self._h, int(pole), int(mode), *(self._dev(t, pole) for t in
                                                                       (rhogq, den, flx_v, frhog, inp, out)),
                                      float(dt), float(bcoef), int(bool(clamp)), st))
 
     def laplacian(self, q, q_pl, y, y_pl, transpose: bool = False):
         """nc_laplacian: y = L(C(q)), or C^T L^T q with transpose"""
-        import torch
-        st = torch.cuda.current_stream(q.device).cuda_stream
+        st = _stream(q)
         _check(self._lib.nc_laplacian(self._h, int(transpose), self._dev(q), self._dev(q_pl, True), self._dev(y),
                                       self._dev(y_pl, True), st))
 
@@ -509,56 +526,49 @@ class NicamCuda:
     def divergence(self, v, v_pl, y, y_pl, transpose: bool = False):
         """nc_divergence: y = D(C(v)) (v of shape (3,) + field shape), or
         v = C^T D^T y with transpose"""
-        import torch
-        st = torch.cuda.current_stream(y.device).cuda_stream
+        st = _stream(y)
         _check(self._lib.nc_divergence(self._h, int(transpose), self._dev(v, comps=3), self._dev(v_pl, True, 3),
                                        self._dev(y), self._dev(y_pl, True), st))
 
     def gradient(self, q, q_pl, g, g_pl, transpose: bool = False):
         """nc_gradient: g = Grad(C(q)) (g of shape (3,) + field shape), or
         q = C^T Grad^T g with transpose"""
-        import torch
-        st = torch.cuda.current_stream(q.device).cuda_stream
+        st = _stream(q)
         _check(self._lib.nc_gradient(self._h, int(transpose), self._dev(q), self._dev(q_pl, True),
                                      self._dev(g, comps=3), self._dev(g_pl, True, 3), st))
 
     def diffusion(self, kh, kh_pl, s, s_pl, y, y_pl, transpose: bool = False):
         """nc_diffusion: y = Dk(C(s)), the kh-weighted diffusion after the halo
         exchange, or s = C^T Dk^T y with transpose (kh fixed)"""
-        import torch
-        st = torch.cuda.current_stream(s.device).cuda_stream
+        st = _stream(s)
         _check(self._lib.nc_diffusion(self._h, int(transpose), self._dev(kh), self._dev(kh_pl, True), self._dev(s),
                                       self._dev(s_pl, True), self._dev(y), self._dev(y_pl, True), st))
 
     def diffusion_kh(self, s, s_pl, y, y_pl, gkh, gkh_pl):
         """nc_diffusion_kh: gkh = d<y, Dk(C(s))>/dkh"""
-        import torch
-        st = torch.cuda.current_stream(s.device).cuda_stream
+        st = _stream(s)
         _check(self._lib.nc_diffusion_kh(self._h, self._dev(s), self._dev(s_pl, True), self._dev(y),
                                          self._dev(y_pl, True), self._dev(gkh), self._dev(gkh_pl, True), st))
 
     def exchange(self, x, x_pl, transpose: bool = False):
         """nc_exchange: the halo exchange of x (nf,) + field shape (or one
         field) in place, or its adjoint with transpose"""
-        import torch
         nf = x.shape[0] if x.dim() == len(self.field_shape) + 1 else 0
-        st = torch.cuda.current_stream(x.device).cuda_stream
+        st = _stream(x)
         _check(self._lib.nc_exchange(self._h, int(transpose), self._dev(x, comps=nf), self._dev(x_pl, True, nf),
                                      max(nf, 1), st))
 
     def divdamp3d(self, v, v_pl, y, y_pl, transpose: bool = False):
         """nc_divdamp3d: y = D3(C(v)) (v of shape (4,) + field shape: the four
         momenta; y (3,) + field shape), or v = C^T D3^T y with transpose"""
-        import torch
-        st = torch.cuda.current_stream(y.device).cuda_stream
+        st = _stream(y)
         _check(self._lib.nc_divdamp3d(self._h, int(transpose), self._dev(v, comps=4), self._dev(v_pl, True, 4),
                                       self._dev(y, comps=3), self._dev(y_pl, True, 3), st))
 
     def divdamp2d(self, v, v_pl, y, y_pl, transpose: bool = False):
         """nc_divdamp2d: y = D2(C(v)) (v and y of shape (3,) + field shape), or
         v = C^T D2^T y with transpose"""
-        import torch
-        st = torch.cuda.current_stream(y.device).cuda_stream
+        st = _stream(y)
         _check(self._lib.nc_divdamp2d(self._h, int(transpose), self._dev(v, comps=3), self._dev(v_pl, True, 3),
                                       self._dev(y, comps=3), self._dev(y_pl, True, 3), st))
 
@@ -572,8 +582,7 @@ class NicamCuda:
         """nc_trc_step_lin: the tracer advection of the handle's last step
         applied to the tracer mass x0 (mode 0), its tangent-linear (1) or
         adjoint (2) applied to inp, into out"""
-        import torch
-        st = torch.cuda.current_stream(out.device).cuda_stream
+        st = _stream(out)
         _check(self._lib.nc_trc_step_lin(self._h, int(mode), self._dev(x0), self._dev(x0_pl, True), self._dev(inp),
                                          self._dev(inp_pl, True), self._dev(out), self._dev(out_pl, True), st))
 
