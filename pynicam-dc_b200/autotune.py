@@ -11,9 +11,11 @@ the device name, the state shape, the precision and the ensemble members, so
 a later handle of the same case applies it without measuring.
 
 The tiled stencil kernels keep their compile-time tile shapes (32 x 8 cells of
-one region, chosen by measurement on B200) and their resident-block targets
-(``NC_F32_*`` / launch bounds in csrc/nc_common.cuh): those are template
-constants of the kernels, not launch parameters.
+one region, 16 x 16 for regions of at most 16 cells a side, chosen by
+measurement on B200) and their resident-block targets (``NC_F32_*`` / launch
+bounds): those are template constants of the kernels, not launch parameters.
+``vi_solve`` and ``vi_energy`` are accepted, but have no effect any more: their
+column kernel has a fixed block.
 
 Tuning advances the handle's state by the profiled steps: upload the state
 again afterwards (the ensemble driver does).

@@ -65,7 +65,7 @@ KERNELS = {
     # PROG_split / PROG_mean initialisation (k_split_init); the first stage reads no PROG0
     "split_init": (_f(*_n("PROG0.", 6), *PROG), _f(*_n("PS.", 6), *_n("PM.", 5)), ()),
     "split_init_first": (_f(*PROG), _f(*_n("PS.", 6), *_n("PM.", 5)), ()),
-    # 3-D divergence damping (k_dd3d_t): momenta of PROG or PROG_split
+    # 3-D divergence damping (k_dd3d_m): momenta of PROG or PROG_split
     "dd3d": (_f("RHOGVX", "RHOGVY", "RHOGVZ", "RHOGW") + C2WGZ + _m("RGSQRTH"), _f(*_n("vtmp2.", 3)),
              _n("coef_intp.", 18) + _n("coef_diff.", 18)),
     # vp0 horizontal terms (k_vp0_hl) and column part with the implicit matrix (k_vp0_cr)
@@ -77,7 +77,7 @@ KERNELS = {
     "vp0_c": (_f(*PROG[:5], "eth", *_n("vph.", 8), "vx", "vy", "vz", *_n("gT0.", 6)) + _f64("pregd", "rhogd") +
               _m("RGSQRTH", "C2W.0", "C2W.1", "W2C.0", "W2C.1", "RGSGAM2", "PHI") + C2WGZ,
               _f(*_n("gT.", 6), "ethtot0") + _f64("Mc", "Mu", "Ml"), ()),
-    # acoustic loop: path 1 (k_path1_l), vi_main horizontal divergences (k_vimain_a_l),
+    # acoustic loop: path 1 (k_path1_l), vi_main horizontal divergences (k_vimain_a_m / k_vimain_a_l),
     # Thomas solve and energy update (k_vi_col)
     "path1": (_f(*_n("vtmp2.", 3), "PS.5", "PS.1", "PS.2", "PS.3", "gT.1", "gT.2", "gT.3", "PM.1", "PM.2", "PM.3") +
               _m("RGAM", "RGAMH") + C2WGZ,
