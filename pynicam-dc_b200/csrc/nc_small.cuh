@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 4, NC_F32_VP0H)) k_vp
 // mass and energy fluxes, buoyancy, vertical pressure gradient, gz, pwh,
 // half-level eth, the vertical kinetic-energy term) are formed and the ones at
 // k and k-1 are carried in registers.  Each value is the expression of
-// vp0_column (the pole form), so regional and pole columns round alike.
+// k_vp0_pl (the pole form), so regional and pole columns round alike.
 // 256-thread blocks capped at 64 registers (four per SM; measured faster
 // than three at 74 registers).  blockIdx.y takes a chunk of nk levels: a whole
 // column per thread walked 42 levels at 9 us each, however few the columns;
@@ -1278,6 +1278,11 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
   const MetT<R> m = met_of<R>(POLE);
   const double dt = a.dt, Rdry = cC.Rdry, CVdry = cC.CVdry, RovCV = a.RovCV;
   const R* const* DV = a.dvh.f;
+  // the pole columns form fluxes, rhog_split1 and the running means in R, the
+  // regional ones in double
+  using F = typename std::conditional<POLE, R, double>::type;
+  const F rweight = F(a.rweight);
+  auto rdgz = [](int k) -> F { return POLE ? F(CC.rdgz[k]) : F(cC.rdgz[k]); };
   double* s0 = sm + lane;
   double* s1 = s0 + KA * VC_COLS;
   double* s2 = s1 + KA * VC_COLS;
@@ -1301,19 +1306,19 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
       z0 = cz(0, q); z1 = cz(1, q); z2 = cz(2, q); z3 = cz(3, q); z4 = cz(4, q); z5 = cz(5, q);
       gh = GU ? R(1.0) : __ldg(m.RGAMH + q);
     };
-    auto flux = [&](double& hd, double& he) {   // half-level fluxes at the loaded level
-      const double a0 = f0, a1 = f1, a2 = f2, e = fe, b0 = m0, b1 = m1, b2 = m2, em = me;
-      hd = (z0 * a0 + z1 * b0 + z2 * a1 + z3 * b1 + z4 * a2 + z5 * b2) * (double)gh;
-      he = (z0 * (a0 * e) + z1 * (b0 * em) + z2 * (a1 * e) + z3 * (b1 * em) + z4 * (a2 * e) + z5 * (b2 * em)) * (double)gh;
+    auto flux = [&](F& hd, F& he) {   // half-level fluxes at the loaded level
+      const F a0 = f0, a1 = f1, a2 = f2, e = fe, b0 = m0, b1 = m1, b2 = m2, em = me;
+      hd = (z0 * a0 + z1 * b0 + z2 * a1 + z3 * b1 + z4 * a2 + z5 * b2) * (F)gh;
+      he = (z0 * (a0 * e) + z1 * (b0 * em) + z2 * (a1 * e) + z3 * (b1 * em) + z4 * (a2 * e) + z5 * (b2 * em)) * (F)gh;
     };
     {
       const int q = c.at(lo - 2);
       m0 = __ldg(DV[0] + q); m1 = __ldg(DV[1] + q); m2 = __ldg(DV[2] + q); me = __ldg(a.eth + q);
     }
     load(lo - 1);
-    double hD, hE;
+    F hD, hE;
     flux(hD, hE);
-    if (lo - 1 == kmin) hD = hE = 0.0;    // zero at kmin and at kmax+1
+    if (lo - 1 == kmin) hD = hE = F(0.0);    // zero at kmin and at kmax+1
     m0 = f0; m1 = f1; m2 = f2; me = fe;
     double T1m = 0.0, T2m = 0.0;
     for (int k = lo - 1; k < hi; ++k) {
@@ -1324,11 +1329,11 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
       const R g4 = __ldg(a.gT[4] + p), ps4 = __ldg(a.PS[4] + p);
       const double mu = __ldg(a.Mu + p), ml = __ldg(a.Ml + p), mcc = __ldg(a.Mc + p);
       const double rgm = GU ? 1.0 : (double)__ldg(m.RGAM + p), rgh = GU ? 1.0 : (double)__ldg(m.RGAMH + p);
-      double hDn, hEn;
+      F hDn, hEn;
       flux(hDn, hEn);
-      if (k == kmax) hDn = hEn = 0.0;
-      const double drhog = -hd0 - (hDn - hD) * cC.rdgz[k];
-      const double drhoge = -hd1 - (hEn - hE) * cC.rdgz[k];
+      if (k == kmax) hDn = hEn = F(0.0);
+      const double drhog = -hd0 - (hDn - hD) * rdgz(k);
+      const double drhoge = -hd1 - (hEn - hE) * rdgz(k);
       const double g1 = g0 + drhog;
       const double gp = (g5 + drhoge) * Rdry / CVdry;
       const double T1 = (ps5 * RovCV + dt * gp) * rs2;
@@ -1344,7 +1349,8 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
           S(s1, kmin) = rw_kmin;
         }
         if (k == kmax) {   // the loaded level is kmax+1
-          const double top = -(z0 * f0 + z1 * m0 + z2 * f1 + z3 * m1 + z4 * f2 + z5 * m2);
+          using W = typename std::conditional<POLE, double, R>::type;   // as the fluxes, the other way round
+          const double top = -(W(z0) * f0 + W(z1) * m0 + W(z2) * f1 + W(z3) * m1 + W(z4) * f2 + W(z5) * m2);
           const double rw_top = top * __ldg(m.RGSGAM2H + c.at(kT));
           b = b - mu * rw_top;
           S(s1, kT) = rw_top;
@@ -1400,7 +1406,7 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
   // values of level kk-1 (d...) and its half-level terms (h...)
   R drg = R(0.0), dr0 = R(0.0), dr1 = R(0.0), dvx = R(0.0), dvy = R(0.0), dvz = R(0.0), dx = R(0.0), dy = R(0.0),
     dz = R(0.0), det = R(0.0), h10 = R(0.0), h11 = R(0.0), hfl = R(0.0);
-  double drs = 0.0, drw = 0.0;
+  F drs = F(0.0), drw = F(0.0);
   for (int kk = kk0; kk <= hi; ++kk) {
     const int ke = min(kk, KA - 1), kn = min(kk + 1, KA - 1), ko = max(kk - 1, 0);
     const int p = c.at(ke), pn = c.at(kn), po = c.at(ko);
@@ -1415,13 +1421,13 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
             re0 = __ldg(a.PS[5] + c.at(min(max(ko, kmin), kmax))), pm0 = a.PM0[po], pm4 = a.PM4[po];
     const R ghh = GU && !POLE ? R(1.0) : gam_at(m.RGAMH, p);
     // rhogw_split1 and its mass flux at the half levels kk and kk+1
-    auto rws_at = [&](int k, R g) -> double { return (k >= kmin && k <= kT) ? S(s1, k) * g : 0.0; };
-    auto v2_at = [&](int k, double r, R q) -> double { return (k > kmin && k <= kmax) ? S(s0, k) + 1.0 * r * q : 0.0; };
-    const double rws = rws_at(ke, gs), rwn = rws_at(kn, gsn);
-    const double v2 = v2_at(ke, rws, rq), v2n = v2_at(kn, rwn, rqn);
+    auto rws_at = [&](int k, R g) -> F { return (k >= kmin && k <= kT) ? F(S(s1, k) * g) : F(0.0); };
+    auto v2_at = [&](int k, F r, R q) -> F { return (k > kmin && k <= kmax) ? F(S(s0, k)) + F(1.0) * r * q : F(0.0); };
+    const F rws = rws_at(ke, gs), rwn = rws_at(kn, gsn);
+    const F v2 = v2_at(ke, rws, rq), v2n = v2_at(kn, rwn, rqn);
     const bool in = kk >= kmin && kk <= kmax;
-    const double drhog2 = in ? -hd0 - (v2n - v2) * cC.rdgz[ke] : 0.0;
-    const double rs = r0 + (g0 + drhog2) * dt;
+    const F drhog2 = in ? -hd0 - (v2n - v2) * rdgz(ke) : F(0.0);
+    const F rs = r0 + (g0 + drhog2) * F(dt);
     const R r1 = R(rs);
     const R x1 = vx + u0, y1 = vy + u1, z1v = vz + u2;
     // between the levels kk and kk-1
@@ -1446,8 +1452,8 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
         a.dwe[0][po] = dr1;
         a.dwe[1][po] = R(drw);
         a.dwe[2][po] = re;
-        a.PM0[po] = pm0 + drs * a.rweight;
-        a.PM4[po] = pm4 + drw * a.rweight;
+        a.PM0[po] = pm0 + drs * rweight;
+        a.PM4[po] = pm4 + drw * rweight;
       }
     }
     drg = rg; dr0 = r0; dr1 = r1; dvx = vx; dvy = vy; dvz = vz; dx = x1; dy = y1; dz = z1v; det = et;
