@@ -25,7 +25,7 @@ struct DiagArgs {
   R *vvx, *vvy, *vvz;
 };
 
-template <class R>
+template <class R, bool POLE>
 __device__ void diag_point(const Col c, const MetT<R> m, const DiagArgs<R>& a, int k, double gx, double gy, double gz) {
   const int kmin = cD.kmin, kmax = cD.kmax;
   if (k == kmin - 1 || k == kmax + 1) return;   // written with the row next to them
@@ -83,7 +83,9 @@ __device__ void diag_point(const Col c, const MetT<R> m, const DiagArgs<R>& a, i
   }
   if (k > kmin && k < kmax) {
     const double wk = w_at(k), wk1 = w_at(k + 1);
-    finish(k, p, d.pre, d.rho, d.ein, d.vx, d.vy, d.vz, wk, wk1);
+    // the pole points form the second pass from the stored (rounded) values
+    auto Q = [](double x) -> double { return POLE ? (double)R(x) : x; };
+    finish(k, p, Q(d.pre), Q(d.rho), Q(d.ein), Q(d.vx), Q(d.vy), Q(d.vz), Q(wk), Q(wk1));
     a.vx[p] = d.vx; a.vy[p] = d.vy; a.vz[p] = d.vz;
     put(p, d.tem, d.pre, d.rho, d.ein);
     a.w[p] = wk;
@@ -148,10 +150,10 @@ __global__ void __launch_bounds__(128, NC_MINB(R, 8, NC_F32_DIAG)) k_diag(const 
   if ((int)blockIdx.x < npb) {
     if (!pole_point((int)(blockIdx.x * blockDim.x + threadIdx.x), q)) return;
     const R* X = CG.GRD_x_pl + (q.g * cD.LP + q.lp) * 3;
-    diag_point(col_pl(q.g, q.lp), met_of<R>(true), ap, q.k, (double)X[0], (double)X[1], (double)X[2]);
+    diag_point<R, true>(col_pl(q.g, q.lp), met_of<R>(true), ap, q.k, (double)X[0], (double)X[1], (double)X[2]);
   } else {
     if (!reg_point((int)((blockIdx.x - npb) * blockDim.x + threadIdx.x), q)) return;
-    diag_point(col_reg(q.i, q.j, q.l), met_of<R>(false), a, q.k, (double)P2(CG.GRD_x, 0, q.i, q.j, q.l),
+    diag_point<R, false>(col_reg(q.i, q.j, q.l), met_of<R>(false), a, q.k, (double)P2(CG.GRD_x, 0, q.i, q.j, q.l),
                (double)P2(CG.GRD_x, 1, q.i, q.j, q.l), (double)P2(CG.GRD_x, 2, q.i, q.j, q.l));
   }
 }
