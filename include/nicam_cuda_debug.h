@@ -31,10 +31,11 @@ int nc_get_field(nc_handle* h, const char* name, double* host_reg, double* host_
  * fused multiply-adds and a multiply.  With y NULL every x[i] is divided by the
  * constant b (reciprocal pair set on the host, as for rscale and 3); otherwise
  * x[i] is divided by y[i] with the pair formed on the device from the
- * correctly rounded reciprocal (as for the density that the diagnostics and
- * the tracer Courant numbers divide by).  Copies the n host doubles in, writes q, copies it
- * back (synchronous).  For finite operands with a normal-range quotient the
- * bits equal the IEEE quotient; the tests compare them.  0 <= n <= 2^28; with
+ * correctly rounded reciprocal, where that is exact, and by the division itself
+ * elsewhere (as the tracer kernels divide).  Copies the n host doubles in, writes q, copies it
+ * back (synchronous).  With y the bits equal the IEEE quotient for every pair
+ * of operands (a NaN for a NaN); with y NULL for finite operands with a
+ * normal-range quotient.  The tests compare them.  0 <= n <= 2^28; with
  * y NULL, b finite and nonzero; else NC_ERR_ARG. */
 int nc_divide_known(const double* x, const double* y, double* q, int64_t n, double b);
 

@@ -34,7 +34,7 @@ static void recip_pair(double b, double& h, double& l) {
 __global__ void k_divide_known(const double* x, const double* y, double* q, int n, double b, double bh, double bl) {
   const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= n) return;
-  q[t] = y ? nc::div_by(x[t], nc::recip_of(y[t])) : nc::div_by(x[t], b, bh, bl);
+  q[t] = y ? nc::DivD(y[t])(x[t]) : nc::div_by(x[t], b, bh, bl);
 }
 
 static int fail(int code, const std::string& msg) {

@@ -227,18 +227,58 @@ struct RecipF {
 __device__ __forceinline__ RecipF recip_of(float b) { return RecipF{__frcp_rn(b)}; }
 __device__ __forceinline__ float div_by(float x, const RecipF& r) { return x * r.h; }
 
-// x / b for a divisor that several quotients share, exactly: through one
-// reciprocal in float64 (div_by), by the division itself in float32 (whose
-// div_by is not the rounded quotient)
+// x / b for a divisor that several quotients share, with the bits of the
+// division itself for every x and b: through one reciprocal in float64 where
+// that is exact, else, and in float32 (whose div_by is not the rounded
+// quotient), by dividing.  The steps of div_by are exact where the divisor is
+// within 2^+-100 (DIV_B) and the quotient within 2^+-700 (DIV_Q): the
+// reciprocal's tail, the numerator and the remainder are then normal numbers.
+// The rest is left to the division: infinities and NaN (the reciprocal form
+// would make inf / b a NaN), zero and subnormal divisors, and tracer masses so
+// small that their quotient is subnormal (it could round twice).  A zero x
+// takes its quotient's sign from x * h.
+#define DIV_B 100
+#define DIV_Q 700
+__device__ __forceinline__ bool exp_within(double x, int e) {   // 2^-e <= |x| < 2^(e+1)
+  return (unsigned)((__double2hiint(x) & 0x7fffffff) - ((1023 - e) << 20)) < (unsigned)(2 * e + 1) << 20;
+}
+// (a call of its own: inlined it takes ten registers more in the tracer kernels)
+static __device__ __noinline__ double slow_quot(double x, double b) { return x / b; }
 struct DivD {
   Recip r;
-  __device__ __forceinline__ explicit DivD(double b) : r(recip_of(b)) {}
-  __device__ __forceinline__ double operator()(double x) const { return div_by(x, r); }
+  __device__ __forceinline__ explicit DivD(double b) : r(recip_of(b)) {
+    if (!exp_within(b, DIV_B)) r.h = __longlong_as_double(0x7ff8000000000000LL);   // no quotient passes
+  }
+  __device__ __forceinline__ double operator()(double x) const {
+    const double q0 = __fma_rn(x, r.h, __dmul_rn(x, r.l));
+    const double q = __fma_rn(__fma_rn(-q0, r.b, x), r.h, q0);
+    if (exp_within(q, DIV_Q)) return q;
+    return (x == 0.0 && r.h == r.h) ? __dmul_rn(x, r.h) : slow(x);
+  }
+  // the same for several quotients that share one test: fast() of each, and if
+  // one of them set bad, slow() of all
+  __device__ __forceinline__ double fast(double x, bool& bad) const {
+    const double q0 = __fma_rn(x, r.h, __dmul_rn(x, r.l));
+    const double q = __fma_rn(__fma_rn(-q0, r.b, x), r.h, q0);
+    const bool zero = x == 0.0;
+    bad |= !(exp_within(q, DIV_Q) || (zero && r.h == r.h));
+    return zero ? __dmul_rn(x, r.h) : q;
+  }
+  __device__ __forceinline__ double slow(double x) const { return slow_quot(x, r.b); }
+  __device__ __forceinline__ void two(double x0, double x1, double& q0, double& q1) const {
+    bool bad = false;
+    q0 = fast(x0, bad);
+    q1 = fast(x1, bad);
+    if (bad) { q0 = slow(x0); q1 = slow(x1); }
+  }
 };
 struct DivF {
   float b;
   __device__ __forceinline__ explicit DivF(float x) : b(x) {}
   __device__ __forceinline__ float operator()(float x) const { return x / b; }
+  __device__ __forceinline__ float fast(float x, bool&) const { return x / b; }
+  __device__ __forceinline__ float slow(float x) const { return x / b; }
+  __device__ __forceinline__ void two(float x0, float x1, float& q0, float& q1) const { q0 = x0 / b; q1 = x1 / b; }
 };
 template <class R> struct DivOf { using type = DivD; };
 template <> struct DivOf<float> { using type = DivF; };

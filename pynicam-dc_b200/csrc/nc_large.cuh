@@ -38,14 +38,17 @@ __device__ void diag_point(const Col c, const MetT<R> m, const DiagArgs<R>& a, i
     D d;
     d.rhog = P[0][p];
     d.rho = d.rhog / m.GSGAM2[p];
-    const auto rr = recip_of(d.rhog);   // the quotients by RHOG
-    d.vx = div_by(P[1][p], rr);
-    d.vy = div_by(P[2][p], rr);
-    d.vz = div_by(P[3][p], rr);
-    d.ein = div_by(P[5][p], rr);
-    const double q0 = div_by(a.Pqw[0][p], rr);
+    // the quotients by RHOG: through one reciprocal for the regional points, by
+    // dividing for the few pole points (the same but for subnormal quotients)
+    const auto rr = recip_of(d.rhog);
+    auto by = [&](double x) -> double { return POLE ? x / d.rhog : div_by(x, rr); };
+    d.vx = by(P[1][p]);
+    d.vy = by(P[2][p]);
+    d.vz = by(P[3][p]);
+    d.ein = by(P[5][p]);
+    const double q0 = by(a.Pqw[0][p]);
     double qd, cv;
-    moist_qd_cv([&](int n) { return div_by(a.Pqw[n][p], rr); }, q0, qd, cv);
+    moist_qd_cv([&](int n) { return by(a.Pqw[n][p]); }, q0, qd, cv);
     d.tem = d.ein / cv;
     d.pre = d.rho * d.tem * (qd * cC.Rdry + q0 * cC.Rvap);
     return d;

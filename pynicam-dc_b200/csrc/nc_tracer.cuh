@@ -124,19 +124,33 @@ __device__ __forceinline__ void trc_vadv_column(const Col c, const TrcVadvArgs<R
       fr_n = __ldg(&a.frhog[c.at(k + 1)]);
     }
     const Div by_p(den_p);
-    const R ck1 = by_k(flx_p) * CC.rdgz[k];
-    const R ck0_p = (k + 1 <= kmax) ? by_p(-flx_p) * CC.rdgz[k + 1] : R(0.0);
+    // the level's quotients by its densities: one tracer a thread is bound by its
+    // chain and tests them together, several test each (see DivD)
+    R q_one = R(0.0), c1k, c0p, dk;
+    if (NT == 1) {
+      bool bad = false;
+      c1k = by_k.fast(flx_p, bad); c0p = by_p.fast(-flx_p, bad); dk = by_k.fast(a.bcoef * fr_k, bad);
+      q_one = by_p.fast(rq_p[0], bad);
+      if (bad) {
+        c1k = by_k.slow(flx_p); c0p = by_p.slow(-flx_p); dk = by_k.slow(a.bcoef * fr_k);
+        q_one = by_p.slow(rq_p[0]);
+      }
+    } else {
+      c1k = by_k(flx_p); c0p = by_p(-flx_p); dk = by_k(a.bcoef * fr_k);
+    }
+    const R ck1 = c1k * CC.rdgz[k];
+    const R ck0_p = (k + 1 <= kmax) ? c0p * CC.rdgz[k + 1] : R(0.0);
+    dk = dk * a.dt;
     const R inL = R(0.5) - copysign(R(0.5), ck0);
     const R inU = R(0.5) + copysign(R(0.5), ck0_p);
     const R c1 = ck0, c2 = ck1;
     const R Cin = inL * c1 + inU * c2;
     const R Cout = (R(1.0) - inL) * c1 + (R(1.0) - inU) * c2;
     const R zsw = R(0.5) - copysign(R(0.5), fabs(Cout) - EPS);
-    const R dk = by_k(a.bcoef * fr_k) * a.dt;
     const Div by_o(Cout + zsw);
 #pragma unroll
     for (int m = 0; m < NT; ++m) {
-      const R q_p = by_p(rq_p[m]);
+      const R q_p = NT == 1 ? q_one : by_p(rq_p[m]);
       const R qh_raw = CC.afact[k] * q_k[m] + CC.bfact[k] * q_m[m];
       const R qc = q_k[m], qb = q_m[m], qa = q_p;
       const R QminL = (inL == R(1.0)) ? npmin(qc, qb) : BIG;
@@ -147,8 +161,13 @@ __device__ __forceinline__ void trc_vadv_column(const Col c, const TrcVadvArgs<R
       const R qnmax = npmax(npmax(QmaxL, QmaxU), qc);
       const R CQmin = inL * c1 * QminL + inU * c2 * QminU;
       const R CQmax = inL * c1 * QmaxL + inU * c2 * QmaxU;
-      const R qomin = by_o((qc - qnmax) + qnmax * (Cin + Cout - dk) - CQmax) * (R(1.0) - zsw) + qc * zsw;
-      const R qomax = by_o((qc - qnmin) + qnmin * (Cin + Cout - dk) - CQmin) * (R(1.0) - zsw) + qc * zsw;
+      const R nmin = (qc - qnmax) + qnmax * (Cin + Cout - dk) - CQmax;
+      const R nmax = (qc - qnmin) + qnmin * (Cin + Cout - dk) - CQmin;
+      R omin, omax;
+      if (NT == 1) by_o.two(nmin, nmax, omin, omax);
+      else { omin = by_o(nmin); omax = by_o(nmax); }
+      const R qomin = omin * (R(1.0) - zsw) + qc * zsw;
+      const R qomax = omax * (R(1.0) - zsw) + qc * zsw;
       R qh = R(0.0);   // the face at kmin stays zero
       if (k > kmin) {
         qh = inL * npmin(npmax(qh_raw, qmin_prev[m]), qmax_prev[m]) + (R(1.0) - inL) * npmin(npmax(qh_raw, qomin), qomax);
@@ -177,10 +196,12 @@ __device__ __forceinline__ void trc_vadv_column(const Col c, const TrcVadvArgs<R
 // column, so one tracer's columns alone leave the SMs waiting (263 us a tracer
 // at gl07 z60 float64).  A thread takes NT tracers of its column: bound by
 // memory (density, fluxes and tendency re-read for each tracer) and by the
-// divisions.  17 tracers at gl07 z60 float64: one a thread 1.87 ms, two 1.54,
-// three 1.47, four 1.64 (166 registers); 6 at gl06 z40 132, 113, 110, 134 us; 6 at
-// gl05 z40 53, 51, 52, 62 us; 6 at gl04 z40 30, 32, 42, 49 us.  Two, where the
-// columns of all tracers are at least 256 for each SM; fewer are bound by the
+// divisions, whose quotients are exact for all operands (DivD; without the test of
+// their range two tracers a thread took 1.54 ms and gave the quotients below 1e-308
+// another rounding, dividing throughout 2.39).  A launch of 17 tracers at gl07 z60
+// float64: one a thread 2.16 ms, two 1.78, three 1.86; 6 at gl06 z40 153, 129,
+// 146 us; 6 at gl05 z40 60, 58, 67 us.  Two, where the columns of all
+// tracers are at least 256 for each SM; fewer are bound by the
 // chain and take a tracer a thread.
 #define TV_THREADS 256
 #define TV_NT 2
@@ -549,11 +570,11 @@ __global__ void __launch_bounds__(TILE_THREADS) k_trc_grad_t(const __grid_consta
       const int ci = min(max(ii, 1), gmax), cj = min(max(jj, 1), gmax);
       mine = ci >= i0 && ci < i0 + T::X && cj >= j0 && cj < j0 + T::Y;
     }
-    const typename DivOf<R>::type den(ok ? __ldg(a.rhog_t + qq) : R(1.0));
+    const R den = ok ? __ldg(a.rhog_t + qq) : R(1.0);
 #pragma unroll
     for (int n = 0; n < TRC_NB; ++n) {
       if (n >= a.nb) break;
-      const R v = ok ? den(__ldg(a.rhogq[n] + qq)) : R(0.0);
+      const R v = ok ? __ldg(a.rhogq[n] + qq) / den : R(0.0);
       s_q[n][p] = v;
       if (mine) {
         a.q[n][qq] = v;
@@ -795,8 +816,10 @@ __global__ void k_trc_qout(const __grid_constant__ TrcLimArgs<R> a) {
     }
     const R zsw = R(0.5) - copysign(R(0.5), fabs(Cout) - EPS);
     const typename DivOf<R>::type den(Cout + zsw);
-    a.Qmin[n][p] = den(qc - CQmax - qnmax * (R(1.0) - Cin - Cout + d)) * (R(1.0) - zsw) + qc * zsw;
-    a.Qmax[n][p] = den(qc - CQmin - qnmin * (R(1.0) - Cin - Cout + d)) * (R(1.0) - zsw) + qc * zsw;
+    R omin, omax;
+    den.two(qc - CQmax - qnmax * (R(1.0) - Cin - Cout + d), qc - CQmin - qnmin * (R(1.0) - Cin - Cout + d), omin, omax);
+    a.Qmin[n][p] = omin * (R(1.0) - zsw) + qc * zsw;
+    a.Qmax[n][p] = omax * (R(1.0) - zsw) + qc * zsw;
   }
 }
 
