@@ -43,7 +43,9 @@ enum { NC_F64 = 0, NC_I32 = 1, NC_I64 = 2, NC_BOOL = 3 };
  * nhm/share/mod_bsstate.py:20, ppm.pntmask and adm.ADM_have_sgp, run
  * constants as 0-d arrays, and the halo plan (halo_r_dst, halo_r_src,
  * halo_p_dst, halo_p_src) composed from comm.Copy_list_* and
- * comm.Singular_list (share/mod_comm.py:1400-1561). */
+ * comm.Singular_list (share/mod_comm.py:1400-1561).  The plan is one gather:
+ * nc_create answers NC_ERR_ARG to an entry outside the grid and to a source
+ * that is itself a destination. */
 typedef struct nc_array {
   const char* name;
   const void* data;

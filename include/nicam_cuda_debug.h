@@ -39,6 +39,13 @@ int nc_get_field(nc_handle* h, const char* name, double* host_reg, double* host_
  * y NULL, b finite and nonzero; else NC_ERR_ARG. */
 int nc_divide_known(const double* x, const double* y, double* q, int64_t n, double b);
 
+/* The check of the exchange plan that nc_create makes (halo_r_dst, halo_r_src,
+ * halo_p_dst, halo_p_src; lall_pl = 2 * members): NC_ERR_ARG, naming the entry,
+ * for a destination or source outside the grid and for a source that is itself
+ * a destination.  Runs on the host; needs no GPU. */
+int nc_check_halo_plan(const int64_t* r_dst, const int64_t* r_src, int64_t nr, const int64_t* p_dst,
+                       const int64_t* p_src, int64_t np, int32_t gall_1d, int32_t lall, int32_t lall_pl);
+
 #ifdef __cplusplus
 }
 #endif

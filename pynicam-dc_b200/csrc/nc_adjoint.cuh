@@ -310,6 +310,8 @@ __global__ void __launch_bounds__(VL_COLS * NC_ADJ_K) k_vadv_lin(const __grid_co
 // and clears the halo, a second forms L^T y at the halo entries and adds it to
 // their sources (atomically: several may share one), instead of writing the
 // halo, adding it up from there and clearing it in launches of their own.
+// inside: the plan writes interior cells as well, whose sources are then looked
+// up for every neighbour (a plan of the model's grids writes halo cells only).
 // ---------------------------------------------------------------------------
 enum { LOP_LAP, LOP_DIV, LOP_GRAD };
 __host__ __device__ constexpr int lop_in(int op) { return op == LOP_DIV ? 3 : 1; }
@@ -325,8 +327,8 @@ __device__ __forceinline__ const double* lop_coef_pl(int g, int lp) {   // of po
 }
 
 template <int OP>
-__global__ void k_lop_fwd(const double* x, const double* x_pl, const int* hsrc, const int* hsrc_pl, double* y,
-                          double* y_pl, int npb) {
+__global__ void k_lop_fwd(const double* x, const double* x_pl, const int* hsrc, const int* hsrc_pl, bool inside,
+                          double* y, double* y_pl, int npb) {
   const int n = cD.npti, np = cD.npl;
   if ((int)blockIdx.x < npb) {   // pole rows: a thread per (level, pole)
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -362,14 +364,14 @@ __global__ void k_lop_fwd(const double* x, const double* x_pl, const int* hsrc, 
   if (interior(c.i, c.j)) {
     const int G = cD.G, c2 = (c.l * G + c.j) * G + c.i;
     const double* cf = lop_coef<OP>();
-    const bool edge = c.i == 1 || c.j == 1 || c.i == G - 2 || c.j == G - 2;
+    const bool edge = inside || c.i == 1 || c.j == 1 || c.i == G - 2 || c.j == G - 2;
     double v[lop_in(OP)][7];
 #pragma unroll
     for (int m = 0; m < 7; ++m) {
       const int off = kNbI[m] + kNbJ[m] * G;
       int s = p + off;
       bool pole = false;
-      if (edge && !interior(c.i + kNbI[m], c.j + kNbJ[m])) {
+      if (edge && (inside || !interior(c.i + kNbI[m], c.j + kNbJ[m]))) {
         const int h = __ldg(hsrc + c2 + off);
         pole = h < 0;
         s = pole ? (-h - 1) + c.k * cD.LP : h + c.k * cD.planei;
@@ -441,8 +443,8 @@ __device__ __forceinline__ void lop_gather_pl(const double* y_pl, int g, int k, 
 }
 
 template <int OP>
-__global__ void k_lop_adj(const double* y, const double* y_pl, const int* hsrc, const int* hsrc_pl, double* x,
-                          double* x_pl, int npb) {
+__global__ void k_lop_adj(const double* y, const double* y_pl, const int* hsrc, const int* hsrc_pl, bool inside,
+                          double* x, double* x_pl, int npb) {
   double o[lop_in(OP)];
   if ((int)blockIdx.x < npb) {
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -459,7 +461,7 @@ __global__ void k_lop_adj(const double* y, const double* y_pl, const int* hsrc, 
   Pt c;
   if (!reg_point(p, c)) return;
   const int G = cD.G;
-  const bool own = interior(c.i, c.j) || __ldg(hsrc + (c.l * G + c.j) * G + c.i) == ix(c.i, c.j, 0, c.l);
+  const bool own = (!inside && interior(c.i, c.j)) || __ldg(hsrc + (c.l * G + c.j) * G + c.i) == ix(c.i, c.j, 0, c.l);
   if (own) lop_gather<OP>(y, c.i, c.j, c.k, c.l, o);
 #pragma unroll
   for (int d = 0; d < lop_in(OP); ++d) x[d * cD.npti + p] = own ? o[d] : 0.0;

@@ -339,6 +339,7 @@ struct nc_handle {
   int nr = 0, np = 0;
   int *c_dst = nullptr, *c_src = nullptr;   // the same in array indices (k_comm)
   int *hsrc = nullptr, *hsrc_pl = nullptr;  // the exchange source of every cell and pole point (itself where none)
+  bool halo_inside = false;                 // the plan writes interior cells too
   // marshal staging
   double *stage = nullptr, *stage_pl = nullptr;
   double* mass_part = nullptr;
@@ -1534,11 +1535,11 @@ static int linear_op(nc_handle* h, int transpose, const double* x, const double*
   const int tb = 128, nreg = (int)((D.npt + tb - 1) / tb);
   if (!transpose) {
     const int npb = (D.KA * D.LP + tb - 1) / tb;
-    k_lop_fwd<OP><<<(unsigned)(npb + nreg), tb, 0, s>>>(x, x_pl, h->hsrc, h->hsrc_pl, y, y_pl, npb);
+    k_lop_fwd<OP><<<(unsigned)(npb + nreg), tb, 0, s>>>(x, x_pl, h->hsrc, h->hsrc_pl, h->halo_inside, y, y_pl, npb);
     return check_launch(h, "lop_fwd");
   }
   const int npb = (D.npl + tb - 1) / tb;
-  k_lop_adj<OP><<<(unsigned)(npb + nreg), tb, 0, s>>>(x, x_pl, h->hsrc, h->hsrc_pl, y, y_pl, npb);
+  k_lop_adj<OP><<<(unsigned)(npb + nreg), tb, 0, s>>>(x, x_pl, h->hsrc, h->hsrc_pl, h->halo_inside, y, y_pl, npb);
   TRY(check_launch(h, "lop_adj"));
   const int nent = h->nr + h->np;
   if (nent > 0) {
@@ -1701,6 +1702,41 @@ static int make_f32_geometry(nc_handle* h) {
     Cf.afact[k] = (float)C.afact[k]; Cf.bfact[k] = (float)C.bfact[k]; Cf.cfact[k] = (float)C.cfact[k];
     Cf.dfact[k] = (float)C.dfact[k]; Cf.rdgz[k] = (float)C.rdgz[k]; Cf.rdgzh[k] = (float)C.rdgzh[k];
     Cf.nl_khmax[k] = (float)C.nl_khmax[k]; Cf.ray_c[k] = (float)C.ray_c[k]; Cf.ray_ch[k] = (float)C.ray_ch[k];
+  }
+  return 0;
+}
+
+// The exchange is one pass that reads its sources while it writes its
+// destinations, and set-up uses both as indices: every entry inside the state,
+// and no source that is itself a destination.  *inside: some destination is an
+// interior cell (the linear operators then look every neighbour's source up).
+static int check_plan(const int64_t* r_dst, const int64_t* r_src, int64_t nr, const int64_t* p_dst, const int64_t* p_src,
+                      int64_t np, int64_t G, int64_t L, int64_t LP, bool* inside) {
+  const int64_t n = L * G * G, m = 6 * LP;
+  auto bad = [](const char* what, int64_t at, int64_t v) {
+    return fail(NC_ERR_ARG, std::string("halo plan: ") + what + " " + std::to_string(at) + " = " + std::to_string(v));
+  };
+  std::vector<char> dst((size_t)(n + m), 0);   // regional cells, then pole points
+  *inside = false;
+  for (int64_t e = 0; e < nr; ++e) {
+    const int64_t d = r_dst[e];
+    if (d < 0 || d >= n) return bad("regional destination outside the grid, entry", e, d);
+    const int64_t i = d % G, j = (d / G) % G;
+    if (i >= 1 && i <= G - 2 && j >= 1 && j <= G - 2) *inside = true;
+    dst[(size_t)d] = 1;
+  }
+  for (int64_t e = 0; e < np; ++e) {
+    if (p_dst[e] < 0 || p_dst[e] >= m) return bad("pole destination outside the grid, entry", e, p_dst[e]);
+    dst[(size_t)(n + p_dst[e])] = 1;
+  }
+  for (int64_t e = 0; e < nr; ++e) {
+    const int64_t s = r_src[e];
+    if (s < -m || s >= n) return bad("source outside the grid, regional entry", e, s);
+    if (dst[(size_t)(s >= 0 ? s : n - s - 1)]) return bad("source that the exchange writes, regional entry", e, s);
+  }
+  for (int64_t e = 0; e < np; ++e) {
+    if (p_src[e] < 0 || p_src[e] >= n) return bad("source outside the grid, pole entry", e, p_src[e]);
+    if (dst[(size_t)p_src[e]]) return bad("source that the exchange writes, pole entry", e, p_src[e]);
   }
   return 0;
 }
@@ -2040,6 +2076,8 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
     if (!a || !b || !c || !d || a->dtype != NC_I64 || b->dtype != NC_I64 || c->dtype != NC_I64 || d->dtype != NC_I64 ||
         numel(a) != numel(b) || numel(c) != numel(d))
       return fail(NC_ERR_ARG, "bad halo plan");
+    TRY(check_plan((const int64_t*)a->data, (const int64_t*)b->data, numel(a), (const int64_t*)c->data,
+                   (const int64_t*)d->data, numel(c), D.G, D.L, D.LP, &h->halo_inside));
     h->nr = (int)numel(a);
     h->np = (int)numel(c);
     const nc_array* src[4] = {a, b, c, d};
@@ -2824,6 +2862,14 @@ int nc_mass_sum_noalloc(const double* rhog, const double* rhogq, const double* g
   k_mass_noalloc_fold<<<1, 1, 0, st>>>(part, (int)blocks, out);
   CU(cudaGetLastError());
   return 0;
+}
+
+int nc_check_halo_plan(const int64_t* r_dst, const int64_t* r_src, int64_t nr, const int64_t* p_dst,
+                       const int64_t* p_src, int64_t np, int32_t gall_1d, int32_t lall, int32_t lall_pl) {
+  if (nr < 0 || np < 0 || gall_1d < 4 || lall < 1 || lall_pl < 1 || (nr && (!r_dst || !r_src)) || (np && (!p_dst || !p_src)))
+    return fail(NC_ERR_ARG, "nc_check_halo_plan: bad argument");
+  bool inside;
+  return check_plan(r_dst, r_src, nr, p_dst, p_src, np, gall_1d, lall, lall_pl, &inside);
 }
 
 int nc_divide_known(const double* x, const double* y, double* q, int64_t n, double b) {
