@@ -301,8 +301,12 @@ enum {
 static const char* const kTuneName[TB_N] = {"diag", "vi_solve", "vi_energy", "vp0_c", "gtend", "hdiff1", "post",
                                             "split_init", "trc_vflux", "trc_vadv", "trc_remap", "trc_qout",
                                             "trc_apply", "trc_rhog"};
+// the sizes nc_set_block accepts, and the largest that the launches use (the
+// launch bounds of kernels that take more registers than 1024 threads leave)
 static const int kTuneMax[TB_N] = {128, 128, 128, NC_VP0C_BLOCK, 1024, 1024, 1024, 1024, 1024, 1024, 1024, 1024,
                                    1024, 1024};
+static const int kLaunchMax[TB_N] = {128, 128, 128, NC_VP0C_BLOCK, 1024, 1024, 1024, 1024, 1024, TV_THREADS,
+                                     TRC_BATCH_THREADS, TRC_BATCH_THREADS, TRC_BATCH_THREADS, 1024};
 
 // "no non-finite value seen": every byte 0x7f, above any variable index
 #define NC_BAD_NONE 0x7f7f7f7f
@@ -622,6 +626,9 @@ static cudaStream_t pole_stream(nc_handle* h) {
   return (h->prof || h->single || !h->stream2) ? h->stream : h->stream2;
 }
 
+// threads per block of a launch
+static int threads_of(const nc_handle* h, int tb) { return std::min(h->blk[tb], kLaunchMax[tb]); }
+
 // tiles per region, and the regions that take the 16-wide tile
 template <class T>
 static int tiles_of(const Dims& D) { return ((D.G - 2 + T::X - 1) / T::X) * ((D.G - 2 + T::Y - 1) / T::Y); }
@@ -718,7 +725,7 @@ static int trc_vadv(nc_handle* h, FieldPair* x, int nx, bool second) {
     va.den = second ? F(h->rhog_t) : F(h->P0[0]);
     va.flx_v = F(h->flx_v); va.frhog = F(h->frhog);
     va.dt = h->dtl; va.bcoef = 0.0; va.clamp = second ? 1 : 0; va.dtl = h->dtl;
-    const int tb = std::min(h->blk[TB_TRC_VADV], TV_THREADS);
+    const int tb = threads_of(h, TB_TRC_VADV);
     const unsigned cb = (unsigned)((D.npt2 + tb - 1) / tb);
     if (pole) k_trc_vadv<R, 1><<<dim3(pcb, (unsigned)nx), 32, 0, ps>>>(va, 1, nx);
     else if (nx == 1 || (long long)D.npt2 * nx < 256LL * h->sms) k_trc_vadv<R, 1><<<dim3(cb, (unsigned)nx), tb, 0, s>>>(va, 0, nx);
@@ -822,17 +829,17 @@ static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
     k_trc_grad_pl<<<pg, 32, 0, ps>>>(ga[1]);
     TRY(check_launch(h, "trc_grad_pl"));
     TRY(comm_fields_of<R>(h, cq.data(), (int)cq.size(), "comm"));
-    auto pts = [&](int tb) { return (unsigned)((D.npt + h->blk[tb] - 1) / h->blk[tb]); };
-    k_trc_remap<<<pts(TB_TRC_REMAP), h->blk[TB_TRC_REMAP], 0, s>>>(ra);
+    auto pts = [&](int tb) { return (unsigned)((D.npt + threads_of(h, tb) - 1) / threads_of(h, tb)); };
+    k_trc_remap<<<pts(TB_TRC_REMAP), threads_of(h, TB_TRC_REMAP), 0, s>>>(ra);
     TRY(check_launch(h, "trc_remap"));
     k_trc_remap_pl<<<pg, 32, 0, ps>>>(rp);
     TRY(check_launch(h, "trc_remap_pl"));
-    k_trc_qout<<<pts(TB_TRC_QOUT), h->blk[TB_TRC_QOUT], 0, s>>>(la);
+    k_trc_qout<<<pts(TB_TRC_QOUT), threads_of(h, TB_TRC_QOUT), 0, s>>>(la);
     TRY(check_launch(h, "trc_qout"));
     k_trc_qout_pl<<<pg, 32, 0, ps>>>(lp);
     TRY(check_launch(h, "trc_qout_pl"));
     TRY(comm_fields_of<R>(h, cl.data(), (int)cl.size(), "comm"));
-    k_trc_apply<<<pts(TB_TRC_APPLY), h->blk[TB_TRC_APPLY], 0, s>>>(la);
+    k_trc_apply<<<pts(TB_TRC_APPLY), threads_of(h, TB_TRC_APPLY), 0, s>>>(la);
     TRY(check_launch(h, "trc_apply"));
     k_trc_apply_pl<<<pg, 32, 0, ps>>>(lp);
     TRY(check_launch(h, "trc_apply_pl"));

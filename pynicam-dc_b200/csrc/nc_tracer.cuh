@@ -645,8 +645,14 @@ struct TrcRemapArgs {
   int nb;
 };
 
+// The largest block of the three kernels of a batch (80, 80 and 125 registers a
+// thread in the float64 form; 1024 threads leave 64).  The float64 remap and
+// outflow bounds are compiled for 768, which holds them to 80 registers, six
+// blocks of 128 an SM: 17 tracers at gl07 z60, a step: remap 3.13 ms (for 512
+// threads 3.70), outflow bounds 3.43 (unbounded 3.84).
+#define TRC_BATCH_THREADS 512
 template <class R>
-__global__ void k_trc_remap(const __grid_constant__ TrcRemapArgs<R> a) {
+__global__ void __launch_bounds__(NC_MINB(R, 768, TRC_BATCH_THREADS)) k_trc_remap(const __grid_constant__ TrcRemapArgs<R> a) {
   Pt c;
   const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (!reg_point(p, c)) return;
@@ -775,7 +781,7 @@ __device__ __forceinline__ int hex_off(int n) { return kNbI[n] + kNbJ[n] * cD.G;
 // Outflow bounds, one thread per point; the Courant numbers and masks are read
 // once for the tracers of the batch.
 template <class R>
-__global__ void k_trc_qout(const __grid_constant__ TrcLimArgs<R> a) {
+__global__ void __launch_bounds__(NC_MINB(R, 768, TRC_BATCH_THREADS)) k_trc_qout(const __grid_constant__ TrcLimArgs<R> a) {
   Pt t;
   const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (!reg_point(p, t)) return;
@@ -829,7 +835,7 @@ __global__ void k_trc_qout(const __grid_constant__ TrcLimArgs<R> a) {
 // (A tile that shares the faces through shared memory was slower for one tracer,
 // 0.94 against 0.62 ms at gl08 mixed: two barriers and 22 KB a block.)
 template <class R>
-__global__ void k_trc_apply(const __grid_constant__ TrcLimArgs<R> a) {
+__global__ void __launch_bounds__(TRC_BATCH_THREADS) k_trc_apply(const __grid_constant__ TrcLimArgs<R> a) {
   Pt t;
   const int p = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (!reg_point(p, t) || !interior(t.i, t.j)) return;

@@ -133,3 +133,36 @@ def test_linear_operators_in_place(pkg):
                     assert float((a - b).abs().max()) <= 1e-15 * float(b.abs().max()) + 0.0, (op.__name__, transpose)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("prec", ["float64", "mixed"])
+def test_largest_blocks(pkg, prec):
+    """a step with every tunable kernel at the largest block nc_set_block accepts equals the default's"""
+    g = _ig().Grid(4, vlayer=9, ztop=30000.0, device="cuda")
+    geo = g.setup(dtl=600.0, gamma=9.6e16, nq=3)
+    s, sp = g.jw_state(nq=3)
+    for q in range(3):
+        s[..., 6 + q], sp[..., 6 + q] = 0.01 * s[..., 0] / (q + 1), 0.01 * sp[..., 0] / (q + 1)
+    names = ("diag", "vi_solve", "vi_energy", "vp0_c", "gtend", "hdiff1", "post", "split_init", "trc_vflux", "trc_vadv",
+             "trc_remap", "trc_qout", "trc_apply", "trc_rhog")
+
+    def run(top):
+        c = pkg.NicamCuda(geo, graph=not top, precision=prec)
+        try:
+            for n in names if top else ():
+                with pytest.raises(pkg.NicamError):
+                    c.set_block(n, 1056)
+                for t in (1024, 256, 128):
+                    try:
+                        c.set_block(n, t)
+                        break
+                    except pkg.NicamError:
+                        continue
+                assert c.get_block(n) == t
+            c.upload(s, sp)
+            c.step(1)
+            return c.download()
+        finally:
+            c.close()
+    (a, ap), (b, bp) = run(False), run(True)
+    assert np.array_equal(a, b) and np.array_equal(ap, bp)
