@@ -108,3 +108,20 @@ def test_autotune_picks_fastest_and_caches(tmp_path):
     assert list(stored.values())[0] == choice
     core2 = FakeCore()
     assert at.tune(core2, members=2, cache=cache) == choice and core2.blk == choice
+
+
+def test_autotune_measures_what_the_kernels_run_now(tmp_path):
+    """the kernels whose block is fixed are not measured; a table measured on
+    kernels of another form is not applied"""
+    at = importlib.import_module("pynicam-dc_b200.autotune")
+    core = FakeCore()
+    timed = []
+    core.kernel_stats = lambda: (timed.append(dict(core.blk)), {k: (1.0, 1) for k in core.blk})[1]
+    cache = str(tmp_path / "tune.json")
+    old_key = "|".join([at._device_name(), "x".join(str(x) for x in core.shape), core.precision, "members=2"])
+    with open(cache, "w") as f:
+        json.dump({old_key: {"diag": 32, "trc_apply": 512}}, f)
+    choice = at.tune(core, members=2, cache=cache)
+    assert choice["vi_solve"] == choice["vi_energy"] == 128 and choice["diag"] != 32
+    assert {b[k] for b in timed for k in at.FIXED if k in b} == {128}
+    assert max(b.get("trc_vadv", 0) for b in timed) == 256
