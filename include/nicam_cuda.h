@@ -57,7 +57,10 @@ typedef struct nc_array {
 typedef struct nc_handle nc_handle;
 
 /* Replaces Dyn.dynamics_setup (mod_dynamics.py:164) for the device: uploads
- * geometry, metrics and the halo plan, allocates all device work arrays.
+ * geometry, metrics and the halo plan, allocates all device work arrays.  With
+ * several tracers up to 27 further fields, whose batches the horizontal tracer
+ * advection works in, are allocated as far as a sixth of the memory that is
+ * left allows; with less it takes fewer tracers at a time, with equal results.
  *
  * The optional scalar entry "precision" selects the arithmetic, as the
  * reference's Backend.configure(name, precision) does

@@ -39,6 +39,12 @@ int nc_get_field(nc_handle* h, const char* name, double* host_reg, double* host_
  * y NULL, b finite and nonzero; else NC_ERR_ARG. */
 int nc_divide_known(const double* x, const double* y, double* q, int64_t n, double b);
 
+/* The tracers a batch of the horizontal advection takes (1..4) in a handle with
+ * nq tracers when free_bytes of device memory are left after its other fields and
+ * the work fields of one tracer take set_bytes; a negative status on a bad
+ * argument.  Runs on the host; needs no GPU. */
+int nc_trc_batch(int64_t free_bytes, int64_t set_bytes, int32_t nq);
+
 /* The check of the exchange plan that nc_create makes (halo_r_dst, halo_r_src,
  * halo_p_dst, halo_p_src; lall_pl = 2 * members): NC_ERR_ARG, naming the entry,
  * for a destination or source outside the grid and for a source that is itself

@@ -364,7 +364,8 @@ struct nc_handle {
   FieldPair gadv[4], vt[6], vt2[6], gT0[6], frhog;
   FieldPair PSa[6], PSb[6], PM[5], vtmp2[3], gT[6], Mc, Mu, Ml, ethtot0, hdiv[3];
   FieldPair flx_v, rhog_t, flx[6], xc[9], ch[6], cm[6];
-  TrcWork tw[TRC_NB];           // horizontal advection of a batch of tracers
+  TrcWork tw[TRC_NB];           // horizontal advection of a batch of tracers, of which
+  int trc_nb = 1;               // this many are allocated (trc_sets)
   FieldPair vph[8];             // horizontal terms of vp0 (div1, div2, dd, dpg)
   const double* hs_lat = nullptr;   // Held-Suarez latitude planes (optional)
   // DCMIP forcing with Kessler microphysics (optional): full-level heights,
@@ -777,7 +778,7 @@ static int trc_hflux(nc_handle* h) {
 }
 
 // horizontal advection of the tracer masses x[0..nx-1] in place (gradient,
-// exchange, face values, Qout, exchange, flux update), in batches of TRC_NB
+// exchange, face values, Qout, exchange, flux update), in batches of trc_nb
 // whose kernels read the winds' fields (centroids, masks, Courant numbers, mass
 // fluxes) once; leaves q, gq, qa, Qmin / Qmax of the last batch behind
 template <class R>
@@ -786,8 +787,8 @@ static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
   const cudaStream_t s = h->stream, ps = pole_stream(h);
   const unsigned pkb = (unsigned)((D.KA * D.LP + 31) / 32);
   const double dt = h->dtl;
-  for (int at = 0; at < nx; at += TRC_NB) {
-    const int nb = std::min(nx - at, TRC_NB);
+  for (int at = 0; at < nx; at += h->trc_nb) {
+    const int nb = std::min(nx - at, h->trc_nb);
     FieldPair* xb = x + at;
     const dim3 pg(pkb, (unsigned)nb);
     const dim3 gt((unsigned)D.KA, (unsigned)(narrow(D) ? tiles_of<Tile16>(D) : tiles_of<Tile32>(D)), (unsigned)D.L);
@@ -1748,6 +1749,45 @@ static int check_plan(const int64_t* r_dst, const int64_t* r_src, int64_t nr, co
   return 0;
 }
 
+// Tracers a batch of the horizontal advection takes when free_bytes of device
+// memory are left and the work fields of one tracer (a set) take set_bytes: the
+// first set is always there, each further one needs sixteen times its size to be
+// free.  A batch of four is 1.9 times as fast as one tracer at a time (17
+// tracers at gl07 z60 float64), but its sets are 27 whole fields, which a run that
+// just fits must not fail for: three take at most a sixth of what is left.
+static int trc_batch_of(long long free_bytes, long long set_bytes, int nq) {
+  int n = 1;
+  for (; n < std::min(nq, TRC_NB) && set_bytes <= free_bytes / 16; ++n) free_bytes -= set_bytes;
+  return n;
+}
+// the sets beyond the first, one allocation each
+static int trc_sets(nc_handle* h) {
+  const Dims& D = h->D;
+  const int es = h->mixed ? (int)sizeof(float) : (int)sizeof(double);
+  auto round = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t rb = round((size_t)D.npt * es), pb = round((size_t)D.npl * es), set = 9 * (rb + pb);
+  size_t free_b = 0, total_b = 0;
+  CU(cudaMemGetInfo(&free_b, &total_b));
+  const int nb = trc_batch_of((long long)free_b, (long long)set, D.nq);
+  for (int n = 1; n < nb; ++n) {
+    char* at = nullptr;
+    if (cudaMalloc((void**)&at, set) != cudaSuccess) {   // taken by another program meanwhile: the batch stays smaller
+      cudaGetLastError();
+      break;
+    }
+    h->allocs.push_back(at);
+    CU(cudaMemset(at, 0, set));
+    TrcWork& w = h->tw[n];
+    for (FieldPair* f : {&w.q, &w.gq[0], &w.gq[1], &w.gq[2], &w.qa[0], &w.qa[1], &w.qa[2], &w.Qmin, &w.Qmax}) {
+      f->r = reinterpret_cast<double*>(at);
+      f->p = reinterpret_cast<double*>(at + rb);
+      at += rb + pb;
+    }
+    h->trc_nb = n + 1;
+  }
+  return 0;
+}
+
 static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
   {
     int dev = 0;
@@ -2158,15 +2198,10 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
   TRY(field(h, h->Mc, "Mc", true)); TRY(field(h, h->Mu, "Mu", true)); TRY(field(h, h->Ml, "Ml", true));
   TRY(field(h, h->ethtot0, "ethtot0"));
   TRY(field(h, h->flx_v, "flx_v")); TRY(field(h, h->rhog_t, "rhog_t"));
-  for (int n = 0; n < std::min(std::max(D.nq, 1), TRC_NB); ++n) {   // named as one tracer's fields for the first of a batch
-    const std::string sfx = n ? "#" + std::to_string(n) : "";
-    TrcWork& w = h->tw[n];
-    TRY(field(h, w.q, ("q" + sfx).c_str()));
-    TRY(field(h, w.Qmin, ("Qmin" + sfx).c_str())); TRY(field(h, w.Qmax, ("Qmax" + sfx).c_str()));
-    for (int d = 0; d < 3; ++d) {
-      TRY(field(h, w.gq[d], ("gq." + std::to_string(d) + sfx).c_str()));
-      TRY(field(h, w.qa[d], ("qa." + std::to_string(d) + sfx).c_str()));
-    }
+  TRY(field(h, h->tw[0].q, "q")); TRY(field(h, h->tw[0].Qmin, "Qmin")); TRY(field(h, h->tw[0].Qmax, "Qmax"));
+  for (int d = 0; d < 3; ++d) {
+    snprintf(nm, sizeof nm, "gq.%d", d); TRY(field(h, h->tw[0].gq[d], nm));
+    snprintf(nm, sizeof nm, "qa.%d", d); TRY(field(h, h->tw[0].qa[d], nm));
   }
   for (int n = 0; n < 8; ++n) { snprintf(nm, sizeof nm, "vph.%d", n); TRY(field(h, h->vph[n], nm)); }
   for (int f = 0; f < 6; ++f) {
@@ -2208,7 +2243,7 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
   CU(cudaStreamCreateWithFlags(&h->s_d2h, cudaStreamNonBlocking));
   for (cudaEvent_t* e : {&h->ev_in_ready, &h->ev_in_free, &h->ev_out_ready, &h->ev_out_done, &h->ev_user})
     CU(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-  return 0;
+  return trc_sets(h);   // last: what it may take depends on the memory that is left
 }
 
 int nc_create(const nc_array* arrays, int32_t narrays, nc_handle** out) {
@@ -2869,6 +2904,11 @@ int nc_mass_sum_noalloc(const double* rhog, const double* rhogq, const double* g
   k_mass_noalloc_fold<<<1, 1, 0, st>>>(part, (int)blocks, out);
   CU(cudaGetLastError());
   return 0;
+}
+
+int nc_trc_batch(int64_t free_bytes, int64_t set_bytes, int32_t nq) {
+  if (free_bytes < 0 || set_bytes < 1 || nq < 1) return -fail(NC_ERR_ARG, "nc_trc_batch: bad argument");
+  return trc_batch_of(free_bytes, set_bytes, nq);
 }
 
 int nc_check_halo_plan(const int64_t* r_dst, const int64_t* r_src, int64_t nr, const int64_t* p_dst,

@@ -34,7 +34,7 @@ EXPORTS = ("nc_create", "nc_upload_state", "nc_download_state", "nc_download_sta
            "nc_upload_state_device", "nc_download_state_device", "nc_check_finite", "nc_set_block", "nc_get_block",
            "nc_step", "nc_set_graph", "nc_run_phases", "nc_sync", "nc_mass_sums", "nc_get_field", "nc_state_pointers", "nc_kernel_launches", "nc_stream", "nc_profile",
            "nc_kernel_stats", "nc_grid_spring", "nc_mass_sum_noalloc", "nc_forcing_step", "nc_history_vars", "nc_restart_pack",
-           "nc_restart_unpack", "nc_restart_finish", "nc_divide_known", "nc_check_halo_plan", "nc_vsolve", "nc_vadv_lin", "nc_laplacian",
+           "nc_restart_unpack", "nc_restart_finish", "nc_divide_known", "nc_check_halo_plan", "nc_trc_batch", "nc_vsolve", "nc_vadv_lin", "nc_laplacian",
            "nc_trc_step_lin", "nc_set_time", "nc_trc_prepare", "nc_divergence", "nc_gradient", "nc_diffusion", "nc_divdamp3d", "nc_divdamp2d", "nc_exchange", "nc_diffusion_kh", "nc_forcing_precip", "nc_last_error", "nc_destroy")
 
 
@@ -89,6 +89,8 @@ def load_library(path: str = LIB_PATH):
     lib.nc_divide_known.restype = ctypes.c_int
     lib.nc_check_halo_plan.argtypes = [dp, dp, i64, dp, dp, i64, i32, i32, i32]
     lib.nc_check_halo_plan.restype = ctypes.c_int
+    lib.nc_trc_batch.argtypes = [i64, i64, i32]
+    lib.nc_trc_batch.restype = ctypes.c_int
     lib.nc_vsolve.argtypes = [vp, i32, i32] + [dp] * 9 + [vp]
     lib.nc_vadv_lin.argtypes = [vp, i32, i32] + [dp] * 6 + [ctypes.c_double, ctypes.c_double, i32, vp]
     lib.nc_laplacian.argtypes = [vp, i32, dp, dp, dp, dp, vp]
