@@ -290,9 +290,11 @@ __global__ void __launch_bounds__(VL_COLS * NC_ADJ_K) k_vadv_lin(const __grid_co
   s_a[0] = up;
   s_b[0] = dn;
   __syncthreads();
-  // raw_k = afact_k q_k + bfact_k q_{k-1}
-  gq += s_a[-VL_COLS] + s_b[VL_COLS] + cC.afact[k] * graw;
-  if (k + 1 < KA) gq += cC.bfact[k + 1] * s_d[VL_COLS];
+  // raw_k = afact_k q_k + bfact_k q_{k-1}, on the faces alone: the factors of the
+  // other rows are not read
+  gq += s_a[-VL_COLS] + s_b[VL_COLS];
+  if (face) gq += cC.afact[k] * graw;
+  if (k >= kmin && k < kmax) gq += cC.bfact[k + 1] * s_d[VL_COLS];
   if (act) a.out[p] = gy + gq / den;
 }
 

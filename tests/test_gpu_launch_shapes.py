@@ -166,3 +166,62 @@ def test_largest_blocks(pkg, prec):
             c.close()
     (a, ap), (b, bp) = run(False), run(True)
     assert np.array_equal(a, b) and np.array_equal(ap, bp)
+
+
+def _column_case(pkg, vlayer, geo_edit=None):
+    """a gl03 handle and random column fields: tracer mass, density, vertical flux, two directions"""
+    import torch
+    g = _ig().Grid(3, vlayer=vlayer, ztop=30000.0, device="cuda")
+    geo = g.setup(dtl=600.0, gamma=7.68e17, nq=1)
+    if geo_edit:
+        geo_edit(geo)
+    c = pkg.NicamCuda(geo, graph=False)
+    gen = torch.Generator(device="cuda").manual_seed(vlayer)
+    f = lambda lo, hi: lo + (hi - lo) * torch.rand(tuple(c.field_shape), generator=gen, dtype=torch.float64, device="cuda")
+    den = f(0.5, 1.0)
+    flx = f(-40.0, 40.0) * (30000.0 / vlayer / 500.0)      # Courant numbers below 0.2
+    flx[:, :c.kmin + 1] = 0.0
+    flx[:, c.kmax + 1:] = 0.0
+    return c, den * f(0.5, 1.0), den, flx, torch.zeros_like(den), f(-1.0, 1.0), f(-1.0, 1.0)
+
+
+@pytest.mark.parametrize("vlayer", [2, 3, 29, 62])
+def test_column_operators_smallest_and_tallest(pkg, vlayer):
+    """the linearised vertical step and the tridiagonal solve from the fewest layers to the most:
+    the adjoint against the tangent-linear and the transpose against the solve (dot products)"""
+    import torch
+    c, rq, den, flx, fr, x, y = _column_case(pkg, vlayer)
+    try:
+        tl, ad = torch.empty_like(x), torch.empty_like(x)
+        c.vadv_lin(1, rq, den, flx, fr, x, tl, 300.0, 0.0, True)
+        c.vadv_lin(2, rq, den, flx, fr, y, ad, 300.0, 0.0, True)
+        size = float((tl * y).abs().sum())
+        assert size > 0 and abs(float((tl * y).sum() - (x * ad).sum())) <= 1e-13 * size
+        Mc, Mu, Ml = 3.0 + 0.3 * x, -1.0 + 0.1 * y, -1.0 + 0.1 * rq
+        c.vsolve(Mc, Mu, Ml, x, tl)
+        c.vsolve(Mc, Mu, Ml, y, ad, transpose=True)
+        k = slice(c.kmin + 1, c.kmax + 1)              # the rows of the solve
+        size = float((tl * y)[:, k].abs().sum())
+        assert size > 0 and abs(float((tl * y)[:, k].sum() - (x * ad)[:, k].sum())) <= 1e-13 * size
+    finally:
+        c.close()
+
+
+def test_vertical_adjoint_reads_the_faces_factors_only(pkg):
+    """the half-level factors below the lowest layer have no face: nothing of them enters the adjoint"""
+    import torch
+
+    def spoil(geo):
+        for n in ("GRD_afact", "GRD_bfact"):
+            geo[n] = np.array(geo[n], np.float64)
+            geo[n][0] = np.nan
+    out = []
+    for edit in (None, spoil):
+        c, rq, den, flx, fr, _, y = _column_case(pkg, 9, edit)
+        try:
+            o = torch.empty_like(y)
+            c.vadv_lin(2, rq, den, flx, fr, y, o, 300.0, 0.0, True)
+            out.append(o.clone())
+        finally:
+            c.close()
+    assert bool(torch.isfinite(out[0]).all()) and torch.equal(out[0], out[1])
