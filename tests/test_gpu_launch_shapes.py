@@ -225,3 +225,33 @@ def test_vertical_adjoint_reads_the_faces_factors_only(pkg):
         finally:
             c.close()
     assert bool(torch.isfinite(out[0]).all()) and torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("vlayer", [100, 126])
+def test_tall_columns_equal_oracle(pkg, vlayer):
+    test_odd_layers_equal_oracle(pkg, vlayer)
+
+
+@pytest.mark.parametrize("vlayer", [61, 126])
+def test_tall_mixed_step_near_float64(pkg, vlayer):
+    """the mixed step of tall columns against the float64 step (measured at 61 and 126 layers:
+    RHOG and RHOGE 5e-8, RHOGVX and RHOGVY 1.6e-7, RHOGVZ 1.2e-4, RHOGW 5e-6; pole momentum 9e-6)"""
+    g = _ig().Grid(4, vlayer=vlayer, ztop=30000.0, device="cuda")
+    geo = g.setup(dtl=300.0, gamma=9.6e16, nq=1)
+    s, sp = _perturbed(geo, *g.jw_state(nq=1), seed=7)
+    out = []
+    for prec in ("float64", "mixed"):
+        c = pkg.NicamCuda(geo, graph=True, precision=prec)
+        try:
+            c.upload(s, sp)
+            c.step(1)
+            out.append(c.download())
+        finally:
+            c.close()
+    (a, ap), (b, bp) = out
+    for v, tol in enumerate((1e-6, 1e-5, 1e-5, 1e-3, 1e-4, 1e-6)):
+        assert np.linalg.norm(b[..., v] - a[..., v]) <= tol * np.linalg.norm(a[..., v]), v
+    # the pole points: horizontal momentum as one vector, then density, vertical momentum, energy
+    assert np.linalg.norm((bp - ap)[..., 1:4]) <= 1e-4 * np.linalg.norm(ap[..., 1:4])
+    for v, tol in ((0, 1e-6), (4, 1e-4), (5, 1e-6)):
+        assert np.linalg.norm(bp[..., v] - ap[..., v]) <= tol * np.linalg.norm(ap[..., v]), v

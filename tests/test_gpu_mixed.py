@@ -131,3 +131,39 @@ def test_mixed_day_mass(day):
     drift = np.abs(m[1] - m[0]) / np.abs(m[0])
     print("mixed mass drift over the day:", drift)
     assert drift[0] <= 1e-8 and drift[1] <= 1e-7, drift
+
+
+# relative differences of the pole points (both poles, g = 0, levels kmin..kmax) after one
+# and two steps from the jet with a 0.5 K perturbation, mixed against float64; measured on
+# B200 at gl03 z10, gl04 z20, gl05 z40 and gl06 z40: RHOG 6.6e-8, RHOGE 6.2e-8, RHOGQ1
+# 3.1e-7, RHOGW 1.2e-4, the horizontal momentum (as a vector: RHOGVZ is what its terms leave
+# after they cancel) 5.3e-4, RHOGVZ 3.5e-15 of that vector; the bounds are about four times these
+POLE_TOL = {"RHOG": 3e-7, "RHOGE": 3e-7, "RHOGQ1": 1.2e-6, "RHOGW": 5e-4, "momentum": 2e-3, "RHOGVZ": 1.5e-14}
+
+
+@pytest.mark.parametrize("glevel, vlayer", [(3, 10), (4, 20), (5, 40)])
+def test_mixed_pole_points_near_float64(pkg, dg, glevel, vlayer):
+    import importlib
+    ig = importlib.import_module("pynicam-dc_b200.icogrid")
+    ens = importlib.import_module("pynicam-dc_b200.ensemble")
+    g = ig.Grid(glevel, vlayer=vlayer, ztop=30000.0, device="cuda")
+    geo = g.setup(dtl={3: 1200.0, 4: 900.0, 5: 600.0}[glevel], gamma={3: 7.68e17, 4: 9.6e16, 5: 1.2e16}[glevel], nq=1)
+    s, sp = ens.perturbed_members(geo, *g.jw_state(nq=1), 1, seed=3, sigma=0.5, length=1500e3)[0]
+    s[..., 6], sp[..., 6] = 0.01 * s[..., 0], 0.01 * sp[..., 0]
+    out = {}
+    for prec in ("float64", "mixed"):
+        c = pkg.NicamCuda(geo, graph=True, precision=prec)
+        try:
+            c.upload(s, sp)
+            for n in (1, 2):
+                c.step(1)
+                out[prec, n] = c.download()[1][0, 1:vlayer + 1]
+        finally:
+            c.close()
+    for n in (1, 2):
+        a, b = out["mixed", n], out["float64", n]
+        e = {nm: dg.rel_l2(a[..., v], b[..., v]) for v, nm in ((0, "RHOG"), (4, "RHOGW"), (5, "RHOGE"), (6, "RHOGQ1"))}
+        e["momentum"] = dg.rel_l2(a[..., 1:4], b[..., 1:4])
+        e["RHOGVZ"] = float(np.linalg.norm(a[..., 3] - b[..., 3]) / np.linalg.norm(b[..., 1:4]))
+        for nm, tol in POLE_TOL.items():
+            assert e[nm] <= tol, (n, nm, e)
