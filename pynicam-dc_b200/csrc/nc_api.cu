@@ -861,6 +861,22 @@ static int trc_rhog(nc_handle* h) {
   return 0;
 }
 
+// vi_main's columns: the regional ones, and on the pole stream the pole's
+// divergences and columns
+template <class R, bool DEEP>
+static int vi_column(nc_handle* h, const VimainArgs<R>* vi, int ncol, cudaStream_t s, cudaStream_t ps, unsigned pkb) {
+  const Dims& D = h->D;
+  const size_t sm = vi_col_smem(D.KA, DEEP);
+  const unsigned nb = (unsigned)((ncol + VC_COLS - 1) / VC_COLS);
+  if (h->C.gam_unit) k_vi_col<R, true, false, DEEP><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
+  else k_vi_col<R, false, false, DEEP><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
+  TRY(check_launch(h, "vi_solve"));
+  k_vimain_a_pl<<<pkb, 32, 0, ps>>>(vi[1]);
+  TRY(check_launch(h, "vimain_a_pl"));
+  k_vi_col<R, false, true, DEEP><<<(6 * D.LP + VC_COLS - 1) / VC_COLS, 32 * VC_MAXW, sm, ps>>>(vi[1]);
+  return check_launch(h, "vi_solve_pl");
+}
+
 // Levels per thread of a column kernel split along the levels
 static int column_chunks(const nc_handle* h, int levels) {
   const long long want = 4LL * 1024 * h->sms;
@@ -1088,15 +1104,7 @@ static int run_step(nc_handle* h) {
       TRY(check_launch(h, "vimain_a"));
       {
         const int ncol = D.L * (D.G - 2) * (D.G - 2);
-        const size_t sm = vi_col_smem(D.KA);
-        const unsigned nb = (unsigned)((ncol + VC_COLS - 1) / VC_COLS);
-        if (h->C.gam_unit) k_vi_col<R, true, false><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
-        else k_vi_col<R, false, false><<<nb, 32 * VC_MAXW, sm, s>>>(vi[0]);
-        TRY(check_launch(h, "vi_solve"));
-        k_vimain_a_pl<<<pkb, 32, 0, ps>>>(vi[1]);
-        TRY(check_launch(h, "vimain_a_pl"));
-        k_vi_col<R, false, true><<<(6 * D.LP + VC_COLS - 1) / VC_COLS, 32 * VC_MAXW, sm, ps>>>(vi[1]);
-        TRY(check_launch(h, "vi_solve_pl"));
+        TRY(vi_deep(D.KA, h->mixed) ? (vi_column<R, true>(h, vi, ncol, s, ps, pkb)) : (vi_column<R, false>(h, vi, ncol, s, ps, pkb)));
       }
       TRY(comm<R>(h, {PN[0], PN[4], PN[5]}));
       PHASE();
@@ -1804,11 +1812,16 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
   CU(cudaFuncSetAttribute(k_dd3d_m<double, Tile16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double, Tile16>()));
   CU(cudaFuncSetAttribute(k_dd3d_m<float, Tile32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float, Tile32>()));
   CU(cudaFuncSetAttribute(k_dd3d_m<float, Tile16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float, Tile16>()));
-  // the column kernel of vi_main: five doubles per level of 32 columns (164 KB at NC_MAXK levels)
-  for (const void* f : {(const void*)k_vi_col<double, true, false>, (const void*)k_vi_col<double, false, false>,
-                        (const void*)k_vi_col<double, false, true>, (const void*)k_vi_col<float, true, false>,
-                        (const void*)k_vi_col<float, false, false>, (const void*)k_vi_col<float, false, true>})
-    CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vi_col_smem(NC_MAXK)));
+  // the column kernel of vi_main: three or five doubles per level of 32 columns
+  // (98 KB at NC_MAXK levels, 82 KB at the most that take five)
+  for (const void* f : {(const void*)k_vi_col<double, true, false, false>, (const void*)k_vi_col<double, false, false, false>,
+                        (const void*)k_vi_col<double, false, true, false>, (const void*)k_vi_col<float, true, false, false>,
+                        (const void*)k_vi_col<float, false, false, false>, (const void*)k_vi_col<float, false, true, false>})
+    CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vi_col_smem(VI_DEEP_F64, false)));
+  for (const void* f : {(const void*)k_vi_col<double, true, false, true>, (const void*)k_vi_col<double, false, false, true>,
+                        (const void*)k_vi_col<double, false, true, true>, (const void*)k_vi_col<float, true, false, true>,
+                        (const void*)k_vi_col<float, false, false, true>, (const void*)k_vi_col<float, false, true, true>})
+    CU(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vi_col_smem(NC_MAXK, true)));
   CU(cudaFuncSetAttribute(k_vadv_lin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vadv_lin_smem(NC_ADJ_K)));
   CU(cudaFuncSetAttribute(k_tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem(NC_ADJ_K)));
   ArrTab T;

@@ -1253,9 +1253,18 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) k_vimain_a_m(const __grid_con
 //   0 horizontal part of the half-level mass flux
 //   1 the right-hand side, then the solution
 //   2 Mu, then the sweep's gamma      3 Ml      4 Mc
+// DEEP, for tall columns: the first three slots alone (98 KB at 128 levels).  The
+// sweep then reads the matrix from memory, VC_PF levels ahead of the ones it works
+// on (eight instead of four spill in float: gl07 z80 0.91 -> 1.22 ms).  Five slots a
+// level take a block of 82 levels to 105 KB: fewer blocks an SM, or hardly any L1
+// beside them.  A step's eleven launches at gl07, the two kernels before / five
+// slots / three: float64 82 levels 23.1 / 24.7 / 15.8 ms, 128 levels 36.9 / 33.4 /
+// 24.6 (five: one block); mixed 82 levels 16.0 / 15.3 / 10.0, 128 levels 25.1 /
+// 29.8 / 18.4.
 #define VC_COLS 32
 #define VC_MAXW 8
-static inline size_t vi_col_smem(int KA) { return (size_t)5 * KA * VC_COLS * sizeof(double); }
+#define VC_PF 4
+static inline size_t vi_col_smem(int KA, bool deep) { return (size_t)(deep ? 3 : 5) * KA * VC_COLS * sizeof(double); }
 
 // the contiguous part [lo, hi) of the levels first..last that a warp takes
 __device__ __forceinline__ void warp_levels(int first, int last, int& lo, int& hi) {
@@ -1265,7 +1274,7 @@ __device__ __forceinline__ void warp_levels(int first, int last, int& lo, int& h
   hi = min(lo + per, last + 1);
 }
 
-template <class R, bool GU, bool POLE>
+template <class R, bool GU, bool POLE, bool DEEP>
 __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* sm) {
   const int KA = cD.KA, kmin = cD.kmin, kmax = cD.kmax, kT = kmax + 1;
   const int lane = (int)(threadIdx.x % 32);
@@ -1286,7 +1295,7 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
   double* s0 = sm + lane;
   double* s1 = s0 + KA * VC_COLS;
   double* s2 = s1 + KA * VC_COLS;
-  double* s3 = s2 + KA * VC_COLS;
+  double* s3 = s2 + KA * VC_COLS;   // not there with DEEP
   double* s4 = s3 + KA * VC_COLS;
   auto S = [](double* s, int k) -> double& { return s[k * VC_COLS]; };
   auto cz = [&](int comp, int q) -> R { return __ldg(POLE ? m.C2WGz + q * 6 + comp : m.C2WGz + comp * cD.npti + q); };
@@ -1327,7 +1336,8 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
       const R hd0 = __ldg(a.hdiv[0] + p), hd1 = __ldg(a.hdiv[1] + p), g0 = __ldg(a.gT[0] + p), g5 = __ldg(a.gT[5] + p);
       const R ps5 = __ldg(a.PS[5] + p), ps0 = __ldg(a.PS[0] + p), rs2 = __ldg(m.RGSGAM2 + p);
       const R g4 = __ldg(a.gT[4] + p), ps4 = __ldg(a.PS[4] + p);
-      const double mu = __ldg(a.Mu + p), ml = __ldg(a.Ml + p), mcc = __ldg(a.Mc + p);
+      const double mu = !DEEP || k == kmax ? __ldg(a.Mu + p) : 0.0, ml = !DEEP || k == kmin + 1 ? __ldg(a.Ml + p) : 0.0;
+      const double mcc = DEEP ? 0.0 : __ldg(a.Mc + p);
       const double rgm = GU ? 1.0 : (double)__ldg(m.RGAM + p), rgh = GU ? 1.0 : (double)__ldg(m.RGAMH + p);
       F hDn, hEn;
       flux(hDn, hEn);
@@ -1357,9 +1367,11 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
         }
         S(s0, k) = hD;
         S(s1, k) = b;
-        S(s2, k) = mu;
-        S(s3, k) = ml;
-        S(s4, k) = mcc;
+        if (!DEEP) {
+          S(s2, k) = mu;
+          S(s3, k) = ml;
+          S(s4, k) = mcc;
+        }
       }
       T1m = T1; T2m = T2; hD = hDn; hE = hEn;
       m0 = f0; m1 = f1; m2 = f2; me = fe;
@@ -1370,20 +1382,53 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
   // read before this level's are overwritten
   if (threadIdx.x < 32) {
     const int k0 = kmin + 1;
-    double beta = S(s4, k0), u = S(s1, k0) / beta;
-    double mu = S(s2, k0);
-    double mc_ = S(s4, k0 + 1), ml = S(s3, k0 + 1), b = S(s1, k0 + 1), mu1 = S(s2, k0 + 1);   // k0+1 <= kT < KA
-    S(s1, k0) = u;
-    for (int k = k0 + 1; k <= kmax; ++k) {
-      const int kn = min(k + 1, kmax);
-      const double mcn = S(s4, kn), mln = S(s3, kn), bn = S(s1, kn), mun = S(s2, kn);
-      const double gg = mu / beta;
-      beta = mc_ - ml * gg;
-      u = (b - ml * u) / beta;
-      S(s2, k - 1) = gg;      // gamma of level k beside the level below, whose Mu is spent
-      S(s1, k) = u;
-      mu = mu1;
-      mu1 = mun; mc_ = mcn; ml = mln; b = bn;
+    double u;
+    if constexpr (DEEP) {
+      double mc_[VC_PF], mu_[VC_PF], ml_[VC_PF];
+      auto fetch = [&](int k) {
+#pragma unroll
+        for (int e = 0; e < VC_PF; ++e) {
+          const int p = c.at(min(k + e, kmax));
+          mc_[e] = __ldg(a.Mc + p); mu_[e] = __ldg(a.Mu + p); ml_[e] = __ldg(a.Ml + p);
+        }
+      };
+      double beta = __ldg(a.Mc + c.at(k0)), mu = __ldg(a.Mu + c.at(k0));
+      fetch(k0 + 1);
+      u = S(s1, k0) / beta;
+      S(s1, k0) = u;
+      for (int k = k0 + 1; k <= kmax; k += VC_PF) {
+        double mc0[VC_PF], mu0[VC_PF], ml0[VC_PF];
+#pragma unroll
+        for (int e = 0; e < VC_PF; ++e) { mc0[e] = mc_[e]; mu0[e] = mu_[e]; ml0[e] = ml_[e]; }
+        if (k + VC_PF <= kmax) fetch(k + VC_PF);
+#pragma unroll
+        for (int e = 0; e < VC_PF; ++e) {
+          if (k + e > kmax) break;
+          const double gg = mu / beta;
+          beta = mc0[e] - ml0[e] * gg;
+          u = (S(s1, k + e) - ml0[e] * u) / beta;
+          S(s2, k + e - 1) = gg;      // gamma of level k + e
+          S(s1, k + e) = u;
+          mu = mu0[e];
+        }
+      }
+    } else {
+      double beta = S(s4, k0);
+      u = S(s1, k0) / beta;
+      double mu = S(s2, k0);
+      double mc_ = S(s4, k0 + 1), ml = S(s3, k0 + 1), b = S(s1, k0 + 1), mu1 = S(s2, k0 + 1);   // k0+1 <= kT < KA
+      S(s1, k0) = u;
+      for (int k = k0 + 1; k <= kmax; ++k) {
+        const int kn = min(k + 1, kmax);
+        const double mcn = S(s4, kn), mln = S(s3, kn), bn = S(s1, kn), mun = S(s2, kn);
+        const double gg = mu / beta;
+        beta = mc_ - ml * gg;
+        u = (b - ml * u) / beta;
+        S(s2, k - 1) = gg;      // gamma of level k beside the level below, whose Mu is spent
+        S(s1, k) = u;
+        mu = mu1;
+        mu1 = mun; mc_ = mcn; ml = mln; b = bn;
+      }
     }
     double x = u, un = S(s1, kmax - 1), gn = S(s2, kmax - 1);
     for (int k = kmax - 1; k >= k0; --k) {
@@ -1464,11 +1509,19 @@ __device__ __forceinline__ void vi_col(const VimainArgs<R>& a, int blk, double* 
 }
 
 // GU: the gamma factors are all 1 and are not loaded
-template <class R, bool GU, bool POLE>
+template <class R, bool GU, bool POLE, bool DEEP>
 __global__ void __launch_bounds__(32 * VC_MAXW, NC_MINB(R, 2, 3)) k_vi_col(const __grid_constant__ VimainArgs<R> a) {
   extern __shared__ __align__(16) double vi_sm[];
-  vi_col<R, GU, POLE>(a, (int)blockIdx.x, vi_sm);
+  vi_col<R, GU, POLE, DEEP>(a, (int)blockIdx.x, vi_sm);
 }
+// Three slots above 64 levels in float64 and 43 in float, where the five no
+// longer fit in 164 KB for the blocks an SM that the registers allow (two and
+// three).  A step at gl07, five and three slots: float64 42 levels 7.87 and 8.19 ms,
+// 62 11.7 and 12.2, 68 14.0 and 13.3; mixed 42 levels 4.73 and 4.77 ms, 46 5.49
+// and 5.23, 52 8.88 and 5.93; gl05 mixed 52 levels 0.89 and 0.57.
+#define VI_DEEP_F64 64
+#define VI_DEEP_F32 43
+static inline bool vi_deep(int KA, bool mixed) { return KA > (mixed ? VI_DEEP_F32 : VI_DEEP_F64); }
 
 // ---------------------------------------------------------------------------
 // elementwise helpers of the small step

@@ -227,12 +227,12 @@ def test_vertical_adjoint_reads_the_faces_factors_only(pkg):
     assert bool(torch.isfinite(out[0]).all()) and torch.equal(out[0], out[1])
 
 
-@pytest.mark.parametrize("vlayer", [100, 126])
+@pytest.mark.parametrize("vlayer", [62, 63, 100, 126])
 def test_tall_columns_equal_oracle(pkg, vlayer):
     test_odd_layers_equal_oracle(pkg, vlayer)
 
 
-@pytest.mark.parametrize("vlayer", [61, 126])
+@pytest.mark.parametrize("vlayer", [41, 42, 61, 126])
 def test_tall_mixed_step_near_float64(pkg, vlayer):
     """the mixed step of tall columns against the float64 step (measured at 61 and 126 layers:
     RHOG and RHOGE 5e-8, RHOGVX and RHOGVY 1.6e-7, RHOGVZ 1.2e-4, RHOGW 5e-6; pole momentum 9e-6)"""
