@@ -5,8 +5,10 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -681,9 +683,10 @@ static Prog<R> prog_pl(nc_handle* h) {
 // halo exchange of the whole PRG_var: PROG and every tracer
 template <class R>
 static int comm_prg(nc_handle* h) {
-  std::vector<FieldPair> fl(h->P, h->P + 6);
-  fl.insert(fl.end(), h->Pq, h->Pq + h->D.nq);
-  return comm_fields_of<R>(h, fl.data(), (int)fl.size(), "comm_final");
+  FieldPair fl[6 + NC_MAXNQ];
+  std::copy(h->P, h->P + 6, fl);
+  std::copy(h->Pq, h->Pq + h->D.nq, fl + 6);
+  return comm_fields_of<R>(h, fl, 6 + h->D.nq, "comm_final");
 }
 
 // ---------------------------------------------------------------------------
@@ -797,7 +800,7 @@ static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
     TrcRemapPlArgs<R> rp;
     TrcLimArgs<R> la;
     TrcLimPlArgs<R> lp;
-    std::vector<FieldPair> cq, cl;
+    FieldPair cq[3 * TRC_NB], cl[2 * TRC_NB];   // exchanged: gradients, outflow bounds
     for (int n = 0; n < nb; ++n) {
       TrcWork& w = h->tw[n];
       for (int pole = 0; pole < 2; ++pole) {
@@ -809,12 +812,12 @@ static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
       for (int d = 0; d < 3; ++d) {
         ra.gq[n][d] = RG<R>(w.gq[d]); rp.gq[n][d] = PL<R>(w.gq[d]);
         ra.qa[n][d] = RG<R>(w.qa[d]); la.qa[n][d] = RG<R>(w.qa[d]);
-        cq.push_back(w.gq[d]);
+        cq[3 * n + d] = w.gq[d];
       }
       rp.qa[n] = PL<R>(w.qa[0]); lp.qa[n] = PL<R>(w.qa[0]);
       la.q[n] = RG<R>(w.q); la.Qmin[n] = RG<R>(w.Qmin); la.Qmax[n] = RG<R>(w.Qmax); la.rhogq[n] = RG<R>(xb[n]);
       lp.q_of[n] = PL<R>(w.q); lp.Qmin[n] = PL<R>(w.Qmin); lp.Qmax[n] = PL<R>(w.Qmax); lp.rhogq[n] = PL<R>(xb[n]);
-      cl.push_back(w.Qmin); cl.push_back(w.Qmax);
+      cl[2 * n] = w.Qmin; cl[2 * n + 1] = w.Qmax;
     }
     ga[0].rhog_t = RG<R>(h->rhog_t); ga[1].rhog_t = PL<R>(h->rhog_t);
     ga[0].nb = ga[1].nb = ra.nb = la.nb = nb;
@@ -829,7 +832,7 @@ static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
     TRY(check_launch(h, "trc_grad"));
     k_trc_grad_pl<<<pg, 32, 0, ps>>>(ga[1]);
     TRY(check_launch(h, "trc_grad_pl"));
-    TRY(comm_fields_of<R>(h, cq.data(), (int)cq.size(), "comm"));
+    TRY(comm_fields_of<R>(h, cq, 3 * nb, "comm"));
     auto pts = [&](int tb) { return (unsigned)((D.npt + threads_of(h, tb) - 1) / threads_of(h, tb)); };
     k_trc_remap<<<pts(TB_TRC_REMAP), threads_of(h, TB_TRC_REMAP), 0, s>>>(ra);
     TRY(check_launch(h, "trc_remap"));
@@ -839,7 +842,7 @@ static int trc_horizontal(nc_handle* h, FieldPair* x, int nx) {
     TRY(check_launch(h, "trc_qout"));
     k_trc_qout_pl<<<pg, 32, 0, ps>>>(lp);
     TRY(check_launch(h, "trc_qout_pl"));
-    TRY(comm_fields_of<R>(h, cl.data(), (int)cl.size(), "comm"));
+    TRY(comm_fields_of<R>(h, cl, 2 * nb, "comm"));
     k_trc_apply<<<pts(TB_TRC_APPLY), threads_of(h, TB_TRC_APPLY), 0, s>>>(la);
     TRY(check_launch(h, "trc_apply"));
     k_trc_apply_pl<<<pg, 32, 0, ps>>>(lp);
@@ -2264,8 +2267,14 @@ int nc_create(const nc_array* arrays, int32_t narrays, nc_handle** out) {
   *out = nullptr;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return fail(NC_ERR_CUDA, "no CUDA device");
-  nc_handle* h = new nc_handle();
-  int rc = create_impl(arrays, narrays, h);
+  nc_handle* h = new (std::nothrow) nc_handle();
+  if (!h) return fail(NC_ERR_STATE, "nc_create: out of host memory");
+  int rc;
+  try {
+    rc = create_impl(arrays, narrays, h);
+  } catch (const std::exception& e) {   // host memory for the set-up's tables
+    rc = fail(NC_ERR_STATE, std::string("nc_create: ") + e.what());
+  }
   if (rc) {
     std::string keep = g_err;
     nc_destroy(h);
@@ -2926,10 +2935,14 @@ int nc_trc_batch(int64_t free_bytes, int64_t set_bytes, int32_t nq) {
 
 int nc_check_halo_plan(const int64_t* r_dst, const int64_t* r_src, int64_t nr, const int64_t* p_dst,
                        const int64_t* p_src, int64_t np, int32_t gall_1d, int32_t lall, int32_t lall_pl) {
-  if (nr < 0 || np < 0 || gall_1d < 4 || lall < 1 || lall_pl < 1 || (nr && (!r_dst || !r_src)) || (np && (!p_dst || !p_src)))
+  if (nr < 0 || np < 0 || gall_1d < 4 || lall < 1 || lall_pl < 1 || (double)lall * gall_1d * gall_1d > 2147483647.0 || (nr && (!r_dst || !r_src)) || (np && (!p_dst || !p_src)))
     return fail(NC_ERR_ARG, "nc_check_halo_plan: bad argument");
   bool inside;
-  return check_plan(r_dst, r_src, nr, p_dst, p_src, np, gall_1d, lall, lall_pl, &inside);
+  try {
+    return check_plan(r_dst, r_src, nr, p_dst, p_src, np, gall_1d, lall, lall_pl, &inside);
+  } catch (const std::exception& e) {
+    return fail(NC_ERR_STATE, std::string("nc_check_halo_plan: ") + e.what());
+  }
 }
 
 int nc_divide_known(const double* x, const double* y, double* q, int64_t n, double b) {

@@ -65,6 +65,8 @@ def test_refused_plans(pkg, plan):
         from make_golden import load
         geo, _ = load(os.path.join(HERE, "golden", "gl03_z10_trc.npz"))
         pkg.runtime.check_halo_plan(ens._stacked_plan(geo, 2), *plan[1:])
+    with pytest.raises(pkg.NicamError, match="bad argument"):    # more cells than a handle can index
+        pkg.runtime.check_halo_plan(plan[0], 2 ** 30, 2 ** 30)
 
 
 @pytest.mark.gpu
