@@ -412,10 +412,11 @@ struct nc_handle {
   cudaEvent_t ev_in_ready = nullptr, ev_in_free = nullptr, ev_out_ready = nullptr, ev_out_done = nullptr;
   cudaEvent_t ev_user = nullptr;   // ordering against a caller's stream (device-pointer marshal)
   double *stage_out = nullptr, *stage_out_pl = nullptr;
-  double* adj_work = nullptr;   // exchanged copy of the Laplacian's input (allocated on first use)
+  double* adj_work = nullptr;   // exchanged copy of the scalar of the Kh-weighted diffusion (first use)
   double* adj_work6 = nullptr;   // the diffusion / divergence-damping adjoints' triangle cotangents (6 fields)
   double* adj_work4 = nullptr;   // exchanged copy of the 3-D divergence damping's four momenta (first use)
-  double* adj_work3 = nullptr;  // exchanged copy of the divergence's three components (first use)
+  double* adj_work3 = nullptr;  // copy of an input that overlaps its output (linear_op), exchanged copy of the
+                                // 2-D divergence damping's three components (first use)
   // linearised tracer step (nc_trc_step_lin): work fields allocated on first use
   FieldPair lin[20];
   bool lin_ready = false;
@@ -566,11 +567,6 @@ static int load_consts(nc_handle* h) {
 // launch helpers
 // ---------------------------------------------------------------------------
 static const int kBlock = 128;
-static unsigned grid_cols_kl(const nc_handle* h) {   // regional columns + (k, lp) pole threads
-  long long n = h->D.npt2 + (long long)h->D.KA * h->D.LP;
-  return (unsigned)((n + kBlock - 1) / kBlock);
-}
-
 static int mark(nc_handle* h, const char* what) {
   if (h->ev_used == h->ev_pool.size()) {
     cudaEvent_t e;
@@ -880,7 +876,12 @@ static int vi_column(nc_handle* h, const VimainArgs<R>* vi, int ncol, cudaStream
   return check_launch(h, "vi_solve_pl");
 }
 
-// Levels per thread of a column kernel split along the levels
+// Levels per thread of a column kernel split along the levels: enough chunks for
+// 1024 threads on every SM and four times over, of at least 4 levels, and whole
+// columns where those alone are as many.  k_vp0_cr, a step at z40 with one, two and
+// four chunks, and with these: gl05 float64 645, 351, 231 and 166 us (ten chunks),
+// gl07 float64 1.80, 1.87, 1.73 and 1.73 ms (four), gl07 mixed 1.27, 1.26, 1.17
+// and 1.17 (four), 12 x gl06 mixed 3.31, 3.38, 3.50 and 3.37 (two).
 static int column_chunks(const nc_handle* h, int levels) {
   const long long want = 4LL * 1024 * h->sms;
   const long long n = std::max(1LL, std::min((want + h->D.npt2 - 1) / h->D.npt2, (long long)levels / 4));
@@ -893,7 +894,6 @@ static int run_step(nc_handle* h) {
   const cudaStream_t ps = pole_stream(h);
   h->phase = 0;
   const Dims& D = h->D;
-  const unsigned gkl = grid_cols_kl(h);
   // pole kernels: one thread per pole point (6 * LP * kall) or per pole level
   // (kall * LP), in blocks of a warp to spread the few threads over SMs; LP = 2
   // per ensemble member.  They stay launches of their own on the pole stream:
@@ -1023,7 +1023,7 @@ static int run_step(nc_handle* h) {
       const unsigned tx = (unsigned)((D.G - 2 + T::X - 1) / T::X), ty = (unsigned)((D.G - 2 + T::Y - 1) / T::Y);
       const int nk = tile_chunks(h, tiles * D.L, levels);
       const dim3 gt(tx, ty, (unsigned)(D.L * ((levels + nk - 1) / nk)));
-      k_dd3d_m<R, T, true><<<gt, TILE_THREADS, dd3d_m_smem<R, T>(), s>>>(v, o, nk);
+      k_dd3d_m<R, T><<<gt, TILE_THREADS, dd3d_m_smem<R, T>(), s>>>(v, o, nk);
       TRY(check_launch(h, "dd3d"));
       k_dd3d_pl<<<(unsigned)((D.KA * D.LP * 8 + 31) / 32), 32, 0, ps>>>(vp, op);
       TRY(check_launch(h, "dd3d_pl"));
@@ -1811,10 +1811,10 @@ static int create_impl(const nc_array* arrays, int32_t narrays, nc_handle* h) {
   CU(cudaFuncSetAttribute(k_hdiff2_m<double, Tile16>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<double, Tile16>()));
   CU(cudaFuncSetAttribute(k_hdiff2_m<float, Tile32>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<float, Tile32>()));
   CU(cudaFuncSetAttribute(k_hdiff2_m<float, Tile16>, cudaFuncAttributeMaxDynamicSharedMemorySize, hdiff2_m_smem<float, Tile16>()));
-  CU(cudaFuncSetAttribute(k_dd3d_m<double, Tile32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double, Tile32>()));
-  CU(cudaFuncSetAttribute(k_dd3d_m<double, Tile16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double, Tile16>()));
-  CU(cudaFuncSetAttribute(k_dd3d_m<float, Tile32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float, Tile32>()));
-  CU(cudaFuncSetAttribute(k_dd3d_m<float, Tile16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float, Tile16>()));
+  CU(cudaFuncSetAttribute(k_dd3d_m<double, Tile32>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double, Tile32>()));
+  CU(cudaFuncSetAttribute(k_dd3d_m<double, Tile16>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<double, Tile16>()));
+  CU(cudaFuncSetAttribute(k_dd3d_m<float, Tile32>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float, Tile32>()));
+  CU(cudaFuncSetAttribute(k_dd3d_m<float, Tile16>, cudaFuncAttributeMaxDynamicSharedMemorySize, dd3d_m_smem<float, Tile16>()));
   // the column kernel of vi_main: three or five doubles per level of 32 columns
   // (98 KB at NC_MAXK levels, 82 KB at the most that take five)
   for (const void* f : {(const void*)k_vi_col<double, true, false, false>, (const void*)k_vi_col<double, false, false, false>,

@@ -160,12 +160,10 @@ template <> __device__ __forceinline__ const GeomT<float>& geom<float>() { retur
 #ifndef NC_F32_VP0C
 #define NC_F32_VP0C 3
 #endif
-#ifndef NC_F32_VIMAINA
-#define NC_F32_VIMAINA 6
-#endif
 
-// a * b + c with two roundings in both forms, as the reference rounds them
-// (fused multiply-adds in the float form: 0.8 % of the gl08 mixed step)
+// a * b + c with two roundings in both forms, as the reference rounds them (a
+// fused multiply-add in the float form would save 0.8 % of the gl08 mixed step,
+// but moves its results)
 template <class R>
 __device__ __forceinline__ R mad(R a, R b, R c) { return a * b + c; }
 

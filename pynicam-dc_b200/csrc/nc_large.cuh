@@ -146,7 +146,10 @@ __device__ void diag_point(const Col c, const MetT<R> m, const DiagArgs<R>& a, i
 
 // A thread per point (a column per thread was bound by the chain of a level's
 // loads, stores and divisions: 4 us a level at any grid level); w at the
-// half levels k and k+1 is formed by both neighbours.
+// half levels k and k+1 is formed by both neighbours.  Eight and nine blocks of 128
+// an SM although they spill (72 and 80 bytes stored a thread): a step at gl07 z40
+// float64 0.96 ms, six blocks without spills 1.10, five 1.25; mixed nine 0.75,
+// eight 0.81, six 1.00.
 template <class R>
 __global__ void __launch_bounds__(128, NC_MINB(R, 8, NC_F32_DIAG)) k_diag(const __grid_constant__ DiagArgs<R> a, const __grid_constant__ DiagArgs<R> ap, int npb) {
   Pt q;

@@ -116,52 +116,6 @@ __device__ __forceinline__ R mc(const R* a, const Col& c, int comp, int ncomp, i
   return c.pole ? a[c.at(k) * ncomp + comp] : a[comp * cD.npti + c.at(k)];
 }
 
-// ---- horizontal 7-point operators (regional, interior (i,j) only) ---------
-
-// divergence of (vx,vy,vz) at (i,j,k,l) given a functor returning the three
-// components at a neighbour: kernels/fluxconv.py:52-78
-template <class R, class F>
-__device__ __forceinline__ R div7(int i, int j, int k, int l, F vel) {
-  R acc[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    R s = R(0);
-#pragma unroll
-    for (int m = 0; m < 7; ++m) {
-      R v = vel(i + kNbI[m], j + kNbJ[m], k, d);
-      R t = P2(CG.coef_div, d * 7 + m, i, j, l) * v;
-      s = (m == 0) ? t : s + t;
-    }
-    acc[d] = s;
-  }
-  return acc[0] + acc[1] + acc[2];
-}
-
-// gradient components (kernels/oprtgradient.py:45-70): np.sum over the 7
-// stencil points, left to right
-template <class R, class F>
-__device__ __forceinline__ void grad7(int i, int j, int k, int l, F scl, R out[3]) {
-  R s[7];
-#pragma unroll
-  for (int m = 0; m < 7; ++m) s[m] = scl(i + kNbI[m], j + kNbJ[m], k);
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    R a = P2(CG.coef_grad, d * 7 + 0, i, j, l) * s[0];
-#pragma unroll
-    for (int m = 1; m < 7; ++m) a = a + P2(CG.coef_grad, d * 7 + m, i, j, l) * s[m];
-    out[d] = a;
-  }
-}
-
-// laplacian (kernels/oprtlaplacian.py:41-55)
-template <class R, class F>
-__device__ __forceinline__ R lap7(int i, int j, int k, int l, F scl) {
-  R a = P2(CG.coef_lap, 0, i, j, l) * scl(i, j, k);
-#pragma unroll
-  for (int m = 1; m < 7; ++m) a = a + P2(CG.coef_lap, m, i, j, l) * scl(i + kNbI[m], j + kNbJ[m], k);
-  return a;
-}
-
 // tangent-plane projection of one vector at an interior point
 // (kernels/horizontalizevec.py:51-54)
 template <class R>

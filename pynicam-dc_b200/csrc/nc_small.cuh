@@ -16,16 +16,6 @@ struct Three { R* f[3]; };
 template <class R>
 struct CThree { const R* f[3]; };
 
-// the six-edge divergence-damping combination for direction d at (i,j)
-// (kernels/oprtdivdamp.py:110-120)
-template <class R>
-__device__ __forceinline__ R ddivd(int i, int j, int l, int d, const R aTI, const R aTJ,
-                                        const R bTI, const R cTJ, const R cTI, const R dTJ) {
-  return P2(CG.coef_diff, d * 6 + 0, i, j, l) * (aTI + aTJ) + P2(CG.coef_diff, d * 6 + 1, i, j, l) * (aTJ + bTI) +
-         P2(CG.coef_diff, d * 6 + 2, i, j, l) * (bTI + cTJ) + P2(CG.coef_diff, d * 6 + 3, i, j, l) * (cTJ + cTI) +
-         P2(CG.coef_diff, d * 6 + 4, i, j, l) * (cTI + dTJ) + P2(CG.coef_diff, d * 6 + 5, i, j, l) * (dTJ + aTI);
-}
-
 // Tiled 3-D divergence damping: one block per T::X x T::Y tile of output
 // cells of one region, marching upward in k.  Per level the block stages the
 // haloed tile of RGAM-scaled momentum and the vertical mass flux rwv(k+1) in
@@ -38,15 +28,12 @@ __device__ __forceinline__ R ddivd(int i, int j, int l, int d, const R aTI, cons
 // are added left to right in the reference's order.
 // The tile's k-invariant coefficients are read once per block instead of
 // once per level: the triangle weights coef_intp (18 planes) staged in shared
-// memory, the cell's coef_diff (18) held in registers (CDR) or read per
-// level.  Dynamic shared memory dd3d_m_smem<R, T>().
+// memory, the cell's coef_diff (18) held in registers.  Dynamic shared memory
+// dd3d_m_smem<R, T>().
 template <class R, class T>
 constexpr int dd3d_m_smem() {
   return (18 * (T::X + 1) * (T::Y + 1) + 9 * (T::X + 2) * (T::Y + 2) + 4 * (T::X + 1) * (T::Y + 1)) * (int)sizeof(R);
 }
-#ifndef DD_M_MINB
-#define DD_M_MINB 2
-#endif
 // The march takes two levels at a time: a triangle's coefficients are read once
 // for both, and a pair of levels costs two barriers.  Bound by shared-memory
 // reads and barriers: gl08 mixed 636 -> 509 us, gl06 mixed 66 -> 58 us, gl07
@@ -126,8 +113,8 @@ __global__ void k_dd3d_pl(const __grid_constant__ Four<R> v, const __grid_consta
 
 // The levels are split into chunks of nk where the tiles alone leave SMs idle
 // (see tile_chunks); blockIdx.z counts (region, chunk).
-template <class R, class T, bool CDR>
-__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, DD_M_MINB, 4)) k_dd3d_m(Four<R> v, Three<R> out,
+template <class R, class T>
+__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 2, 4)) k_dd3d_m(Four<R> v, Three<R> out,
                                                                                            int nk) {
   constexpr int PX = T::X + 2, PY = T::Y + 2, NP = PX * PY;
   constexpr int TX = T::X + 1, TY = T::Y + 1, NT = TX * TY;
@@ -152,10 +139,10 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, DD_M_MINB, 4)) k_dd3d
 #pragma unroll
     for (int m = 0; m < 18; ++m) s_ci[m * NT + p] = ok ? P2c(CG.coef_intp, m, ii, jj, l) : R(0.0);
   }
-  R cd[CDR ? 18 : 1];
-  if (CDR && own) {
+  R cd[18];
+  if (own) {
 #pragma unroll
-    for (int m = 0; m < (CDR ? 18 : 1); ++m) cd[m] = P2c(CG.coef_diff, m, i, j, l);
+    for (int m = 0; m < 18; ++m) cd[m] = P2c(CG.coef_diff, m, i, j, l);
   }
   // vertical mass flux at the half level of q from the momenta at q (u) and below (d)
   auto rwv = [&](int q, const R* u, const R* d, R w) -> R {
@@ -246,7 +233,6 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, DD_M_MINB, 4)) k_dd3d
     }
     if (own) {
       const int ta = (ty + 1) * TX + (tx + 1);   // triangle (i, j)
-      auto D = [&](int m) { return CDR ? cd[CDR ? m : 0] : P2c(CG.coef_diff, m, i, j, l); };
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         if (k + e > kb) break;
@@ -259,8 +245,8 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, DD_M_MINB, 4)) k_dd3d
         const int q = ix(i, j, k + e, l);
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-          out.f[d][q] = mad(D(d * 6 + 5), dTJ + aTI, mad(D(d * 6 + 4), cTI + dTJ, mad(D(d * 6 + 3), cTJ + cTI,
-                        mad(D(d * 6 + 2), bTI + cTJ, mad(D(d * 6 + 1), aTJ + bTI, D(d * 6 + 0) * (aTI + aTJ))))));
+          out.f[d][q] = mad(cd[d * 6 + 5], dTJ + aTI, mad(cd[d * 6 + 4], cTI + dTJ, mad(cd[d * 6 + 3], cTJ + cTI,
+                        mad(cd[d * 6 + 2], bTI + cTJ, mad(cd[d * 6 + 1], aTJ + bTI, cd[d * 6 + 0] * (aTI + aTJ))))));
       }
     }
     c0 = c2;
@@ -351,14 +337,6 @@ __device__ void presgrad_pl(int g, int k, int lp, const Col& c, const MetT<R>& m
     for (int d = 0; d < 3; ++d) out[d] = gh[d] + (pvmh(kk + 1, d) - pvmh(kk, d)) * CC.rdgz[kk];
   }
   horiz_pl(g, lp, out[0], out[1], out[2]);
-}
-
-// vertical pressure gradient (kernels/presgrad.py:196-204)
-template <class R, class PF>
-__device__ __forceinline__ R presgradw(const Col& c, const MetT<R>& m, int k, PF Pk) {
-  if (k < cD.kmin + 1 || k > cD.kmax) return R(0.0);
-  int p = c.at(k), pm = c.at(k - 1);
-  return gam_at(m.GAM2H, p) * (Pk(k) * m.RGSGAM2[p] - Pk(k - 1) * m.RGSGAM2[pm]) * CC.rdgzh[k];
 }
 
 // flux convergence at level k of a regional or pole column given the
@@ -510,7 +488,7 @@ struct Vp0H {
 // vp0 horizontal terms, one block per (NK levels, tile): like k_path1_l, each of
 // the 78 coefficients is loaded once and applied to the block's NK levels (the
 // float32 instance; two float64 levels do not leave room for four blocks of
-// shared memory). 
+// shared memory).
 template <class R> constexpr int VP_NK = sizeof(R) == 8 ? 1 : 2;
 template <class R, class T, int NK>
 __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 4, NC_F32_VP0H)) k_vp0_hl(Vp0Args<R> a, Vp0H<R> h) {
@@ -692,10 +670,10 @@ __global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 4, NC_F32_VP0H)) k_vp
 // half-level eth, the vertical kinetic-energy term) are formed and the ones at
 // k and k-1 are carried in registers.  Each value is the expression of
 // k_vp0_pl (the pole form), so regional and pole columns round alike.
-// 256-thread blocks capped at 64 registers (four per SM; measured faster
-// than three at 74 registers).  blockIdx.y takes a chunk of nk levels: a whole
-// column per thread walked 42 levels at 9 us each, however few the columns;
-// a chunk forms the half-level values of its first two levels again.
+// 256-thread blocks, three an SM (80 registers).  blockIdx.y takes a chunk of nk
+// levels: a whole column per thread walked 42 levels at 9 us each, however few the
+// columns; a chunk forms the half-level values of its first two levels again (see
+// column_chunks).
 #define NC_VP0C_BLOCK 256
 template <class R>
 __global__ void __launch_bounds__(NC_VP0C_BLOCK, NC_MINB(R, 3, NC_F32_VP0C)) k_vp0_cr(Vp0Args<R> a, Vp0H<R> h,
@@ -1072,9 +1050,10 @@ __global__ void k_vimain_a_pl(const __grid_constant__ VimainArgs<R> a) {
 }
 
 // vi_main kernel A, one block per (level, tile): the horizontal divergences
-// of RGAM*diff_vh, RGAM*diff_vh*eth and RGAM*(rhogv + diff_vh)*ethtot0.
+// of RGAM*diff_vh, RGAM*diff_vh*eth and RGAM*(rhogv + diff_vh)*ethtot0 (the
+// double form; the float form marches, see k_vimain_a_m).
 template <class R, class T>
-__global__ void __launch_bounds__(TILE_THREADS, NC_MINB(R, 6, NC_F32_VIMAINA)) k_vimain_a_l(VimainArgs<R> a) {
+__global__ void __launch_bounds__(TILE_THREADS, 6) k_vimain_a_l(VimainArgs<R> a) {
   constexpr int PX = T::X + 2, PY = T::Y + 2;
   __shared__ R s_h[3][3][PY * PX];
   const TileLv tl = tile_level<T>(cD.kmin);
