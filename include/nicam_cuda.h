@@ -383,8 +383,9 @@ int nc_history_vars(nc_handle* h, const int32_t* items, int32_t nitems, int64_t 
  * transpose = 1 writes y = C^T L^T q, the adjoint, with the exchange's
  * adjoint adding each halo value into its source cell (atomically: the
  * order of those additions, and so the last bits, may vary between calls).
- * q and y must not alias.  The forward form allocates one scratch copy of
- * a field in the handle on its first call. */
+ * q and y must not be the same buffer.  A call whose input overlaps its output
+ * otherwise copies the input first, to scratch in the handle (three fields,
+ * allocated on the first such call). */
 int nc_vsolve(nc_handle* h, int32_t pole, int32_t transpose, const double* Mc, const double* Mu, const double* Ml,
               const double* b, double* x, const double* x_fwd, double* gMc, double* gMu, double* gMl,
               void* stream);
@@ -401,9 +402,9 @@ int nc_laplacian(nc_handle* h, int32_t transpose, const double* q, const double*
  * 3 x 6*kall*2 pole values).  transpose = 1 reads y and writes v = C^T D^T y.
  * nc_gradient: g = Grad(C(q)) (kernels/oprtgradient.py:45-88,
  * OPRT_gradient), g the three components one after the other; transpose = 1
- * reads g and writes q = C^T Grad^T g.  The buffer written must not alias the
- * one read.  The forward forms allocate a scratch copy in the handle on their
- * first call; the adjoints add with atomics (last bits may vary). */
+ * reads g and writes q = C^T Grad^T g.  The buffer written may overlap the one
+ * read (the input is then copied first, to the scratch of nc_laplacian); the
+ * adjoints add with atomics (last bits may vary). */
 int nc_divergence(nc_handle* h, int32_t transpose, double* v, double* v_pl, double* y, double* y_pl, void* stream);
 int nc_gradient(nc_handle* h, int32_t transpose, double* q, double* q_pl, double* g, double* g_pl, void* stream);
 

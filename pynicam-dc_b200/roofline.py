@@ -54,7 +54,7 @@ KERNELS = {
     "advmom": (_f(*PROG[:5], "vvx", "vvy", "vvz") + C2WGZ + _m("RGSQRTH", "C2W.0", "C2W.1"),
                _f(*_n("gadv.", 4)),
                _n("coef_div.", 21) + _n("GRD_x.", 3)),
-    # hyperdiffusion, first and second Laplacian pass (k_hdiff1, k_hdiff2_l)
+    # hyperdiffusion, first and second Laplacian pass (k_hdiff1, k_hdiff2_m)
     "hdiff1": (_f("vx", "vy", "vz", "w", "tem", "rho") + _m("tem_bs", "rho_bs"), _f(*_n("vt.", 6)),
                _n("coef_lap.", 7)),
     "hdiff2": (_f(*_n("vt.", 6), "RHOG"), _f(*_n("vt2.", 6)),
@@ -114,17 +114,24 @@ def esize(cls: str, precision: str) -> int:
     return 4 if precision == "mixed" else 8
 
 
-def kernel_bytes(name: str, npt: int, npt2: int, precision: str = "float64") -> int:
-    """algorithmic bytes of one launch of a regional kernel"""
+# fields that a tracer kernel reads or writes once for each tracer of its launch (the others once a launch)
+TRACER_FIELDS = frozenset(("RHOGQ1", "q", "gq.0", "gq.1", "gq.2", "qa.0", "qa.1", "qa.2", "Qmin", "Qmax"))
+TRACER_BATCH = 4     # tracers a launch of trc_grad, trc_remap, trc_qout, trc_apply; trc_vadv takes all
+
+
+def kernel_bytes(name: str, npt: int, npt2: int, precision: str = "float64", tracers: int = 1) -> int:
+    """algorithmic bytes of one launch of a regional kernel (the tracer kernels: on so many tracers)"""
     reads, writes, planes = KERNELS[name]
-    b = sum(esize(c, precision) for _, c in reads + writes) * npt
+    many = tracers if name.startswith("trc_") else 1
+    b = sum(esize(c, precision) * (many if n in TRACER_FIELDS else 1) for n, c in reads + writes) * npt
     return b + len(planes) * esize("p", precision) * npt2
 
 
-def kernel_passes(name: str) -> tuple:
+def kernel_passes(name: str, tracers: int = 1) -> tuple:
     """(3-D array passes, planes) of one launch"""
     reads, writes, planes = KERNELS[name]
-    return len(reads) + len(writes), len(planes)
+    many = tracers if name.startswith("trc_") else 1
+    return sum(many if n in TRACER_FIELDS else 1 for n, _ in reads + writes), len(planes)
 
 
 def step_launches(sstep=(2, 3, 6), nq: int = 1) -> dict:
@@ -132,10 +139,28 @@ def step_launches(sstep=(2, 3, 6), nq: int = 1) -> dict:
     steps sstep per stage, nq tracers)"""
     ns = sum(sstep)
     nst = len(sstep)
+    batches = -(-nq // TRACER_BATCH)
     return {"diag": nst, "advmom": nst, "hdiff1": nst, "hdiff2": nst, "gtend": nst, "split_init": nst - 1,
             "split_init_first": 1, "dd3d": nst + ns, "vp0_h": nst, "vp0_c": nst, "path1": ns, "vimain_a": ns,
-            "vi_solve": ns, "post": nst, "trc_vflux": 1, "trc_vadv": 2 * nq, "trc_hflux": 1,
-            "trc_grad": nq, "trc_remap": nq, "trc_qout": nq, "trc_apply": nq, "trc_rhog": 1}
+            "vi_solve": ns, "post": nst, "trc_vflux": 1, "trc_vadv": 2, "trc_hflux": 1,
+            "trc_grad": batches, "trc_remap": batches, "trc_qout": batches, "trc_apply": batches, "trc_rhog": 1}
+
+
+def launch_tracers(name: str, nq: int) -> list:
+    """the tracers of each launch of a kernel that step_launches counts"""
+    if name == "trc_vadv":
+        return [nq, nq]
+    return [min(TRACER_BATCH, nq - at) for at in range(0, nq, TRACER_BATCH)]
+
+
+def _launches(sstep, nq):
+    """(kernel, launches, tracers of each) of one large step"""
+    for k, n in step_launches(sstep, nq).items():
+        if k in ("trc_vadv", "trc_grad", "trc_remap", "trc_qout", "trc_apply"):
+            for m in launch_tracers(k, nq):
+                yield k, 1, m
+        else:
+            yield k, n, 1
 
 
 def exchange_fields(sstep=(2, 3, 6), nq: int = 1) -> int:
@@ -153,7 +178,9 @@ def step_bytes(npt: int, npt2: int, halo_points: int, sstep=(2, 3, 6), nq: int =
     exchanges (halo_points = halo values per level and field: regional halo
     cells + pole neighbours; kall levels), and the PROG0 snapshot copy"""
     e = esize("f", precision)
-    out = {k: n * kernel_bytes(k, npt, npt2, precision) for k, n in step_launches(sstep, nq).items()}
+    out = {}
+    for k, n, m in _launches(sstep, nq):
+        out[k] = out.get(k, 0) + n * kernel_bytes(k, npt, npt2, precision, m)
     kall_pts = npt // max(npt2, 1)
     out["comm"] = 2 * e * halo_points * kall_pts * exchange_fields(sstep, nq)
     out["prog0_copy"] = 2 * 6 * e * npt
@@ -165,7 +192,7 @@ def field_passes(sstep=(2, 3, 6), nq: int = 1, kall: int = 42) -> float:
     """F: float64-equivalent field passes per step (3-D passes + planes / kall),
     the halo exchanges and the PROG0 copy included at their own sizes"""
     F = 0.0
-    for k, n in step_launches(sstep, nq).items():
-        f3, p2 = kernel_passes(k)
+    for k, n, m in _launches(sstep, nq):
+        f3, p2 = kernel_passes(k, m)
         F += n * (f3 + p2 / kall)
     return F + 12
