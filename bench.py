@@ -51,12 +51,12 @@ PUBLISHED_F64 = 26_214_480 / 0.190
 PUBLISHED_F32 = 26_214_480 / 0.100
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per 3-D point of one
-# launch, from ncu captures of kernels that move the same fields as today's: the
-# float64 path 1 on the gl07 z40 case (7,318,080 points), the divergence damping
-# and the float32 path 1 on gl06 z40 (1,942,080 points; every field pass larger
-# than L2 in both); the traffic of a launch grows with its points, so the bench
-# scales this to its own grid.  Kernels without a capture report null.
-NCU_TRAFFIC_PER_POINT = {"float64": {"path1": 224.7, "dd3d": 104.9}, "mixed": {"path1": 99.3, "dd3d": 49.2}}
+# launch, from ncu captures of the present kernels on gl06 z40 (1,942,080 points,
+# profiles/vi_col_path1_dd3d_gl06_ncu.md; every launch's fields exceed L2); the
+# traffic of a launch grows with its points, so the bench scales this to its own
+# grid.  Kernels without a capture report null.
+NCU_TRAFFIC_PER_POINT = {"float64": {"path1": 205.4, "dd3d": 113.1, "vi_solve": 471.0},
+                         "mixed": {"path1": 100.6, "dd3d": 51.3, "vi_solve": 225.5}}
 
 
 def _pkg():
